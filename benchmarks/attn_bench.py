@@ -48,7 +48,7 @@ def ours(iters):
     q = qkv.detach()
     o = torch.empty(a.b, a.s, a.h * a.d, dtype=q.dtype, device=dev)
     lse = torch.empty(a.b, a.h, a.s, dtype=torch.float32, device=dev)
-    delta = torch.empty(2, a.b, a.h, a.s, dtype=torch.float32, device=dev)
+    delta = torch.empty(2, a.b, a.h, (a.s + 127) // 128 * 128, dtype=torch.float32, device=dev)
     dqkv = torch.empty_like(q)
     scale = a.d ** -0.5
     st, stream = _bind.status_ptr(dev), _bind.stream_ptr(dev)

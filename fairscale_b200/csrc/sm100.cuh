@@ -1,7 +1,7 @@
 // Inline-PTX wrappers for the Blackwell (sm_100a) execution model: mbarriers with bounded
 // waits, TMA tile loads/stores (per-CTA only), tcgen05 tensor-core MMA with TMEM accumulators.
 //
-// Every wait in this file is bounded: after `kWaitLimitNs` without progress the waiter raises
+// Every wait in this file is bounded: after `kWaitLimitCycles` without progress the waiter raises
 // the CTA-wide abort flag and returns false; callers then skip their work, the kernel records
 // FSB_ERR_WAIT_TIMEOUT in its status word, lets in-flight copies drain, frees TMEM and returns.
 #pragma once
@@ -10,7 +10,10 @@
 
 namespace fsb {
 
-constexpr uint64_t kWaitLimitNs = 1000ull * 1000ull * 1000ull;  // 1 s
+// Limit of one wait, counted in SM cycles: 1 s at 1.965 GHz (the highest SM clock), longer at lower clocks.  The cycle
+// counter is read in a few cycles, the nanosecond timer (%globaltimer) is not, and the first read of every wait that has
+// to block sits on the critical path of the pipeline stage behind it.
+constexpr long long kWaitLimitCycles = 1965ll * 1000ll * 1000ll;
 
 // ------------------------------------------------------------------------------------------------
 // mbarrier
@@ -52,7 +55,7 @@ static __device__ unsigned int g_blocked_wait_sites[8];
 // the kernel reports it in bits 8..15 of the status word.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int site = 1) {
   if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = globaltimer_ns();
+  const long long t0 = clock64();
   uint32_t spins = 0;
   while (!mbar_try_wait(bar, parity)) {
     if (((++spins) & 63u) == 0u) {
@@ -60,7 +63,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
         atomicOr(&g_blocked_wait_sites[(site >> 5) & 7], 1u << (site & 31));
         return false;
       }
-      if (globaltimer_ns() - t0 > kWaitLimitNs) {
+      if (clock64() - t0 > kWaitLimitCycles) {
         if (*abort_flag == 0) *abort_flag = site;
         atomicOr(&g_blocked_wait_sites[(site >> 5) & 7], 1u << (site & 31));
         return false;
@@ -85,12 +88,12 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t pa
 }
 __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int site = 1) {
   if (mbar_try_wait_cluster(bar, parity)) return true;
-  const uint64_t t0 = globaltimer_ns();
+  const long long t0 = clock64();
   uint32_t spins = 0;
   while (!mbar_try_wait_cluster(bar, parity)) {
     if (((++spins) & 63u) == 0u) {
       if (*abort_flag) return false;
-      if (globaltimer_ns() - t0 > kWaitLimitNs) {
+      if (clock64() - t0 > kWaitLimitCycles) {
         if (*abort_flag == 0) *abort_flag = site;
         return false;
       }
@@ -249,6 +252,11 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r
         "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
+__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
@@ -272,12 +280,24 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t local_smem_addr, uint32_
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// The same without making this thread's earlier writes visible to the cluster: for an arrival that only says "I have read
+// it".  The release above waits until every global store of the thread has been acknowledged, over a microsecond after an
+// epilogue.
+__device__ __forceinline__ void mbar_arrive_cluster_read_done(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
 // TMA tile load into THIS CTA's shared memory that reports its bytes to an mbarrier given by its
 // shared::cluster address (the pair leader's barrier). No data is shared between CTAs by the load.
 __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, uint32_t bar_cluster_addr, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorMap* map, uint32_t bar_cluster_addr, int x, int y, int z) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_slot, uint32_t ncols) {

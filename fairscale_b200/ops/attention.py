@@ -36,12 +36,25 @@ def _native_available() -> bool:
         return False
 
 
+def _native_takes(qkv: torch.Tensor, n_heads: int, D: int, scale: float) -> bool:
+    """Does this call run the tcgen05 kernels?  bf16 and head size 64 or 128; whole tiles (a length that is a multiple of 128)
+    always, any other length unless the call asks for what only torch's own operator offers: a functorch transform, forward-mode
+    differentiation, tracing, a softmax scale that is not positive, an empty tensor."""
+    if not (_bind.use_native(qkv) and qkv.dtype == torch.bfloat16 and D in (64, 128) and _native_available()):
+        return False
+    if qkv.shape[1] % 128 == 0:
+        return True
+    if qkv.numel() == 0 or qkv.shape[2] != 3 * n_heads * D or not (0.0 < scale < math.inf):
+        return False
+    return not (torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0 or torch.compiler.is_compiling())
+
+
 def causal_attention(qkv: torch.Tensor, n_heads: int, scale: Optional[float] = None) -> torch.Tensor:
     global BACKEND
     B, S, three_hd = qkv.shape
     D = three_hd // (3 * n_heads)
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
-    if _bind.use_native(qkv) and qkv.dtype == torch.bfloat16 and _native_available() and D in (64, 128) and S % 128 == 0:
+    if _native_takes(qkv, n_heads, D, scale):
         from .attention_native import flash_attention_packed
 
         BACKEND = "tcgen05"
@@ -52,8 +65,8 @@ def causal_attention(qkv: torch.Tensor, n_heads: int, scale: Optional[float] = N
         if not _WARNED_LIBRARY_PATH:
             _WARNED_LIBRARY_PATH = True
             warnings.warn(
-                f"causal_attention: the tcgen05 kernels take bf16 with head size 64 or 128 and a sequence length that is a multiple "
-                f"of 128 (got {qkv.dtype}, head size {D}, length {S}); this call runs torch's scaled_dot_product_attention instead",
+                f"causal_attention: the tcgen05 kernels take bf16 with head size 64 or 128 (got {qkv.dtype}, head size {D}, length {S}); "
+                f"this call runs torch's scaled_dot_product_attention instead",
                 stacklevel=2,
             )
         BACKEND = "torch-sdpa"

@@ -1,0 +1,101 @@
+"""Edge sizes of the kernels whose dispatch depends on the shape, against plain PyTorch in fp32 or fp64 (needs a B200).
+
+Tolerances: a bf16 result differs from the exact one by up to 2^-9 relative per element from its own rounding; attention rounds
+the probabilities and dS to bf16 as well, which the products average over many keys.  So 1e-2 in the 2-norm for one product and
+2e-2 / 3e-2 for attention forward / backward, as in the kernels' main tests; copies and single-rounding sums are exact.
+"""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _dev():
+    return torch.device("cuda", 0)
+
+
+def _status_ok():
+    from fairscale_b200 import _native
+
+    torch.cuda.synchronize()
+    assert _native.read_status(_dev()) == 0
+
+
+def _rel_err(a, b):
+    return ((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-12)).item()
+
+
+def _attention_ref(x, H):
+    B, S, W = x.shape
+    D = W // (3 * H)
+    q, k, v = x.view(B, S, 3, H, D).permute(2, 0, 3, 1, 4)
+    s = (q @ k.transpose(-1, -2)) / math.sqrt(D)
+    s = s.masked_fill(torch.ones(S, S, dtype=torch.bool, device=x.device).triu(1), float("-inf"))
+    return (torch.softmax(s, -1) @ v).transpose(1, 2).reshape(B, S, H * D)
+
+
+# one row, less than a tile, one row more or less than a tile of 128 and a pair of tiles, an odd number of tiles whose last
+# pair has one tile (with more items than SMs too, so that the persistent kernels meet both kinds of item), a long ragged one
+@pytest.mark.parametrize("B,S,H,D", [(1, 1, 1, 64), (2, 5, 2, 128), (2, 77, 3, 64), (1, 127, 2, 128), (2, 129, 2, 128), (1, 255, 2, 64),
+                                     (3, 257, 2, 128), (1, 385, 2, 64), (2, 384, 3, 64), (40, 300, 8, 64), (24, 650, 16, 128), (2, 1543, 4, 128)])
+def test_attention_any_length(B, S, H, D):
+    from fairscale_b200.ops import attention
+
+    torch.manual_seed(S)
+    x = (torch.randn(B, S, 3 * H * D, device=_dev()) * 0.7).bfloat16().requires_grad_()
+    o = attention.causal_attention(x, H)
+    assert attention.BACKEND == "tcgen05"
+    go = torch.randn_like(o)
+    o.backward(go)
+    _status_ok()
+    ref = x.detach().float().requires_grad_()
+    oref = _attention_ref(ref, H)
+    oref.backward(go.float())
+    assert _rel_err(o, oref) < 2e-2
+    g, gr = x.grad.view(B, S, 3, H, D), ref.grad.view(B, S, 3, H, D)
+    for i in range(3):
+        # with one or five keys dQ and dK are (almost) zero: measure them against the whole gradient there
+        scale = gr[:, :, i].norm() if S > 64 else gr.norm()
+        assert ((g[:, :, i].float() - gr[:, :, i]).norm() / scale).item() < 3e-2, i
+
+
+def test_attention_ragged_rows_do_not_mix():
+    """A sequence's last tile must not see the next sequence of the batch, and rows past the end are not written."""
+    from fairscale_b200.ops.attention import causal_attention
+
+    torch.manual_seed(0)
+    B, S, H, D = 3, 200, 2, 64
+    x = torch.randn(B, S, 3 * H * D, device=_dev()).bfloat16()
+    go = torch.randn(B, S, H * D, device=_dev()).bfloat16()
+    whole = x.clone().requires_grad_()
+    o = causal_attention(whole, H)
+    o.backward(go)
+    for b in range(B):
+        one = x[b : b + 1].clone().requires_grad_()
+        ob = causal_attention(one, H)
+        ob.backward(go[b : b + 1])
+        assert torch.equal(ob[0], o[b]) and torch.equal(one.grad[0], whole.grad[b])
+    # a view that starts off a 16-byte boundary, and a gradient that is not contiguous
+    flat = torch.empty(B * S * 3 * H * D + 1, device=_dev(), dtype=torch.bfloat16)
+    odd = flat[1:].view(B, S, -1)
+    odd.copy_(x)
+    odd.requires_grad_()
+    od = causal_attention(odd, H)
+    od.backward(go.transpose(0, 1).contiguous().transpose(0, 1))
+    assert torch.equal(od, o) and torch.equal(odd.grad, whole.grad)
+    _status_ok()
+
+
+def test_attention_ragged_infinities_stay_where_they_are():
+    from fairscale_b200.ops.attention import causal_attention
+
+    torch.manual_seed(0)
+    S, D = 150, 64
+    x = torch.randn(1, S, 3 * D, device=_dev()).bfloat16()
+    x[0, 140, D : 2 * D] = float("inf")  # one key: no query before it may notice
+    a = causal_attention(x, 1)
+    y = x.clone()
+    y[0, 140, D : 2 * D] = 0
+    assert torch.equal(a[0, :140], causal_attention(y, 1)[0, :140])
