@@ -24,10 +24,11 @@
 // but need the packed tensor permuted, copied and concatenated: B4 S1543 H16 D128 forward + backward 539 us, now 330 us.)
 //
 // The kernel is persistent: one CTA per SM walks a list of work items (256 query rows of one head), longest rows first,
-// dealt forwards and backwards in turn (snake_item; S8192: 508 -> 471 us against plain round-robin).  TMEM, barriers and the K / V ring live for the whole kernel, and the next item's query tiles are
-// loaded as soon as the last Q K^T products of the current item have completed, i.e. during its final softmax and
-// output write.  (With one CTA per item an SM sat idle for 7-10 us between consecutive CTAs - launch, 197 KB of shared
-// memory, TMEM allocation - which was a third of the kernel's run time.)
+// dealt forwards and backwards in turn (snake_item; B2 S8192 H16 D64: 508 -> 471 us against plain round-robin).  TMEM,
+// barriers and the K / V ring live for the whole kernel, and the next item's query tiles are loaded as soon as the last
+// Q K^T products of the current item have completed, i.e. during its final softmax and output write.  (With one CTA per
+// item an SM sat idle for 7-10 us between consecutive CTAs - launch, 197 KB of shared memory, TMEM allocation - which was
+// a third of the kernel's run time.)
 //
 // Replaces nn.MultiheadAttention / bmm+softmax in the reference's models
 // (benchmarks/models/transformer_lm.py:107,150-152,169-183).

@@ -27,8 +27,8 @@
 
 namespace fsb {
 
-// BATCHED: the tensor maps are 3-D (K / MN, rows, problem) and a tile index also selects the problem; used for the
-// local experts of an MoE layer (equal capacity per expert), where one launch replaces a Python loop of GEMMs.
+// BATCHED (both kernels): the tensor maps are 3-D (K / MN, rows, problem) and a tile index also selects the problem; used
+// for the local experts of an MoE layer (equal capacity per expert), where one launch replaces a Python loop of GEMMs.
 template <int BLOCK_N, bool BATCHED>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, GemmParams p) {
@@ -311,6 +311,7 @@ __device__ __forceinline__ bool wait_a_rows(const GemmParams& p, int r0, int r1,
   return true;
 }
 
+template <bool BATCHED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, GemmParams p) {
   using L = PairSmem;
@@ -339,8 +340,13 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
 
   const int tiles_m = (p.M + 2 * BLOCK_M - 1) / (2 * BLOCK_M);
   const int tiles_n = (p.N + PAIR_BLOCK_N - 1) / PAIR_BLOCK_N;
-  const int num_tiles = tiles_m * tiles_n;
+  const int tiles_per_problem = tiles_m * tiles_n;
+  const int num_tiles = tiles_per_problem * (BATCHED ? p.batch : 1);
   const int num_kb = (p.K + BLOCK_K - 1) / BLOCK_K;
+  auto load_tile = [&](void* dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
+    if (BATCHED) tma_load_3d_pair(dst, map, bar, x, y, z);
+    else         tma_load_2d_pair(dst, map, bar, x, y);
+  };
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -432,8 +438,9 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
           if (++q == PAIR_SCHED_DEPTH) { q = 0; qphase ^= 1u; }
         }
         if (tile < 0) break;
+        const int pb = BATCHED ? tile / tiles_per_problem : 0;
         int tm, tn;
-        pair_tile_coords(p, tile, tiles_m, tiles_n, tm, tn);
+        pair_tile_coords(p, tile - pb * tiles_per_problem, tiles_m, tiles_n, tm, tn);
         const int m0 = tm * 2 * BLOCK_M + static_cast<int>(rank) * BLOCK_M;
         const int n0 = tn * PAIR_BLOCK_N + static_cast<int>(rank) * PAIR_HALF_N;
         if (p.b_ready != nullptr && n0 < p.N) {
@@ -452,16 +459,16 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
           const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0);
           const int k0 = kb * BLOCK_K;
           if (!p.a_mn_major) {
-            tma_load_2d_pair(sa, &tmap_a, bar, k0, m0);
+            load_tile(sa, &tmap_a, bar, k0, m0, pb);
           } else {
 #pragma unroll
-            for (int j = 0; j < BLOCK_M / 64; ++j) tma_load_2d_pair(sa + j * 8192, &tmap_a, bar, m0 + j * 64, k0);
+            for (int j = 0; j < BLOCK_M / 64; ++j) load_tile(sa + j * 8192, &tmap_a, bar, m0 + j * 64, k0, pb);
           }
           if (!p.b_mn_major) {
-            tma_load_2d_pair(sb, &tmap_b, bar, k0, n0);
+            load_tile(sb, &tmap_b, bar, k0, n0, pb);
           } else {
 #pragma unroll
-            for (int j = 0; j < PAIR_HALF_N / 64; ++j) tma_load_2d_pair(sb + j * 8192, &tmap_b, bar, n0 + j * 64, k0);
+            for (int j = 0; j < PAIR_HALF_N / 64; ++j) load_tile(sb + j * 8192, &tmap_b, bar, n0 + j * 64, k0, pb);
           }
           if (++stage == PAIR_STAGES) { stage = 0; phase ^= 1u; }
         }
@@ -534,7 +541,8 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
     const int quad = warp & 3;            // TMEM lane quadrant this warp may access
     const int half = (warp - 2) >> 2;     // which 128 columns of the 256 this warp drains
     uint8_t* stage = smem + L::EPI_OFFSET + (warp - 2) * 4096;
-    const bool coalesce = epilogue_can_coalesce(p);
+    // in a batch every problem's base has to keep the alignment of the first one
+    const bool coalesce = epilogue_can_coalesce(p) && (!BATCHED || (p.stride_c % 8 == 0 && p.stride_aux % 8 == 0));
     int acc = 0;
     uint32_t acc_phase = 0;
     int q = 0;
@@ -546,18 +554,20 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
       tile = __shfl_sync(0xffffffffu, tile, 0);
       if (++q == PAIR_SCHED_DEPTH) { q = 0; qphase ^= 1u; }
       if (tile < 0) break;
+      const int pb = BATCHED ? tile / tiles_per_problem : 0;
       int tm, tn;
-      pair_tile_coords(p, tile, tiles_m, tiles_n, tm, tn);
+      pair_tile_coords(p, tile - pb * tiles_per_problem, tiles_m, tiles_n, tm, tn);
+      const GemmParams pt = BATCHED ? gemm_params_of_batch(p, pb) : p;
       const int row0 = tm * 2 * BLOCK_M + static_cast<int>(rank) * BLOCK_M + quad * 32;
       const int n0 = tn * PAIR_BLOCK_N + half * (PAIR_BLOCK_N / 2);
       uint4 pre[8];
-      if (coalesce && epilogue_needs_aux(p.epilogue) && n0 < p.N) epi_slab_prefetch(pre, p.aux, p.ld_aux, row0, n0, p.M, p.N, lane);
+      if (coalesce && epilogue_needs_aux(p.epilogue) && n0 < p.N) epi_slab_prefetch(pre, pt.aux, pt.ld_aux, row0, n0, pt.M, pt.N, lane);
       if (!mbar_wait(&tmem_full_bar[acc], acc_phase, abort_flag, 9)) { ok = false; break; }
       tc_fence_after_sync();
       const uint32_t t_base = tmem_base + static_cast<uint32_t>(acc * PAIR_BLOCK_N + half * (PAIR_BLOCK_N / 2)) +
                               (static_cast<uint32_t>(quad * 32) << 16);
-      if (coalesce) epilogue_rows_coalesced(t_base, row0, n0, PAIR_BLOCK_N / 2, p, stage, lane, pre);
-      else          epilogue_rows<PAIR_BLOCK_N / 2>(t_base, row0 + lane, n0, p);
+      if (coalesce) epilogue_rows_coalesced(t_base, row0, n0, PAIR_BLOCK_N / 2, pt, stage, lane, pre);
+      else          epilogue_rows<PAIR_BLOCK_N / 2>(t_base, row0 + lane, n0, pt);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty_bar[acc]), 0));
@@ -711,7 +721,7 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* bia
     if (!b_mn_major && !fsb_host::encode_2d_16bit(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BLOCK_K, PAIR_HALF_N)) return -1;
     static bool pair_attr_set[64] = {false};
     if (!pair_attr_set[di]) {
-      cudaFuncSetAttribute(gemm_bf16_tcgen05_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem::TOTAL);
+      cudaFuncSetAttribute(gemm_bf16_tcgen05_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem::TOTAL);
       pair_attr_set[di] = true;
     }
     const int pair_tiles = ((M + 2 * BLOCK_M - 1) / (2 * BLOCK_M)) * ((N + PAIR_BLOCK_N - 1) / PAIR_BLOCK_N);
@@ -719,7 +729,7 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* bia
     const int pairs = pair_tiles < max_pairs ? pair_tiles : max_pairs;
     p.sched = next_sched_slot(di);
     if (p.sched == nullptr) return -1;
-    gemm_bf16_tcgen05_pair_kernel<<<2 * pairs, PAIR_THREADS, PairSmem::TOTAL, stream>>>(ta, tb, p);
+    gemm_bf16_tcgen05_pair_kernel<false><<<2 * pairs, PAIR_THREADS, PairSmem::TOTAL, stream>>>(ta, tb, p);
     return static_cast<int>(cudaGetLastError());
   }
   if (block_n == 256) {
@@ -779,6 +789,21 @@ FSB_API int fsb_gemm_bf16_batched(const void* A, const void* B, void* C, const v
   cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
   const long long tiles = static_cast<long long>(batch) * ((M + BLOCK_M - 1) / BLOCK_M) * ((N + block_n - 1) / block_n);
   const int grid = tiles < num_sms ? static_cast<int>(tiles) : num_sms;
+  if (M >= 256 && N >= 256) {
+    // the rule of fsb_gemm_bf16: 256 x 256 tiles by CTA pairs once a problem has a whole one
+    if (!b_mn_major && !fsb_host::encode_3d_16bit(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)batch, (uint64_t)ldb, (uint64_t)stride_b, BLOCK_K, PAIR_HALF_N, 1)) return -1;
+    static bool pair_attr_set[64] = {false};
+    if (!pair_attr_set[dev & 63]) {
+      cudaFuncSetAttribute(gemm_bf16_tcgen05_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem::TOTAL);
+      pair_attr_set[dev & 63] = true;
+    }
+    const long long pair_tiles = static_cast<long long>(batch) * ((M + 2 * BLOCK_M - 1) / (2 * BLOCK_M)) * ((N + PAIR_BLOCK_N - 1) / PAIR_BLOCK_N);
+    const int pairs = pair_tiles < num_sms / 2 ? static_cast<int>(pair_tiles) : num_sms / 2;
+    p.sched = next_sched_slot(dev & 63);
+    if (p.sched == nullptr) return -1;
+    gemm_bf16_tcgen05_pair_kernel<true><<<2 * pairs, PAIR_THREADS, PairSmem::TOTAL, stream>>>(ta, tb, p);
+    return static_cast<int>(cudaGetLastError());
+  }
   static bool attr_set_dev[64][2] = {{false}};  // the attribute is per device
   bool* attr_set = attr_set_dev[dev & 63];
   if (block_n == 256) {

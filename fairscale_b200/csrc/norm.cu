@@ -351,9 +351,13 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_bwd_dx_kernel(const __nv_bf
 
 // out[c] = sum_r part[r, c]  (fp32 partials -> bf16 or fp32 result).  block = (32 columns, 8 row groups): a thread
 // adds rows ty, ty + 8, ... of its column in a fixed order, the eight sums are combined through shared memory.
+// blockIdx.y: independent matrices stored one after the other.
 __global__ void __launch_bounds__(256) column_reduce_kernel(const float* __restrict__ part, int rows, int H, __nv_bfloat16* out_bf16, float* out_f32) {
   __shared__ float red[8][33];
   const int c = blockIdx.x * 32 + threadIdx.x;
+  part += static_cast<long long>(blockIdx.y) * rows * H;
+  if (out_bf16 != nullptr) out_bf16 += static_cast<long long>(blockIdx.y) * H;
+  if (out_f32 != nullptr) out_f32 += static_cast<long long>(blockIdx.y) * H;
   float acc = 0.f;
   if (c < H) {
 #pragma unroll 4
@@ -370,11 +374,14 @@ __global__ void __launch_bounds__(256) column_reduce_kernel(const float* __restr
   }
 }
 
-// Column sums of a bf16 matrix [rows, H] (bias gradient): strip partials then reduce.
+// Column sums of a bf16 matrix [rows, H] (bias gradient): strip partials then reduce.  blockIdx.z: independent matrices
+// stored one after the other (the experts of an MoE layer).
 __global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16* __restrict__ x, long long rows, int H, float* __restrict__ part) {
   // block = 32 x 8 threads; a block handles 256 columns (8 per thread along x) for a strip of rows
   const int col0 = (blockIdx.x * 32 + threadIdx.x) * 8;
   const bool active = col0 < H;
+  x += static_cast<long long>(blockIdx.z) * rows * H;
+  part += static_cast<long long>(blockIdx.z) * gridDim.y * H;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   for (long long r = blockIdx.y * 8 + threadIdx.y; active && r < rows; r += static_cast<long long>(gridDim.y) * 8) {
     const Vec16<__nv_bfloat16> t = ld16(x + r * H + col0);
@@ -510,18 +517,20 @@ FSB_API int fsb_colsum_num_strips(long long rows) {
   return static_cast<int>(want < 1 ? 1 : (want > 48 ? 48 : want));
 }
 
-// out[c] = sum_r x[r, c]; x bf16 [rows, H] (H % 8 == 0); partials fp32 [n_strips, H]; out bf16 [H].
-FSB_API int fsb_colsum(const void* x, long long rows, int H, float* partials, void* out, cudaStream_t stream) {
+// out[b, c] = sum_r x[b, r, c]; x bf16 [batch, rows, H] (H % 8 == 0); partials fp32 [batch, n_strips, H]; out bf16 [batch, H].
+FSB_API int fsb_colsum_batched(const void* x, int batch, long long rows, int H, float* partials, void* out, cudaStream_t stream) {
   using namespace fsb;
-  if (rows <= 0 || H <= 0) return 0;
-  if (H % 8 != 0) return -1;
+  if (batch <= 0 || rows <= 0 || H <= 0) return 0;
+  if (H % 8 != 0 || batch > 65535) return -1;
   const int strips = fsb_colsum_num_strips(rows);
-  dim3 block(32, 8), grid((H / 8 + 31) / 32, strips);
+  const dim3 block(32, 8), grid((H / 8 + 31) / 32, strips, batch);
   colsum_partial_kernel<<<grid, block, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), rows, H, partials);
-  const dim3 threads(32, 8);
-  const int blocks = (H + 31) / 32;
-  column_reduce_kernel<<<blocks, threads, 0, stream>>>(partials, strips, H, static_cast<__nv_bfloat16*>(out), nullptr);
+  column_reduce_kernel<<<dim3((H + 31) / 32, batch), block, 0, stream>>>(partials, strips, H, static_cast<__nv_bfloat16*>(out), nullptr);
   return static_cast<int>(cudaGetLastError());
+}
+
+FSB_API int fsb_colsum(const void* x, long long rows, int H, float* partials, void* out, cudaStream_t stream) {
+  return fsb_colsum_batched(x, 1, rows, H, partials, out, stream);
 }
 
 // ---------------------------------------------------------------------------------------------------------

@@ -9,7 +9,8 @@ Two data paths:
   ``(expert, slot)`` rows and gathered back with their gate weights; no ``[S, E, C]`` tensor exists.  With an
   NVLink workspace for the group the scatter writes rows *directly into the destination rank's expert buffer*
   and the combine reads rows directly from the owners' output buffers (``csrc/comm.cu``), fusing dispatch /
-  combine with the all-to-all; otherwise a local scatter + ``all_to_all_single`` is used (NCCL / gloo).
+  combine with the all-to-all; otherwise the rows are moved within this GPU (``csrc/moe_rows.cu``; index ops on the CPU)
+  and exchanged with ``all_to_all_single`` (NCCL / gloo).
 * **dense path** (any other gate): the reference's einsum formulation.
 """
 
@@ -102,6 +103,70 @@ def _routes(route: Top2Route, world: int, n_local: int, rank: int) -> Tuple[Tens
     return dst_rank.to(torch.int32).contiguous(), dst_row.to(torch.int32).contiguous(), flat
 
 
+def _local_rows(t: Tensor) -> bool:
+    """Do the row kernels of ``csrc/moe_rows.cu`` move this tensor's rows?"""
+    return t.is_cuda and t.dtype in (torch.float32, torch.float16, torch.bfloat16)
+
+
+def _flat_rows(route: Top2Route) -> Tensor:
+    """int32 ``[S, 2]``: row of the global ``[E * C, M]`` view that each choice claims, -1 if it was dropped."""
+    if getattr(route, "flat", None) is not None:
+        return route.flat
+    flat = route.expert * route.capacity + route.slot
+    return torch.where(route.keep, flat, torch.full_like(flat, -1)).to(torch.int32).contiguous()
+
+
+def _scatter_local(x: Tensor, flat: Tensor, w: Optional[Tensor], counts: Optional[Tensor], E: int, C: int) -> Tensor:
+    """``out[flat[s, k]] = x[s] (* w[s, k])`` as ``[E * C, M]``; rows nobody claimed are zero."""
+    from ctypes import c_int, c_longlong, c_void_p
+
+    from ...ops import _bind
+
+    _bind._SIGNATURES.setdefault("fsb_moe_scatter_local", [c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p])
+    x = x.contiguous()
+    S, M = x.shape
+    # without per-expert counts the kernel cannot tell which rows stay unclaimed
+    out = x.new_empty((E * C, M)) if counts is not None else x.new_zeros((E * C, M))
+    _bind.call("fsb_moe_scatter_local", x.data_ptr(), _bind.dtype_code(x.dtype), flat.data_ptr(), _bind.ptr(w), S, M, out.data_ptr(),
+               _bind.ptr(counts), E, C, _bind.stream_ptr(x.device))
+    return out
+
+
+def _gather_local(buf: Tensor, flat: Tensor, w: Optional[Tensor], grad: Optional[Tensor] = None) -> Tensor:
+    """``sum_k w[s, k] * buf[flat[s, k]]`` as ``[S, M]``, or with ``grad`` the fp32 dots ``<buf[flat[s, k]], grad[s]>`` ``[S, 2]``."""
+    from ctypes import c_int, c_longlong, c_void_p
+
+    from ...ops import _bind
+
+    _bind._SIGNATURES.setdefault("fsb_moe_gather_local", [c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_void_p])
+    S, M = flat.shape[0], buf.shape[1]
+    out = None if grad is not None else buf.new_empty((S, M))
+    dots = buf.new_empty((S, 2), dtype=torch.float32) if grad is not None else None
+    _bind.call("fsb_moe_gather_local", buf.data_ptr(), _bind.dtype_code(buf.dtype), flat.data_ptr(), _bind.ptr(w), S, M, _bind.ptr(out),
+               _bind.ptr(grad), _bind.ptr(dots), _bind.stream_ptr(buf.device))
+    return out if dots is None else dots
+
+
+def _to_experts(rows: Tensor, group: Any, world: int, n_local: int, C: int) -> Tensor:
+    """``[E * C, M]`` rows of this rank's tokens -> ``[n_local, world * C, M]`` rows of this rank's experts."""
+    if world == 1:
+        return rows.view(n_local, C, -1)
+    out = torch.empty_like(rows)
+    comm.all_to_all_single(out, rows, group)  # [world, n_local, C, M] by source rank
+    return out.view(world, n_local, C, -1).transpose(0, 1).reshape(n_local, world * C, -1)
+
+
+def _to_tokens(rows: Tensor, group: Any, world: int, n_local: int, C: int) -> Tensor:
+    """The way back: ``[n_local, world * C, M]`` -> ``[E * C, M]`` rows that belong to this rank's tokens."""
+    M = rows.shape[-1]
+    if world == 1:
+        return rows.reshape(n_local * C, M).contiguous()
+    rows = rows.view(n_local, world, C, M).transpose(0, 1).contiguous().view(-1, M)
+    out = torch.empty_like(rows)
+    comm.all_to_all_single(out, rows, group)
+    return out
+
+
 class _Dispatch(torch.autograd.Function):
     """tokens ``[S, M]`` -> expert inputs ``[n_local, world * C, M]`` on the owning ranks."""
 
@@ -109,13 +174,18 @@ class _Dispatch(torch.autograd.Function):
     def forward(ctx: Any, x: Tensor, route: Top2Route, group: Any, n_local: int, owner: Optional[_LayerBuffers] = None) -> Tensor:  # type: ignore[override]
         world, rank = comm.group_size(group), comm.group_rank(group)
         C, E, M = route.capacity, route.num_experts, x.shape[1]
-        dst_rank, dst_row, flat = _routes(route, world, n_local, rank)
         ctx.meta = (group, n_local, world, rank, C, E, M, x.dtype)
         ctx.owner, ctx.claimed = owner, False
-        ctx.save_for_backward(dst_rank, dst_row, flat, route.keep)
         ws = symm.workspace_for(group) if (x.is_cuda and comm.comm_mode() == "fused" and x.dtype == torch.bfloat16) else None
         if owner is not None:
             owner._mine = False
+        ctx.local = ws is None and _local_rows(x)
+        if ctx.local:
+            flat = _flat_rows(route)
+            ctx.save_for_backward(flat)
+            return _to_experts(_scatter_local(x, flat, None, route.counts, E, C), group, world, n_local, C)
+        dst_rank, dst_row, flat = _routes(route, world, n_local, rank)
+        ctx.save_for_backward(dst_rank, dst_row, flat, route.keep)
         if ws is not None:
             private = owner is not None and owner.claim(ws, n_local * world * C, M, x.dtype)
             ctx.claimed = private and owner.expect_backward
@@ -138,6 +208,9 @@ class _Dispatch(torch.autograd.Function):
     @staticmethod
     def backward(ctx: Any, grad: Tensor):  # type: ignore[override]
         group, n_local, world, rank, C, E, M, dtype = ctx.meta
+        if ctx.local:
+            (flat,) = ctx.saved_tensors
+            return _gather_local(_to_tokens(grad.contiguous(), group, world, n_local, C), flat, None), None, None, None, None
         dst_rank, dst_row, flat, keep = ctx.saved_tensors
         S = dst_rank.shape[0]
         if ctx.claimed:
@@ -167,14 +240,21 @@ class _Combine(torch.autograd.Function):
                 owner: Optional[_LayerBuffers] = None) -> Tensor:  # type: ignore[override]
         world, rank = comm.group_size(group), comm.group_rank(group)
         C, E, M = route.capacity, route.num_experts, expert_out.shape[-1]
-        dst_rank, dst_row, flat = _routes(route, world, n_local, rank)
-        S = dst_rank.shape[0]
-        w = (gate * route.keep).to(torch.float32).contiguous()
         ctx.meta = (group, n_local, world, rank, C, E, M)
         ctx.fill = (route.counts, E, C, n_local) if route.counts is not None else None
         ws = symm.workspace_for(group) if (expert_out.is_cuda and comm.comm_mode() == "fused" and expert_out.dtype == torch.bfloat16) else None
         ctx.private = ws is not None and owner is not None and owner.holds()
         ctx.owner = owner
+        ctx.local = ws is None and _local_rows(expert_out)
+        if ctx.local:
+            flat = _flat_rows(route)
+            w = gate.to(torch.float32).contiguous()  # the kernels look at flat: a dropped choice's weight is not read
+            home = _to_tokens(expert_out.contiguous(), group, world, n_local, C)
+            ctx.save_for_backward(flat, w, home)
+            return _gather_local(home, flat, w)
+        dst_rank, dst_row, flat = _routes(route, world, n_local, rank)
+        S = dst_rank.shape[0]
+        w = (gate * route.keep).to(torch.float32).contiguous()
         if ws is not None:
             buf = owner.bufs["out"] if ctx.private else ws.scratch("moe_out", (n_local * world * C, M), expert_out.dtype)
             buf.copy_(expert_out.reshape(-1, M))
@@ -194,6 +274,12 @@ class _Combine(torch.autograd.Function):
     @staticmethod
     def backward(ctx: Any, dy: Tensor):  # type: ignore[override]
         group, n_local, world, rank, C, E, M = ctx.meta
+        if ctx.local:
+            flat, w, home = ctx.saved_tensors
+            dy = dy.to(home.dtype).contiguous()
+            counts = ctx.fill[0] if ctx.fill is not None else None
+            d_eo = _to_experts(_scatter_local(dy, flat, w, counts, E, C), group, world, n_local, C)
+            return d_eo, _gather_local(home, flat, None, grad=dy), None, None, None, None
         dst_rank, dst_row, flat, keep, w, saved = ctx.saved_tensors
         S = dst_rank.shape[0]
         dy = dy.contiguous()

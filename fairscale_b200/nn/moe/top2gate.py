@@ -55,6 +55,7 @@ class Top2Route(NamedTuple):
     capacity: int
     num_experts: int
     counts: Optional[Tensor] = None  # int32 [2 * E]: tokens per expert as first / second choice (CUDA index kernels only)
+    flat: Optional[Tensor] = None  # int32 [S, 2]: expert * C + slot, -1 for a dropped choice (CUDA index kernels only)
 
 
 def _route_indices_native(logits: Tensor, noise: Tensor) -> Optional[Tuple[Tensor, Tensor, Tensor, Tensor, Tensor]]:
@@ -76,6 +77,23 @@ def _route_indices_native(logits: Tensor, noise: Tensor) -> Optional[Tuple[Tenso
     _bind.call("fsb_top2_route", logits.data_ptr(), _bind.dtype_code(logits.dtype), noise.data_ptr(), S, E, out[0].data_ptr(),
                out[1].data_ptr(), out[2].data_ptr(), out[3].data_ptr(), ws.data_ptr(), totals.data_ptr(), _bind.stream_ptr(dev), launches=3)
     return out, totals
+
+
+def _pack_route(route: Tensor, capacity: int) -> Tuple[Tensor, Tensor, Tensor, Tensor]:
+    """``expert``, ``slot`` (int64), ``keep`` (bool) and ``flat`` (int32), all ``[S, 2]``, from the index kernels' ``[4, S]``."""
+    from ctypes import c_int, c_void_p
+
+    from ...ops import _bind
+
+    _bind._SIGNATURES.setdefault("fsb_moe_route_pack", [c_void_p, c_int, c_int] + [c_void_p] * 5)
+    S, dev = route.shape[1], route.device
+    expert = torch.empty((S, 2), dtype=torch.int64, device=dev)
+    slot = torch.empty((S, 2), dtype=torch.int64, device=dev)
+    keep = torch.empty((S, 2), dtype=torch.bool, device=dev)
+    flat = torch.empty((S, 2), dtype=torch.int32, device=dev)
+    _bind.call("fsb_moe_route_pack", route.data_ptr(), S, capacity, expert.data_ptr(), slot.data_ptr(), keep.data_ptr(),
+               flat.data_ptr(), _bind.stream_ptr(dev))
+    return expert, slot, keep, flat
 
 
 class _GateValues(torch.autograd.Function):
@@ -135,15 +153,13 @@ def top2_route(logits: torch.Tensor, noise: Optional[Tensor] = None) -> Top2Rout
         logits = logits.contiguous()
     native = _route_indices_native(logits.detach(), noise) if logits.is_cuda else None
     if native is not None:
-        # five launches in all: three for the indices, one for softmax + gate values + auxiliary loss, one memset
+        # six launches in all: three for the indices, one that lays them out per (token, choice), one for softmax + gate
+        # values + auxiliary loss, one memset
         route, counts2 = native
         count1 = counts2[:E]
         gate, l_aux = _GateValues.apply(logits, route, count1, capacity)
-        r = route.long()
-        keep = torch.stack([r[2] < capacity, r[3] < capacity], dim=1)
-        expert = torch.stack([r[0], r[1]], dim=1)
-        slot = torch.stack([r[2], r[3]], dim=1) * keep
-        return Top2Route(l_aux.to(logits.dtype), expert, slot, keep, gate, capacity, E, counts2)
+        expert, slot, keep, flat = _pack_route(route, capacity)
+        return Top2Route(l_aux.to(logits.dtype), expert, slot, keep, gate, capacity, E, counts2, flat)
     gates = F.softmax(logits, dim=1, dtype=torch.float)
     idx1 = torch.argmax(gates, dim=1)
     noisy = (logits + noise).scatter(1, idx1.unsqueeze(1), float("-inf"))

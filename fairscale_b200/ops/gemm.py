@@ -331,13 +331,15 @@ class _GroupedMLPFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):  # type: ignore[override]
+        from .reduce import batched_column_sum
+
         x, w1, w2, pre, h = ctx.saved_tensors
         dy = dy.contiguous()
         dw2 = batched_linear_wgrad(dy, h)
-        db2 = dy.float().sum(1).to(dy.dtype)
+        db2 = batched_column_sum(dy)
         dpre = batched_linear_dgrad(dy, w2, dgelu_pre=pre)
         dw1 = batched_linear_wgrad(dpre, x)
-        db1 = dpre.float().sum(1).to(dy.dtype)
+        db1 = batched_column_sum(dpre)
         dx = batched_linear_dgrad(dpre, w1)
         return dx, dw1, db1, dw2, db2
 

@@ -19,3 +19,18 @@ def column_sum(x: torch.Tensor) -> torch.Tensor:
     out = torch.empty((H,), dtype=torch.bfloat16, device=x.device)
     _bind.call("fsb_colsum", x2.data_ptr(), rows, H, partials.data_ptr(), out.data_ptr(), _bind.stream_ptr(x.device), launches=2)
     return out
+
+
+def batched_column_sum(x: torch.Tensor) -> torch.Tensor:
+    """``x.sum(1)`` for a 3-D tensor: the bias gradients of stacked experts, accumulated in fp32."""
+    E, rows, H = x.shape
+    if not _bind.use_native(x) or x.dtype != torch.bfloat16 or H % 8 or rows == 0:
+        return x.float().sum(1).to(x.dtype)
+    x = x.contiguous()
+    if x.data_ptr() % 16:  # the kernel reads 16 bytes at a time
+        x = x.clone()
+    strips = _bind.fn("fsb_colsum_num_strips")(rows)
+    partials = torch.empty((E, strips, H), dtype=torch.float32, device=x.device)
+    out = torch.empty((E, H), dtype=torch.bfloat16, device=x.device)
+    _bind.call("fsb_colsum_batched", x.data_ptr(), E, rows, H, partials.data_ptr(), out.data_ptr(), _bind.stream_ptr(x.device), launches=2)
+    return out

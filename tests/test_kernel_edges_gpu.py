@@ -99,3 +99,68 @@ def test_attention_ragged_infinities_stay_where_they_are():
     y = x.clone()
     y[0, 140, D : 2 * D] = 0
     assert torch.equal(a[0, :140], causal_attention(y, 1)[0, :140])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("S,E,M", [(64, 4, 1024), (820, 4, 512), (48, 16, 33), (8, 2, 8)])
+def test_moe_rows_match_index_ops(S, E, M, dtype):
+    """Dispatch and combine of one rank on the row kernels against the index formulation that the CPU runs."""
+    import torch.distributed as dist
+
+    from fairscale_b200.nn.moe import top2gate
+    from fairscale_b200.nn.moe.moe_layer import _Combine, _Dispatch
+
+    if not dist.is_initialized():
+        dist.init_process_group("nccl", store=dist.HashStore(), rank=0, world_size=1)
+    group = dist.group.WORLD
+    torch.manual_seed(S + M)
+    logits = torch.randn(S, E, device=_dev()) + torch.linspace(2, 0, E, device=_dev())  # crowded first experts: some choices overflow
+    noise = top2gate.gumbel_rsample(logits.shape, logits.device)
+    x = torch.randn(S, M, device=_dev()).to(dtype)
+    dy = torch.randn(S, M, device=_dev()).to(dtype)
+    got = {}
+    for where, cast in (("gpu", lambda t: t), ("cpu", lambda t: t.cpu())):
+        lg, xx = (cast(t).detach().clone().requires_grad_() for t in (logits, x))
+        route = top2gate.top2_route(lg, cast(noise))
+        rows = _Dispatch.apply(xx, route, group, E)
+        weight = cast(torch.arange(1, E + 1, device=_dev())).to(dtype).view(E, 1, 1)  # experts that differ, or the gates' gradient is zero
+        out = _Combine.apply(rows * weight, route.gate, route, group, E)
+        out.backward(cast(dy))
+        got[where] = [t.detach().cpu() for t in (rows, out, xx.grad, lg.grad)]
+    _status_ok()
+    assert torch.equal(got["gpu"][0], got["cpu"][0])
+    eps = {torch.float32: 1e-5, torch.float16: 2e-3, torch.bfloat16: 1.6e-2}[dtype]  # gates differ by fp32 rounding, so results by a last bit
+    for a, b in zip(got["gpu"][1:], got["cpu"][1:]):
+        torch.testing.assert_close(a.float(), b.float(), rtol=eps, atol=eps * b.float().abs().max().item())
+
+
+@pytest.mark.parametrize("E,C,K,N", [(2, 256, 256, 256), (3, 257, 72, 264), (4, 410, 512, 2048), (1, 300, 64, 256)])
+def test_batched_pair_gemm_edges(E, C, K, N):
+    """Problems with whole 256 x 256 tiles run on CTA pairs; remainders must not leak into the next problem."""
+    from fairscale_b200.ops.gemm import batched_linear_dgrad, batched_linear_forward, batched_linear_wgrad
+
+    torch.manual_seed(C)
+    x = torch.randn(E, C, K, device=_dev()).bfloat16()
+    w = torch.randn(E, N, K, device=_dev()).bfloat16()
+    dy = torch.randn(E, C, N, device=_dev()).bfloat16()
+    b = torch.randn(E, N, device=_dev()).bfloat16()
+    y, _ = batched_linear_forward(x, w, b)
+    want = torch.baddbmm(b.double().unsqueeze(1), x.double(), w.double().transpose(1, 2))
+    dx, dw = batched_linear_dgrad(dy, w), batched_linear_wgrad(dy, x)
+    _status_ok()
+    for e in range(E):
+        assert _rel_err(y[e], want[e]) < 1e-2
+        assert _rel_err(dx[e], dy[e].double() @ w[e].double()) < 1e-2
+        assert _rel_err(dw[e], dy[e].double().t() @ x[e].double()) < 1e-2
+
+
+@pytest.mark.parametrize("E,rows,H", [(1, 1, 8), (3, 63, 256), (4, 410, 2048), (2, 5000, 264)])
+def test_batched_column_sum(E, rows, H):
+    from fairscale_b200.ops.reduce import batched_column_sum
+
+    torch.manual_seed(rows)
+    x = torch.randn(E, rows, H, device=_dev()).bfloat16()
+    want = x.double().sum(1)
+    # fp32 sums of `rows` terms and one rounding to bf16
+    torch.testing.assert_close(batched_column_sum(x).double(), want, rtol=2**-8, atol=1e-5 * rows)
+    assert torch.equal(batched_column_sum(x)[-1], batched_column_sum(x[-1:])[0])
