@@ -1,4 +1,4 @@
-"""Softmax cross-entropy on bf16 logits (``csrc/cross_entropy.cu``)."""
+"""Softmax cross-entropy on bf16 or fp32 logits (``csrc/cross_entropy.cu``)."""
 
 from __future__ import annotations
 
@@ -9,11 +9,21 @@ import torch
 from . import _bind
 
 
+def _native_takes(logits: torch.Tensor, targets: torch.Tensor) -> bool:
+    """bf16 or dense fp32 rows that start on 16-byte boundaries, int64 targets beside them."""
+    if not _bind.use_native(logits):
+        return False
+    if logits.dtype == torch.bfloat16:
+        return logits.stride(0) % 8 == 0
+    return (logits.dtype == torch.float32 and logits.is_contiguous() and logits.shape[1] % 4 == 0 and logits.data_ptr() % 16 == 0
+            and targets.is_cuda and targets.dtype == torch.int64 and targets.is_contiguous())
+
+
 def ce_forward(logits: torch.Tensor, targets: torch.Tensor, ignore_index: int = -100, vocab_start: int = 0,
                want_stats: bool = False) -> Tuple[torch.Tensor, torch.Tensor, Optional[torch.Tensor]]:
     """Per-row loss and log-sum-exp of ``logits[rows, V]``; optional ``(max, sumexp, target_logit)`` stats."""
     rows, V = logits.shape
-    if not _bind.use_native(logits) or logits.dtype != torch.bfloat16 or logits.stride(0) % 8:
+    if not _native_takes(logits, targets):
         lf = logits.float()
         lse = torch.logsumexp(lf, dim=-1)
         local = targets - vocab_start
@@ -28,16 +38,16 @@ def ce_forward(logits: torch.Tensor, targets: torch.Tensor, ignore_index: int = 
     loss = torch.empty(rows, dtype=torch.float32, device=logits.device)
     lse = torch.empty(rows, dtype=torch.float32, device=logits.device)
     stats = torch.empty((rows, 3), dtype=torch.float32, device=logits.device) if want_stats else None
-    _bind.call("fsb_ce_fwd", logits.data_ptr(), targets.data_ptr(), loss.data_ptr(), lse.data_ptr(), _bind.ptr(stats), rows, V,
+    _bind.call("fsb_ce_fwd_dtype", logits.data_ptr(), _bind.dtype_code(logits.dtype), targets.data_ptr(), loss.data_ptr(), lse.data_ptr(), _bind.ptr(stats), rows, V,
                logits.stride(0), vocab_start, ignore_index, _bind.stream_ptr(logits.device))
     return loss, lse, stats
 
 
 def ce_backward(logits: torch.Tensor, targets: torch.Tensor, lse: torch.Tensor, grad_out: torch.Tensor, scale: float,
                 ignore_index: int = -100, vocab_start: int = 0, inplace: bool = True) -> torch.Tensor:
-    """``(softmax - onehot) * grad_out * scale``; overwrites ``logits`` when ``inplace``."""
+    """``(softmax - onehot) * grad_out * scale``; overwrites bf16 ``logits`` when ``inplace``."""
     rows, V = logits.shape
-    if not _bind.use_native(logits) or logits.dtype != torch.bfloat16 or logits.stride(0) % 8:
+    if not _native_takes(logits, targets):
         p = torch.exp(logits.float() - lse.unsqueeze(1))
         local = targets - vocab_start
         inside = (local >= 0) & (local < V)
@@ -47,9 +57,10 @@ def ce_backward(logits: torch.Tensor, targets: torch.Tensor, lse: torch.Tensor, 
         g = g.expand(rows) if g.numel() == 1 else g
         g = torch.where(targets == ignore_index, torch.zeros_like(g), g)
         return ((p - onehot) * g.unsqueeze(1)).to(logits.dtype)
-    out = logits if inplace else torch.empty_like(logits)
+    # fp32 logits may be the caller's own (bf16 ones are a projection's output that nothing else reads): never overwritten
+    out = logits if inplace and logits.dtype == torch.bfloat16 else torch.empty_like(logits)
     g = grad_out.float().contiguous()
-    _bind.call("fsb_ce_bwd", logits.data_ptr(), targets.data_ptr(), lse.data_ptr(), g.data_ptr(), int(g.numel() == 1), scale,
+    _bind.call("fsb_ce_bwd_dtype", logits.data_ptr(), _bind.dtype_code(logits.dtype), targets.data_ptr(), lse.data_ptr(), g.data_ptr(), int(g.numel() == 1), scale,
                out.data_ptr(), rows, V, logits.stride(0), vocab_start, ignore_index, _bind.stream_ptr(logits.device))
     return out
 

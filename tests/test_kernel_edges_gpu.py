@@ -164,3 +164,40 @@ def test_batched_column_sum(E, rows, H):
     # fp32 sums of `rows` terms and one rounding to bf16
     torch.testing.assert_close(batched_column_sum(x).double(), want, rtol=2**-8, atol=1e-5 * rows)
     assert torch.equal(batched_column_sum(x)[-1], batched_column_sum(x[-1:])[0])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,V", [(1, 8), (3, 512), (5, 32000), (7, 2056)])
+def test_vocab_cross_entropy_pieces(rows, V, dtype):
+    """Loss, statistics and gradient of one vocabulary shard; masked (-inf, lowest finite) logits, targets of other shards."""
+    from fairscale_b200.ops.loss import ce_backward, ce_forward
+
+    torch.manual_seed(V)
+    x = (torch.randn(rows, V, device=_dev()) * 4).to(dtype)
+    x[:, : V // 4] = float("-inf")  # a thread's first logits among them
+    if V > 8:
+        x[:, V // 4 : V // 2] = torch.finfo(dtype).min
+    v0 = 1000
+    t = torch.randint(V // 2, V, (rows,), device=_dev()) + v0
+    if rows > 1:
+        t[0] = 3  # another rank's token
+    loss, lse, stats = ce_forward(x, t, ignore_index=-(2**62), vocab_start=v0, want_stats=True)
+    xd = x.double()
+    want = torch.logsumexp(xd, -1)
+    tl = torch.where(t >= v0, xd.gather(1, (t - v0).clamp(min=0).unsqueeze(1)).squeeze(1), torch.zeros((), device=_dev(), dtype=torch.float64))
+    tol = 2e-6 if dtype == torch.float32 else 1e-4  # fp32 logits: expf and fp32 sums; bf16: the fast exponential
+    torch.testing.assert_close(lse.double(), want, rtol=tol, atol=tol)
+    torch.testing.assert_close(loss.double(), want - tl, rtol=tol, atol=10 * tol)
+    torch.testing.assert_close((stats[:, 0] + stats[:, 1].log()).double(), want, rtol=tol, atol=tol)
+    g = torch.rand(rows, device=_dev())
+    before = x.clone()
+    dx = ce_backward(x, t, lse, g, 1.0, ignore_index=-(2**62), vocab_start=v0, inplace=True)
+    p = torch.softmax(before.double(), -1)
+    onehot = torch.zeros_like(p)
+    for r in range(rows):
+        if t[r] >= v0:
+            onehot[r, t[r] - v0] = 1
+    torch.testing.assert_close(dx.double(), (p - onehot) * g.double().unsqueeze(1), rtol=2e-5 if dtype == torch.float32 else 1e-2, atol=1e-6 if dtype == torch.float32 else 1e-4)
+    if dtype == torch.float32:
+        assert torch.equal(x, before)  # fp32 logits may be the caller's own
+    _status_ok()
