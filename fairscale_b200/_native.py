@@ -133,7 +133,10 @@ def use_native(*tensors: Any) -> bool:
     CUDA tensors always take the native path (and fail loudly if the library is absent);
     CPU tensors take the reference path.
     """
-    return len(tensors) > 0 and all(getattr(t, "is_cuda", False) for t in tensors if t is not None)
+    for t in tensors:
+        if t is not None and not getattr(t, "is_cuda", False):
+            return False
+    return len(tensors) > 0
 
 
 def check(code: int, what: str) -> None:
@@ -148,7 +151,9 @@ def status_word(device: Any) -> Any:
     """Per-device int32 status word that kernels with bounded waits write on timeout."""
     import torch
 
-    key = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
+    key = torch.device("cuda", device).index if isinstance(device, int) else torch.device(device).index
+    if key is None:
+        key = torch.cuda.current_device()
     if key not in _status_tensors:
         _status_tensors[key] = torch.zeros(1, dtype=torch.int32, device=f"cuda:{key}")
     return _status_tensors[key]

@@ -81,8 +81,16 @@ def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
 
+def _device_index(device: Any) -> int:
+    index = device.index if isinstance(device, torch.device) else (device if isinstance(device, int) else None)
+    if index is None:
+        index = torch.device(device).index if device is not None and not isinstance(device, torch.device) else None
+    return torch.cuda.current_device() if index is None else index
+
+
 def stream_ptr(device: Any = None) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """Raw handle of the current stream (without building a ``torch.cuda.Stream`` around it for every launch)."""
+    return torch._C._cuda_getCurrentRawStream(_device_index(device))
 
 
 def dtype_code(dt: torch.dtype) -> int:
@@ -93,5 +101,19 @@ def use_native(*tensors: Any) -> bool:
     return _native.use_native(*tensors)
 
 
+_status_ptrs: dict = {}  # device index -> address of its status word (allocated once per process)
+
+
 def status_ptr(device: Any) -> int:
-    return _native.status_word(device).data_ptr()
+    index = _device_index(device)
+    ptr_ = _status_ptrs.get(index)
+    if ptr_ is None:
+        ptr_ = _status_ptrs[index] = _native.status_word(index).data_ptr()
+    return ptr_
+
+
+def no_graph() -> bool:
+    """True when an operation may run without its autograd node: gradients are off, and nothing else (forward-mode
+    differentiation, a functorch transform, a tracer) has to see the node either."""
+    return not (torch.is_grad_enabled() or torch.autograd.forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active()
+                or torch.compiler.is_compiling())

@@ -242,6 +242,8 @@ class _LinearFn(torch.autograd.Function):
 def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, *, gelu: bool = False,
            residual: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Differentiable fused linear: ``gelu(x w^T + b)`` or ``x w^T + b + residual``."""
+    if _bind.no_graph():
+        return linear_forward(x, w, bias, gelu=gelu, residual=residual)[0]
     return _LinearFn.apply(x, w, bias, gelu, residual)
 
 

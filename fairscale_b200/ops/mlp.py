@@ -11,6 +11,7 @@ from typing import Optional
 
 import torch
 
+from . import _bind
 from .gemm import grad_slot_info, linear_dgrad, linear_forward, wgrad_into_slot
 from .reduce import column_sum
 
@@ -41,4 +42,7 @@ class _MLPFn(torch.autograd.Function):
 
 def mlp(x: torch.Tensor, w1: torch.Tensor, b1: torch.Tensor, w2: torch.Tensor, b2: torch.Tensor,
         residual: Optional[torch.Tensor] = None) -> torch.Tensor:
+    if _bind.no_graph():
+        h, _ = linear_forward(x, w1, b1, gelu=True)
+        return linear_forward(h, w2, b2, residual=residual)[0]
     return _MLPFn.apply(x, w1, b1, w2, b2, residual)

@@ -84,10 +84,14 @@ class _NormFn(torch.autograd.Function):
 
 
 def layer_norm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], eps: float = 1e-5) -> torch.Tensor:
+    if _bind.no_graph():
+        return norm_forward(x, weight, bias, eps, False)[0]
     return _NormFn.apply(x, weight, bias, eps, False)
 
 
 def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6) -> torch.Tensor:
+    if _bind.no_graph():
+        return norm_forward(x, weight, None, eps, True)[0]
     return _NormFn.apply(x, weight, None, eps, True)
 
 
