@@ -1,10 +1,10 @@
 // LayerNorm / RMSNorm forward and backward for bf16 activations, fp32 statistics.
 //
-// Forward: one CTA per row, the row is read once with 16-byte loads, kept in registers, reduced
-// (mean / variance) and written once; mean and rstd are saved for backward.
-// Backward: same one-pass structure for dx; dgamma / dbeta are accumulated per CTA over a strip of
-// rows into fp32 partials [n_strips, H], reduced by a second small kernel (no atomics, so the
-// result is deterministic).
+// Forward: a row is read once with 16-byte loads, kept in registers, reduced (mean / variance) and written once; mean
+// and rstd are saved for backward.  Backward: same one-pass structure for dx; dgamma / dbeta are accumulated per CTA into
+// fp32 partials [n_strips, H], reduced by a second small kernel (no atomics, so the result is deterministic).
+// Rows of up to 4096 columns take a warp each forwards and the row-group kernel backwards, longer ones (up to 8192) one
+// CTA per row.
 // Replaces nn.LayerNorm in the reference's benchmark models (benchmarks/models/transformer_lm.py:109-110).
 
 #include "common.cuh"
@@ -13,9 +13,11 @@ namespace fsb {
 
 constexpr int NORM_THREADS = 256;
 constexpr int NORM_MAX_VEC = 4;  // block-per-row path: up to 4 x 8 bf16 per thread -> H <= 8192
-constexpr int NORM_WARPS = 4;    // warp-per-row path: rows handled per CTA
+constexpr int NORM_WARPS = 4;    // warp-per-row forward: rows handled per CTA
+constexpr int NORM_ROWS_MAX_H = 4096;  // row-group backward: up to 512 threads of 8 columns
+constexpr int NORM_ROWS_MAX_CTAS = 2 * 148;
 
-// ---- warp-per-row kernels (H <= 4096): a lane keeps VPL 16-byte vectors of the row in registers, all
+// ---- warp-per-row forward (H <= 4096): a lane keeps VPL 16-byte vectors of the row in registers, all
 // reductions are warp shuffles, no shared memory and no block barriers.
 template <bool RMS, int VPL>
 __global__ void __launch_bounds__(NORM_WARPS * 32) norm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
@@ -74,138 +76,115 @@ __global__ void __launch_bounds__(NORM_WARPS * 32) norm_fwd_warp_kernel(const __
   }
 }
 
-// dx only (dgamma / dbeta come from norm_dparam_partial_kernel)
-template <bool RMS, int VPL>
-__global__ void __launch_bounds__(NORM_WARPS * 32) norm_bwd_dx_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                                                                           const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
-                                                                           const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx,
-                                                                           long long rows, int H) {
-  const int lane = threadIdx.x & 31;
-  const long long row = static_cast<long long>(blockIdx.x) * NORM_WARPS + (threadIdx.x >> 5);
-  if (row >= rows) return;
-  const int nvec = H / 8;
-  const float mean = RMS ? 0.f : mean_in[row];
-  const float rstd = rstd_in[row];
-  float xh[VPL][8], wdy[VPL][8];
-  float s1 = 0.f, s2 = 0.f;
+// ---- row-group backward (H <= 4096): a thread owns the same 8 columns of every row, so gamma and the dgamma / dbeta sums
+// stay in its registers; a CTA of H / 8 threads walks groups of R rows, one group after the other (persistent grid, 512
+// threads per SM: the 128 registers per thread hold two groups).  Bound by memory, and what counts is bytes in flight: the
+// next group's vectors are loaded before the current group's reductions, and R rows share one round of block reductions.
+// A warp per row, with all of a row's sums in one warp's registers, had room for one row only: 16384 x 2048 71 -> 53 us,
+// 8192 x 1024 31 -> 25 us, 4096 x 4096 (two kernels there) 43 -> 34 us.  (The forward has no sums to keep and is faster
+// with a warp per row: 35 against 41 us.)
+
+// Block-wide sums of N values per thread for blocks of whole warps; `red` holds 2 * 16 * N floats and is used in turn
+// (`turn` alternates), so one barrier per call is enough.
+template <int N>
+__device__ __forceinline__ void block_sums(float (&v)[N], float* red, int turn) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
 #pragma unroll
-  for (int it = 0; it < VPL; ++it) {
-    const int j = lane + it * 32;
-    if (j < nvec) {
-      const Vec16<__nv_bfloat16> tx = ld16(x + row * H + j * 8);
-      const Vec16<__nv_bfloat16> td = ld16(dy + row * H + j * 8);
-      const Vec16<__nv_bfloat16> tg = ld16(gamma + j * 8);
+  for (int i = 0; i < N; ++i) v[i] = warp_sum(v[i]);
+  if (warps == 1) return;
+  float* buf = red + (turn & 1) * 16 * N;
+  if (lane == 0) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        xh[it][k] = (__bfloat162float(tx.v[k]) - mean) * rstd;
-        wdy[it][k] = __bfloat162float(td.v[k]) * __bfloat162float(tg.v[k]);
-        s1 += wdy[it][k];
-        s2 += wdy[it][k] * xh[it][k];
-      }
-    }
+    for (int i = 0; i < N; ++i) buf[warp * N + i] = v[i];
   }
-  s1 = RMS ? 0.f : warp_sum(s1) / H;
-  s2 = warp_sum(s2) / H;
+  __syncthreads();
 #pragma unroll
-  for (int it = 0; it < VPL; ++it) {
-    const int j = lane + it * 32;
-    if (j < nvec) {
-      Vec16<__nv_bfloat16> o;
+  for (int i = 0; i < N; ++i) v[i] = 0.f;
+  for (int w = 0; w < warps; ++w) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) o.v[k] = __float2bfloat16_rn(rstd * (wdy[it][k] - s1 - xh[it][k] * s2));
-      st16(dx + row * H + j * 8, o);
-    }
+    for (int i = 0; i < N; ++i) v[i] += buf[w * N + i];
   }
 }
 
-// dx and the dgamma / dbeta partials in one pass over dy and x (H <= 2048).  Persistent: a warp walks rows
-// blockIdx.x * 4 + warp, + 4 * gridDim.x, ...; a lane owns the same VPL x 8 columns in every row, so it accumulates
-// their dgamma / dbeta contributions in registers.  dy and x stay packed in registers between the statistics pass and
-// the output pass.  At the end the four warps of a CTA are summed through shared memory and the CTA writes one
-// partial row: dgamma_part / dbeta_part are [gridDim.x, H].
-template <bool RMS, int VPL>
-__global__ void __launch_bounds__(NORM_WARPS * 32, 2) norm_bwd_fused_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                                                                            const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
-                                                                            const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx,
-                                                                            float* __restrict__ dgamma_part, float* __restrict__ dbeta_part,
-                                                                            long long rows, int H) {
-  extern __shared__ float fused_red[];  // [NORM_WARPS][H]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nvec = H / 8;
-  float dg[VPL][8], db[VPL][8];
+// dx and the dgamma / dbeta partials in one pass over dy and x: dgamma_part / dbeta_part are [gridDim.x, H].
+template <bool RMS, int MAX_THREADS>
+__global__ void __launch_bounds__(MAX_THREADS, 512 / MAX_THREADS) norm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+                                                               const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
+                                                               const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx,
+                                                               float* __restrict__ dgamma_part, float* __restrict__ dbeta_part, long long rows,
+                                                               int H) {
+  constexpr int R = 2;
+  __shared__ float red[2 * 16 * 2 * R];
+  const int col = threadIdx.x * 8;
+  const bool mine = col < H;
+  float dg[8], db[8];
 #pragma unroll
-  for (int it = 0; it < VPL; ++it) {
+  for (int k = 0; k < 8; ++k) dg[k] = db[k] = 0.f;
+  Vec16<__nv_bfloat16> tg, cx[R], cd[R], nx[R], nd[R];
+  tg.raw = make_uint4(0u, 0u, 0u, 0u);
+  if (mine) tg = ld16(gamma + col);
+  float cm[R], cr[R], nm[R], nr[R];
+  auto load = [&](Vec16<__nv_bfloat16> (&tx)[R], Vec16<__nv_bfloat16> (&td)[R], float (&m)[R], float (&r)[R], long long row0) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) { dg[it][k] = 0.f; db[it][k] = 0.f; }
-  }
-  for (long long row = static_cast<long long>(blockIdx.x) * NORM_WARPS + warp; row < rows; row += static_cast<long long>(gridDim.x) * NORM_WARPS) {
-    const float mean = RMS ? 0.f : mean_in[row];
-    const float rstd = rstd_in[row];
-    Vec16<__nv_bfloat16> tx[VPL], td[VPL];
-    float s1 = 0.f, s2 = 0.f;
-#pragma unroll
-    for (int it = 0; it < VPL; ++it) {
-      const int j = lane + it * 32;
-      if (j < nvec) {
-        tx[it] = ld16(x + row * H + j * 8);
-        td[it] = ld16(dy + row * H + j * 8);
-      }
-    }
-#pragma unroll
-    for (int it = 0; it < VPL; ++it) {
-      const int j = lane + it * 32;
-      if (j < nvec) {
-        const Vec16<__nv_bfloat16> tg = ld16(gamma + j * 8);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float xh = (__bfloat162float(tx[it].v[k]) - mean) * rstd;
-          const float w = __bfloat162float(td[it].v[k]) * __bfloat162float(tg.v[k]);
-          s1 += w;
-          s2 = fmaf(w, xh, s2);
+    for (int i = 0; i < R; ++i) {
+      tx[i].raw = td[i].raw = make_uint4(0u, 0u, 0u, 0u);
+      m[i] = r[i] = 0.f;
+      if (row0 + i < rows) {
+        if (mine) {
+          tx[i] = ld16(x + (row0 + i) * H + col);
+          td[i] = ld16(dy + (row0 + i) * H + col);
         }
+        if (!RMS) m[i] = mean_in[row0 + i];
+        r[i] = rstd_in[row0 + i];
       }
     }
-    s1 = RMS ? 0.f : warp_sum(s1) / H;
-    s2 = warp_sum(s2) / H;
+  };
+  const long long step = static_cast<long long>(gridDim.x) * R;
+  long long row0 = static_cast<long long>(blockIdx.x) * R;
+  int turn = 0;
+  load(cx, cd, cm, cr, row0);
+  for (; row0 < rows; row0 += step) {
+    load(nx, nd, nm, nr, row0 + step);
+    float s[2 * R];  // sum of w, sum of w * xhat, per row
 #pragma unroll
-    for (int it = 0; it < VPL; ++it) {
-      const int j = lane + it * 32;
-      if (j < nvec) {
-        const Vec16<__nv_bfloat16> tg = ld16(gamma + j * 8);
-        Vec16<__nv_bfloat16> o;
+    for (int i = 0; i < R; ++i) {
+      s[2 * i] = s[2 * i + 1] = 0.f;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float xh = (__bfloat162float(tx[it].v[k]) - mean) * rstd;
-          const float d = __bfloat162float(td[it].v[k]);
-          const float w = d * __bfloat162float(tg.v[k]);
-          o.v[k] = __float2bfloat16_rn(rstd * (w - s1 - xh * s2));
-          dg[it][k] = fmaf(d, xh, dg[it][k]);
-          if (!RMS) db[it][k] += d;
-        }
-        st16(dx + row * H + j * 8, o);
+      for (int k = 0; k < 8; ++k) {
+        const float xh = (__bfloat162float(cx[i].v[k]) - cm[i]) * cr[i];
+        const float w = __bfloat162float(cd[i].v[k]) * __bfloat162float(tg.v[k]);
+        s[2 * i] += w;
+        s[2 * i + 1] = fmaf(w, xh, s[2 * i + 1]);
       }
     }
+    block_sums<2 * R>(s, red, turn++);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      if (row0 + i >= rows || !mine) break;
+      const float s1 = RMS ? 0.f : s[2 * i] / H, s2 = s[2 * i + 1] / H;
+      Vec16<__nv_bfloat16> o;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float xh = (__bfloat162float(cx[i].v[k]) - cm[i]) * cr[i];
+        const float d = __bfloat162float(cd[i].v[k]);
+        const float w = d * __bfloat162float(tg.v[k]);
+        o.v[k] = __float2bfloat16_rn(cr[i] * (w - s1 - xh * s2));
+        dg[k] = fmaf(d, xh, dg[k]);
+        if (!RMS) db[k] += d;
+      }
+      st16(dx + (row0 + i) * H + col, o);
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) { cx[i] = nx[i]; cd[i] = nd[i]; cm[i] = nm[i]; cr[i] = nr[i]; }
   }
-  // the CTA's partial row: sum of its four warps, dgamma first and dbeta second through the same buffer
-#pragma unroll 1
-  for (int which = 0; which < (RMS ? 1 : 2); ++which) {
-    float* out = which == 0 ? dgamma_part : dbeta_part;
-    if (out == nullptr) break;  // uniform
-    __syncthreads();
-#pragma unroll
-    for (int it = 0; it < VPL; ++it) {
-      const int j = lane + it * 32;
-      if (j < nvec) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) fused_red[warp * H + j * 8 + k] = which == 0 ? dg[it][k] : db[it][k];
-      }
-    }
-    __syncthreads();
-    for (int c = threadIdx.x; c < H; c += NORM_WARPS * 32) {
-      float acc = 0.f;
-#pragma unroll
-      for (int w = 0; w < NORM_WARPS; ++w) acc += fused_red[w * H + c];
-      out[static_cast<long long>(blockIdx.x) * H + c] = acc;
+  if (mine) {
+    float* pg = dgamma_part + static_cast<long long>(blockIdx.x) * H + col;
+    *reinterpret_cast<float4*>(pg) = make_float4(dg[0], dg[1], dg[2], dg[3]);
+    *reinterpret_cast<float4*>(pg + 4) = make_float4(dg[4], dg[5], dg[6], dg[7]);
+    if (!RMS && dbeta_part != nullptr) {
+      float* pb = dbeta_part + static_cast<long long>(blockIdx.x) * H + col;
+      *reinterpret_cast<float4*>(pb) = make_float4(db[0], db[1], db[2], db[3]);
+      *reinterpret_cast<float4*>(pb + 4) = make_float4(db[4], db[5], db[6], db[7]);
     }
   }
 }
@@ -349,15 +328,16 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_bwd_dx_kernel(const __nv_bf
   }
 }
 
-// out[c] = sum_r part[r, c]  (fp32 partials -> bf16 or fp32 result).  block = (32 columns, 8 row groups): a thread
+// out[c] = sum_r part[r, c]  (fp32 partials -> bf16 result).  block = (32 columns, 8 row groups): a thread
 // adds rows ty, ty + 8, ... of its column in a fixed order, the eight sums are combined through shared memory.
-// blockIdx.y: independent matrices stored one after the other.
-__global__ void __launch_bounds__(256) column_reduce_kernel(const float* __restrict__ part, int rows, int H, __nv_bfloat16* out_bf16, float* out_f32) {
+// blockIdx.y: independent matrices stored one after the other; with `out_second` the second one's result goes there (dgamma
+// and dbeta of a norm in one launch), otherwise results are stored one after the other as well.
+__global__ void __launch_bounds__(256) column_reduce_kernel(const float* __restrict__ part, int rows, int H, __nv_bfloat16* out, __nv_bfloat16* out_second) {
   __shared__ float red[8][33];
   const int c = blockIdx.x * 32 + threadIdx.x;
   part += static_cast<long long>(blockIdx.y) * rows * H;
-  if (out_bf16 != nullptr) out_bf16 += static_cast<long long>(blockIdx.y) * H;
-  if (out_f32 != nullptr) out_f32 += static_cast<long long>(blockIdx.y) * H;
+  if (out_second != nullptr) out = blockIdx.y == 0 ? out : out_second;
+  else out += static_cast<long long>(blockIdx.y) * H;
   float acc = 0.f;
   if (c < H) {
 #pragma unroll 4
@@ -369,8 +349,7 @@ __global__ void __launch_bounds__(256) column_reduce_kernel(const float* __restr
     float t = 0.f;
 #pragma unroll
     for (int y = 0; y < 8; ++y) t += red[y][threadIdx.x];
-    if (out_bf16 != nullptr) out_bf16[c] = __float2bfloat16_rn(t);
-    if (out_f32 != nullptr) out_f32[c] = t;
+    out[c] = __float2bfloat16_rn(t);
   }
 }
 
@@ -383,7 +362,19 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16
   x += static_cast<long long>(blockIdx.z) * rows * H;
   part += static_cast<long long>(blockIdx.z) * gridDim.y * H;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (long long r = blockIdx.y * 8 + threadIdx.y; active && r < rows; r += static_cast<long long>(gridDim.y) * 8) {
+  // bound by memory: four loads in flight per thread (16384 x 8192: one load gave 4 TB/s)
+  const long long step = static_cast<long long>(gridDim.y) * 8;
+  long long r = blockIdx.y * 8 + threadIdx.y;
+  for (; active && r + 3 * step < rows; r += 4 * step) {
+    Vec16<__nv_bfloat16> t[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) t[u] = ld16(x + (r + u * step) * H + col0);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int k = 0; k < 8; ++k) acc[k] += __bfloat162float(t[u].v[k]);
+  }
+  for (; active && r < rows; r += step) {
     const Vec16<__nv_bfloat16> t = ld16(x + r * H + col0);
 #pragma unroll
     for (int k = 0; k < 8; ++k) acc[k] += __bfloat162float(t.v[k]);
@@ -407,6 +398,8 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16
 
 // H must be a multiple of 8 and <= 8192. mean/rstd are fp32 [rows]. rms != 0 selects RMSNorm
 // (beta and mean ignored).
+static int norm_rows_threads(int H) { return (H / 8 + 31) / 32 * 32; }
+
 template <bool RMS>
 static void launch_norm_fwd(const __nv_bfloat16* x, const __nv_bfloat16* g, const __nv_bfloat16* b, __nv_bfloat16* y, float* mean,
                             float* rstd, long long rows, int H, float eps, cudaStream_t stream) {
@@ -418,18 +411,6 @@ static void launch_norm_fwd(const __nv_bfloat16* x, const __nv_bfloat16* g, cons
   else if (vpl <= 8)  norm_fwd_warp_kernel<RMS, 8><<<grid, NORM_WARPS * 32, 0, stream>>>(x, g, b, y, mean, rstd, rows, H, eps);
   else if (vpl <= 16) norm_fwd_warp_kernel<RMS, 16><<<grid, NORM_WARPS * 32, 0, stream>>>(x, g, b, y, mean, rstd, rows, H, eps);
   else norm_fwd_kernel<RMS><<<static_cast<unsigned>(rows), NORM_THREADS, 0, stream>>>(x, g, b, y, mean, rstd, H, eps);
-}
-
-template <bool RMS>
-static void launch_norm_bwd_dx(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* g, const float* mean,
-                               const float* rstd, __nv_bfloat16* dx, long long rows, int H, cudaStream_t stream) {
-  using namespace fsb;
-  const unsigned grid = static_cast<unsigned>((rows + NORM_WARPS - 1) / NORM_WARPS);
-  const int vpl = (H / 8 + 31) / 32;
-  if (vpl <= 2)       norm_bwd_dx_warp_kernel<RMS, 2><<<grid, NORM_WARPS * 32, 0, stream>>>(dy, x, g, mean, rstd, dx, rows, H);
-  else if (vpl <= 4)  norm_bwd_dx_warp_kernel<RMS, 4><<<grid, NORM_WARPS * 32, 0, stream>>>(dy, x, g, mean, rstd, dx, rows, H);
-  else if (vpl <= 8)  norm_bwd_dx_warp_kernel<RMS, 8><<<grid, NORM_WARPS * 32, 0, stream>>>(dy, x, g, mean, rstd, dx, rows, H);
-  else norm_bwd_dx_kernel<RMS><<<static_cast<unsigned>(rows), NORM_THREADS, 0, stream>>>(dy, x, g, mean, rstd, dx, H);
 }
 
 FSB_API int fsb_norm_fwd(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd,
@@ -446,14 +427,11 @@ FSB_API int fsb_norm_fwd(const void* x, const void* gamma, const void* beta, voi
   return static_cast<int>(cudaGetLastError());
 }
 
-// Rows of fp32 partials the backward needs room for: the fused kernel (H <= 2048) writes one row per CTA of its
-// persistent grid (two CTAs per SM, never more CTAs than groups of four rows), the two-kernel path at most 48.
-constexpr int NORM_FUSED_MAX_H = 2048;
-constexpr int NORM_FUSED_MAX_CTAS = 2 * 148;
-
-static int norm_bwd_fused_ctas(long long rows) {
-  const long long want = (rows + fsb::NORM_WARPS - 1) / fsb::NORM_WARPS;
-  return static_cast<int>(want < 1 ? 1 : (want > NORM_FUSED_MAX_CTAS ? NORM_FUSED_MAX_CTAS : want));
+// Rows of fp32 partials the backward needs room for: the row-group kernel (H <= 4096) writes one row per CTA of its
+// persistent grid (two CTAs per SM, never more CTAs than groups of two rows), the two-kernel path at most 48.
+static int norm_bwd_rows_ctas(long long rows) {
+  const long long want = (rows + 1) / 2;
+  return static_cast<int>(want < 1 ? 1 : (want > fsb::NORM_ROWS_MAX_CTAS ? fsb::NORM_ROWS_MAX_CTAS : want));
 }
 static int norm_bwd_split_strips(long long rows) {
   const long long want = (rows + 7) / 8;
@@ -461,19 +439,8 @@ static int norm_bwd_split_strips(long long rows) {
 }
 
 FSB_API int fsb_norm_bwd_num_strips(long long rows) {
-  const int a = norm_bwd_fused_ctas(rows), b = norm_bwd_split_strips(rows);
+  const int a = norm_bwd_rows_ctas(rows), b = norm_bwd_split_strips(rows);
   return a > b ? a : b;
-}
-
-template <bool RMS>
-static void launch_norm_bwd_fused(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* g, const float* mean, const float* rstd,
-                                  __nv_bfloat16* dx, float* pg, float* pb, long long rows, int H, int ctas, cudaStream_t stream) {
-  using namespace fsb;
-  const size_t smem = static_cast<size_t>(NORM_WARPS) * H * sizeof(float);  // <= 32 KB
-  const int vpl = (H / 8 + 31) / 32;
-  if (vpl <= 2)      norm_bwd_fused_kernel<RMS, 2><<<ctas, NORM_WARPS * 32, smem, stream>>>(dy, x, g, mean, rstd, dx, pg, pb, rows, H);
-  else if (vpl <= 4) norm_bwd_fused_kernel<RMS, 4><<<ctas, NORM_WARPS * 32, smem, stream>>>(dy, x, g, mean, rstd, dx, pg, pb, rows, H);
-  else               norm_bwd_fused_kernel<RMS, 8><<<ctas, NORM_WARPS * 32, smem, stream>>>(dy, x, g, mean, rstd, dx, pg, pb, rows, H);
 }
 
 // partials: fp32 workspace of 2 * n_strips * H floats (n_strips from fsb_norm_bwd_num_strips).
@@ -483,8 +450,8 @@ FSB_API int fsb_norm_bwd(const void* dy, const void* x, const void* gamma, const
   using namespace fsb;
   if (rows <= 0) return 0;
   if (H % 8 != 0 || H > 8 * NORM_THREADS * NORM_MAX_VEC) return -1;
-  const bool fused = H <= NORM_FUSED_MAX_H;
-  const int strips = fused ? norm_bwd_fused_ctas(rows) : norm_bwd_split_strips(rows);
+  const bool fused = H <= NORM_ROWS_MAX_H;
+  const int strips = fused ? norm_bwd_rows_ctas(rows) : norm_bwd_split_strips(rows);
   float* pg = partials;
   float* pb = partials + static_cast<long long>(strips) * H;
   auto* d = static_cast<const __nv_bfloat16*>(dy);
@@ -493,22 +460,29 @@ FSB_API int fsb_norm_bwd(const void* dy, const void* x, const void* gamma, const
   auto* o = static_cast<__nv_bfloat16*>(dx);
   const bool want_beta = !rms && dbeta != nullptr;
   if (fused) {
-    if (rms) launch_norm_bwd_fused<true>(d, xx, gg, mean, rstd, o, pg, nullptr, rows, H, strips, stream);
-    else     launch_norm_bwd_fused<false>(d, xx, gg, mean, rstd, o, pg, want_beta ? pb : nullptr, rows, H, strips, stream);
+    const int threads = norm_rows_threads(H);
+    if (threads <= 256) {
+      if (rms) norm_bwd_rows_kernel<true, 256><<<strips, threads, 0, stream>>>(d, xx, gg, mean, rstd, o, pg, nullptr, rows, H);
+      else     norm_bwd_rows_kernel<false, 256><<<strips, threads, 0, stream>>>(d, xx, gg, mean, rstd, o, pg, want_beta ? pb : nullptr, rows, H);
+    } else {
+      if (rms) norm_bwd_rows_kernel<true, 512><<<strips, threads, 0, stream>>>(d, xx, gg, mean, rstd, o, pg, nullptr, rows, H);
+      else     norm_bwd_rows_kernel<false, 512><<<strips, threads, 0, stream>>>(d, xx, gg, mean, rstd, o, pg, want_beta ? pb : nullptr, rows, H);
+    }
   } else {
     dim3 block(32, 8), grid((H / 8 + 31) / 32, strips);
     if (rms) {
-      launch_norm_bwd_dx<true>(d, xx, gg, mean, rstd, o, rows, H, stream);
+      norm_bwd_dx_kernel<true><<<static_cast<unsigned>(rows), NORM_THREADS, 0, stream>>>(d, xx, gg, mean, rstd, o, H);
       norm_dparam_partial_kernel<true><<<grid, block, 0, stream>>>(d, xx, mean, rstd, pg, nullptr, rows, H);
     } else {
-      launch_norm_bwd_dx<false>(d, xx, gg, mean, rstd, o, rows, H, stream);
+      norm_bwd_dx_kernel<false><<<static_cast<unsigned>(rows), NORM_THREADS, 0, stream>>>(d, xx, gg, mean, rstd, o, H);
       norm_dparam_partial_kernel<false><<<grid, block, 0, stream>>>(d, xx, mean, rstd, pg, want_beta ? pb : nullptr, rows, H);
     }
   }
   const dim3 threads(32, 8);
   const int blocks = (H + 31) / 32;
-  column_reduce_kernel<<<blocks, threads, 0, stream>>>(pg, strips, H, static_cast<__nv_bfloat16*>(dgamma), nullptr);
-  if (want_beta) column_reduce_kernel<<<blocks, threads, 0, stream>>>(pb, strips, H, static_cast<__nv_bfloat16*>(dbeta), nullptr);
+  // the beta partials follow the gamma partials
+  column_reduce_kernel<<<dim3(blocks, want_beta ? 2 : 1), threads, 0, stream>>>(pg, strips, H, static_cast<__nv_bfloat16*>(dgamma),
+                                                                                want_beta ? static_cast<__nv_bfloat16*>(dbeta) : nullptr);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -200,6 +200,15 @@ def wgrad_into_slot(dy: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, slo
     return linear_wgrad(dy, x, out=slot)
 
 
+def grad_window(info, dtype: torch.dtype, device: torch.device) -> Optional[torch.Tensor]:  # type: ignore[no-untyped-def]
+    """The flat-gradient window behind a view's descriptor, for kernels that write bf16 gradients element by element
+    (bias and norm parameters), or None; a window is handed out once per backward."""
+    if info is None or dtype != torch.bfloat16 or device.type != "cuda":
+        return None
+    arena, offset, shape = info
+    return arena.slot(offset, shape, dtype, device)
+
+
 def matmul_nt(a: torch.Tensor, b: torch.Tensor, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """``a[M,K] @ b[N,K]^T`` for 2-D bf16 tensors."""
     y, _ = linear_forward(a, b, None, out_dtype=out_dtype)
@@ -217,6 +226,7 @@ class _LinearFn(torch.autograd.Function):
         ctx.has_bias = bias is not None
         ctx.has_residual = residual is not None
         ctx.w_slot = grad_slot_info(w)
+        ctx.b_slot = grad_slot_info(bias) if bias is not None else None
         ctx.save_for_backward(x, w, pre)
         return y
 
@@ -235,7 +245,7 @@ class _LinearFn(torch.autograd.Function):
         if ctx.has_bias and ctx.needs_input_grad[2]:
             from .reduce import column_sum
 
-            db = column_sum(dy2)
+            db = column_sum(dy2, grad_window(ctx.b_slot, dy2.dtype, dy2.device))
         return dx, dw, db, None, d_res
 
 

@@ -2,12 +2,13 @@
 
 from __future__ import annotations
 
-from typing import Optional, Tuple
+from typing import Any, Optional, Tuple
 
 import torch
 from torch import nn
 
 from . import _bind
+from .gemm import grad_slot_info, grad_window
 
 
 def _native_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
@@ -42,7 +43,8 @@ def norm_forward(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Ten
 
 
 def norm_backward(dy: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, mean: Optional[torch.Tensor], rstd: torch.Tensor,
-                  rms: bool, has_bias: bool) -> Tuple[torch.Tensor, torch.Tensor, Optional[torch.Tensor]]:
+                  rms: bool, has_bias: bool, slots: Tuple[Any, Any] = (None, None)) -> Tuple[torch.Tensor, torch.Tensor, Optional[torch.Tensor]]:
+    """``slots``: flat-gradient descriptors of weight and bias, whose windows the kernel then writes in place."""
     H = x.shape[-1]
     if not _native_ok(x, weight):
         xf, dyf, wf = x.float(), dy.float(), weight.float()
@@ -59,11 +61,17 @@ def norm_backward(dy: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, mean:
     strips = _bind.fn("fsb_norm_bwd_num_strips")(rows)
     partials = torch.empty((2, strips, H), dtype=torch.float32, device=x.device)
     dx = torch.empty_like(x2)
-    dw = torch.empty(H, dtype=torch.bfloat16, device=x.device)
-    db = torch.empty(H, dtype=torch.bfloat16, device=x.device) if (has_bias and not rms) else None
+    dw = grad_window(slots[0], weight.dtype, x.device)
+    if dw is None:
+        dw = torch.empty(H, dtype=torch.bfloat16, device=x.device)
+    db = None
+    if has_bias and not rms:
+        db = grad_window(slots[1], weight.dtype, x.device)
+        if db is None:
+            db = torch.empty(H, dtype=torch.bfloat16, device=x.device)
     _bind.call("fsb_norm_bwd", dy2.data_ptr(), x2.data_ptr(), weight.data_ptr(), _bind.ptr(mean), rstd.data_ptr(), dx.data_ptr(),
                dw.data_ptr(), _bind.ptr(db), partials.data_ptr(), rows, H, int(rms), _bind.stream_ptr(x.device),
-               launches=4 if db is not None else 3)
+               launches=2 if H <= 4096 else 3)
     return dx.view_as(x), dw, db
 
 
@@ -73,13 +81,14 @@ class _NormFn(torch.autograd.Function):
         y, mean, rstd = norm_forward(x, weight, bias, eps, rms)
         ctx.rms = rms
         ctx.has_bias = bias is not None
+        ctx.slots = (grad_slot_info(weight), grad_slot_info(bias) if bias is not None else None)
         ctx.save_for_backward(x, weight, mean, rstd)
         return y
 
     @staticmethod
     def backward(ctx, dy):  # type: ignore[override]
         x, weight, mean, rstd = ctx.saved_tensors
-        dx, dw, db = norm_backward(dy, x, weight, mean, rstd, ctx.rms, ctx.has_bias)
+        dx, dw, db = norm_backward(dy, x, weight, mean, rstd, ctx.rms, ctx.has_bias, ctx.slots)
         return dx, dw, db, None, None
 
 

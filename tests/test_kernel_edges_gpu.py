@@ -166,6 +166,60 @@ def test_batched_column_sum(E, rows, H):
     assert torch.equal(batched_column_sum(x)[-1], batched_column_sum(x[-1:])[0])
 
 
+# one column group per thread up to 4096 columns (whole and partial warps), one CTA per row beyond; row counts that are no
+# multiple of the rows a CTA takes at a time, and more rows than the persistent grid takes in one round
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("rows,H", [(1, 8), (3, 264), (5, 2048), (7, 2056), (2, 4096), (3, 4104), (1801, 768)])
+def test_norm_backward_edges(rows, H, rms):
+    from fairscale_b200.ops import norm
+
+    torch.manual_seed(rows + H)
+    x, dy = (torch.randn(rows, H, device=_dev()).bfloat16() for _ in range(2))
+    w = torch.randn(H, device=_dev()).bfloat16()
+    b = None if rms else torch.randn(H, device=_dev()).bfloat16()
+    y, mean, rstd = norm.norm_forward(x, w, b, 1e-5, rms)
+    dx, dw, db = norm.norm_backward(dy, x, w, mean, rstd, rms, b is not None)
+    _status_ok()
+    xd, wd = x.double(), w.double()
+    mu = 0 if rms else xd.mean(-1, keepdim=True)
+    rs = torch.rsqrt((xd - mu).pow(2).mean(-1, keepdim=True) + 1e-5)
+    xh, g = (xd - mu) * rs, dy.double() * wd
+    assert _rel_err(y, xh * wd + (0 if b is None else b.double())) < 4e-3  # one rounding to bf16
+    assert _rel_err(dx, rs * (g - (0 if rms else g.mean(-1, keepdim=True)) - xh * (g * xh).mean(-1, keepdim=True))) < 4e-3
+    assert _rel_err(dw, (dy.double() * xh).sum(0)) < 4e-3
+    if not rms:
+        assert _rel_err(db, dy.double().sum(0)) < 4e-3
+
+
+def test_small_gradients_land_in_their_flat_window():
+    """Bias and norm gradients are written where the flat gradient wants them; a second use goes through autograd's sum."""
+    from fairscale_b200.nn.misc.flatten_params_wrapper import GradArena
+    from fairscale_b200.ops import norm
+    from fairscale_b200.ops.gemm import linear
+
+    torch.manual_seed(0)
+    d = 64
+    arena = GradArena(d * d + 3 * d)
+    w, b, g, be = ((torch.randn(s, device=_dev()) * 0.1).bfloat16().requires_grad_() for s in ((d, d), (d,), (d,), (d,)))
+    x = torch.randn(100, d, device=_dev()).bfloat16()
+
+    def grads():
+        y = linear(norm.layer_norm(x, g, be), w, b)
+        return torch.autograd.grad(linear(y, w, b).float().sum(), (w, b, g, be))
+
+    want = grads()
+    off = 0
+    for p in (w, b, g, be):
+        p._fsb_grad_slot = (arena, off, p.shape)
+        off += p.numel()
+    got = grads()
+    _status_ok()
+    for a, r in zip(got, want):
+        assert torch.equal(a, r)
+    base = arena.buffer.data_ptr()
+    assert got[2].data_ptr() == base + 2 * (d * d + d) and got[3].data_ptr() == base + 2 * (d * d + 2 * d)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rows,V", [(1, 8), (3, 512), (5, 32000), (7, 2056)])
 def test_vocab_cross_entropy_pieces(rows, V, dtype):
