@@ -595,6 +595,11 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
 
 }  // namespace fsb
 
+namespace fsb_host {
+// gemm_cluster_k.cu
+int gemm_cluster_k(const CUtensorMap& ta, const void* B, int ldb, const fsb::GemmParams& p, int block_n, int splits, int dev, cudaStream_t stream);
+}  // namespace fsb_host
+
 // Counter pairs of the dynamic tile scheduler: a ring of slots per device, one slot per launch, so that GEMMs running
 // at the same time on different streams never share a counter.  A slot is all zero whenever no kernel is using it (the
 // kernel resets it), hence 64 launches would have to be in flight at once on one device before two could collide.
@@ -613,6 +618,60 @@ static unsigned int* next_sched_slot(int di) {
   return base[di] + 2 * ((seq[di]++) % kSlots);
 }
 
+static bool pair_enabled() {  // FSB_GEMM_PAIR=0 disables the CTA-pair kernel
+  static const bool on = [] {
+    const char* e = getenv("FSB_GEMM_PAIR");
+    return e == nullptr || e[0] != '0';
+  }();
+  return on;
+}
+
+// Kernel for a product that is not streamed and has no CTA cap.  Measured on B200 (us; 64-wide K blocks = kb):
+//
+//   M, N, K              pair   one CTA 128x256   cluster split-K, block_n / splits
+//   77, 1024, 4096         -         24.7          64/1 20.6   64/2 16.5   64/4 12.4   64/8 16.5
+//   128, 1024, 8192        -         55.4          64/1 41.1   64/4 16.9   128/4 19.3  128/8 14.8
+//   768, 768, 3575       32.9        28.8          64/1 21.9   64/2 16.8   128/1 24.1  128/4 24.7
+//   1024, 1024, 8192     57.4        56.2          64/1 44.0   128/1 48.4  128/2 32.5
+//   2048, 1024, 1024     20.5        12.4          64/1 16.6   128/1 10.3
+//   2048, 2048, 2048     26.0        18.3          128/1 27.2
+//
+// One wave of independent CTAs takes about 6.3 us + K blocks x 0.28 / 0.32 / 0.39 us (tiles 64 / 128 / 256 wide): one CTA's
+// operand stream is bound by latency, not by the tensor cores, so shorter slices win until the SMs run out.  A cluster
+// costs about 2 us more for its barriers, 4 us at eight CTAs, and clusters of four or eight do not fit the SMs to the last
+// one (144 CTAs in clusters of four run in two waves), hence the limits on their number.  With more tiles than one wave
+// of single CTAs the pair's halved operand traffic decides.
+struct GemmPlan {
+  enum Kind { PAIR, ONE_CTA, CLUSTER_K } kind;
+  int block_n, splits;
+};
+static GemmPlan choose_gemm_plan(int M, int N, int K, int num_sms, bool pair_allowed) {
+  const long long tiles_m = (M + fsb::BLOCK_M - 1) / fsb::BLOCK_M;
+  const int num_kb = (K + fsb::BLOCK_K - 1) / fsb::BLOCK_K;
+  const int one_n = N <= 128 ? 128 : 256;  // tile width of the one-CTA kernel
+  auto tiles = [&](int bn) -> long long { return tiles_m * ((N + bn - 1) / bn); };
+  GemmPlan best = {GemmPlan::ONE_CTA, one_n, 1};
+  if (tiles(one_n) > num_sms) {
+    if (pair_allowed && M >= 256 && N >= 256) best.kind = GemmPlan::PAIR;
+    return best;
+  }
+  float cost = 6.5f + (one_n == 128 ? 0.32f : 0.39f) * num_kb;
+  for (int bn = 64; bn <= 128; bn *= 2) {
+    for (int c = 1; c <= 8 && c <= num_kb; c *= 2) {
+      const long long ctas = tiles(bn) * c;
+      const int limit = c <= 2 ? num_sms : c == 4 ? 128 : 64;
+      if (ctas > limit) break;
+      const float base = c == 1 ? 6.2f : c == 8 ? 10.f : 8.3f;
+      const float t = base + (bn == 64 ? 0.28f : 0.32f) * ((num_kb + c - 1) / c);
+      if (t < cost) {
+        cost = t;
+        best = {GemmPlan::CLUSTER_K, bn, c};
+      }
+    }
+  }
+  return best;
+}
+
 // C ABI ------------------------------------------------------------------------------------------
 // lda / ldb: elements between consecutive rows of the *stored* matrix ([rows,K] when K-major,
 // [K,rows] when MN-major). All leading dimensions must be multiples of 8; pointers 16-byte aligned.
@@ -622,13 +681,23 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* bia
                           int epilogue, int out_f32, int accumulate_c, int max_ctas, int* status, cudaStream_t stream,
                           const unsigned int* b_ready, unsigned int b_ready_epoch, long long b_piece_bytes, unsigned long long b_wait_ns,
                           const unsigned int* a_ready = nullptr, int a_shard_rows = 0, int a_piece_rows = 0, int a_first_shard = 0,
-                          int a_num_shards = 0, int b_first_piece = 0);
+                          int a_num_shards = 0, int b_first_piece = 0, int ck_block_n = 0, int ck_splits = 0);
 
 FSB_API int fsb_gemm_bf16(const void* A, const void* B, void* C, const void* bias, const void* aux, void* aux_out,
                           int M, int N, int K, int lda, int ldb, int ldc, int ld_aux, int a_mn_major, int b_mn_major,
                           int epilogue, int out_f32, int accumulate_c, int max_ctas, int* status, cudaStream_t stream) {
   return gemm_bf16_impl(A, B, C, bias, aux, aux_out, M, N, K, lda, ldb, ldc, ld_aux, a_mn_major, b_mn_major, epilogue, out_f32,
                         accumulate_c, max_ctas, status, stream, nullptr, 0u, 0, 0ull);
+}
+
+// The same product by the cluster split-K kernel (gemm_cluster_k.cu) whatever its shape: block_n 64 or 128, splits 1, 2, 4
+// or 8 and no more than the number of 64-wide K blocks (-1 otherwise).  fsb_gemm_bf16 chooses these by itself.
+FSB_API int fsb_gemm_bf16_cluster_k(const void* A, const void* B, void* C, const void* bias, const void* aux, void* aux_out,
+                                    int M, int N, int K, int lda, int ldb, int ldc, int ld_aux, int a_mn_major, int b_mn_major,
+                                    int epilogue, int out_f32, int accumulate_c, int block_n, int splits, int* status, cudaStream_t stream) {
+  if (splits < 1) return -1;
+  return gemm_bf16_impl(A, B, C, bias, aux, aux_out, M, N, K, lda, ldb, ldc, ld_aux, a_mn_major, b_mn_major, epilogue, out_f32,
+                        accumulate_c, 0, status, stream, nullptr, 0u, 0, 0ull, nullptr, 0, 0, 0, 0, 0, block_n, splits);
 }
 
 // C[M, N] = epilogue(A[M, K] * B^T + bias) with B ([N, K], rows contiguous: ldb == K) arriving while the kernel runs:
@@ -665,7 +734,7 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* bia
                           int epilogue, int out_f32, int accumulate_c, int max_ctas, int* status, cudaStream_t stream,
                           const unsigned int* b_ready, unsigned int b_ready_epoch, long long b_piece_bytes, unsigned long long b_wait_ns,
                           const unsigned int* a_ready, int a_shard_rows, int a_piece_rows, int a_first_shard, int a_num_shards,
-                          int b_first_piece) {
+                          int b_first_piece, int ck_block_n, int ck_splits) {
   using namespace fsb;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) % 16) || (reinterpret_cast<uintptr_t>(B) % 16)) return -1;
@@ -709,14 +778,15 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* bia
   int grid = tiles < num_sms ? tiles : num_sms;
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
 
-  cudaError_t err;
-  static int pair_mode = -1;  // FSB_GEMM_PAIR=0 disables the CTA-pair kernel
-  if (pair_mode < 0) {
-    const char* e = getenv("FSB_GEMM_PAIR");
-    pair_mode = (e != nullptr && e[0] == '0') ? 0 : 1;
-  }
-  if ((b_ready != nullptr || a_ready != nullptr) && !(pair_mode == 1 && M >= 256 && N >= 256 && max_ctas == 0)) return -1;
-  if (pair_mode == 1 && M >= 256 && N >= 256 && max_ctas == 0) {
+  if (ck_splits > 0) return fsb_host::gemm_cluster_k(ta, B, ldb, p, ck_block_n, ck_splits, dev, stream);
+
+  if ((b_ready != nullptr || a_ready != nullptr) && !(pair_enabled() && M >= 256 && N >= 256 && max_ctas == 0)) return -1;
+  const bool streamed = b_ready != nullptr || a_ready != nullptr;  // only the pair kernel waits for arriving operands
+  GemmPlan plan = {GemmPlan::ONE_CTA, block_n, 1};
+  if (streamed) plan.kind = GemmPlan::PAIR;
+  else if (max_ctas == 0) plan = choose_gemm_plan(M, N, K, num_sms, pair_enabled());
+  if (plan.kind == GemmPlan::CLUSTER_K) return fsb_host::gemm_cluster_k(ta, B, ldb, p, plan.block_n, plan.splits, dev, stream);
+  if (plan.kind == GemmPlan::PAIR) {
     // the B map's box is this CTA's 128 columns (K-major) / 64 (MN-major, unchanged)
     if (!b_mn_major && !fsb_host::encode_2d_16bit(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BLOCK_K, PAIR_HALF_N)) return -1;
     static bool pair_attr_set[64] = {false};
@@ -745,8 +815,7 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* bia
     }
     gemm_bf16_tcgen05_kernel<128, false><<<grid, GEMM_THREADS, SmemLayout<128>::TOTAL, stream>>>(ta, tb, p);
   }
-  err = cudaGetLastError();
-  return static_cast<int>(err);
+  return static_cast<int>(cudaGetLastError());
 }
 
 // `batch` independent products of one shape in a single launch (the local experts of an MoE layer):
@@ -789,7 +858,7 @@ FSB_API int fsb_gemm_bf16_batched(const void* A, const void* B, void* C, const v
   cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
   const long long tiles = static_cast<long long>(batch) * ((M + BLOCK_M - 1) / BLOCK_M) * ((N + block_n - 1) / block_n);
   const int grid = tiles < num_sms ? static_cast<int>(tiles) : num_sms;
-  if (M >= 256 && N >= 256) {
+  if (pair_enabled() && M >= 256 && N >= 256) {
     // the rule of fsb_gemm_bf16: 256 x 256 tiles by CTA pairs once a problem has a whole one
     if (!b_mn_major && !fsb_host::encode_3d_16bit(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)batch, (uint64_t)ldb, (uint64_t)stride_b, BLOCK_K, PAIR_HALF_N, 1)) return -1;
     static bool pair_attr_set[64] = {false};

@@ -134,6 +134,52 @@ def test_moe_rows_match_index_ops(S, E, M, dtype):
         torch.testing.assert_close(a.float(), b.float(), rtol=eps, atol=eps * b.float().abs().max().item())
 
 
+# (M, N, K): below, at and above the 128 x 64 / 128 x 128 tiles, K of one block, K no multiple of a block, K with fewer
+# blocks than a cluster could split
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("M,N,K", [(8, 8, 64), (77, 1000, 1024), (128, 64, 512), (136, 72, 520), (256, 200, 136), (264, 128, 4096)])
+@pytest.mark.parametrize("block_n,splits", [(64, 1), (64, 8), (128, 1), (128, 2), (128, 4)])
+def test_cluster_split_k_gemm(M, N, K, a_mn, b_mn, block_n, splits):
+    from ctypes import c_int, c_void_p
+
+    from fairscale_b200.ops import _bind
+
+    _bind._SIGNATURES.setdefault("fsb_gemm_bf16_cluster_k", [c_void_p] * 6 + [c_int] * 14 + [c_void_p, c_void_p])
+    torch.manual_seed(M + N + K)
+    a = torch.randn((K, -(-M // 8) * 8), device=_dev()).bfloat16()[:, :M] if a_mn else torch.randn((M, K), device=_dev()).bfloat16()
+    b = torch.randn((K, N) if b_mn else (N, K), device=_dev()).bfloat16()
+    bias = torch.randn(N, device=_dev()).bfloat16()
+    aux = torch.randn(M, N, device=_dev()).bfloat16()
+    ref = (a.t() if a_mn else a).double() @ (b if b_mn else b.t()).double()
+
+    def run(epi, dtype=torch.bfloat16, use_bias=False, use_aux=False, pre=None, into=None, accumulate=0):
+        c = into if into is not None else torch.full((M, N), float("nan"), device=_dev(), dtype=dtype)
+        code = _bind.fn("fsb_gemm_bf16_cluster_k")(
+            a.data_ptr(), b.data_ptr(), c.data_ptr(), bias.data_ptr() if use_bias else None, aux.data_ptr() if use_aux else None,
+            _bind.ptr(pre), M, N, K, a.stride(0), b.stride(0), N, N, int(a_mn), int(b_mn), epi, int(dtype == torch.float32), accumulate,
+            block_n, splits, _bind.status_ptr(_dev()), _bind.stream_ptr(_dev()))
+        assert code == (-1 if splits > -(-K // 64) else 0)
+        return c
+
+    if splits > -(-K // 64):
+        run(0)  # refused: a CTA of the cluster would have no K block
+        return
+    assert _rel_err(run(0), ref) < 1e-2
+    f32 = run(0, torch.float32)
+    assert _rel_err(f32, ref) < 1e-5
+    assert _rel_err(run(0, torch.float32, into=f32.clone(), accumulate=1), 2 * ref) < 1e-5
+    with_bias = ref + bias.double()
+    pre = torch.empty(M, N, device=_dev(), dtype=torch.bfloat16)
+    assert _rel_err(run(2, use_bias=True, pre=pre), torch.nn.functional.gelu(with_bias)) < 1e-2
+    assert _rel_err(pre, with_bias) < 1e-2
+    assert _rel_err(run(3, use_bias=True, use_aux=True), with_bias + aux.double()) < 1e-2
+    z = aux.double().requires_grad_()
+    torch.nn.functional.gelu(z).sum().backward()
+    assert _rel_err(run(4, use_aux=True), ref * z.grad) < 1e-2
+    assert torch.equal(run(0, torch.float32), f32)  # the cluster sums in a fixed order
+    _status_ok()
+
+
 @pytest.mark.parametrize("E,C,K,N", [(2, 256, 256, 256), (3, 257, 72, 264), (4, 410, 512, 2048), (1, 300, 64, 256)])
 def test_batched_pair_gemm_edges(E, C, K, N):
     """Problems with whole 256 x 256 tiles run on CTA pairs; remainders must not leak into the next problem."""
