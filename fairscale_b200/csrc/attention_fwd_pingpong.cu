@@ -11,11 +11,19 @@
 //
 // Roles (320 threads): warp 0 TMA producer, warp 1 MMA issuer and TMEM owner, warps 2-5 softmax of tile A, warps 6-9
 // softmax of tile B; one thread per query row (TMEM lane), so the row maximum and row sum need no exchange.
-// TMEM (512 columns): S_A [0,128)  S_B [128,256)  O_A [256,256+D)  O_B [384,384+D).  The bf16 probabilities overwrite
+// TMEM (512 columns): S_A [0,128)  S_B [128,256)  O_A [256,256+D)  O_B [384,384+D).  With head size 128 the bf16 probabilities overwrite
 // the first 64 columns of their own score tile (two values per 32-bit column) and feed P V as the TMEM A operand of
 // tcgen05.mma, so they never pass through shared memory.  The tensor pipe executes in issue order: S_t(j+1) is issued
 // after PV_t(j) and therefore cannot overwrite P_t(j) early.
 // Tile A skips the last key tile of the item (it lies wholly above A's diagonal).  Every mbarrier wait is bounded.
+//
+// Head size 64 leaves 128 TMEM columns free, and the probabilities get them (P_A [384,448)  P_B [448,512), O_B [320,384)).
+// Then S_t(j+1) need not wait for PV_t(j): it is issued as soon as the softmax warps have read the last scores of step j,
+// half-way through their exponentials, and is ready when they come back for it:
+//
+//   tensor pipe :  S_A(j+1)  S_B(j+1)  PV_A(j)  PV_B(j)  S_A(j+2) ...
+//
+// (In place, the chain exponentials -> PV -> S -> maximum kept the exponential unit, which bounds this head size, at 57 %.)
 //
 // Any sequence length: the tensor map is three-dimensional (columns, positions, batch), so a tile that overhangs the
 // sequence reads zeros instead of the next sequence's rows; keys past the end lie above every real query's diagonal and
@@ -65,6 +73,7 @@ struct Bars {
   uint64_t s_full[2];   // per query tile: scores of the current step are in TMEM
   uint64_t p_full[2];   // per query tile: probabilities written (4 warp arrivals)
   uint64_t o_done[2];   // per query tile: P V of the current step has completed
+  uint64_t s_read[2];   // per query tile, head size 64: the softmax warps hold all scores of the step (4 warp arrivals)
   uint64_t q_empty;     // the item's last Q K^T products have completed: the query tiles may be replaced
   uint64_t o_free[2];   // per query tile: the softmax warps have read the item's output accumulator (4 warp arrivals)
   uint32_t tmem_slot;
@@ -139,6 +148,9 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
   constexpr int SLABS = D / 64;
   constexpr uint32_t SLAB = BM * 128;  // bytes of a [128 x 64] bf16 slab
   constexpr uint32_t TMEM_COLS = 512;
+  constexpr bool SEP = D == 64;                    // probabilities in columns of their own
+  constexpr uint32_t O_COL = 256, O_STEP = SEP ? 64 : 128;
+  constexpr uint32_t P_COL = SEP ? 384 : 0, P_STEP = SEP ? 64 : 128;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   Bars* bars = reinterpret_cast<Bars*>(smem + L::BAR_OFF);
@@ -165,6 +177,7 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
       mbar_init(&bars->p_full[i], 4);
       mbar_init(&bars->o_done[i], 1);
       mbar_init(&bars->o_free[i], 4);
+      mbar_init(&bars->s_read[i], 4);
     }
     bars->abort_flag = 0;
     fence_barrier_init();
@@ -225,10 +238,13 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
     uint32_t cs[2] = {0, 0};   // steps issued so far per query tile (phase of p_full)
     uint32_t it = 0;
     uint32_t it_b = 0;         // items with a second query tile so far (phase of o_free[1])
+    uint32_t ss[2] = {0, 0};   // score products issued so far per query tile (phase of s_read)
     bool ok = true;
     auto issue_s = [&](int t, uint32_t kt) -> bool {
       const int st = kt & 1;
       if (!mbar_wait_warp(&bars->k_full[st], (kt >> 1) & 1u, abort_flag)) return false;
+      if (SEP && ss[t] > 0 && !mbar_wait_warp(&bars->s_read[t], (ss[t] - 1u) & 1u, abort_flag)) return false;
+      ++ss[t];
       tc_fence_after_sync();
       const uint32_t sk = smem_u32(smem + L::K_OFF + st * L::TILE);
       if (elect_one()) {
@@ -247,7 +263,7 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
       if (elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < BN / 16; ++ks)
-          umma_f16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + ks * 8, desc_mnmajor(sv, ks, SLAB), idesc_o, (!first || ks != 0) ? 1u : 0u);
+          umma_f16_ts(tmem_base + O_COL + t * O_STEP, tmem_base + P_COL + t * P_STEP + ks * 8, desc_mnmajor(sv, ks, SLAB), idesc_o, (!first || ks != 0) ? 1u : 0u);
         umma_commit(&bars->o_done[t]);
       }
       __syncwarp();
@@ -274,6 +290,15 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
         if (!mbar_wait_warp(&bars->v_full[st], (kt >> 1) & 1u, abort_flag)) { ok = false; break; }
         if (item == static_cast<int>(blockIdx.x)) { PP_TRACE(0, j, 0); }
         if (p.trace != nullptr && item == 0 && j < 32 && lane == 0) p.trace[384 + j] = clock64();
+        if (SEP) {
+          // the next step's scores first: they wait for reads half-way through the exponentials of this one
+          if (j + 1 < n_a && !issue_s(0, kt + 1)) { ok = false; break; }
+          if (j + 1 < n_kv) {
+            if (has_b && !issue_s(1, kt + 1)) { ok = false; break; }
+            commit(&bars->k_empty[(kt + 1) & 1]);
+            if (j + 2 == n_kv) commit(&bars->q_empty);  // that was the item's last use of the query tiles
+          }
+        }
         if (j == 0) {
           // the output accumulators still belong to the previous item until its softmax warps have read them
           if (!mbar_wait_warp(&bars->o_free[0], (it & 1u) ^ 1u, abort_flag)) { ok = false; break; }
@@ -282,13 +307,13 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
         if (j < n_a) {
           if (!issue_pv(0, kt, j == 0)) { ok = false; break; }
           if (item == static_cast<int>(blockIdx.x)) { PP_TRACE(0, j, 1); }
-          if (j + 1 < n_a && !issue_s(0, kt + 1)) { ok = false; break; }
+          if (!SEP && j + 1 < n_a && !issue_s(0, kt + 1)) { ok = false; break; }
         }
         if (item == static_cast<int>(blockIdx.x)) { PP_TRACE(0, j, 2); }
         if (has_b && !issue_pv(1, kt, j == 0)) { ok = false; break; }
         if (item == static_cast<int>(blockIdx.x)) { PP_TRACE(0, j, 3); }
         commit(&bars->v_empty[st]);
-        if (j + 1 < n_kv) {
+        if (!SEP && j + 1 < n_kv) {
           if (has_b && !issue_s(1, kt + 1)) { ok = false; break; }
           commit(&bars->k_empty[(kt + 1) & 1]);
           if (j + 2 == n_kv) commit(&bars->q_empty);  // that was the item's last use of the query tiles
@@ -303,8 +328,9 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
     const int quad = warp & 3;
     const int row = quad * 32 + lane;
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
-    const uint32_t ts = tmem_base + t * 128 + lane_off;        // scores; probabilities overwrite columns [0, 64)
-    const uint32_t to = tmem_base + 256 + t * 128 + lane_off;  // output accumulator
+    const uint32_t ts = tmem_base + t * 128 + lane_off;                   // scores
+    const uint32_t tp = tmem_base + P_COL + t * P_STEP + lane_off;         // probabilities (columns [0, 64) of the scores unless SEP)
+    const uint32_t to = tmem_base + O_COL + t * O_STEP + lane_off;         // output accumulator
     const float sl2 = p.scale * LOG2E;
     uint32_t cs = 0;  // steps of this tile so far, over all items (phase of s_full / o_done)
     bool ok = true;
@@ -342,10 +368,14 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
         const float alpha = (m_run == -INFINITY) ? 0.f : ex2_approx((m_run - m_new) * sl2);
         const float mb = m_new * sl2;
         if (traced) { PP_TRACE(1 + t, j, 1); }
-        if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-          // O_t belongs to P V of step j-1 until that has completed (it has: S_t(j) was issued behind it)
+        const bool rescale = j > 0 && __any_sync(0xffffffffu, alpha != 1.f);
+        if (j > 0 && (SEP || rescale)) {
+          // O_t (and P_t, where it has columns of its own) belongs to P V of step j-1 until that has completed; in place it
+          // has, because S_t(j) was issued behind it
           if (!mbar_wait(&bars->o_done[t], (cs - 1u) & 1u, abort_flag)) { ok = false; break; }
           tc_fence_after_sync();
+        }
+        if (rescale) {
 #pragma unroll 1
           for (int c = 0; c < D / 32; ++c) {
             uint32_t r[32];
@@ -362,7 +392,7 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
           }
         }
         if (traced) { PP_TRACE(1 + t, j, 2); }
-        // pass 2: exponentials; chunk c of 32 keys becomes 16 packed columns at [16 c, 16 c + 16), always behind the reads
+        // pass 2: exponentials; chunk c of 32 keys becomes 16 packed columns at [16 c, 16 c + 16), in place always behind the reads
         float rs = 0.f;
         uint32_t pk[16];
         tmem_ld_32x32(ts, r0);
@@ -370,15 +400,20 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
         tmem_ld_wait();
         if (!diag) rs += chunk_exp<false>(r0, 0, row, sl2, mb, pk); else rs += chunk_exp<true>(r0, 0, row, sl2, mb, pk);
         tmem_ld_32x32(ts + 64, r0);  // in flight during the next exponentials
-        tmem_st_32x16(ts, pk);
+        tmem_st_32x16(tp, pk);
         if (!diag) rs += chunk_exp<false>(r1, 32, row, sl2, mb, pk); else rs += chunk_exp<true>(r1, 32, row, sl2, mb, pk);
         tmem_ld_32x32(ts + 96, r1);
-        tmem_st_32x16(ts + 16, pk);
+        tmem_st_32x16(tp + 16, pk);
         tmem_ld_wait();
+        if (SEP) {
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->s_read[t]);
+        }
         if (!diag) rs += chunk_exp<false>(r0, 64, row, sl2, mb, pk); else rs += chunk_exp<true>(r0, 64, row, sl2, mb, pk);
-        tmem_st_32x16(ts + 32, pk);
+        tmem_st_32x16(tp + 32, pk);
         if (!diag) rs += chunk_exp<false>(r1, 96, row, sl2, mb, pk); else rs += chunk_exp<true>(r1, 96, row, sl2, mb, pk);
-        tmem_st_32x16(ts + 48, pk);
+        tmem_st_32x16(tp + 48, pk);
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
