@@ -64,15 +64,14 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// K-major operand descriptor for k-step `ks` (16 elements) of a tile made of [rows x 64] slabs of `slab_bytes`
-__device__ __forceinline__ uint64_t desc_kmajor(uint32_t base, int ks, uint32_t slab_bytes) {
-  return make_smem_desc(base + static_cast<uint32_t>(ks >> 2) * slab_bytes + static_cast<uint32_t>(ks & 3) * 32u, 16u, 1024u);
+// Operand descriptors of tiles made of [rows x 64] slabs of `slab_bytes`, and the byte offsets of their k-steps: K-major 16
+// elements (32 bytes inside the swizzle row); MN-major (the same bytes as [k_rows x 64] slabs) 16 k_rows = 2048 bytes.
+__device__ __forceinline__ uint64_t desc_kmajor(uint32_t base) { return make_smem_desc(base, 16u, 1024u); }
+__device__ __forceinline__ uint64_t desc_mnmajor(uint32_t base, uint32_t slab_bytes) { return make_smem_desc(base, slab_bytes, 1024u); }
+__device__ __forceinline__ constexpr uint32_t kstep_kmajor(int ks, uint32_t slab_bytes) {
+  return static_cast<uint32_t>(ks >> 2) * slab_bytes + static_cast<uint32_t>(ks & 3) * 32u;
 }
-// MN-major operand descriptor: the tile is [k_rows x 64] slabs (one per 64 MN elements, `slab_bytes` apart);
-// k-step `ks` covers 16 k_rows = 2048 bytes.
-__device__ __forceinline__ uint64_t desc_mnmajor(uint32_t base, int ks, uint32_t slab_bytes) {
-  return make_smem_desc(base + static_cast<uint32_t>(ks) * 2048u, slab_bytes, 1024u);
-}
+__device__ __forceinline__ constexpr uint32_t kstep_mnmajor(int ks) { return static_cast<uint32_t>(ks) * 2048u; }
 
 struct AttnBars {
   uint64_t stat_full;     // stationary tiles landed
@@ -229,10 +228,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    // MMA issuer: all lanes run the loop, one elected lane issues each group
+    // MMA issuer: the whole warp, see umma_f16_ss_warp
     const uint32_t idesc_s = make_idesc_f16(ATT_BM, 64, true, false, false);
     const uint32_t idesc_q = make_idesc_f16(ATT_BM, D, true, false, true);  // dS K : dS from TMEM, K tile read MN-major
-    const uint32_t sq = smem_u32(smem + L::Q_OFF), sdo = smem_u32(smem + L::DO_OFF);
+    const uint64_t dq = desc_kmajor(smem_u32(smem + L::Q_OFF)), ddo = desc_kmajor(smem_u32(smem + L::DO_OFF));
+    const uint64_t dk0 = desc_kmajor(smem_u32(smem + L::K_OFF)), dv0 = desc_kmajor(smem_u32(smem + L::V_OFF));
+    const uint64_t dkt0 = desc_mnmajor(smem_u32(smem + L::K_OFF), SLAB);
     uint32_t jt0 = 0, ut0 = 0, it = 0;  // key tiles / steps of earlier items, items so far
     bool ok = true;
     // step u = key tile u / 2, keys [64 (u & 1), +64) of it; S and dP of step u go to accumulator buffer u & 1
@@ -241,19 +242,16 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_cons
       const int hh = u & 1, st = jt & 1, buf = u & 1;
       if (hh == 0 && !mbar_wait_warp(&bars->str_full[st], (jt >> 1) & 1u, abort_flag, 35)) return false;
       tc_fence_after_sync();
-      const uint32_t sk = smem_u32(smem + L::K_OFF + st * L::TILE) + hh * 8192u;  // rows 64 hh .. of every slab
-      const uint32_t sv = smem_u32(smem + L::V_OFF + st * L::TILE) + hh * 8192u;
-      if (elect_one()) {
+      const uint32_t off = st * L::TILE + hh * 8192u;  // rows 64 hh .. of every slab
+      const uint64_t dk = desc_offset(dk0, off), dv = desc_offset(dv0, off);
 #pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks)
-          umma_f16_ss(tmem_base + buf * 128, desc_kmajor(sq, ks, SLAB), desc_kmajor(sk, ks, SLAB), idesc_s, ks != 0);
+      for (int ks = 0; ks < D / 16; ++ks)
+        umma_f16_ss_warp(tmem_base + buf * 128, desc_offset(dq, kstep_kmajor(ks, SLAB)), desc_offset(dk, kstep_kmajor(ks, SLAB)), idesc_s, ks != 0);
 #pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks)
-          umma_f16_ss(tmem_base + buf * 128 + 64, desc_kmajor(sdo, ks, SLAB), desc_kmajor(sv, ks, SLAB), idesc_s, ks != 0);
-        umma_commit(&bars->s_full[buf]);
-        if (u == n_steps - 1) umma_commit(&bars->stat_empty);  // the item's last use of Q and dO
-      }
-      __syncwarp();
+      for (int ks = 0; ks < D / 16; ++ks)
+        umma_f16_ss_warp(tmem_base + buf * 128 + 64, desc_offset(ddo, kstep_kmajor(ks, SLAB)), desc_offset(dv, kstep_kmajor(ks, SLAB)), idesc_s, ks != 0);
+      umma_commit_warp(&bars->s_full[buf]);
+      if (u == n_steps - 1) umma_commit_warp(&bars->stat_empty);  // the item's last use of Q and dO
       return true;
     };
     for (int item; ok && (item = snake_item(static_cast<int>(it))) < n_items; ++it) {
@@ -268,15 +266,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_cons
         if (u == 0 && !mbar_wait_warp(&bars->acc_free, (it & 1u) ^ 1u, abort_flag, 38)) { ok = false; break; }
         if (!mbar_wait_warp(&bars->p_full[buf], (ut >> 1) & 1u, abort_flag, 39)) { ok = false; break; }
         tc_fence_after_sync();
-        const uint32_t sk = smem_u32(smem + L::K_OFF + st * L::TILE);
-        if (elect_one()) {
+        const uint64_t dkt = desc_offset(dkt0, st * L::TILE + hh * 4 * 2048u);
 #pragma unroll
-          for (int ks = 0; ks < 64 / 16; ++ks)
-            umma_f16_ts(tmem_base + 256, tmem_base + buf * 128 + (ks >> 1) * 32 + (ks & 1) * 8, desc_mnmajor(sk, hh * 4 + ks, SLAB), idesc_q, (u | ks) != 0);
-          if (hh == 1) umma_commit(&bars->str_empty[st]);
-          if (u == n_steps - 1) umma_commit(&bars->acc_done);
-        }
-        __syncwarp();
+        for (int ks = 0; ks < 64 / 16; ++ks)
+          umma_f16_ts_warp(tmem_base + 256, tmem_base + buf * 128 + (ks >> 1) * 32 + (ks & 1) * 8, desc_offset(dkt, kstep_mnmajor(ks)), idesc_q, (u | ks) != 0);
+        if (hh == 1) umma_commit_warp(&bars->str_empty[st]);
+        if (u == n_steps - 1) umma_commit_warp(&bars->acc_done);
         if (u + 2 < n_steps && !issue_sp(u + 2, n_steps)) { ok = false; break; }
       }
       jt0 += static_cast<uint32_t>(n_steps >> 1);
@@ -477,10 +472,12 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    // MMA issuer: all lanes run the loop, one elected lane issues each group
+    // MMA issuer: the whole warp, see umma_f16_ss_warp
     const uint32_t idesc_s = make_idesc_f16(ATT_BM, KV_QSUB, true, false, false);  // K Q^T, V dO^T
     const uint32_t idesc_a = make_idesc_f16(ATT_BM, D, true, false, true);         // P^T dO, dS^T Q (A in TMEM, B MN-major)
-    const uint32_t sk = smem_u32(smem + L::K_OFF), sv = smem_u32(smem + L::V_OFF);
+    const uint64_t dk = desc_kmajor(smem_u32(smem + L::K_OFF)), dv = desc_kmajor(smem_u32(smem + L::V_OFF));
+    const uint64_t dq0 = desc_kmajor(smem_u32(smem + L::Q_OFF)), ddo0 = desc_kmajor(smem_u32(smem + L::DO_OFF));
+    const uint64_t dqt0 = desc_mnmajor(smem_u32(smem + L::Q_OFF), QSLAB), ddot0 = desc_mnmajor(smem_u32(smem + L::DO_OFF), QSLAB);
     uint32_t tt0 = 0, it = 0;
     bool ok = true;
     // S^T(t) = K Q_t^T and dP^T(t) = V dO_t^T into accumulator buffer t & 1
@@ -489,20 +486,16 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_cons
       const int st = tt % L::STAGES, buf = t & 1;
       if (!mbar_wait_warp(&bars->str_full[st], (tt / L::STAGES) & 1u, abort_flag, 67)) return false;
       tc_fence_after_sync();
-      const uint32_t sq = smem_u32(smem + L::Q_OFF + st * L::QTILE);
-      const uint32_t sdo = smem_u32(smem + L::DO_OFF + st * L::QTILE);
+      const uint64_t dq = desc_offset(dq0, st * L::QTILE), ddo = desc_offset(ddo0, st * L::QTILE);
       const uint32_t t_s = tmem_base + (buf ? 384u : 0u);
-      if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks)
-          umma_f16_ss(t_s, desc_kmajor(sk, ks, SLAB), desc_kmajor(sq, ks, QSLAB), idesc_s, ks != 0);
+      for (int ks = 0; ks < D / 16; ++ks)
+        umma_f16_ss_warp(t_s, desc_offset(dk, kstep_kmajor(ks, SLAB)), desc_offset(dq, kstep_kmajor(ks, QSLAB)), idesc_s, ks != 0);
 #pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks)
-          umma_f16_ss(t_s + 64, desc_kmajor(sv, ks, SLAB), desc_kmajor(sdo, ks, QSLAB), idesc_s, ks != 0);
-        umma_commit(&bars->s_full[buf]);
-        if (t == n_sub - 1) umma_commit(&bars->stat_empty);  // the item's last use of the K and V tiles
-      }
-      __syncwarp();
+      for (int ks = 0; ks < D / 16; ++ks)
+        umma_f16_ss_warp(t_s + 64, desc_offset(dv, kstep_kmajor(ks, SLAB)), desc_offset(ddo, kstep_kmajor(ks, QSLAB)), idesc_s, ks != 0);
+      umma_commit_warp(&bars->s_full[buf]);
+      if (t == n_sub - 1) umma_commit_warp(&bars->stat_empty);  // the item's last use of the K and V tiles
       return true;
     };
     for (int item; ok && (item = snake_item(static_cast<int>(it))) < n_items; ++it) {
@@ -513,25 +506,21 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_cons
       for (int t = 0; t < n_sub && ok; ++t) {
         const uint32_t tt = tt0 + t;
         const int st = tt % L::STAGES;
-        const uint32_t sq = smem_u32(smem + L::Q_OFF + st * L::QTILE);
-        const uint32_t sdo = smem_u32(smem + L::DO_OFF + st * L::QTILE);
+        const uint64_t dqt = desc_offset(dqt0, st * L::QTILE), ddot = desc_offset(ddot0, st * L::QTILE);
         // dK / dV still belong to the previous item until its threads have read them
         if (t == 0 && !mbar_wait_warp(&bars->acc_free, (it & 1u) ^ 1u, abort_flag, 70)) { ok = false; break; }
         const int buf = t & 1;
         if (!mbar_wait_warp(&bars->p_full[buf], (tt >> 1) & 1u, abort_flag, 71)) { ok = false; break; }
         tc_fence_after_sync();
         const uint32_t t_s = tmem_base + (buf ? 384u : 0u);
-        if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < KV_QSUB / 16; ++ks)
-            umma_f16_ts(tmem_base + 128, t_s + (ks >> 1) * 32 + (ks & 1) * 8, desc_mnmajor(sdo, ks, QSLAB), idesc_a, (t | ks) != 0);
+        for (int ks = 0; ks < KV_QSUB / 16; ++ks)
+          umma_f16_ts_warp(tmem_base + 128, t_s + (ks >> 1) * 32 + (ks & 1) * 8, desc_offset(ddot, kstep_mnmajor(ks)), idesc_a, (t | ks) != 0);
 #pragma unroll
-          for (int ks = 0; ks < KV_QSUB / 16; ++ks)
-            umma_f16_ts(tmem_base + 256, t_s + 64 + (ks >> 1) * 32 + (ks & 1) * 8, desc_mnmajor(sq, ks, QSLAB), idesc_a, (t | ks) != 0);
-          umma_commit(&bars->str_empty[st]);
-          if (t == n_sub - 1) umma_commit(&bars->acc_done);
-        }
-        __syncwarp();
+        for (int ks = 0; ks < KV_QSUB / 16; ++ks)
+          umma_f16_ts_warp(tmem_base + 256, t_s + 64 + (ks >> 1) * 32 + (ks & 1) * 8, desc_offset(dqt, kstep_mnmajor(ks)), idesc_a, (t | ks) != 0);
+        umma_commit_warp(&bars->str_empty[st]);
+        if (t == n_sub - 1) umma_commit_warp(&bars->acc_done);
         if (t + 2 < n_sub && !issue_sp(t + 2, n_sub)) { ok = false; break; }
       }
       tt0 += static_cast<uint32_t>(n_sub);

@@ -105,14 +105,14 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&v);
 }
-// K-major operand: [rows x 64] slabs of `slab_bytes`; k-step ks covers 16 elements (32 bytes inside the swizzle row)
-__device__ __forceinline__ uint64_t desc_kmajor(uint32_t base, int ks, uint32_t slab_bytes) {
-  return make_smem_desc(base + static_cast<uint32_t>(ks >> 2) * slab_bytes + static_cast<uint32_t>(ks & 3) * 32u, 16u, 1024u);
+// Operand descriptors: K-major [rows x 64] slabs of `slab_bytes`, k-step ks covers 16 elements (32 bytes inside the swizzle
+// row); MN-major the same bytes read as [k_rows x 64] slabs, k-step ks covers 16 k_rows = 2048 bytes.
+__device__ __forceinline__ uint64_t desc_kmajor(uint32_t base) { return make_smem_desc(base, 16u, 1024u); }
+__device__ __forceinline__ uint64_t desc_mnmajor(uint32_t base, uint32_t slab_bytes) { return make_smem_desc(base, slab_bytes, 1024u); }
+__device__ __forceinline__ constexpr uint32_t kstep_kmajor(int ks, uint32_t slab_bytes) {
+  return static_cast<uint32_t>(ks >> 2) * slab_bytes + static_cast<uint32_t>(ks & 3) * 32u;
 }
-// MN-major operand: the same bytes read as [k_rows x 64] slabs; k-step ks covers 16 k_rows = 2048 bytes
-__device__ __forceinline__ uint64_t desc_mnmajor(uint32_t base, int ks, uint32_t slab_bytes) {
-  return make_smem_desc(base + static_cast<uint32_t>(ks) * 2048u, slab_bytes, 1024u);
-}
+__device__ __forceinline__ constexpr uint32_t kstep_mnmajor(int ks) { return static_cast<uint32_t>(ks) * 2048u; }
 
 template <bool DIAG>
 __device__ __forceinline__ float chunk_max(const uint32_t (&r)[32], int col0, int row, float m) {
@@ -230,10 +230,11 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer (all lanes run the loop, one is elected per group)
+    // ------------------------------------------------------------------ MMA issuer (the whole warp, see umma_f16_ss_warp)
     const uint32_t idesc_s = make_idesc_f16(BM, BN, true, false, false);  // Q K^T: both K-major
     const uint32_t idesc_o = make_idesc_f16(BM, D, true, false, true);    // P V: P from TMEM, V MN-major
-    const uint32_t sq = smem_u32(smem + L::Q_OFF);
+    const uint64_t dq0 = desc_kmajor(smem_u32(smem + L::Q_OFF)), dk0 = desc_kmajor(smem_u32(smem + L::K_OFF));
+    const uint64_t dv0 = desc_mnmajor(smem_u32(smem + L::V_OFF), SLAB);
     uint32_t kt0 = 0;          // key tiles consumed by earlier items
     uint32_t cs[2] = {0, 0};   // steps issued so far per query tile (phase of p_full)
     uint32_t it = 0;
@@ -246,34 +247,26 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
       if (SEP && ss[t] > 0 && !mbar_wait_warp(&bars->s_read[t], (ss[t] - 1u) & 1u, abort_flag)) return false;
       ++ss[t];
       tc_fence_after_sync();
-      const uint32_t sk = smem_u32(smem + L::K_OFF + st * L::TILE);
-      if (elect_one()) {
+      const uint64_t dq = desc_offset(dq0, t * L::TILE), dk = desc_offset(dk0, st * L::TILE);
 #pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks)
-          umma_f16_ss(tmem_base + t * 128, desc_kmajor(sq + t * L::TILE, ks, SLAB), desc_kmajor(sk, ks, SLAB), idesc_s, ks != 0);
-        umma_commit(&bars->s_full[t]);
-      }
-      __syncwarp();
+      for (int ks = 0; ks < D / 16; ++ks)
+        umma_f16_ss_warp(tmem_base + t * 128, desc_offset(dq, kstep_kmajor(ks, SLAB)), desc_offset(dk, kstep_kmajor(ks, SLAB)), idesc_s, ks != 0);
+      umma_commit_warp(&bars->s_full[t]);
       return true;
     };
     auto issue_pv = [&](int t, uint32_t kt, bool first) -> bool {
       if (!mbar_wait_warp(&bars->p_full[t], cs[t] & 1u, abort_flag)) return false;
       tc_fence_after_sync();
-      const uint32_t sv = smem_u32(smem + L::V_OFF + (kt & 1) * L::TILE);
-      if (elect_one()) {
+      const uint64_t dv = desc_offset(dv0, (kt & 1) * L::TILE);
 #pragma unroll
-        for (int ks = 0; ks < BN / 16; ++ks)
-          umma_f16_ts(tmem_base + O_COL + t * O_STEP, tmem_base + P_COL + t * P_STEP + ks * 8, desc_mnmajor(sv, ks, SLAB), idesc_o, (!first || ks != 0) ? 1u : 0u);
-        umma_commit(&bars->o_done[t]);
-      }
-      __syncwarp();
+      for (int ks = 0; ks < BN / 16; ++ks)
+        umma_f16_ts_warp(tmem_base + O_COL + t * O_STEP, tmem_base + P_COL + t * P_STEP + ks * 8, desc_offset(dv, kstep_mnmajor(ks)), idesc_o,
+                         (!first || ks != 0) ? 1u : 0u);
+      umma_commit_warp(&bars->o_done[t]);
       ++cs[t];
       return true;
     };
-    auto commit = [&](uint64_t* bar) {
-      if (elect_one()) umma_commit(bar);
-      __syncwarp();
-    };
+    auto commit = [&](uint64_t* bar) { umma_commit_warp(bar); };
     for (int item; ok && (item = snake_item(static_cast<int>(it))) < n_items; ++it) {
       const int q2 = n_q2 - 1 - item / HB;
       const bool has_b = 2 * q2 + 1 < n_tiles;

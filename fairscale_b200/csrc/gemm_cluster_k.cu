@@ -181,30 +181,25 @@ gemm_cluster_k_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer (all lanes run the loop, one elected lane issues)
+    // ------------------------------------------------------------------ MMA issuer (the whole warp)
     const uint32_t idesc = make_idesc_f16(BLOCK_M, BN, true, p.a_mn_major != 0, p.b_mn_major != 0);
     const uint32_t a_lbo = p.a_mn_major ? 8192u : 16u, b_lbo = p.b_mn_major ? 8192u : 16u;
     const uint32_t a_kstep = p.a_mn_major ? 2048u : 32u, b_kstep = p.b_mn_major ? 2048u : 32u;
+    const uint64_t adesc0 = make_smem_desc(smem_u32(smem), a_lbo, 1024u), bdesc0 = make_smem_desc(smem_u32(smem) + L::A_BYTES, b_lbo, 1024u);
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
     for (int kb = kb0; kb < kb1; ++kb) {
       if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag, 101)) { ok = false; break; }
       tc_fence_after_sync();
-      const uint32_t sa = smem_u32(smem + stage * L::STAGE_BYTES);
-      const uint32_t sb = sa + L::A_BYTES;
-      if (elect_one()) {
+      const uint64_t ad = desc_offset(adesc0, stage * L::STAGE_BYTES), bd = desc_offset(bdesc0, stage * L::STAGE_BYTES);
 #pragma unroll
-        for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
-          umma_f16_ss(tmem_base, make_smem_desc(sa + k * a_kstep, a_lbo, 1024u), make_smem_desc(sb + k * b_kstep, b_lbo, 1024u), idesc,
-                      (kb != kb0 || k != 0) ? 1u : 0u);
-        umma_commit(&empty_bar[stage]);
-      }
-      __syncwarp();
+      for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
+        umma_f16_ss_warp(tmem_base, desc_offset(ad, k * a_kstep), desc_offset(bd, k * b_kstep), idesc, (kb != kb0 || k != 0) ? 1u : 0u);
+      umma_commit_warp(&empty_bar[stage]);
       if (++stage == NST) { stage = 0; phase ^= 1u; }
     }
-    if (ok && elect_one()) umma_commit(done_bar);
-    __syncwarp();
+    if (ok) umma_commit_warp(done_bar);
   } else {
     // ------------------------------------------------------------------ accumulator -> partial tile, or straight to the epilogue
     const int quad = warp & 3;

@@ -113,13 +113,14 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer (all lanes run the loop, one elected lane issues)
+    // ------------------------------------------------------------------ MMA issuer (the whole warp, see umma_f16_ss_warp)
     {
       const uint32_t idesc = make_idesc_f16(BLOCK_M, BLOCK_N, true, p.a_mn_major != 0, p.b_mn_major != 0);
       // K-major: LBO unused, SBO 1024; UMMA_K advance = 32 B inside the swizzle row.
       // MN-major: LBO = 8192 (next 64 MN elements), SBO 1024; UMMA_K advance = 16 k-rows = 2048 B.
       const uint32_t a_lbo = p.a_mn_major ? 8192u : 16u, b_lbo = p.b_mn_major ? 8192u : 16u;
       const uint32_t a_kstep = p.a_mn_major ? 2048u : 32u, b_kstep = p.b_mn_major ? 2048u : 32u;
+      const uint64_t adesc0 = make_smem_desc(smem_u32(smem), a_lbo, 1024u), bdesc0 = make_smem_desc(smem_u32(smem) + L::A_BYTES, b_lbo, 1024u);
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -132,23 +133,15 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
           tc_fence_after_sync();
-          const uint32_t sa = smem_u32(smem + stage * L::STAGE_BYTES);
-          const uint32_t sb = sa + L::A_BYTES;
-          if (elect_one()) {
+          const uint64_t ad = desc_offset(adesc0, stage * L::STAGE_BYTES), bd = desc_offset(bdesc0, stage * L::STAGE_BYTES);
 #pragma unroll
-            for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
-              const uint64_t adesc = make_smem_desc(sa + k * a_kstep, a_lbo, 1024u);
-              const uint64_t bdesc = make_smem_desc(sb + k * b_kstep, b_lbo, 1024u);
-              umma_f16_ss(d_tmem, adesc, bdesc, idesc, (kb | k) != 0 ? 1u : 0u);
-            }
-            umma_commit(&empty_bar[stage]);  // frees the smem slot once these MMAs have read it
-          }
-          __syncwarp();
+          for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
+            umma_f16_ss_warp(d_tmem, desc_offset(ad, k * a_kstep), desc_offset(bd, k * b_kstep), idesc, (kb | k) != 0 ? 1u : 0u);
+          umma_commit_warp(&empty_bar[stage]);  // frees the smem slot once these MMAs have read it
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
-        if (elect_one()) umma_commit(&tmem_full_bar[acc]);
-        __syncwarp();
+        umma_commit_warp(&tmem_full_bar[acc]);
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1u;
       }
@@ -484,12 +477,13 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer (leader only; all lanes run the loop,
-    // one elected lane issues, so that addresses and descriptors stay warp-uniform)
+    // ------------------------------------------------------------------ MMA issuer (the leader's whole warp, see umma_f16_ss_warp)
     if (leader) {
       const uint32_t idesc = make_idesc_f16(2 * BLOCK_M, PAIR_BLOCK_N, true, p.a_mn_major != 0, p.b_mn_major != 0);
       const uint32_t a_lbo = p.a_mn_major ? 8192u : 16u, b_lbo = p.b_mn_major ? 8192u : 16u;
       const uint32_t a_kstep = p.a_mn_major ? 2048u : 32u, b_kstep = p.b_mn_major ? 2048u : 32u;
+      const uint64_t adesc0 = make_smem_desc(smem_u32(smem), a_lbo, 1024u), bdesc0 = make_smem_desc(smem_u32(smem) + L::A_BYTES, b_lbo, 1024u);
+      const uint32_t empty0 = map_to_cta(smem_u32(empty_bar), 0), empty1 = map_to_cta(smem_u32(empty_bar), 1);
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -509,29 +503,18 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag, 7)) { ok = false; break; }
           tc_fence_after_sync();
-          const uint32_t sa = smem_u32(smem + stage * L::STAGE_BYTES);
-          const uint32_t sb = sa + L::A_BYTES;
-          const uint32_t eb = smem_u32(&empty_bar[stage]);
-          if (elect_one()) {
+          const uint64_t ad = desc_offset(adesc0, stage * L::STAGE_BYTES), bd = desc_offset(bdesc0, stage * L::STAGE_BYTES);
 #pragma unroll
-            for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
-              const uint64_t adesc = make_smem_desc(sa + k * a_kstep, a_lbo, 1024u);
-              const uint64_t bdesc = make_smem_desc(sb + k * b_kstep, b_lbo, 1024u);
-              umma_f16_ss_pair(d_tmem, adesc, bdesc, idesc, (kb | k) != 0 ? 1u : 0u);
-            }
-            umma_commit_pair(map_to_cta(eb, 0));
-            umma_commit_pair(map_to_cta(eb, 1));
-          }
-          __syncwarp();
+          for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
+            umma_f16_ss_pair_warp(d_tmem, desc_offset(ad, k * a_kstep), desc_offset(bd, k * b_kstep), idesc, (kb | k) != 0 ? 1u : 0u);
+          umma_commit_pair_warp(empty0 + stage * 8);
+          umma_commit_pair_warp(empty1 + stage * 8);
           if (++stage == PAIR_STAGES) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
         const uint32_t fb = smem_u32(&tmem_full_bar[acc]);
-        if (elect_one()) {
-          umma_commit_pair(map_to_cta(fb, 0));
-          umma_commit_pair(map_to_cta(fb, 1));
-        }
-        __syncwarp();
+        umma_commit_pair_warp(map_to_cta(fb, 0));
+        umma_commit_pair_warp(map_to_cta(fb, 1));
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1u;
       }
