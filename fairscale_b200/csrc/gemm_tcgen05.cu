@@ -9,7 +9,7 @@
 //   dgrad    dX = dY W   : A = dY (K-major),  B = W  (MN-major, stored [N_out... see gemm.py)
 //   wgrad    dW = dY^T X : A = dY (MN-major), B = X  (MN-major)
 //
-// Structure: persistent kernel, one CTA per SM, 192 threads.
+// Structure: persistent kernel, one CTA per SM, 192 threads, tiles handed out at run time.
 //   warp 0      TMA producer: 128-byte-swizzled 64-wide K slabs of A and B into a 4-stage smem ring
 //   warp 1      allocates TMEM (2 x BLOCK_N fp32 columns) and issues tcgen05.mma (one elected lane)
 //   warps 2..5  epilogue: tcgen05.ld the finished accumulator (each warp its 32-lane quadrant),
@@ -27,6 +27,8 @@
 
 namespace fsb {
 
+constexpr int SCHED_DEPTH = 4;  // tile indices in flight between a CTA's (pair's) scheduler and its readers
+
 // BATCHED (both kernels): the tensor maps are 3-D (K / MN, rows, problem) and a tile index also selects the problem; used
 // for the local experts of an MoE layer (equal capacity per expert), where one launch replaces a Python loop of GEMMs.
 template <int BLOCK_N, bool BATCHED>
@@ -40,7 +42,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* tmem_full_bar = empty_bar + STAGES;
   uint64_t* tmem_empty_bar = tmem_full_bar + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty_bar + 2);
+  uint64_t* sched_full = tmem_empty_bar + 2;              // [SCHED_DEPTH] the slot holds a tile index
+  uint64_t* sched_empty = sched_full + SCHED_DEPTH;       // [SCHED_DEPTH] every reader has taken it
+  volatile int* sched_tile = reinterpret_cast<volatile int*>(sched_empty + SCHED_DEPTH);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(const_cast<int*>(sched_tile) + SCHED_DEPTH);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // warp-uniform
@@ -66,6 +71,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
       mbar_init(&tmem_full_bar[a], 1);
       mbar_init(&tmem_empty_bar[a], 4);  // one arrival per epilogue warp
     }
+    for (int q = 0; q < SCHED_DEPTH; ++q) {
+      mbar_init(&sched_full[q], 1);
+      mbar_init(&sched_empty[q], 5);  // the MMA warp and the epilogue warps
+    }
     fence_barrier_init();
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
@@ -79,13 +88,36 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   tc_fence_after_sync();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
+  // Every CTA starts with the tile of its own index; the tiles after those are handed out at run time, as in the CTA-pair
+  // kernel below and for the same reason: the producer takes the next index from a counter in global memory and publishes it
+  // (or -1 at the end) through a small ring that the other roles read in order.  A launch with one tile per CTA never
+  // touches the counter; one without a counter (p.sched null) strides through the tiles, which is up to 3 % faster on a
+  // device that nothing else uses (16384 x 2048 x 2048: 100 against 102 us).
+  int q = 0;            // this role's position in the ring
+  uint32_t qphase = 0;
+  const bool counted = num_tiles > static_cast<int>(gridDim.x) && p.sched != nullptr;
+  // Reader side, by all lanes of a warp: the next tile (-1: no more, -2: the wait ran out).
+  auto take_tile = [&]() -> int {
+    int t = -2;
+    if (lane == 0 && mbar_wait(&sched_full[q], qphase, abort_flag)) {
+      t = sched_tile[q];
+      mbar_arrive(&sched_empty[q]);
+    }
+    if (++q == SCHED_DEPTH) { q = 0; qphase ^= 1u; }
+    return __shfl_sync(0xffffffffu, t, 0);
+  };
+
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      auto fetch = [&](int before) -> int {  // `before`: the last index this CTA was given
+        return static_cast<int>(gridDim.x) + (counted ? static_cast<int>(atomicAdd(&p.sched[0], 1u)) : before);
+      };
+      int nxt = fetch(static_cast<int>(blockIdx.x));  // needed when the first tile's loads are all on their way
+      for (int tile = blockIdx.x, next_tile = -1; tile >= 0 && ok; tile = next_tile) {
         const int pb = BATCHED ? tile / tiles_per_problem : 0;
         int tm, tn;
         tile_coords(tile - pb * tiles_per_problem, tiles_m, tiles_n, tm, tn);
@@ -110,6 +142,22 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
+        if (!ok) break;
+        // the other roles are a ring of loads behind and look for the next index after this
+        next_tile = nxt < num_tiles ? nxt : -1;
+        if (!mbar_wait(&sched_empty[q], qphase ^ 1u, abort_flag)) break;
+        sched_tile[q] = next_tile;
+        mbar_arrive(&sched_full[q]);
+        if (++q == SCHED_DEPTH) { q = 0; qphase ^= 1u; }
+        if (next_tile >= 0) nxt = fetch(next_tile);  // used one tile from now
+      }
+      if (counted) {
+        // The last CTA to get here has seen every CTA's final fetch (each adds to sched[1] after the value of its last fetch
+        // came back, so no fence is needed): put the counters back for the next launch.
+        if (atomicAdd(&p.sched[1], 1u) == gridDim.x - 1u) {
+          p.sched[0] = 0u;
+          p.sched[1] = 0u;
+        }
       }
     }
   } else if (warp == 1) {
@@ -126,7 +174,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      for (int tile = blockIdx.x; tile >= 0 && ok; tile = take_tile()) {
         if (!mbar_wait_warp(&tmem_empty_bar[acc], acc_phase ^ 1u, abort_flag)) { ok = false; break; }
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BLOCK_N);
@@ -152,7 +200,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+    for (int tile = blockIdx.x; tile >= 0 && ok; tile = take_tile()) {
       const int pb = BATCHED ? tile / tiles_per_problem : 0;
       int tm, tn;
       tile_coords(tile - pb * tiles_per_problem, tiles_m, tiles_n, tm, tn);
@@ -203,7 +251,6 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
 constexpr int PAIR_BLOCK_N = 256;
 constexpr int PAIR_HALF_N = 128;
 constexpr int PAIR_STAGES = 6;
-constexpr int PAIR_SCHED_DEPTH = 4;                      // tile indices in flight between the scheduler and its readers
 constexpr int PAIR_EPI_WARPS = 8;                        // two per TMEM lane quadrant, 128 columns each
 constexpr int PAIR_THREADS = 64 + 32 * PAIR_EPI_WARPS;   // producer warp + MMA warp + epilogue warps
 
@@ -319,10 +366,10 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
   uint64_t* empty_bar = full_bar + PAIR_STAGES;
   uint64_t* tmem_full_bar = empty_bar + PAIR_STAGES;
   uint64_t* tmem_empty_bar = tmem_full_bar + 2;
-  uint64_t* sched_full = tmem_empty_bar + 2;           // [PAIR_SCHED_DEPTH] in every CTA: the slot holds a tile index
-  uint64_t* sched_empty = sched_full + PAIR_SCHED_DEPTH;  // [PAIR_SCHED_DEPTH] in the leader: every reader has taken it
-  volatile int* sched_tile = reinterpret_cast<volatile int*>(sched_empty + PAIR_SCHED_DEPTH);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(const_cast<int*>(sched_tile) + PAIR_SCHED_DEPTH);
+  uint64_t* sched_full = tmem_empty_bar + 2;           // [SCHED_DEPTH] in every CTA: the slot holds a tile index
+  uint64_t* sched_empty = sched_full + SCHED_DEPTH;  // [SCHED_DEPTH] in the leader: every reader has taken it
+  volatile int* sched_tile = reinterpret_cast<volatile int*>(sched_empty + SCHED_DEPTH);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(const_cast<int*>(sched_tile) + SCHED_DEPTH);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // warp-uniform
@@ -351,7 +398,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
       mbar_init(&tmem_full_bar[a], 1);
       mbar_init(&tmem_empty_bar[a], 2 * PAIR_EPI_WARPS);  // the epilogue warps of both CTAs of the pair
     }
-    for (int q = 0; q < PAIR_SCHED_DEPTH; ++q) {
+    for (int q = 0; q < SCHED_DEPTH; ++q) {
       mbar_init(&sched_full[q], 1);
       mbar_init(&sched_empty[q], 2 + 2 * PAIR_EPI_WARPS);  // the peer's producer, the MMA warp, all epilogue warps of the pair
     }
@@ -405,7 +452,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
         st_shared_cluster_u32(map_to_cta(smem_u32(const_cast<int*>(&sched_tile[q])), 1), static_cast<uint32_t>(t));
         mbar_arrive_cluster(map_to_cta(smem_u32(&sched_full[q]), 0));
         mbar_arrive_cluster(map_to_cta(smem_u32(&sched_full[q]), 1));
-        if (++q == PAIR_SCHED_DEPTH) { q = 0; qphase ^= 1u; }
+        if (++q == SCHED_DEPTH) { q = 0; qphase ^= 1u; }
         return true;
       };
       int cur = -1, nxt = -1;
@@ -428,7 +475,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
           }
         } else {
           tile = take_tile(q, qphase, 3);
-          if (++q == PAIR_SCHED_DEPTH) { q = 0; qphase ^= 1u; }
+          if (++q == SCHED_DEPTH) { q = 0; qphase ^= 1u; }
         }
         if (tile < 0) break;
         const int pb = BATCHED ? tile / tiles_per_problem : 0;
@@ -495,7 +542,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
         int tile = 0;
         if (lane == 0) tile = take_tile(q, qphase, 5);
         tile = __shfl_sync(0xffffffffu, tile, 0);
-        if (++q == PAIR_SCHED_DEPTH) { q = 0; qphase ^= 1u; }
+        if (++q == SCHED_DEPTH) { q = 0; qphase ^= 1u; }
         if (tile < 0) break;
         if (!mbar_wait_warp(&tmem_empty_bar[acc], acc_phase ^ 1u, abort_flag, 6)) { ok = false; break; }
         tc_fence_after_sync();
@@ -535,7 +582,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
       int tile = 0;
       if (lane == 0) tile = take_tile(q, qphase, 8);
       tile = __shfl_sync(0xffffffffu, tile, 0);
-      if (++q == PAIR_SCHED_DEPTH) { q = 0; qphase ^= 1u; }
+      if (++q == SCHED_DEPTH) { q = 0; qphase ^= 1u; }
       if (tile < 0) break;
       const int pb = BATCHED ? tile / tiles_per_problem : 0;
       int tm, tn;
@@ -622,12 +669,26 @@ static bool pair_enabled() {  // FSB_GEMM_PAIR=0 disables the CTA-pair kernel
 // One wave of independent CTAs takes about 6.3 us + K blocks x 0.28 / 0.32 / 0.39 us (tiles 64 / 128 / 256 wide): one CTA's
 // operand stream is bound by latency, not by the tensor cores, so shorter slices win until the SMs run out.  A cluster
 // costs about 2 us more for its barriers, 4 us at eight CTAs, and clusters of four or eight do not fit the SMs to the last
-// one (144 CTAs in clusters of four run in two waves), hence the limits on their number.  With more tiles than one wave
-// of single CTAs the pair's halved operand traffic decides.
+// one (144 CTAs in clusters of four run in two waves), hence the limits on their number.
+//
+// With more tiles than one wave of single CTAs it is one CTA per tile or a pair per 256 x 256 tile:
+//
+//   M, N, K                  pair   one CTA          M, N, K (in a loop of a second)  pair   one CTA, strided
+//   4096, 2048, 2048         36.1    30.0            16384, 6144, 2048               338.5   330.7
+//   8192, 4096, 1024         64.3    56.5            16384, 2048, 8192               440.0   448.0
+//   5970, 6144, 2048        114.6   111.8            4096, 12288, 4096               323.0   334.0
+//   16384, 2048, 2048       104.1   102.1            8192, 2048, 16384 (wgrad)       490.0   513.0
+//
+// A pair costs some 6 us more per launch and rounds up to larger tiles, but moves a third less operand data, which counts
+// once a product is long enough to run at the card's power limit: beyond 2.56e11 operations, unless K is so short that the
+// output, which one CTA drains in smaller pieces, is what takes the time (16 x 8192 x 2048 x K 256: 316 against 178 us).
 struct GemmPlan {
   enum Kind { PAIR, ONE_CTA, CLUSTER_K } kind;
   int block_n, splits;
 };
+static bool pair_pays(long long problems, int M, int N, int K) {
+  return M >= 256 && N >= 256 && K > 512 && 2.0 * problems * M * N * K > 2.56e11;
+}
 static GemmPlan choose_gemm_plan(int M, int N, int K, int num_sms, bool pair_allowed) {
   const long long tiles_m = (M + fsb::BLOCK_M - 1) / fsb::BLOCK_M;
   const int num_kb = (K + fsb::BLOCK_K - 1) / fsb::BLOCK_K;
@@ -635,7 +696,7 @@ static GemmPlan choose_gemm_plan(int M, int N, int K, int num_sms, bool pair_all
   auto tiles = [&](int bn) -> long long { return tiles_m * ((N + bn - 1) / bn); };
   GemmPlan best = {GemmPlan::ONE_CTA, one_n, 1};
   if (tiles(one_n) > num_sms) {
-    if (pair_allowed && M >= 256 && N >= 256) best.kind = GemmPlan::PAIR;
+    if (pair_allowed && pair_pays(1, M, N, K)) best.kind = GemmPlan::PAIR;
     return best;
   }
   float cost = 6.5f + (one_n == 128 ? 0.32f : 0.39f) * num_kb;
@@ -769,6 +830,11 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* bia
   if (streamed) plan.kind = GemmPlan::PAIR;
   else if (max_ctas == 0) plan = choose_gemm_plan(M, N, K, num_sms, pair_enabled());
   if (plan.kind == GemmPlan::CLUSTER_K) return fsb_host::gemm_cluster_k(ta, B, ldb, p, plan.block_n, plan.splits, dev, stream);
+  // Run-time tile hand-out for products large enough to share the device with a collective; small ones stride.
+  if (max_ctas == 0 && M >= 256 && N >= 256 && (plan.kind == GemmPlan::PAIR || tiles > num_sms)) {
+    p.sched = next_sched_slot(di);
+    if (p.sched == nullptr) return -1;
+  }
   if (plan.kind == GemmPlan::PAIR) {
     // the B map's box is this CTA's 128 columns (K-major) / 64 (MN-major, unchanged)
     if (!b_mn_major && !fsb_host::encode_2d_16bit(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BLOCK_K, PAIR_HALF_N)) return -1;
@@ -780,8 +846,6 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* bia
     const int pair_tiles = ((M + 2 * BLOCK_M - 1) / (2 * BLOCK_M)) * ((N + PAIR_BLOCK_N - 1) / PAIR_BLOCK_N);
     const int max_pairs = num_sms / 2;
     const int pairs = pair_tiles < max_pairs ? pair_tiles : max_pairs;
-    p.sched = next_sched_slot(di);
-    if (p.sched == nullptr) return -1;
     gemm_bf16_tcgen05_pair_kernel<false><<<2 * pairs, PAIR_THREADS, PairSmem::TOTAL, stream>>>(ta, tb, p);
     return static_cast<int>(cudaGetLastError());
   }
@@ -841,8 +905,7 @@ FSB_API int fsb_gemm_bf16_batched(const void* A, const void* B, void* C, const v
   cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
   const long long tiles = static_cast<long long>(batch) * ((M + BLOCK_M - 1) / BLOCK_M) * ((N + block_n - 1) / block_n);
   const int grid = tiles < num_sms ? static_cast<int>(tiles) : num_sms;
-  if (pair_enabled() && M >= 256 && N >= 256) {
-    // the rule of fsb_gemm_bf16: 256 x 256 tiles by CTA pairs once a problem has a whole one
+  if (pair_enabled() && pair_pays(batch, M, N, K)) {
     if (!b_mn_major && !fsb_host::encode_3d_16bit(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)batch, (uint64_t)ldb, (uint64_t)stride_b, BLOCK_K, PAIR_HALF_N, 1)) return -1;
     static bool pair_attr_set[64] = {false};
     if (!pair_attr_set[dev & 63]) {

@@ -36,8 +36,8 @@ struct GemmParams {
   // batched (grouped) products: `batch` independent problems of the same shape; element strides between them
   int batch;
   long long stride_c, stride_aux, stride_bias;
-  // dynamic tile scheduler of the CTA-pair kernel: sched[0] = next tile to hand out, sched[1] = pairs that have finished
-  // (both zero before the launch; the last pair to finish resets them)
+  // dynamic tile scheduler: sched[0] = tiles handed out, sched[1] = CTA pairs (CTAs) that have finished; both zero before the
+  // launch, the last one to finish resets them.  Null for the one-CTA kernel: no hand-out.
   unsigned int* sched;
   // Optional arrival flags of the B operand (CTA-pair kernel, B K-major with contiguous rows): the operand is being
   // written by somebody else (copy engines gathering a sharded weight) while the kernel runs.  Bytes

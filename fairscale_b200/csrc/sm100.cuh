@@ -184,21 +184,12 @@ __device__ __forceinline__ void umma_f16_ss(uint32_t tmem_d, uint64_t adesc, uin
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem]
-__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // Arrive on `bar` once every tcgen05 operation issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// The same three for a whole converged warp: every lane calls, one elected lane issues.  The election is part of the
+// MMA (A from shared memory or, _ts, from TMEM) and commit for a whole converged warp: every lane calls, one elected lane issues.  The election is part of the
 // instruction's predicate, not a branch around a group of them, so the descriptors are computed in uniform control flow and
 // stay in uniform registers; inside a one-lane branch each operand had to be moved there first, about 100 cycles per MMA,
 // which is more than a 128 x 64 x 16 product takes.
@@ -313,12 +304,6 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t local_smem_addr, uint32_
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// The same without making this thread's earlier writes visible to the cluster: for an arrival that only says "I have read
-// it".  The release above waits until every global store of the thread has been acknowledged, over a microsecond after an
-// epilogue.
-__device__ __forceinline__ void mbar_arrive_cluster_read_done(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
 // TMA tile load into THIS CTA's shared memory that reports its bytes to an mbarrier given by its
 // shared::cluster address (the pair leader's barrier). No data is shared between CTAs by the load.
 __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, uint32_t bar_cluster_addr, int x, int y) {
@@ -345,14 +330,6 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
 }
 // One MMA spanning both SMs of the pair: D rows 0..127 live in the leader's TMEM, 128..255 in the peer's;
 // each CTA supplies its half of A (rows) and its half of B (columns) from its own shared memory.
-__device__ __forceinline__ void umma_f16_ss_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // For a whole converged warp, as umma_f16_ss_warp.
 __device__ __forceinline__ void umma_f16_ss_pair_warp(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -363,6 +340,7 @@ __device__ __forceinline__ void umma_f16_ss_pair_warp(uint32_t tmem_d, uint64_t 
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// Arrive (once the pair's MMAs issued so far are complete) on the barrier at a shared::cluster address.
 __device__ __forceinline__ void umma_commit_pair_warp(uint32_t bar_cluster_addr) {
   asm volatile(
       "{\n\t.reg .pred q;\n\t"
@@ -370,11 +348,6 @@ __device__ __forceinline__ void umma_commit_pair_warp(uint32_t bar_cluster_addr)
       "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar_cluster_addr)
       : "memory");
 }
-// Arrive (once the pair's MMAs issued so far are complete) on the barrier at a shared::cluster address.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster_addr) : "memory");
-}
-
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(
