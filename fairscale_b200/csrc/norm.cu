@@ -106,13 +106,14 @@ __device__ __forceinline__ void block_sums(float (&v)[N], float* red, int turn) 
   }
 }
 
-// dx and the dgamma / dbeta partials in one pass over dy and x: dgamma_part / dbeta_part are [gridDim.x, H].
+// dx and the dgamma / dbeta partials in one pass over dy and x: dgamma_part / dbeta_part are [gridDim.x, H].  `res` (may be
+// null): a gradient of x from elsewhere - the residual branch around the norm - that is added before dx is rounded.
 template <bool RMS, int MAX_THREADS>
 __global__ void __launch_bounds__(MAX_THREADS, 512 / MAX_THREADS) norm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                                                const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
-                                                               const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx,
-                                                               float* __restrict__ dgamma_part, float* __restrict__ dbeta_part, long long rows,
-                                                               int H) {
+                                                               const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ res,
+                                                               __nv_bfloat16* __restrict__ dx, float* __restrict__ dgamma_part,
+                                                               float* __restrict__ dbeta_part, long long rows, int H) {
   constexpr int R = 2;
   __shared__ float red[2 * 16 * 2 * R];
   const int col = threadIdx.x * 8;
@@ -120,7 +121,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 512 / MAX_THREADS) norm_bwd_rows_
   float dg[8], db[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) dg[k] = db[k] = 0.f;
-  Vec16<__nv_bfloat16> tg, cx[R], cd[R], nx[R], nd[R];
+  Vec16<__nv_bfloat16> tg, cx[R], cd[R], nx[R], nd[R], tr[R];
   tg.raw = make_uint4(0u, 0u, 0u, 0u);
   if (mine) tg = ld16(gamma + col);
   float cm[R], cr[R], nm[R], nr[R];
@@ -145,6 +146,11 @@ __global__ void __launch_bounds__(MAX_THREADS, 512 / MAX_THREADS) norm_bwd_rows_
   load(cx, cd, cm, cr, row0);
   for (; row0 < rows; row0 += step) {
     load(nx, nd, nm, nr, row0 + step);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      tr[i].raw = make_uint4(0u, 0u, 0u, 0u);
+      if (res != nullptr && mine && row0 + i < rows) tr[i] = ld16(res + (row0 + i) * H + col);
+    }
     float s[2 * R];  // sum of w, sum of w * xhat, per row
 #pragma unroll
     for (int i = 0; i < R; ++i) {
@@ -168,7 +174,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 512 / MAX_THREADS) norm_bwd_rows_
         const float xh = (__bfloat162float(cx[i].v[k]) - cm[i]) * cr[i];
         const float d = __bfloat162float(cd[i].v[k]);
         const float w = d * __bfloat162float(tg.v[k]);
-        o.v[k] = __float2bfloat16_rn(cr[i] * (w - s1 - xh * s2));
+        o.v[k] = __float2bfloat16_rn(fmaf(cr[i], w - s1 - xh * s2, __bfloat162float(tr[i].v[k])));
         dg[k] = fmaf(d, xh, dg[k]);
         if (!RMS) db[k] += d;
       }
@@ -290,7 +296,8 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_fwd_kernel(const __nv_bfloa
 template <bool RMS>
 __global__ void __launch_bounds__(NORM_THREADS) norm_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                                                    const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
-                                                                   const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx, int H) {
+                                                                   const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ res,
+                                                                   __nv_bfloat16* __restrict__ dx, int H) {
   __shared__ float scratch[32];
   const int nvec = H / 8;
   const long long row = blockIdx.x;
@@ -320,9 +327,11 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_bwd_dx_kernel(const __nv_bf
   for (int it = 0; it < NORM_MAX_VEC; ++it) {
     const int j = threadIdx.x + it * NORM_THREADS;
     if (j < nvec) {
-      Vec16<__nv_bfloat16> o;
+      Vec16<__nv_bfloat16> o, tr;
+      tr.raw = make_uint4(0u, 0u, 0u, 0u);
+      if (res != nullptr) tr = ld16(res + row * H + j * 8);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) o.v[k] = __float2bfloat16_rn(rstd * (wdy[it][k] - s1 - xh[it][k] * s2));
+      for (int k = 0; k < 8; ++k) o.v[k] = __float2bfloat16_rn(fmaf(rstd, wdy[it][k] - s1 - xh[it][k] * s2, __bfloat162float(tr.v[k])));
       st16(dx + row * H + j * 8, o);
     }
   }
@@ -444,9 +453,9 @@ FSB_API int fsb_norm_bwd_num_strips(long long rows) {
 }
 
 // partials: fp32 workspace of 2 * n_strips * H floats (n_strips from fsb_norm_bwd_num_strips).
-// dgamma / dbeta are bf16 [H] outputs (dbeta may be null, and is ignored for RMSNorm).
-FSB_API int fsb_norm_bwd(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd, void* dx,
-                         void* dgamma, void* dbeta, float* partials, long long rows, int H, int rms, cudaStream_t stream) {
+// dgamma / dbeta are bf16 [H] outputs (dbeta may be null, and is ignored for RMSNorm).  res: bf16 [rows, H] added to dx, or null.
+FSB_API int fsb_norm_bwd_res(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd, const void* res, void* dx,
+                             void* dgamma, void* dbeta, float* partials, long long rows, int H, int rms, cudaStream_t stream) {
   using namespace fsb;
   if (rows <= 0) return 0;
   if (H % 8 != 0 || H > 8 * NORM_THREADS * NORM_MAX_VEC) return -1;
@@ -457,24 +466,25 @@ FSB_API int fsb_norm_bwd(const void* dy, const void* x, const void* gamma, const
   auto* d = static_cast<const __nv_bfloat16*>(dy);
   auto* xx = static_cast<const __nv_bfloat16*>(x);
   auto* gg = static_cast<const __nv_bfloat16*>(gamma);
+  auto* rr = static_cast<const __nv_bfloat16*>(res);
   auto* o = static_cast<__nv_bfloat16*>(dx);
   const bool want_beta = !rms && dbeta != nullptr;
   if (fused) {
     const int threads = norm_rows_threads(H);
     if (threads <= 256) {
-      if (rms) norm_bwd_rows_kernel<true, 256><<<strips, threads, 0, stream>>>(d, xx, gg, mean, rstd, o, pg, nullptr, rows, H);
-      else     norm_bwd_rows_kernel<false, 256><<<strips, threads, 0, stream>>>(d, xx, gg, mean, rstd, o, pg, want_beta ? pb : nullptr, rows, H);
+      if (rms) norm_bwd_rows_kernel<true, 256><<<strips, threads, 0, stream>>>(d, xx, gg, mean, rstd, rr, o, pg, nullptr, rows, H);
+      else     norm_bwd_rows_kernel<false, 256><<<strips, threads, 0, stream>>>(d, xx, gg, mean, rstd, rr, o, pg, want_beta ? pb : nullptr, rows, H);
     } else {
-      if (rms) norm_bwd_rows_kernel<true, 512><<<strips, threads, 0, stream>>>(d, xx, gg, mean, rstd, o, pg, nullptr, rows, H);
-      else     norm_bwd_rows_kernel<false, 512><<<strips, threads, 0, stream>>>(d, xx, gg, mean, rstd, o, pg, want_beta ? pb : nullptr, rows, H);
+      if (rms) norm_bwd_rows_kernel<true, 512><<<strips, threads, 0, stream>>>(d, xx, gg, mean, rstd, rr, o, pg, nullptr, rows, H);
+      else     norm_bwd_rows_kernel<false, 512><<<strips, threads, 0, stream>>>(d, xx, gg, mean, rstd, rr, o, pg, want_beta ? pb : nullptr, rows, H);
     }
   } else {
     dim3 block(32, 8), grid((H / 8 + 31) / 32, strips);
     if (rms) {
-      norm_bwd_dx_kernel<true><<<static_cast<unsigned>(rows), NORM_THREADS, 0, stream>>>(d, xx, gg, mean, rstd, o, H);
+      norm_bwd_dx_kernel<true><<<static_cast<unsigned>(rows), NORM_THREADS, 0, stream>>>(d, xx, gg, mean, rstd, rr, o, H);
       norm_dparam_partial_kernel<true><<<grid, block, 0, stream>>>(d, xx, mean, rstd, pg, nullptr, rows, H);
     } else {
-      norm_bwd_dx_kernel<false><<<static_cast<unsigned>(rows), NORM_THREADS, 0, stream>>>(d, xx, gg, mean, rstd, o, H);
+      norm_bwd_dx_kernel<false><<<static_cast<unsigned>(rows), NORM_THREADS, 0, stream>>>(d, xx, gg, mean, rstd, rr, o, H);
       norm_dparam_partial_kernel<false><<<grid, block, 0, stream>>>(d, xx, mean, rstd, pg, want_beta ? pb : nullptr, rows, H);
     }
   }
@@ -484,6 +494,11 @@ FSB_API int fsb_norm_bwd(const void* dy, const void* x, const void* gamma, const
   column_reduce_kernel<<<dim3(blocks, want_beta ? 2 : 1), threads, 0, stream>>>(pg, strips, H, static_cast<__nv_bfloat16*>(dgamma),
                                                                                 want_beta ? static_cast<__nv_bfloat16*>(dbeta) : nullptr);
   return static_cast<int>(cudaGetLastError());
+}
+
+FSB_API int fsb_norm_bwd(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd, void* dx,
+                         void* dgamma, void* dbeta, float* partials, long long rows, int H, int rms, cudaStream_t stream) {
+  return fsb_norm_bwd_res(dy, x, gamma, mean, rstd, nullptr, dx, dgamma, dbeta, partials, rows, H, rms, stream);
 }
 
 FSB_API int fsb_colsum_num_strips(long long rows) {

@@ -92,11 +92,11 @@ class Block(nn.Module):
             nn.init.normal_(w, 0.0, cfg.init_std)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        h = self.ln1(x)
+        h, x = self.ln1(x, with_residual=True)
         qkv = linear(h, self.qkv_w, self.qkv_b)
         a = causal_attention(qkv, self.n_heads)
         x = linear(a, self.proj_w, self.proj_b, residual=x)
-        h = self.ln2(x)
+        h, x = self.ln2(x, with_residual=True)
         return mlp(h, self.fc1_w, self.fc1_b, self.fc2_w, self.fc2_b, residual=x)
 
 

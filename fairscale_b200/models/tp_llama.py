@@ -110,12 +110,14 @@ class TPBlock(nn.Module):
 
     def forward(self, x: torch.Tensor, batch: int) -> torch.Tensor:  # x: [T / world, D], rows in (batch, seq) order
         cfg = self.cfg
-        qkv = self.qkv(self.norm1(x))  # [T, 3 * D / world]
+        h, x = self.norm1(x, with_residual=True)
+        qkv = self.qkv(h)  # [T, 3 * D / world]
         S = qkv.shape[0] // batch
         qkv = rope_qkv(qkv.view(batch, S, 3, self.local_heads, cfg.d_model // cfg.n_heads), cfg.rope_theta)
         o = causal_attention(qkv.reshape(batch, S, -1), self.local_heads)
         x = x + self.proj(o.reshape(batch * S, -1))
-        return x + self.down(swiglu(self.gate_up(self.norm2(x))))
+        h, x = self.norm2(x, with_residual=True)
+        return x + self.down(swiglu(self.gate_up(h)))
 
 
 class TPLlama(nn.Module):

@@ -43,8 +43,10 @@ def norm_forward(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Ten
 
 
 def norm_backward(dy: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, mean: Optional[torch.Tensor], rstd: torch.Tensor,
-                  rms: bool, has_bias: bool, slots: Tuple[Any, Any] = (None, None)) -> Tuple[torch.Tensor, torch.Tensor, Optional[torch.Tensor]]:
-    """``slots``: flat-gradient descriptors of weight and bias, whose windows the kernel then writes in place."""
+                  rms: bool, has_bias: bool, slots: Tuple[Any, Any] = (None, None), residual: Optional[torch.Tensor] = None
+                  ) -> Tuple[torch.Tensor, torch.Tensor, Optional[torch.Tensor]]:
+    """``slots``: flat-gradient descriptors of weight and bias, whose windows the kernel then writes in place.  ``residual``:
+    another gradient of ``x``, added to ``dx`` in the same pass."""
     H = x.shape[-1]
     if not _native_ok(x, weight):
         xf, dyf, wf = x.float(), dy.float(), weight.float()
@@ -55,6 +57,8 @@ def norm_backward(dy: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, mean:
         dx = (wdy - c1 - xhat * c2) * rstd
         dw = (dyf * xhat).reshape(-1, H).sum(0)
         db = dyf.reshape(-1, H).sum(0) if has_bias else None
+        if residual is not None:
+            dx = dx + residual.float()
         return dx.to(x.dtype), dw.to(weight.dtype), None if db is None else db.to(weight.dtype)
     x2, dy2 = x.contiguous().view(-1, H), dy.contiguous().view(-1, H)
     rows = x2.shape[0]
@@ -69,7 +73,8 @@ def norm_backward(dy: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, mean:
         db = grad_window(slots[1], weight.dtype, x.device)
         if db is None:
             db = torch.empty(H, dtype=torch.bfloat16, device=x.device)
-    _bind.call("fsb_norm_bwd", dy2.data_ptr(), x2.data_ptr(), weight.data_ptr(), _bind.ptr(mean), rstd.data_ptr(), dx.data_ptr(),
+    res2 = None if residual is None else residual.contiguous().view(-1, H)
+    _bind.call("fsb_norm_bwd_res", dy2.data_ptr(), x2.data_ptr(), weight.data_ptr(), _bind.ptr(mean), rstd.data_ptr(), _bind.ptr(res2), dx.data_ptr(),
                dw.data_ptr(), _bind.ptr(db), partials.data_ptr(), rows, H, int(rms), _bind.stream_ptr(x.device),
                launches=2 if H <= 4096 else 3)
     return dx.view_as(x), dw, db
@@ -90,6 +95,37 @@ class _NormFn(torch.autograd.Function):
         x, weight, mean, rstd = ctx.saved_tensors
         dx, dw, db = norm_backward(dy, x, weight, mean, rstd, ctx.rms, ctx.has_bias, ctx.slots)
         return dx, dw, db, None, None
+
+
+class _NormResidualFn(torch.autograd.Function):
+    """``(norm(x), x)``: a residual block reads its input twice, through the norm and past it.  As one node its backward adds
+    the two gradients inside the norm's kernel; autograd's own sum is one more pass over both."""
+
+    @staticmethod
+    def forward(ctx, x, weight, bias, eps: float, rms: bool):  # type: ignore[override]
+        ctx.set_materialize_grads(False)
+        y, mean, rstd = norm_forward(x, weight, bias, eps, rms)
+        ctx.rms = rms
+        ctx.has_bias = bias is not None
+        ctx.slots = (grad_slot_info(weight), grad_slot_info(bias) if bias is not None else None)
+        ctx.save_for_backward(x, weight, mean, rstd)
+        return y, x.view_as(x)
+
+    @staticmethod
+    def backward(ctx, dy, d_res):  # type: ignore[override]
+        x, weight, mean, rstd = ctx.saved_tensors
+        if dy is None:
+            return d_res, None, None, None, None
+        dx, dw, db = norm_backward(dy, x, weight, mean, rstd, ctx.rms, ctx.has_bias, ctx.slots, d_res)
+        return dx, dw, db, None, None
+
+
+def norm_and_residual(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], eps: float, rms: bool
+                      ) -> Tuple[torch.Tensor, torch.Tensor]:
+    """``norm(x)`` and ``x`` itself for the residual branch that goes past it."""
+    if _bind.no_graph():
+        return norm_forward(x, weight, bias, eps, rms)[0], x
+    return _NormResidualFn.apply(x, weight, bias, eps, rms)
 
 
 def layer_norm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], eps: float = 1e-5) -> torch.Tensor:
@@ -113,7 +149,10 @@ class LayerNorm(nn.Module):
         self.bias = nn.Parameter(torch.zeros(hidden)) if bias else None
         self.eps = eps
 
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
+    def forward(self, x: torch.Tensor, with_residual: bool = False) -> Any:
+        """``with_residual``: also return ``x``, for the branch past the norm (see :func:`norm_and_residual`)."""
+        if with_residual:
+            return norm_and_residual(x, self.weight, self.bias, self.eps, False)
         return layer_norm(x, self.weight, self.bias, self.eps)
 
 
@@ -123,5 +162,7 @@ class RMSNorm(nn.Module):
         self.weight = nn.Parameter(torch.ones(hidden))
         self.eps = eps
 
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
+    def forward(self, x: torch.Tensor, with_residual: bool = False) -> Any:
+        if with_residual:
+            return norm_and_residual(x, self.weight, None, self.eps, True)
         return rms_norm(x, self.weight, self.eps)

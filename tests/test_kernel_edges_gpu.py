@@ -235,6 +235,11 @@ def test_norm_backward_edges(rows, H, rms):
     assert _rel_err(dw, (dy.double() * xh).sum(0)) < 4e-3
     if not rms:
         assert _rel_err(db, dy.double().sum(0)) < 4e-3
+    # the residual branch's gradient goes into dx before it is rounded
+    res = torch.randn(rows, H, device=_dev()).bfloat16()
+    both, dw2, _ = norm.norm_backward(dy, x, w, mean, rstd, rms, b is not None, residual=res)
+    want = rs * (g - (0 if rms else g.mean(-1, keepdim=True)) - xh * (g * xh).mean(-1, keepdim=True)) + res.double()
+    assert _rel_err(both, want) < 4e-3 and torch.equal(dw, dw2)
 
 
 def test_small_gradients_land_in_their_flat_window():
