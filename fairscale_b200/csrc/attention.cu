@@ -25,8 +25,6 @@
 
 #include "sm100.cuh"
 
-#include <cstdlib>
-
 namespace fsb {
 
 constexpr int ATT_THREADS = 576;  // TMA warp + MMA warp + 16 compute warps (four per TMEM lane quadrant)
@@ -602,8 +600,9 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_cons
   attn_teardown(bars, warp, tmem_base, TMEM_COLS, p.status);
 }
 
-// delta[b, h, s] = scale * sum_d dO[b, s, h, d] * O[b, s, h, d].  D / 8 lanes share one (token, head) pair (16 bytes per
-// lane and tensor), so a warp covers 256 / D pairs per step and keeps several independent loads in flight.
+// delta[b, h, s] = scale * sum_d dO[b, s, h, d] * O[b, s, h, d].  A warp takes one token at a time; D / 8 lanes share one head
+// (16 bytes per lane and tensor), 256 / D heads per step.  Bound by memory once the indices cost nothing: one division per
+// token, in 32 bits (two 64-bit divisions per token and head took longer than the loads: 46 us for 16384 tokens of 16 x 128).
 // Also writes the base-2 log-sum-exp right behind it, and fills the rows between S and S_pad (see AttnParams::delta).
 __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                                                          const float* __restrict__ lse, float* __restrict__ delta, float scale, int B,
@@ -611,27 +610,30 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
   const int lanes_per = D >> 3;             // 8 or 16
   const int lane = threadIdx.x & 31;
   const int sub = lane / lanes_per, sl = lane - sub * lanes_per;
-  const int pairs_per_warp = 32 / lanes_per;
-  const long long total = static_cast<long long>(B) * S * H;
+  const int heads_per_step = 32 / lanes_per;
+  const int tokens = B * S;
   const long long total_pad = static_cast<long long>(B) * S_pad * H;
-  const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const long long n_warps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
-  for (long long base = warp * pairs_per_warp; base < total; base += n_warps * pairs_per_warp) {
-    const long long pair = base + sub;  // (token, head) index in [B*S, H] order == element offset / D
-    float acc = 0.f;
-    if (pair < total) {
-      const Vec16<__nv_bfloat16> a = ld16(o + pair * D + sl * 8), c = ld16(d_o + pair * D + sl * 8);
+  const int n_warps = static_cast<int>((gridDim.x * blockDim.x) >> 5);
+  for (int tok = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5); tok < tokens; tok += n_warps) {
+    const int bb = tok / S, ss = tok - bb * S;
+    const long long row0 = static_cast<long long>(bb) * H;
+    const __nv_bfloat16* po = o + static_cast<long long>(tok) * H * D + sl * 8;
+    const __nv_bfloat16* pd = d_o + static_cast<long long>(tok) * H * D + sl * 8;
+#pragma unroll 4
+    for (int h0 = 0; h0 < H; h0 += heads_per_step) {
+      const int h = h0 + sub;
+      float acc = 0.f;
+      if (h < H) {
+        const Vec16<__nv_bfloat16> a = ld16(po + h * D), c = ld16(pd + h * D);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) acc += __bfloat162float(a.v[k]) * __bfloat162float(c.v[k]);
-    }
-    for (int off = lanes_per >> 1; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    if (sl == 0 && pair < total) {
-      const long long tok = pair / H;
-      const int h = static_cast<int>(pair - tok * H);
-      const long long bb = tok / S, ss = tok - bb * S;
-      const long long row = bb * H + h;
-      delta[row * S_pad + ss] = acc * scale;
-      delta[total_pad + row * S_pad + ss] = lse[row * S + ss] * LOG2E;
+        for (int k = 0; k < 8; ++k) acc += __bfloat162float(a.v[k]) * __bfloat162float(c.v[k]);
+      }
+      for (int off = lanes_per >> 1; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+      if (sl == 0 && h < H) {
+        const long long row = row0 + h;
+        delta[row * S_pad + ss] = acc * scale;
+        delta[total_pad + row * S_pad + ss] = lse[row * S + ss] * LOG2E;
+      }
     }
   }
   const int pad = S_pad - S;  // < 128
@@ -680,7 +682,7 @@ FSB_API int fsb_attn_fwd(const void* qkv, void* o, float* lse, int B, int S, int
 FSB_API int fsb_attn_bwd(const void* qkv, const void* o, const void* d_o, const float* lse, float* delta, void* dqkv, int B, int S,
                          int H, int D, float scale, int* status, cudaStream_t stream) {
   using namespace fsb;
-  if (B < 1 || S < 1 || H < 1 || (D != 64 && D != 128)) return -1;
+  if (B < 1 || S < 1 || H < 1 || (D != 64 && D != 128) || static_cast<long long>(B) * S > 0x7fffffffll) return -1;
   const int S_pad = (S + ATT_BM - 1) / ATT_BM * ATT_BM;
   // (columns, positions, batch): a tile that overhangs the sequence reads zeros
   const uint64_t w_qkv = (uint64_t)3 * H * D, w_o = (uint64_t)H * D;
@@ -694,10 +696,9 @@ FSB_API int fsb_attn_bwd(const void* qkv, const void* o, const void* d_o, const 
   p.o = const_cast<__nv_bfloat16*>(static_cast<const __nv_bfloat16*>(o));
   p.lse = const_cast<float*>(lse); p.delta = delta; p.dqkv = static_cast<__nv_bfloat16*>(dqkv); p.status = status;
   {
-    const long long pairs = static_cast<long long>(B) * S * H;
     const int threads = 256;
-    long long blocks = (pairs * (D / 8) + threads - 1) / threads;  // one step per warp at most ...
-    if (blocks > 148 * 16) blocks = 148 * 16;                       // ... but no more CTAs than keep every SM busy
+    long long blocks = (static_cast<long long>(B) * S + threads / 32 - 1) / (threads / 32);  // one token per warp at most ...
+    if (blocks > 148 * 8) blocks = 148 * 8;                                                  // ... but no more CTAs than fill every SM
     attn_delta_kernel<<<static_cast<unsigned>(blocks), threads, 0, stream>>>(static_cast<const __nv_bfloat16*>(o),
                                                                              static_cast<const __nv_bfloat16*>(d_o), lse, delta, scale, B, S, S_pad, H, D);
   }

@@ -24,9 +24,18 @@ template <typename T> __device__ __forceinline__ float ce_log(float x);
 template <> __device__ __forceinline__ float ce_log<__nv_bfloat16>(float x) { return __logf(x); }
 template <> __device__ __forceinline__ float ce_log<float>(float x) { return logf(x); }
 
-template <typename T> __device__ __forceinline__ void online_update(float& m, float& s, float x) {
-  if (x > m) { s = s * ce_exp<T>(m - x) + 1.f; m = x; }
-  else if (x != -INFINITY) { s += ce_exp<T>(x - m); }  // a masked logit adds nothing, also before the first finite one (-inf - -inf)
+// Online softmax over N values at once: one rescaling per vector instead of a branch per value, which made the bf16 forward
+// compute-bound (16384 x 50304: 671 us against 250 us of memory time).  Masked logits (-inf) add nothing, also before the
+// first finite one.
+template <typename T, int N> __device__ __forceinline__ void online_update(float& m, float& s, const float (&x)[N]) {
+  float mx = m;
+#pragma unroll
+  for (int k = 0; k < N; ++k) mx = fmaxf(mx, x[k]);
+  const float ref = mx == -INFINITY ? 0.f : mx;
+  s *= ce_exp<T>(m - ref);
+#pragma unroll
+  for (int k = 0; k < N; ++k) s += ce_exp<T>(x[k] - ref);
+  m = mx;
 }
 
 // stats_out (optional): per row {max, sumexp(at max), target_logit or 0 if target outside [v0, v0+V)}
@@ -42,13 +51,19 @@ __global__ void __launch_bounds__(CE_THREADS) ce_fwd_kernel(const T* __restrict_
   const int nvec = V / VN;
   for (int j = threadIdx.x; j < nvec; j += CE_THREADS) {
     const Vec16<T> t = ld16(lr + j * VN);
+    float x[VN];
 #pragma unroll
-    for (int k = 0; k < VN; ++k) online_update<T>(m, s, to_f32(t.v[k]));
+    for (int k = 0; k < VN; ++k) x[k] = to_f32(t.v[k]);
+    online_update<T, VN>(m, s, x);
   }
-  for (int j = nvec * VN + threadIdx.x; j < V; j += CE_THREADS) online_update<T>(m, s, to_f32(lr[j]));
+  for (int j = nvec * VN + threadIdx.x; j < V; j += CE_THREADS) {
+    const float x[1] = {to_f32(lr[j])};
+    online_update<T, 1>(m, s, x);
+  }
   const float gmax = block_max(m, scratch);
   const float contrib = (m == -INFINITY) ? 0.f : s * ce_exp<T>(m - gmax);
-  const float gsum = block_sum(contrib, scratch);
+  float gsum = block_sum(contrib, scratch);
+  if (gmax == INFINITY) gsum = 1.f;  // inf - inf in the sums: the log-sum-exp of a row with an infinite logit is infinite
   if (threadIdx.x == 0) {
     const long long tgt = targets[row];
     const long long local = tgt - vocab_start;
