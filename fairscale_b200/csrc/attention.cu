@@ -74,10 +74,10 @@ __device__ __forceinline__ constexpr uint32_t kstep_mnmajor(int ks) { return sta
 struct AttnBars {
   uint64_t stat_full;     // stationary tiles landed
   uint64_t stat_empty;    // the item's last products that read the stationary tiles have completed
-  uint64_t str_full[4];   // streamed stage landed
-  uint64_t str_empty[4];  // streamed stage free again
-  uint64_t s_full[2];     // scores and dP of a step of buffer b are in TMEM
-  uint64_t p_full[2];     // the 8 warps of buffer b have written dS (dQ kernel) / P^T and dS^T (dK/dV kernel) of its step
+  uint64_t str_full[6];   // streamed stage landed
+  uint64_t str_empty[6];  // streamed stage free again
+  uint64_t s_full[3];     // scores and dP of a step are in buffer b
+  uint64_t p_full[3];     // the 8 warps of the step have written dS (dQ kernel) / P^T and dS^T (dK/dV kernel) over them
   uint64_t acc_done;      // the item's accumulating products have completed
   uint64_t acc_free;      // the 16 compute warps have read the item's output accumulators
   uint32_t tmem_slot;
@@ -89,11 +89,11 @@ static_assert(sizeof(AttnBars) <= 256, "the barrier block of the shared-memory l
 __device__ __forceinline__ void attn_init_bars(AttnBars* b) {
   mbar_init(&b->stat_full, 1);
   mbar_init(&b->stat_empty, 1);
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < 6; ++i) {
     mbar_init(&b->str_full[i], 1);
     mbar_init(&b->str_empty[i], 1);
   }
-  for (int i = 0; i < 2; ++i) {
+  for (int i = 0; i < 3; ++i) {
     mbar_init(&b->s_full[i], 1);
     mbar_init(&b->p_full[i], 8);
   }
@@ -139,25 +139,28 @@ __device__ __forceinline__ void dq_cols16(const uint32_t (&rs)[16], const uint32
 // =================================================================================================
 // Backward, dQ: one CTA per 128 query rows; streams K and V tiles and consumes them in steps of 64 keys.
 //
-// Two sets of eight warps take alternate steps (set b the steps u with u & 1 == b, accumulator buffer b; two threads per
-// query row with 32 keys each): while one set is in its exponentials the other one waits for TMEM loads, stores or the
+// Two sets of eight warps take alternate steps (set b the steps u with u & 1 == b; two threads per query row with 32 keys
+// each): while one set is in its exponentials the other one waits for TMEM loads, stores or the
 // tensor pipe.  What bounds the kernel is the length of that chain, not a pipe (exponentials 34 %, tensor pipe 25 % busy on
 // the busiest SM with one thread per row and set), hence the short slices per thread and the many warps.
-// Forward and backward of B2 S8192 H16 D64 together: 2420 us with eight warps that all worked on the same step and passed dS
-// through shared memory, 1917 us now (backward alone 1870 -> 1447; B8 S2048 H16 D128 750 -> 690).
+// Backward of B2 S8192 H16 D64: 1870 us with eight warps that all worked on the same step and passed dS through shared
+// memory, 1447 us with the two sets (B8 S2048 H16 D128 750 -> 690 us).
 // dS overwrites scores that the same thread has read (32 keys become the first 16 of their 32 columns) and feeds dS K as
 // the TMEM A operand, so it does not pass through shared memory.  The tensor pipe executes in issue order,
-//   S,dP(0)  S,dP(1) | dQ(0)  S,dP(2)  dQ(1)  S,dP(3) ...
-// so S(u+2), issued behind dQ(u), cannot overwrite dS(u) early and the buffers need no "empty" barriers.
+//   S,dP(0) .. S,dP(n-1) | dQ(0)  S,dP(n)  dQ(1)  S,dP(n+1) ...        with n score buffers, step u in buffer u mod n,
+// so S(u+n), issued behind dQ(u), cannot overwrite dS(u) early and the buffers need no "empty" barriers.  Head size 64
+// leaves TMEM for three buffers: a set that has finished step u then finds the scores of step u + 2 ready, where with two
+// it waits for dQ(u) and those products (backward of B2 S8192 H16 D64 1447 -> 1315 us).
 // =================================================================================================
 template <int D>
 struct DqSmem {
   static constexpr int TILE = ATT_BM * D * 2;
   static constexpr int Q_OFF = 0;
   static constexpr int DO_OFF = TILE;
-  static constexpr int K_OFF = 2 * TILE;   // 2 stages
-  static constexpr int V_OFF = 4 * TILE;   // 2 stages
-  static constexpr int BAR_OFF = 6 * TILE;
+  static constexpr int STAGES = D == 64 ? 4 : 2;  // K / V tiles in flight
+  static constexpr int K_OFF = 2 * TILE;
+  static constexpr int V_OFF = (2 + STAGES) * TILE;
+  static constexpr int BAR_OFF = (2 + 2 * STAGES) * TILE;
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
 };
 
@@ -179,7 +182,9 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_cons
   const int HB = p.H * p.B;
   const int n_items = n_qt * HB;
   const int HD = p.H * D;
-  constexpr uint32_t TMEM_COLS = 512;  // buffer b: S [128 b, +64) dP [128 b + 64, +64); dQ [256, 256+D)
+  constexpr uint32_t TMEM_COLS = 512;  // buffer b: S [128 b, +64) dP [128 b + 64, +64); then dQ
+  constexpr int NBUF = D == 64 ? 3 : 2;
+  constexpr uint32_t DQ_COL = NBUF * 128;
 
   if (threadIdx.x == 0) {
     attn_init_bars(bars);
@@ -213,8 +218,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_cons
           tma_load_3d(smem + L::DO_OFF + c * SLAB, &tm_do, &bars->stat_full, h * D + c * 64, row0, b);
         }
         for (int j = 0; j < n_kv; ++j, ++jt) {
-          const int st = jt & 1;
-          if (!mbar_wait(&bars->str_empty[st], ((jt >> 1) & 1u) ^ 1u, abort_flag, 34)) { ok = false; break; }
+          const int st = jt % L::STAGES;
+          if (!mbar_wait(&bars->str_empty[st], ((jt / L::STAGES) & 1u) ^ 1u, abort_flag, 34)) { ok = false; break; }
           const int krow = j * ATT_BM;
           mbar_expect_tx(&bars->str_full[st], 2 * L::TILE);
 #pragma unroll
@@ -234,11 +239,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_cons
     const uint64_t dkt0 = desc_mnmajor(smem_u32(smem + L::K_OFF), SLAB);
     uint32_t jt0 = 0, ut0 = 0, it = 0;  // key tiles / steps of earlier items, items so far
     bool ok = true;
-    // step u = key tile u / 2, keys [64 (u & 1), +64) of it; S and dP of step u go to accumulator buffer u & 1
+    // step u = key tile u / 2, keys [64 (u & 1), +64) of it; buffers go round over the steps of all items
     auto issue_sp = [&](int u, int n_steps) -> bool {
       const uint32_t jt = jt0 + (u >> 1);
-      const int hh = u & 1, st = jt & 1, buf = u & 1;
-      if (hh == 0 && !mbar_wait_warp(&bars->str_full[st], (jt >> 1) & 1u, abort_flag, 35)) return false;
+      const int hh = u & 1, st = jt % L::STAGES, buf = (ut0 + u) % NBUF;
+      if (hh == 0 && !mbar_wait_warp(&bars->str_full[st], (jt / L::STAGES) & 1u, abort_flag, 35)) return false;
       tc_fence_after_sync();
       const uint32_t off = st * L::TILE + hh * 8192u;  // rows 64 hh .. of every slab
       const uint64_t dk = desc_offset(dk0, off), dv = desc_offset(dv0, off);
@@ -256,21 +261,21 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_cons
       const int qt = n_qt - 1 - item / HB;
       const int n_steps = 2 * (qt + 1);
       if (!mbar_wait_warp(&bars->stat_full, it & 1u, abort_flag, 37)) { ok = false; break; }
-      ok = issue_sp(0, n_steps) && issue_sp(1, n_steps);
+      for (int u = 0; u < NBUF && u < n_steps && ok; ++u) ok = issue_sp(u, n_steps);
       for (int u = 0; u < n_steps && ok; ++u) {
         const uint32_t jt = jt0 + (u >> 1), ut = ut0 + u;
-        const int hh = u & 1, st = jt & 1, buf = u & 1;
+        const int hh = u & 1, st = jt % L::STAGES, buf = ut % NBUF;
         // the dQ accumulator still belongs to the previous item until its threads have read it
         if (u == 0 && !mbar_wait_warp(&bars->acc_free, (it & 1u) ^ 1u, abort_flag, 38)) { ok = false; break; }
-        if (!mbar_wait_warp(&bars->p_full[buf], (ut >> 1) & 1u, abort_flag, 39)) { ok = false; break; }
+        if (!mbar_wait_warp(&bars->p_full[buf], (ut / NBUF) & 1u, abort_flag, 39)) { ok = false; break; }
         tc_fence_after_sync();
         const uint64_t dkt = desc_offset(dkt0, st * L::TILE + hh * 4 * 2048u);
 #pragma unroll
         for (int ks = 0; ks < 64 / 16; ++ks)
-          umma_f16_ts_warp(tmem_base + 256, tmem_base + buf * 128 + (ks >> 1) * 32 + (ks & 1) * 8, desc_offset(dkt, kstep_mnmajor(ks)), idesc_q, (u | ks) != 0);
+          umma_f16_ts_warp(tmem_base + DQ_COL, tmem_base + buf * 128 + (ks >> 1) * 32 + (ks & 1) * 8, desc_offset(dkt, kstep_mnmajor(ks)), idesc_q, (u | ks) != 0);
         if (hh == 1) umma_commit_warp(&bars->str_empty[st]);
         if (u == n_steps - 1) umma_commit_warp(&bars->acc_done);
-        if (u + 2 < n_steps && !issue_sp(u + 2, n_steps)) { ok = false; break; }
+        if (u + NBUF < n_steps && !issue_sp(u + NBUF, n_steps)) { ok = false; break; }
       }
       jt0 += static_cast<uint32_t>(n_steps >> 1);
       ut0 += static_cast<uint32_t>(n_steps);
@@ -278,13 +283,13 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_cons
   } else {
     const int quad = warp & 3;
     const int grp = (warp - 2) >> 2;          // which D/4 output columns
-    const int buf = grp >> 1, half = grp & 1;  // which of two consecutive steps, which 32 of its 64 keys
+    const int set = grp >> 1, half = grp & 1;  // which of two consecutive steps, which 32 of its 64 keys
     const int row = quad * 32 + lane;
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
-    const uint32_t ts = tmem_base + buf * 128 + half * 32 + lane_off;  // this thread's scores; its dS overwrites the first 16 columns
-    const int col0 = buf * 64 + half * 32;                 // first key of this thread inside the 128-key tile
+    const uint32_t ts0 = tmem_base + half * 32 + lane_off;  // this thread's scores in buffer 0; its dS overwrites the first 16 columns
+    const int col0 = set * 64 + half * 32;                  // first key of this thread inside the 128-key tile
     const float sl2 = p.scale * LOG2E;
-    uint32_t cs = 0, it = 0;  // this set's steps / items so far
+    uint32_t ut = set, it = 0;  // this set's next step over all items (every item has an even number), items so far
     bool ok = true;
     for (int item; ok && (item = snake_item(static_cast<int>(it))) < n_items; ++it) {
       const int qt = n_qt - 1 - item / HB;
@@ -294,8 +299,9 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_cons
       const size_t stat_idx = (static_cast<size_t>(b) * p.H + h) * p.S_pad + pos;
       const float lse2 = p.delta[static_cast<size_t>(p.B) * p.H * p.S_pad + stat_idx];  // base-2 lse, written by the delta kernel
       const float delta_s = p.delta[stat_idx];                                       // scale * rowsum(dO * O)
-      for (int j = 0; j <= qt; ++j, ++cs) {
-        if (!mbar_wait(&bars->s_full[buf], cs & 1u, abort_flag, 40)) { ok = false; break; }
+      for (int j = 0; j <= qt; ++j, ut += 2) {
+        const uint32_t buf = ut % NBUF, ts = ts0 + buf * 128;
+        if (!mbar_wait(&bars->s_full[buf], (ut / NBUF) & 1u, abort_flag, 40)) { ok = false; break; }
         tc_fence_after_sync();
         const bool diag = (j == qt);
         uint32_t rs0[16], rp0[16], rs1[16], rp1[16], pk[8];
@@ -322,7 +328,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_cons
 #pragma unroll 1
       for (int c = 0; c < D / 4; c += 16) {
         uint32_t r[16];
-        tmem_ld_32x16(tmem_base + 256 + lane_off + grp * (D / 4) + c, r);
+        tmem_ld_32x16(tmem_base + DQ_COL + lane_off + grp * (D / 4) + c, r);
         tmem_ld_wait();
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -376,7 +382,8 @@ __device__ __forceinline__ void dkv_cols16(const uint32_t (&rs)[16], const uint3
 // Backward, dK / dV: one CTA per 128 key rows; streams 64-row Q / dO sub-tiles with their statistics (copied to shared
 // memory with the tiles: read from global memory where they are used, each first touch cost an L2 round trip inside the
 // softmax chain).  The same scheme as the dQ kernel: two sets of eight warps take alternate sub-tiles, P^T and dS^T overwrite
-// their own scores in TMEM and are the A operands of the accumulating products; the tensor pipe runs  S,dP(0)  S,dP(1) | dV,dK(0)  S,dP(2)  dV,dK(1)  S,dP(3) ...
+// their own scores in TMEM and are the A operands of the accumulating products, and head size 64 has three score buffers;
+// the tensor pipe runs  S,dP(0) .. S,dP(n-1) | dV,dK(0)  S,dP(n)  dV,dK(1)  S,dP(n+1) ...
 // =================================================================================================
 constexpr int KV_QSUB = 64;
 
@@ -386,7 +393,7 @@ struct DkvSmem {
   static constexpr int QTILE = KV_QSUB * D * 2;   // Q or dO sub-tile
   static constexpr int K_OFF = 0;
   static constexpr int V_OFF = TILE;
-  static constexpr int STAGES = 4;                             // Q / dO sub-tiles in flight
+  static constexpr int STAGES = D == 64 ? 6 : 4;               // Q / dO sub-tiles in flight
   static constexpr int Q_OFF = 2 * TILE;
   static constexpr int DO_OFF = 2 * TILE + STAGES * QTILE;
   static constexpr int STAT_OFF = 2 * TILE + 2 * STAGES * QTILE;  // per stage: 64 base-2 lse, then 64 scaled deltas
@@ -410,15 +417,18 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_cons
 
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // warp-uniform
   // Persistent: one CTA per SM walks the work items (one 128-row key tile of one head); small key tiles see the most
-  // query sub-tiles and come first.  Every item has an even number of sub-tiles, so the accumulator buffer of a
-  // sub-tile is its running index & 1 as well.
+  // query sub-tiles and come first.  Every item has an even number of sub-tiles, so a set's sub-tiles are the even or the
+  // odd ones of the running index as well.
   const int n_kt = p.S_pad / ATT_BM;
   const int HB = p.H * p.B;
   const int n_items = n_kt * HB;
   const int HD = p.H * D;
-  // S^T / dP^T are double-buffered so the products of sub-tile t+1 run while the threads work on sub-tile t:
-  // buffer 0: S^T [0,64) dP^T [64,128); buffer 1: S^T [384,448) dP^T [448,512); dV [128,128+D); dK [256,256+D)
+  // Score buffers: S^T 64 columns, dP^T the next 64.  Head size 64: three at 0, 128, 256, then dV and dK; head size 128:
+  // two at 0 and 384, dV and dK between them.
   constexpr uint32_t TMEM_COLS = 512;
+  constexpr int NBUF = D == 64 ? 3 : 2;
+  constexpr uint32_t BUF_STEP = D == 64 ? 128 : 384;
+  constexpr uint32_t DV_COL = D == 64 ? 384 : 128, DK_COL = D == 64 ? 448 : 256;
 
   if (threadIdx.x == 0) {
     attn_init_bars(bars);
@@ -478,14 +488,14 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_cons
     const uint64_t dqt0 = desc_mnmajor(smem_u32(smem + L::Q_OFF), QSLAB), ddot0 = desc_mnmajor(smem_u32(smem + L::DO_OFF), QSLAB);
     uint32_t tt0 = 0, it = 0;
     bool ok = true;
-    // S^T(t) = K Q_t^T and dP^T(t) = V dO_t^T into accumulator buffer t & 1
+    // S^T(t) = K Q_t^T and dP^T(t) = V dO_t^T; buffers go round over the sub-tiles of all items
     auto issue_sp = [&](int t, int n_sub) -> bool {
       const uint32_t tt = tt0 + t;
-      const int st = tt % L::STAGES, buf = t & 1;
+      const int st = tt % L::STAGES, buf = tt % NBUF;
       if (!mbar_wait_warp(&bars->str_full[st], (tt / L::STAGES) & 1u, abort_flag, 67)) return false;
       tc_fence_after_sync();
       const uint64_t dq = desc_offset(dq0, st * L::QTILE), ddo = desc_offset(ddo0, st * L::QTILE);
-      const uint32_t t_s = tmem_base + (buf ? 384u : 0u);
+      const uint32_t t_s = tmem_base + buf * BUF_STEP;
 #pragma unroll
       for (int ks = 0; ks < D / 16; ++ks)
         umma_f16_ss_warp(t_s, desc_offset(dk, kstep_kmajor(ks, SLAB)), desc_offset(dq, kstep_kmajor(ks, QSLAB)), idesc_s, ks != 0);
@@ -500,39 +510,39 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_cons
       const int kt = item / HB;
       const int n_sub = p.S_pad / KV_QSUB - kt * (ATT_BM / KV_QSUB);
       if (!mbar_wait_warp(&bars->stat_full, it & 1u, abort_flag, 69)) { ok = false; break; }
-      ok = issue_sp(0, n_sub) && issue_sp(1, n_sub);
+      for (int t = 0; t < NBUF && t < n_sub && ok; ++t) ok = issue_sp(t, n_sub);
       for (int t = 0; t < n_sub && ok; ++t) {
         const uint32_t tt = tt0 + t;
         const int st = tt % L::STAGES;
         const uint64_t dqt = desc_offset(dqt0, st * L::QTILE), ddot = desc_offset(ddot0, st * L::QTILE);
         // dK / dV still belong to the previous item until its threads have read them
         if (t == 0 && !mbar_wait_warp(&bars->acc_free, (it & 1u) ^ 1u, abort_flag, 70)) { ok = false; break; }
-        const int buf = t & 1;
-        if (!mbar_wait_warp(&bars->p_full[buf], (tt >> 1) & 1u, abort_flag, 71)) { ok = false; break; }
+        const int buf = tt % NBUF;
+        if (!mbar_wait_warp(&bars->p_full[buf], (tt / NBUF) & 1u, abort_flag, 71)) { ok = false; break; }
         tc_fence_after_sync();
-        const uint32_t t_s = tmem_base + (buf ? 384u : 0u);
+        const uint32_t t_s = tmem_base + buf * BUF_STEP;
 #pragma unroll
         for (int ks = 0; ks < KV_QSUB / 16; ++ks)
-          umma_f16_ts_warp(tmem_base + 128, t_s + (ks >> 1) * 32 + (ks & 1) * 8, desc_offset(ddot, kstep_mnmajor(ks)), idesc_a, (t | ks) != 0);
+          umma_f16_ts_warp(tmem_base + DV_COL, t_s + (ks >> 1) * 32 + (ks & 1) * 8, desc_offset(ddot, kstep_mnmajor(ks)), idesc_a, (t | ks) != 0);
 #pragma unroll
         for (int ks = 0; ks < KV_QSUB / 16; ++ks)
-          umma_f16_ts_warp(tmem_base + 256, t_s + 64 + (ks >> 1) * 32 + (ks & 1) * 8, desc_offset(dqt, kstep_mnmajor(ks)), idesc_a, (t | ks) != 0);
+          umma_f16_ts_warp(tmem_base + DK_COL, t_s + 64 + (ks >> 1) * 32 + (ks & 1) * 8, desc_offset(dqt, kstep_mnmajor(ks)), idesc_a, (t | ks) != 0);
         umma_commit_warp(&bars->str_empty[st]);
         if (t == n_sub - 1) umma_commit_warp(&bars->acc_done);
-        if (t + 2 < n_sub && !issue_sp(t + 2, n_sub)) { ok = false; break; }
+        if (t + NBUF < n_sub && !issue_sp(t + NBUF, n_sub)) { ok = false; break; }
       }
       tt0 += static_cast<uint32_t>(n_sub);
     }
   } else {
     const int quad = warp & 3;
     const int grp = (warp - 2) >> 2;
-    const int buf = grp >> 1, half = grp & 1;  // which of two consecutive sub-tiles, which 32 of its 64 queries (and: dK or dV, which D/2 columns)
+    const int set = grp >> 1, half = grp & 1;  // which of two consecutive sub-tiles, which 32 of its 64 queries (and: dK or dV, which D/2 columns)
     const int row = quad * 32 + lane;          // key row inside the tile
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
-    // this thread's S^T columns, its dP^T at +64; P^T / dS^T overwrite the first 16 columns of each
-    const uint32_t ts = tmem_base + (buf ? 384u : 0u) + half * 32 + lane_off;
+    // this thread's S^T columns in buffer 0, its dP^T at +64; P^T / dS^T overwrite the first 16 columns of each
+    const uint32_t ts0 = tmem_base + half * 32 + lane_off;
     const float sl2 = p.scale * LOG2E;
-    uint32_t tt0 = 0, cs = 0, it = 0;  // sub-tiles, this set's sub-tiles, items so far
+    uint32_t tt0 = 0, it = 0;  // sub-tiles / items so far
     bool ok = true;
     for (int item; ok && (item = snake_item(static_cast<int>(it))) < n_items; ++it) {
       const int kt = item / HB;
@@ -541,14 +551,15 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_cons
       const int first_sub = kt * (ATT_BM / KV_QSUB);
       const int n_sub = p.S_pad / KV_QSUB - first_sub;
       const int key = kt * ATT_BM + row;  // this thread's key (sequence index)
-      for (int t = buf; t < n_sub; t += 2, ++cs) {
-        const int st = static_cast<int>((tt0 + t) % L::STAGES);
+      for (int t = set; t < n_sub; t += 2) {
+        const uint32_t tt = tt0 + t, buf = tt % NBUF, ts = ts0 + buf * BUF_STEP;
+        const int st = static_cast<int>(tt % L::STAGES);
         const int qa0 = (first_sub + t) * KV_QSUB + half * 32;  // first query (sequence index) of this thread
         const bool edge = t < ATT_BM / KV_QSUB || qa0 + 32 > p.S;  // may overlap the diagonal block or the sequence's end
-        if (!mbar_wait(&bars->s_full[buf], cs & 1u, abort_flag, 72)) { ok = false; break; }
+        if (!mbar_wait(&bars->s_full[buf], (tt / NBUF) & 1u, abort_flag, 72)) { ok = false; break; }
         tc_fence_after_sync();
         // the statistics landed with the tile that S^T was made of: this wait does not block, it orders the reads behind the copy
-        if (!mbar_wait(&bars->str_full[st], ((tt0 + t) / L::STAGES) & 1u, abort_flag, 73)) { ok = false; break; }
+        if (!mbar_wait(&bars->str_full[st], (tt / L::STAGES) & 1u, abort_flag, 73)) { ok = false; break; }
         const float* lse2 = reinterpret_cast<const float*>(smem + L::STAT_OFF + st * L::STAT_BYTES) + half * 32;
         const float* delta_s = lse2 + KV_QSUB;
         uint32_t rs0[16], rp0[16], rs1[16], rp1[16], pp[8], pd[8];
@@ -573,9 +584,9 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_cons
       if (!ok) break;
       if (!mbar_wait(&bars->acc_done, it & 1u, abort_flag, 74)) { ok = false; break; }
       tc_fence_after_sync();
-      // buf 0: dK (TMEM cols 256..), buf 1: dV (cols 128..)
-      const uint32_t tcol = tmem_base + (buf == 0 ? 256u : 128u) + static_cast<uint32_t>(half * (D / 2)) + lane_off;
-      __nv_bfloat16* drow = p.dqkv + (static_cast<size_t>(b) * p.S + key) * (3 * HD) + (buf == 0 ? HD : 2 * HD) + h * D + half * (D / 2);
+      // set 0: dK, set 1: dV
+      const uint32_t tcol = tmem_base + (set == 0 ? DK_COL : DV_COL) + static_cast<uint32_t>(half * (D / 2)) + lane_off;
+      __nv_bfloat16* drow = p.dqkv + (static_cast<size_t>(b) * p.S + key) * (3 * HD) + (set == 0 ? HD : 2 * HD) + h * D + half * (D / 2);
 #pragma unroll 1
       for (int c = 0; c < D / 2; c += 16) {
         uint32_t r[16];
