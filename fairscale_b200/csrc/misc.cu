@@ -26,7 +26,57 @@ __host__ inline int misc_grid(long long work_items) {
 }
 
 // ------------------------------------------------------------------------------------------------ RoPE
-// One thread handles 8 consecutive elements (4 pairs) of one (b, s, which, h) row of D elements.
+// Rotates 4 pairs by their angles.
+__device__ __forceinline__ void rope_rotate(Vec16<__nv_bfloat16>& x, const float (&sn)[4], const float (&cs)[4]) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float x1 = __bfloat162float(x.v[2 * k]), x2 = __bfloat162float(x.v[2 * k + 1]);
+    x.v[2 * k] = __float2bfloat16_rn(x1 * cs[k] - x2 * sn[k]);
+    x.v[2 * k + 1] = __float2bfloat16_rn(x1 * sn[k] + x2 * cs[k]);
+  }
+}
+// Sine (times `sign`) and cosine of position s for the pairs 4 j .. 4 j + 3 of a row of D elements.
+__device__ __forceinline__ void rope_angles(int s, int j, float log2_theta, float inv_d, float sign, float (&sn)[4], float (&cs)[4]) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int pair = j * 4 + k;  // frequency index i of the pair (2i, 2i+1)
+    const float inv_freq = exp2f(-log2_theta * (2.f * static_cast<float>(pair)) * inv_d);
+    sincosf(static_cast<float>(s) * inv_freq, &sn[k], &cs[k]);
+    sn[k] *= sign;
+  }
+}
+
+// Head sizes up to 2048.  A CTA takes one token at a time and a thread the same 8 elements (4 pairs) of every row of the
+// token, so a token's angles are computed once instead of once per head of q and k; what is left is bound by memory, with
+// four rows in flight per thread.  (4096 tokens of 3 x 32 x 128: 64 us with the angles per row, 37 us now, 30 us of memory time.)
+__global__ void __launch_bounds__(MISC_THREADS) rope_token_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, long long tokens,
+                                                                  int S, int H, int D, float log2_theta, float sign, int pos_offset) {
+  const int vec_per_row = D / 8;  // divides blockDim.x
+  const int j = static_cast<int>(threadIdx.x) % vec_per_row, r0 = static_cast<int>(threadIdx.x) / vec_per_row;
+  const int rows_per_step = static_cast<int>(blockDim.x) / vec_per_row;
+  const float inv_d = 1.f / static_cast<float>(D);
+  for (long long t = blockIdx.x; t < tokens; t += gridDim.x) {
+    float sn[4], cs[4];
+    rope_angles(static_cast<int>(t % S) + pos_offset, j, log2_theta, inv_d, sign, sn, cs);
+    const long long base = t * 3 * H * D + j * 8;
+    for (int r = r0; r < 3 * H; r += 4 * rows_per_step) {
+      Vec16<__nv_bfloat16> x[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int row = r + u * rows_per_step;
+        if (row < 3 * H && (row < 2 * H || in != out)) x[u] = ld16(in + base + static_cast<long long>(row) * D);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int row = r + u * rows_per_step;
+        if (row < 2 * H) rope_rotate(x[u], sn, cs);  // v: untouched
+        if (row < 3 * H && (row < 2 * H || in != out)) st16(out + base + static_cast<long long>(row) * D, x[u]);
+      }
+    }
+  }
+}
+
+// Any head size.  One thread handles 8 consecutive elements (4 pairs) of one (b, s, which, h) row of D elements.
 __global__ void rope_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, long long B, int S, int H, int D,
                             float log2_theta, float sign, int pos_offset) {
   const int vec_per_row = D / 8;
@@ -42,18 +92,10 @@ __global__ void rope_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16*
       continue;
     }
     const int s = static_cast<int>((row / (3ll * H)) % S) + pos_offset;
+    float sn[4], cs[4];
+    rope_angles(s, j, log2_theta, inv_d, sign, sn, cs);
     Vec16<__nv_bfloat16> x = ld16(in + row * D + j * 8);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int pair = j * 4 + k;  // frequency index i of the pair (2i, 2i+1)
-      const float inv_freq = exp2f(-log2_theta * (2.f * static_cast<float>(pair)) * inv_d);
-      float sn, cs;
-      sincosf(static_cast<float>(s) * inv_freq, &sn, &cs);
-      sn *= sign;
-      const float x1 = __bfloat162float(x.v[2 * k]), x2 = __bfloat162float(x.v[2 * k + 1]);
-      x.v[2 * k] = __float2bfloat16_rn(x1 * cs - x2 * sn);
-      x.v[2 * k + 1] = __float2bfloat16_rn(x1 * sn + x2 * cs);
-    }
+    rope_rotate(x, sn, cs);
     st16(out + row * D + j * 8, x);
   }
 }
@@ -122,6 +164,14 @@ FSB_API int fsb_rope(const void* qkv_in, void* qkv_out, long long B, int S, int 
   using namespace fsb;
   if (B <= 0 || S <= 0 || H <= 0) return 0;
   if (D <= 0 || (D % 8) || theta <= 0.f) return -1;
+  if (D <= 8 * MISC_THREADS) {
+    const long long tokens = B * S, cap = 148ll * 8;
+    const int threads = MISC_THREADS / (D / 8) * (D / 8);
+    rope_token_kernel<<<static_cast<unsigned>(tokens < cap ? tokens : cap), threads, 0, stream>>>(
+        reinterpret_cast<const __nv_bfloat16*>(qkv_in), reinterpret_cast<__nv_bfloat16*>(qkv_out), tokens, S, H, D, log2f(theta),
+        backward ? -1.f : 1.f, pos_offset);
+    return static_cast<int>(cudaGetLastError());
+  }
   const long long total = B * S * 3 * H * (D / 8);
   rope_kernel<<<misc_grid(total), MISC_THREADS, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(qkv_in),
                                                               reinterpret_cast<__nv_bfloat16*>(qkv_out), B, S, H, D, log2f(theta),

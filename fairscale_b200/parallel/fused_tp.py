@@ -297,7 +297,10 @@ def _all_gather_rows(x: torch.Tensor, group: Any) -> torch.Tensor:
 
 
 def _reduce_scatter_rows(x: torch.Tensor, group: Any) -> torch.Tensor:
+    """``x`` is a product that nothing else reads: with one rank it is the result."""
     world = comm.group_size(group)
+    if world == 1:
+        return x.contiguous()
     out = torch.empty((x.shape[0] // world,) + tuple(x.shape[1:]), dtype=x.dtype, device=x.device)
     if world > 1 and dist.get_backend(group) == "gloo":  # gloo has no reduce-scatter
         full = x.contiguous().clone()
@@ -378,7 +381,8 @@ class _LinearReduceScatter(torch.autograd.Function):
         if ag_gemm_supported(ws, dout.shape[0], dout.shape[1], w.shape[1]):
             dx, gathered = ag_gemm(ws, dout, w, None, w_is_kn=True)  # dX = all_gather(dOut) @ W
         else:
-            gathered = _all_gather_rows(dout, ctx.group)
+            # with one rank the rows are all here (the forward's gather copies even then: its input stays the caller's to change)
+            gathered = dout if comm.group_size(ctx.group) == 1 else _all_gather_rows(dout, ctx.group)
             dx = gathered @ w if ctx.needs_input_grad[0] else None
         if ctx.needs_input_grad[1]:
             dw = gemm_ops.linear_wgrad(gathered, x).to(w.dtype)

@@ -271,6 +271,21 @@ def test_small_gradients_land_in_their_flat_window():
     assert got[2].data_ptr() == base + 2 * (d * d + d) and got[3].data_ptr() == base + 2 * (d * d + 2 * d)
 
 
+# head sizes whose rows do and do not divide 256 threads, fewer rows than a step of four takes, more tokens than the grid
+@pytest.mark.parametrize("B,S,H,D", [(1, 1, 1, 8), (2, 5, 3, 80), (1, 7, 1, 2048), (1, 3, 1, 2056), (3, 700, 2, 64), (2, 33, 32, 128)])
+def test_rope_edges(B, S, H, D):
+    from fairscale_b200.ops.rope import _rope_apply, rope_reference
+
+    torch.manual_seed(D)
+    qkv = torch.randn(B, S, 3, H, D, device=_dev()).bfloat16()
+    for backward in (False, True):
+        got = _rope_apply(qkv, 10000.0, backward, 3)
+        want = rope_reference(qkv.double(), 10000.0, backward, 3)
+        assert _rel_err(got, want) < 4e-3  # one rounding to bf16, angles in fp32
+        assert torch.equal(got[:, :, 2], qkv[:, :, 2])
+    _status_ok()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rows,V", [(1, 8), (3, 512), (5, 32000), (7, 2056)])
 def test_vocab_cross_entropy_pieces(rows, V, dtype):
