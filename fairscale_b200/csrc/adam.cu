@@ -166,47 +166,99 @@ __global__ void __launch_bounds__(ADAM_THREADS) multi_tensor_adam_kernel(AdamArg
   if (overflow && a.found_inf != nullptr) *a.found_inf = 1;
 }
 
-// Sum of squares of many tensors (one launch) into *out (fp32, must be zeroed by the caller).
+// Sum of squares of many tensors (one launch) into *out (fp32, must be zeroed by the caller), and x[i] *= *scale_dev (clip
+// coefficient computed on the device).  Bound by memory: 16-byte accesses, four in flight per thread, where a tensor starts
+// on a 16-byte boundary; element by element where it does not.  (220 M bf16 gradients: 110 -> 84 us and 166 -> 131 us
+// against element by element for all; 66 us and 132 us of memory time.)
 struct NormTensor { const void* x; long long numel; long long chunk_start; long long pad_; };
 
-__global__ void __launch_bounds__(ADAM_THREADS) multi_tensor_sumsq_kernel(const NormTensor* table, int n, int dtype, float* out) {
-  __shared__ float scratch[32];
+__device__ __forceinline__ NormTensor norm_tensor_of_chunk(const NormTensor* table, int n, long long chunk, long long& begin, long long& end) {
   int lo = 0, hi = n - 1;
-  const long long chunk = blockIdx.x;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (table[mid].chunk_start <= chunk) lo = mid; else hi = mid - 1;
   }
   const NormTensor t = table[lo];
-  const long long begin = (chunk - t.chunk_start) * ADAM_CHUNK;
-  const long long end = min(begin + (long long)ADAM_CHUNK, t.numel);
-  float acc = 0.f;
-  for (long long j = begin + threadIdx.x; j < end; j += ADAM_THREADS) {
-    const float x = load1(t.x, dtype, j);
-    acc += x * x;
-  }
-  acc = block_sum(acc, scratch);
-  if (threadIdx.x == 0) atomicAdd(out, acc);
+  begin = (chunk - t.chunk_start) * ADAM_CHUNK;
+  end = min(begin + static_cast<long long>(ADAM_CHUNK), t.numel);
+  return t;
 }
 
-// x[i] *= *scale_dev (clip coefficient computed on the device), any dtype.
-__global__ void __launch_bounds__(ADAM_THREADS) multi_tensor_scale_kernel(const NormTensor* table, int n, int dtype, const float* scale_dev, int* found_inf) {
-  int lo = 0, hi = n - 1;
-  const long long chunk = blockIdx.x;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (table[mid].chunk_start <= chunk) lo = mid; else hi = mid - 1;
+template <typename T>
+__global__ void __launch_bounds__(ADAM_THREADS) multi_tensor_sumsq_kernel(const NormTensor* table, int n, float* out) {
+  __shared__ float scratch[32];
+  constexpr int N = Vec16<T>::N, U = 4;
+  long long begin, end;
+  const NormTensor t = norm_tensor_of_chunk(table, n, blockIdx.x, begin, end);
+  const T* x = static_cast<const T*>(t.x);
+  float acc[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) acc[k] = 0.f;
+  long long j = begin + threadIdx.x;  // first element that is left to the plain loop
+  if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
+    const long long step = static_cast<long long>(ADAM_THREADS) * N, vec_end = begin + (end - begin) / N * N;
+    long long i = begin + static_cast<long long>(threadIdx.x) * N;
+    for (; i + (U - 1) * step < vec_end; i += U * step) {
+      Vec16<T> v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = ld16(x + i + u * step);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int k = 0; k < N; ++k) acc[k] = fmaf(to_f32(v[u].v[k]), to_f32(v[u].v[k]), acc[k]);
+    }
+    for (; i < vec_end; i += step) {
+      const Vec16<T> v = ld16(x + i);
+#pragma unroll
+      for (int k = 0; k < N; ++k) acc[k] = fmaf(to_f32(v.v[k]), to_f32(v.v[k]), acc[k]);
+    }
+    j = vec_end + threadIdx.x;
   }
-  const NormTensor t = table[lo];
-  const long long begin = (chunk - t.chunk_start) * ADAM_CHUNK;
-  const long long end = min(begin + (long long)ADAM_CHUNK, t.numel);
+  for (; j < end; j += ADAM_THREADS) acc[0] = fmaf(to_f32(x[j]), to_f32(x[j]), acc[0]);
+  float sum = 0.f;
+#pragma unroll
+  for (int k = 0; k < N; ++k) sum += acc[k];
+  sum = block_sum(sum, scratch);
+  if (threadIdx.x == 0) atomicAdd(out, sum);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(ADAM_THREADS) multi_tensor_scale_kernel(const NormTensor* table, int n, const float* scale_dev, int* found_inf) {
+  constexpr int N = Vec16<T>::N, U = 4;
+  long long begin, end;
+  const NormTensor t = norm_tensor_of_chunk(table, n, blockIdx.x, begin, end);
+  T* x = static_cast<T*>(const_cast<void*>(t.x));
   const float s = *scale_dev;
   bool bad = false;
-  for (long long j = begin + threadIdx.x; j < end; j += ADAM_THREADS) {
-    const float x = load1(t.x, dtype, j) * s;
-    if (!isfinite(x)) bad = true;
-    store1(const_cast<void*>(t.x), dtype, j, x);
+  auto scaled = [&](T e) -> T {
+    const float f = to_f32(e) * s;
+    if (!isfinite(f)) bad = true;
+    return from_f32<T>(f);
+  };
+  long long j = begin + threadIdx.x;
+  if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
+    const long long step = static_cast<long long>(ADAM_THREADS) * N, vec_end = begin + (end - begin) / N * N;
+    long long i = begin + static_cast<long long>(threadIdx.x) * N;
+    for (; i + (U - 1) * step < vec_end; i += U * step) {
+      Vec16<T> v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = ld16(x + i + u * step);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) v[u].v[k] = scaled(v[u].v[k]);
+        st16(x + i + u * step, v[u]);
+      }
+    }
+    for (; i < vec_end; i += step) {
+      Vec16<T> v = ld16(x + i);
+#pragma unroll
+      for (int k = 0; k < N; ++k) v.v[k] = scaled(v.v[k]);
+      st16(x + i, v);
+    }
+    j = vec_end + threadIdx.x;
   }
+  for (; j < end; j += ADAM_THREADS) x[j] = scaled(x[j]);
   if (bad && found_inf != nullptr) *found_inf = 1;
 }
 
@@ -239,8 +291,12 @@ FSB_API int fsb_multi_tensor_sumsq(const void* table, int n_tensors, long long t
                                    cudaStream_t stream) {
   using namespace fsb;
   if (n_tensors <= 0 || total_chunks <= 0) return 0;
-  multi_tensor_sumsq_kernel<<<static_cast<unsigned>(total_chunks), ADAM_THREADS, 0, stream>>>(
-      static_cast<const NormTensor*>(table), n_tensors, dtype, out);
+  const auto* t = static_cast<const NormTensor*>(table);
+  const unsigned grid = static_cast<unsigned>(total_chunks);
+  if (dtype == FSB_F32)       multi_tensor_sumsq_kernel<float><<<grid, ADAM_THREADS, 0, stream>>>(t, n_tensors, out);
+  else if (dtype == FSB_F16)  multi_tensor_sumsq_kernel<__half><<<grid, ADAM_THREADS, 0, stream>>>(t, n_tensors, out);
+  else if (dtype == FSB_BF16) multi_tensor_sumsq_kernel<__nv_bfloat16><<<grid, ADAM_THREADS, 0, stream>>>(t, n_tensors, out);
+  else return -1;
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -248,7 +304,11 @@ FSB_API int fsb_multi_tensor_scale(const void* table, int n_tensors, long long t
                                    const float* scale_dev, int* found_inf, cudaStream_t stream) {
   using namespace fsb;
   if (n_tensors <= 0 || total_chunks <= 0) return 0;
-  multi_tensor_scale_kernel<<<static_cast<unsigned>(total_chunks), ADAM_THREADS, 0, stream>>>(
-      static_cast<const NormTensor*>(table), n_tensors, dtype, scale_dev, found_inf);
+  const auto* t = static_cast<const NormTensor*>(table);
+  const unsigned grid = static_cast<unsigned>(total_chunks);
+  if (dtype == FSB_F32)       multi_tensor_scale_kernel<float><<<grid, ADAM_THREADS, 0, stream>>>(t, n_tensors, scale_dev, found_inf);
+  else if (dtype == FSB_F16)  multi_tensor_scale_kernel<__half><<<grid, ADAM_THREADS, 0, stream>>>(t, n_tensors, scale_dev, found_inf);
+  else if (dtype == FSB_BF16) multi_tensor_scale_kernel<__nv_bfloat16><<<grid, ADAM_THREADS, 0, stream>>>(t, n_tensors, scale_dev, found_inf);
+  else return -1;
   return static_cast<int>(cudaGetLastError());
 }

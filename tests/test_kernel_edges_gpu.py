@@ -271,6 +271,29 @@ def test_small_gradients_land_in_their_flat_window():
     assert got[2].data_ptr() == base + 2 * (d * d + d) and got[3].data_ptr() == base + 2 * (d * d + 2 * d)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_multi_tensor_norm_and_scale_edges(dtype):
+    """Less than a vector, whole and ragged chunks, tensors that start off a 16-byte boundary, infinities."""
+    from fairscale_b200.ops import _bind, multi_tensor
+
+    torch.manual_seed(0)
+    chunk = _bind.fn("fsb_adam_chunk_size")()
+    flat = torch.randn(4 * chunk + 64, device=_dev()).to(dtype)
+    ts = [torch.randn(n, device=_dev()).to(dtype) for n in (1, 7, 8, 9, 2049, chunk, chunk + 3, 3 * chunk + 17)] + [flat[3 : chunk + 40], flat[2 * chunk + 1 :]]
+    want = math.sqrt(sum(t.double().pow(2).sum().item() for t in ts))
+    assert abs(multi_tensor.l2_norm(ts).item() / want - 1) < 1e-5  # fp32 sums, split over threads and chunks
+    flag = torch.zeros(1, dtype=torch.int32, device=_dev())
+    copies = [t.clone() for t in ts[:-2]] + [flat.clone()[3 : chunk + 40]]
+    wants = [(c.float() * 0.3).to(dtype) for c in copies]
+    multi_tensor.scale_(copies, torch.tensor([0.3], device=_dev()), flag)
+    for c, r in zip(copies, wants):
+        assert torch.equal(c, r)
+    assert int(flag) == 0
+    copies[-1][-1] = float("inf")
+    multi_tensor.scale_(copies, torch.tensor([1.0], device=_dev()), flag)
+    assert int(flag) == 1
+
+
 # head sizes whose rows do and do not divide 256 threads, fewer rows than a step of four takes, more tokens than the grid
 @pytest.mark.parametrize("B,S,H,D", [(1, 1, 1, 8), (2, 5, 3, 80), (1, 7, 1, 2048), (1, 3, 1, 2056), (3, 700, 2, 64), (2, 33, 32, 128)])
 def test_rope_edges(B, S, H, D):
