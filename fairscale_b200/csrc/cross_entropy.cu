@@ -24,14 +24,18 @@ template <typename T> __device__ __forceinline__ float ce_log(float x);
 template <> __device__ __forceinline__ float ce_log<__nv_bfloat16>(float x) { return __logf(x); }
 template <> __device__ __forceinline__ float ce_log<float>(float x) { return logf(x); }
 
+// Exponents are taken relative to the largest value; a maximum that is infinite leaves nothing to be relative to (inf - inf).
+__device__ __forceinline__ float ce_ref(float m) { return isinf(m) ? 0.f : m; }
+
 // Online softmax over N values at once: one rescaling per vector instead of a branch per value, which made the bf16 forward
-// compute-bound (16384 x 50304: 671 us against 250 us of memory time).  Masked logits (-inf) add nothing, also before the
-// first finite one.
+// compute-bound (16384 x 50304: 671 us against 250 us of memory time).  fmaxf passes over NaN, so `m` never holds one and a
+// NaN shows in `s` alone.  While every value is -inf or NaN, `m` is -inf and `s` is 0 or NaN; from the first +inf on, `s` is
+// +inf or NaN.
 template <typename T, int N> __device__ __forceinline__ void online_update(float& m, float& s, const float (&x)[N]) {
   float mx = m;
 #pragma unroll
   for (int k = 0; k < N; ++k) mx = fmaxf(mx, x[k]);
-  const float ref = mx == -INFINITY ? 0.f : mx;
+  const float ref = ce_ref(mx);
   s *= ce_exp<T>(m - ref);
 #pragma unroll
   for (int k = 0; k < N; ++k) s += ce_exp<T>(x[k] - ref);
@@ -61,15 +65,14 @@ __global__ void __launch_bounds__(CE_THREADS) ce_fwd_kernel(const T* __restrict_
     online_update<T, 1>(m, s, x);
   }
   const float gmax = block_max(m, scratch);
-  const float contrib = (m == -INFINITY) ? 0.f : s * ce_exp<T>(m - gmax);
-  float gsum = block_sum(contrib, scratch);
-  if (gmax == INFINITY) gsum = 1.f;  // inf - inf in the sums: the log-sum-exp of a row with an infinite logit is infinite
+  const float gref = ce_ref(gmax);
+  const float gsum = block_sum(s * ce_exp<T>(m - gref), scratch);  // a thread without a finite value adds its 0 or NaN
   if (threadIdx.x == 0) {
     const long long tgt = targets[row];
     const long long local = tgt - vocab_start;
     const bool mine = tgt != ignore_index && local >= 0 && local < V;
     const float tl = mine ? to_f32(lr[local]) : 0.f;
-    const float lse = gmax + ce_log<T>(gsum);
+    const float lse = gref + ce_log<T>(gsum);
     if (lse_out != nullptr) lse_out[row] = lse;
     if (loss != nullptr) loss[row] = (tgt == ignore_index) ? 0.f : (lse - tl);
     if (stats_out != nullptr) {

@@ -344,3 +344,34 @@ def test_vocab_cross_entropy_pieces(rows, V, dtype):
     if dtype == torch.float32:
         assert torch.equal(x, before)  # fp32 logits may be the caller's own
     _status_ok()
+
+
+# one vector of NaN (with few columns all that its thread sees), a whole row of it, infinities on their own and beside NaN
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("V", [8, 512, 2056, 32000])
+def test_cross_entropy_keeps_nan_and_infinity(V, dtype):
+    from fairscale_b200.ops.loss import ce_forward
+
+    torch.manual_seed(V)
+    inf, nan = float("inf"), float("nan")
+    x = torch.randn(7, V, device=_dev()).to(dtype)
+    x[0, :8] = nan
+    x[1] = nan
+    x[2, 3] = inf
+    x[3, 3], x[3, 5] = inf, inf
+    x[4, 3], x[4, V - 1] = inf, nan
+    x[5] = -inf
+    t = torch.full((7,), V // 2, device=_dev())
+    t[2:4] = 0
+    loss, lse, stats = ce_forward(x, t, want_stats=True)
+    want = torch.logsumexp(x.double(), -1)
+    assert torch.isnan(want[[0, 1, 4]]).all() and (want[2:4] == inf).all() and want[5] == -inf
+    torch.testing.assert_close(lse.double(), want, rtol=1e-4, atol=1e-4, equal_nan=True)
+    torch.testing.assert_close(loss.double(), want - x.double().gather(1, t.unsqueeze(1)).squeeze(1), rtol=1e-4, atol=1e-3, equal_nan=True)
+    # what another rank's shard makes of the pieces: NaN comes through, also from a shard that holds nothing else
+    other = torch.tensor([0.5, 2.0, 0.25], device=_dev()).expand(7, 3)
+    both = torch.stack([stats, other])
+    top = both[..., 0].max(0).values
+    merged = top + (both[..., 1] * torch.exp(both[..., 0] - top)).sum(0).log()
+    assert torch.isnan(merged[[0, 1, 4]]).all() and torch.isfinite(merged[5:]).all()
+    _status_ok()
