@@ -24,10 +24,17 @@
 
 #include <cstdlib>
 #include <mutex>
+#include <unordered_map>
 
 namespace fsb {
 
 constexpr int SCHED_DEPTH = 4;  // tile indices in flight between a CTA's (pair's) scheduler and its readers
+
+// Counters of the run-time tile hand-out, two per slot: tiles handed out, CTAs (pairs) that have finished.  All zero while no
+// kernel uses them (the last CTA of a launch puts its slot back).  A slot belongs to one stream, so the launches that share
+// it are ordered; slot 0 stands for "no counter" (see sched_slot_of).
+constexpr int SCHED_SLOTS = 256;
+__device__ unsigned int g_sched_counters[2 * SCHED_SLOTS];
 
 // BATCHED (both kernels): the tensor maps are 3-D (K / MN, rows, problem) and a tile index also selects the problem; used
 // for the local experts of an MoE layer (equal capacity per expert), where one launch replaces a Python loop of GEMMs.
@@ -91,11 +98,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   // Every CTA starts with the tile of its own index; the tiles after those are handed out at run time, as in the CTA-pair
   // kernel below and for the same reason: the producer takes the next index from a counter in global memory and publishes it
   // (or -1 at the end) through a small ring that the other roles read in order.  A launch with one tile per CTA never
-  // touches the counter; one without a counter (p.sched null) strides through the tiles, which is up to 3 % faster on a
+  // touches the counter; one without a counter (p.sched_slot 0) strides through the tiles, which is up to 3 % faster on a
   // device that nothing else uses (16384 x 2048 x 2048: 100 against 102 us).
   int q = 0;            // this role's position in the ring
   uint32_t qphase = 0;
-  const bool counted = num_tiles > static_cast<int>(gridDim.x) && p.sched != nullptr;
+  unsigned int* const sched = g_sched_counters + 2 * p.sched_slot;
+  const bool counted = num_tiles > static_cast<int>(gridDim.x) && p.sched_slot != 0;
   // Reader side, by all lanes of a warp: the next tile (-1: no more, -2: the wait ran out).
   auto take_tile = [&]() -> int {
     int t = -2;
@@ -114,7 +122,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
       uint32_t phase = 0;
       bool ok = true;
       auto fetch = [&](int before) -> int {  // `before`: the last index this CTA was given
-        return static_cast<int>(gridDim.x) + (counted ? static_cast<int>(atomicAdd(&p.sched[0], 1u)) : before);
+        return static_cast<int>(gridDim.x) + (counted ? static_cast<int>(atomicAdd(&sched[0], 1u)) : before);
       };
       int nxt = fetch(static_cast<int>(blockIdx.x));  // needed when the first tile's loads are all on their way
       for (int tile = blockIdx.x, next_tile = -1; tile >= 0 && ok; tile = next_tile) {
@@ -154,9 +162,9 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
       if (counted) {
         // The last CTA to get here has seen every CTA's final fetch (each adds to sched[1] after the value of its last fetch
         // came back, so no fence is needed): put the counters back for the next launch.
-        if (atomicAdd(&p.sched[1], 1u) == gridDim.x - 1u) {
-          p.sched[0] = 0u;
-          p.sched[1] = 0u;
+        if (atomicAdd(&sched[1], 1u) == gridDim.x - 1u) {
+          sched[0] = 0u;
+          sched[1] = 0u;
         }
       }
     }
@@ -426,7 +434,9 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
   // Tiles are handed out at run time: the leader's producer takes the next index from a counter in global memory and
   // publishes it (or -1 at the end) to both CTAs through a small ring; every role reads the ring in order.  An SM that
   // is slowed down or taken by a kernel of another stream (a collective) then simply works off fewer tiles, instead of
-  // holding back the tiles a static schedule would have given it.
+  // holding back the tiles a static schedule would have given it.  A launch without a counter strides through the tiles.
+  unsigned int* const sched = g_sched_counters + 2 * p.sched_slot;
+  const bool counted = p.sched_slot != 0;
   // Reader side: wait for slot q, take the index, hand the slot back to the leader.
   auto take_tile = [&](int q, uint32_t qphase, int site) -> int {
     if (!mbar_wait_cluster(&sched_full[q], qphase, abort_flag, site)) return -2;
@@ -455,13 +465,16 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
         if (++q == SCHED_DEPTH) { q = 0; qphase ^= 1u; }
         return true;
       };
+      auto fetch = [&](int before) -> int {  // `before`: the last index this pair was given
+        return counted ? static_cast<int>(atomicAdd(&sched[0], 1u)) : before + num_pairs;
+      };
       int cur = -1, nxt = -1;
       int b_upto = -1;  // highest B piece known to have arrived
       if (leader) {
-        cur = static_cast<int>(atomicAdd(&p.sched[0], 1u));
+        cur = fetch(static_cast<int>(blockIdx.x >> 1) - num_pairs);
         if (cur >= num_tiles) cur = -1;
         ok = publish(cur);
-        if (cur >= 0) nxt = static_cast<int>(atomicAdd(&p.sched[0], 1u));
+        if (cur >= 0) nxt = fetch(cur);
       }
       while (ok) {
         int tile;
@@ -471,7 +484,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
             const int nt = nxt < num_tiles ? nxt : -1;
             if (!publish(nt)) break;
             cur = nt;
-            if (nt >= 0) nxt = static_cast<int>(atomicAdd(&p.sched[0], 1u));  // used one tile from now
+            if (nt >= 0) nxt = fetch(nt);  // used one tile from now
           }
         } else {
           tile = take_tile(q, qphase, 3);
@@ -513,12 +526,12 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
           if (++stage == PAIR_STAGES) { stage = 0; phase ^= 1u; }
         }
       }
-      if (leader) {
+      if (leader && counted) {
         // the last pair to get here has seen every pair's final fetch: put the counters back for the next launch
         __threadfence();
-        if (atomicAdd(&p.sched[1], 1u) == static_cast<unsigned int>(num_pairs - 1)) {
-          p.sched[0] = 0u;
-          p.sched[1] = 0u;
+        if (atomicAdd(&sched[1], 1u) == static_cast<unsigned int>(num_pairs - 1)) {
+          sched[0] = 0u;
+          sched[1] = 0u;
           __threadfence();
         }
       }
@@ -630,22 +643,39 @@ namespace fsb_host {
 int gemm_cluster_k(const CUtensorMap& ta, const void* B, int ldb, const fsb::GemmParams& p, int block_n, int splits, int dev, cudaStream_t stream);
 }  // namespace fsb_host
 
-// Counter pairs of the dynamic tile scheduler: a ring of slots per device, one slot per launch, so that GEMMs running
-// at the same time on different streams never share a counter.  A slot is all zero whenever no kernel is using it (the
-// kernel resets it), hence 64 launches would have to be in flight at once on one device before two could collide.
-static unsigned int* next_sched_slot(int di) {
-  constexpr int kSlots = 64;
-  static std::mutex mu;
-  static unsigned int* base[64] = {nullptr};
-  static unsigned int seq[64] = {0};
-  std::lock_guard<std::mutex> lock(mu);
-  if (base[di] == nullptr) {
-    void* ptr = nullptr;
-    if (cudaMalloc(&ptr, kSlots * 2 * sizeof(unsigned int)) != cudaSuccess) return nullptr;
-    if (cudaMemset(ptr, 0, kSlots * 2 * sizeof(unsigned int)) != cudaSuccess) return nullptr;
-    base[di] = static_cast<unsigned int*>(ptr);
+// Slot of the tile counters for a launch on `stream`: every stream keeps one of its own for the life of the process, so two
+// launches that use the same counters are ordered by their stream, however far the host runs ahead.  Streams are told apart
+// by their id, which is never given out twice (a handle is, while the old stream's work may still be running).  0, no
+// counter, for the streams that come after SCHED_SLOTS - 1 others and for a launch under capture: a graph is replayed on
+// any stream, beside eager launches.  Such a launch strides through its tiles.
+static int sched_slot_of(int di, cudaStream_t stream) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {  // the default stream while another one is captured
+    cudaGetLastError();
+    return 0;
   }
-  return base[di] + 2 * ((seq[di]++) % kSlots);
+  if (capture != cudaStreamCaptureStatusNone) return 0;
+  unsigned long long id = 0;
+  if (cudaStreamGetId(stream, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  static std::mutex mu;
+  static std::unordered_map<unsigned long long, int> slots[64];
+  std::lock_guard<std::mutex> lock(mu);
+  const auto it = slots[di].find(id);
+  if (it != slots[di].end()) return it->second;
+  const int slot = static_cast<int>(slots[di].size()) + 1;
+  if (slot >= fsb::SCHED_SLOTS) return 0;
+  slots[di].emplace(id, slot);
+  return slot;
+}
+
+// The slot that a product launched on `stream` of the current device would use (0: none).
+FSB_API int fsb_gemm_sched_slot(cudaStream_t stream) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return sched_slot_of(dev & 63, stream);
 }
 
 static bool pair_enabled() {  // FSB_GEMM_PAIR=0 disables the CTA-pair kernel
@@ -804,7 +834,7 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* bia
   p.epilogue = epilogue; p.out_f32 = out_f32; p.accumulate_c = accumulate_c;
   p.status = status;
   p.batch = 1; p.stride_c = p.stride_aux = p.stride_bias = 0;
-  p.sched = nullptr;
+  p.sched_slot = 0;
   p.b_ready = b_ready; p.b_ready_epoch = b_ready_epoch; p.b_piece_bytes = b_piece_bytes; p.b_wait_ns = b_wait_ns;
   p.b_num_pieces = b_piece_bytes > 0 ? static_cast<int>((static_cast<long long>(N) * K * 2 + b_piece_bytes - 1) / b_piece_bytes) : 1;
   p.b_first_piece = b_ready != nullptr ? b_first_piece % p.b_num_pieces : 0;
@@ -832,8 +862,7 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* bia
   if (plan.kind == GemmPlan::CLUSTER_K) return fsb_host::gemm_cluster_k(ta, B, ldb, p, plan.block_n, plan.splits, dev, stream);
   // Run-time tile hand-out for products large enough to share the device with a collective; small ones stride.
   if (max_ctas == 0 && M >= 256 && N >= 256 && (plan.kind == GemmPlan::PAIR || tiles > num_sms)) {
-    p.sched = next_sched_slot(di);
-    if (p.sched == nullptr) return -1;
+    p.sched_slot = sched_slot_of(di, stream);
   }
   if (plan.kind == GemmPlan::PAIR) {
     // the B map's box is this CTA's 128 columns (K-major) / 64 (MN-major, unchanged)
@@ -896,7 +925,7 @@ FSB_API int fsb_gemm_bf16_batched(const void* A, const void* B, void* C, const v
   p.a_mn_major = a_mn_major; p.b_mn_major = b_mn_major;
   p.epilogue = epilogue; p.out_f32 = out_f32; p.accumulate_c = accumulate_c;
   p.status = status;
-  p.sched = nullptr;
+  p.sched_slot = 0;
   p.b_ready = nullptr; p.b_ready_epoch = 0; p.b_piece_bytes = 0; p.b_wait_ns = 0; p.b_first_piece = 0; p.b_num_pieces = 1;
   p.a_ready = nullptr; p.a_ready_epoch = 0; p.a_shard_rows = p.a_piece_rows = p.a_first_shard = p.a_num_shards = 0;
   p.batch = batch; p.stride_c = stride_c; p.stride_aux = stride_aux > 0 ? stride_aux : stride_c; p.stride_bias = stride_bias;
@@ -914,8 +943,7 @@ FSB_API int fsb_gemm_bf16_batched(const void* A, const void* B, void* C, const v
     }
     const long long pair_tiles = static_cast<long long>(batch) * ((M + 2 * BLOCK_M - 1) / (2 * BLOCK_M)) * ((N + PAIR_BLOCK_N - 1) / PAIR_BLOCK_N);
     const int pairs = pair_tiles < num_sms / 2 ? static_cast<int>(pair_tiles) : num_sms / 2;
-    p.sched = next_sched_slot(dev & 63);
-    if (p.sched == nullptr) return -1;
+    p.sched_slot = sched_slot_of(dev & 63, stream);
     gemm_bf16_tcgen05_pair_kernel<true><<<2 * pairs, PAIR_THREADS, PairSmem::TOTAL, stream>>>(ta, tb, p);
     return static_cast<int>(cudaGetLastError());
   }

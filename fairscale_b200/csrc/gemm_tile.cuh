@@ -36,9 +36,8 @@ struct GemmParams {
   // batched (grouped) products: `batch` independent problems of the same shape; element strides between them
   int batch;
   long long stride_c, stride_aux, stride_bias;
-  // dynamic tile scheduler: sched[0] = tiles handed out, sched[1] = CTA pairs (CTAs) that have finished; both zero before the
-  // launch, the last one to finish resets them.  Null for the one-CTA kernel: no hand-out.
-  unsigned int* sched;
+  // counters of the run-time tile hand-out (g_sched_counters in gemm_tcgen05.cu); 0: none, every CTA strides through the tiles
+  int sched_slot;
   // Optional arrival flags of the B operand (CTA-pair kernel, B K-major with contiguous rows): the operand is being
   // written by somebody else (copy engines gathering a sharded weight) while the kernel runs.  Bytes
   // [i * b_piece_bytes, (i + 1) * b_piece_bytes) of B are valid once b_ready[i] >= b_ready_epoch (epochs only grow).

@@ -375,3 +375,51 @@ def test_cross_entropy_keeps_nan_and_infinity(V, dtype):
     merged = top + (both[..., 1] * torch.exp(both[..., 0] - top)).sum(0).log()
     assert torch.isnan(merged[[0, 1, 4]]).all() and torch.isfinite(merged[5:]).all()
     _status_ok()
+
+
+# one CTA per tile and CTA pairs, both with more tiles than one wave
+@pytest.mark.parametrize("M,N,K", [(4104, 2568, 512), (8200, 8200, 2048)])
+def test_products_on_two_streams_and_in_a_graph_keep_their_tiles(M, N, K):
+    """The run-time tile hand-out belongs to a stream: a product that waits on one stream while many are enqueued on another,
+    and one replayed from a graph, share no counter with them."""
+    from ctypes import c_void_p
+
+    from fairscale_b200.fair_dev.testing.testing import gpu_delay
+    from fairscale_b200.ops import _bind
+    from fairscale_b200.ops.gemm import _launch
+
+    _bind._SIGNATURES.setdefault("fsb_gemm_sched_slot", [c_void_p])
+    slot = _bind.fn("fsb_gemm_sched_slot")
+    torch.manual_seed(0)
+    a, b = torch.randn(M, K, device=_dev()).bfloat16(), torch.randn(N, K, device=_dev()).bfloat16()
+    want = torch.empty(M, N, device=_dev(), dtype=torch.bfloat16)
+
+    def product(out):
+        _launch(a, b, out, M, N, K, False, False)
+
+    product(want)
+    assert _rel_err(want, a.float() @ b.float().t()) < 1e-2
+    outs = [torch.full_like(want, float("nan")) for _ in range(6)]
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    slots = [slot(_bind.stream_ptr(_dev())), slot(s1.cuda_stream), slot(s2.cuda_stream)]
+    assert min(slots) > 0 and len(set(slots)) == 3 and slot(s1.cuda_stream) == slots[1]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        assert slot(_bind.stream_ptr(_dev())) == 0
+        product(outs[0])
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s1):
+        gpu_delay(3.0)  # so that all of the other stream's products are enqueued before these start
+        for i in (1, 2):
+            product(outs[i])
+    with torch.cuda.stream(s2):
+        for _ in range(80):
+            product(outs[3])
+        product(outs[4])
+    with torch.cuda.stream(s1):
+        graph.replay()
+        product(outs[5])
+    torch.cuda.synchronize()
+    for o in outs:
+        assert torch.equal(o, want)
+    _status_ok()
