@@ -1,14 +1,16 @@
 // Row movement of a mixture-of-experts layer inside one GPU's memory: tokens to expert slots and back.
 //
-//   pack    : int32 routing [4, S] (idx1, idx2, loc1, loc2) -> expert / slot (int64 [S, 2]), keep (bool [S, 2]) and
-//             flat (int32 [S, 2]) = expert * C + slot, or -1 for a choice that overflowed its expert's capacity C
+//   pack    : int32 routing [4, S] (idx1, idx2, loc1, loc2) -> expert / slot (int64 [S, 2]) and keep (bool [S, 2])
+//   claim   : expert, slot, keep -> flat (int32 [S, 2]) = expert * C + slot, or -1 for a choice that is not kept, and one
+//             byte per row of the [E * C, M] buffer: does a token claim it?
 //   scatter : out[flat[s, k], :] = x[s, :] (* w[s, k]);   rows of out that no token claimed are zeroed
 //   gather  : out[s, :] = sum_k w[s, k] * buf[flat[s, k], :];   dots[s, k] = <buf[flat[s, k], :], g[s, :]>
 //
 // All three are bound by memory traffic: a warp moves one row with 16-byte accesses (four in flight per lane), scatter
 // reads a token once for both of its slots, gather sums both choices in fp32 registers.  A choice is known to be dropped
 // from its flat index alone, so nothing on the host depends on how many tokens were kept (the index_copy formulation
-// compacts the kept rows first, which makes the host wait for the device twice per direction).
+// compacts the kept rows first, which makes the host wait for the device twice per direction).  Both come from the route as
+// the layer gets it - a gate may have changed what the routing kernels made - and never from counts taken before that.
 // Layer forward + backward, 8192 tokens of 1024 bf16, 8 experts of 4096: 3722 us with index ops, 1278 us with these kernels
 // and the expert products on CTA pairs; 820 tokens of 512, 4 experts of 2048: 2481 -> 1192 us.
 //
@@ -34,27 +36,35 @@ template <typename T, int VEC> __device__ __forceinline__ void row_st(T* p, cons
 }
 
 __global__ void __launch_bounds__(MR_THREADS) moe_route_pack_kernel(const int* __restrict__ route, int S, int C, long long* __restrict__ expert,
-                                                                    long long* __restrict__ slot, unsigned char* __restrict__ keep,
-                                                                    int* __restrict__ flat) {
+                                                                    long long* __restrict__ slot, unsigned char* __restrict__ keep) {
   const int i = blockIdx.x * MR_THREADS + threadIdx.x;  // (token, choice)
   if (i >= 2 * S) return;
   const int s = i >> 1, k = i & 1;
-  const int e = route[k * S + s], l = route[(2 + k) * S + s];
-  const bool kept = l < C;
-  expert[i] = e;
-  slot[i] = kept ? l : 0;
-  keep[i] = kept ? 1 : 0;
-  flat[i] = kept ? e * C + l : -1;
+  const int l = route[(2 + k) * S + s];
+  expert[i] = route[k * S + s];
+  slot[i] = l < C ? l : 0;
+  keep[i] = l < C ? 1 : 0;
+}
+
+// `claimed` is all zero before the launch
+__global__ void __launch_bounds__(MR_THREADS) moe_claim_rows_kernel(const long long* __restrict__ expert, const long long* __restrict__ slot,
+                                                                    const unsigned char* __restrict__ keep, long long choices, long long E, long long C,
+                                                                    int* __restrict__ flat, unsigned char* __restrict__ claimed) {
+  const long long i = static_cast<long long>(blockIdx.x) * MR_THREADS + threadIdx.x;
+  if (i >= choices) return;
+  const long long row = expert[i] * C + slot[i];
+  const bool kept = keep[i] != 0 && row >= 0 && row < E * C;
+  flat[i] = kept ? static_cast<int>(row) : -1;
+  if (kept) claimed[row] = 1;
 }
 
 // Warps 0 .. S-1 (in grid-stride order) each move one token; warps S .. S + E * C - 1 each look at one row of `out`.
 template <typename T, int VEC>
 __global__ void __launch_bounds__(MR_THREADS) moe_scatter_local_kernel(const T* __restrict__ x, const int* __restrict__ flat, const float* __restrict__ w,
-                                                                       long long S, int M, T* __restrict__ out, const int* __restrict__ counts, int E,
-                                                                       int C) {
+                                                                       long long S, int M, T* __restrict__ out, const unsigned char* __restrict__ claimed,
+                                                                       long long rows) {
   const int lane = threadIdx.x & 31;
   const long long warps = static_cast<long long>(gridDim.x) * MR_WARPS;
-  const long long rows = counts != nullptr ? static_cast<long long>(E) * C : 0;
   for (long long i = static_cast<long long>(blockIdx.x) * MR_WARPS + (threadIdx.x >> 5); i < S + rows; i += warps) {
     if (i < S) {
       const int r0 = flat[2 * i], r1 = flat[2 * i + 1];
@@ -83,8 +93,7 @@ __global__ void __launch_bounds__(MR_THREADS) moe_scatter_local_kernel(const T* 
       }
     } else {
       const long long r = i - S;
-      const int e = static_cast<int>(r / C);
-      if (r - static_cast<long long>(e) * C < static_cast<long long>(counts[e]) + counts[E + e]) continue;  // claimed by a token
+      if (claimed[r]) continue;
       RowVec<T, VEC> z;
 #pragma unroll
       for (int k = 0; k < VEC; ++k) z.v[k] = from_f32<T>(0.f);
@@ -156,32 +165,46 @@ static bool mr_vec(int M, int size, const void* a, const void* b, const void* c)
   return (static_cast<long long>(M) * size) % 16 == 0 && (ptrs & 15u) == 0;
 }
 
-// route int32 [4, S]; expert / slot int64 [S, 2]; keep bool [S, 2]; flat int32 [S, 2].  E * C must fit 31 bits.
-FSB_API int fsb_moe_route_pack(const int* route, int S, int C, long long* expert, long long* slot, unsigned char* keep, int* flat, cudaStream_t stream) {
+// route int32 [4, S]; expert / slot int64 [S, 2]; keep bool [S, 2].
+FSB_API int fsb_moe_route_pack(const int* route, int S, int C, long long* expert, long long* slot, unsigned char* keep, cudaStream_t stream) {
   using namespace fsb;
   if (S <= 0) return 0;
-  moe_route_pack_kernel<<<(2 * S + MR_THREADS - 1) / MR_THREADS, MR_THREADS, 0, stream>>>(route, S, C, expert, slot, keep, flat);
+  moe_route_pack_kernel<<<(2 * S + MR_THREADS - 1) / MR_THREADS, MR_THREADS, 0, stream>>>(route, S, C, expert, slot, keep);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// expert / slot int64 [S, 2], keep bool [S, 2]; flat int32 [S, 2]; claimed [E * C] bytes.  E * C must fit 31 bits.
+FSB_API int fsb_moe_claim_rows(const long long* expert, const long long* slot, const unsigned char* keep, long long S, long long E, long long C, int* flat,
+                               unsigned char* claimed, cudaStream_t stream) {
+  using namespace fsb;
+  if (E * C > 0x7fffffffll) return -1;
+  if (E * C > 0) {
+    const cudaError_t e = cudaMemsetAsync(claimed, 0, static_cast<size_t>(E * C), stream);
+    if (e != cudaSuccess) return static_cast<int>(e);
+  }
+  if (S <= 0) return 0;
+  moe_claim_rows_kernel<<<static_cast<unsigned>((2 * S + MR_THREADS - 1) / MR_THREADS), MR_THREADS, 0, stream>>>(expert, slot, keep, 2 * S, E, C, flat, claimed);
   return static_cast<int>(cudaGetLastError());
 }
 
 template <typename T>
-static void moe_scatter_t(const void* x, const int* flat, const float* w, long long S, int M, void* out, const int* counts, int E, int C, cudaStream_t stream) {
+static void moe_scatter_t(const void* x, const int* flat, const float* w, long long S, int M, void* out, const unsigned char* claimed, long long rows,
+                          cudaStream_t stream) {
   using namespace fsb;
-  const int grid = mr_grid(S + (counts != nullptr ? static_cast<long long>(E) * C : 0));
+  const int grid = mr_grid(S + rows);
   if (mr_vec(M, sizeof(T), x, out, nullptr))
-    moe_scatter_local_kernel<T, 16 / sizeof(T)><<<grid, MR_THREADS, 0, stream>>>(static_cast<const T*>(x), flat, w, S, M, static_cast<T*>(out), counts, E, C);
+    moe_scatter_local_kernel<T, 16 / sizeof(T)><<<grid, MR_THREADS, 0, stream>>>(static_cast<const T*>(x), flat, w, S, M, static_cast<T*>(out), claimed, rows);
   else
-    moe_scatter_local_kernel<T, 1><<<grid, MR_THREADS, 0, stream>>>(static_cast<const T*>(x), flat, w, S, M, static_cast<T*>(out), counts, E, C);
+    moe_scatter_local_kernel<T, 1><<<grid, MR_THREADS, 0, stream>>>(static_cast<const T*>(x), flat, w, S, M, static_cast<T*>(out), claimed, rows);
 }
 
-// x [S, M], out [E * C, M] (fp32 / fp16 / bf16); w fp32 [S, 2] or null; counts int32 [2 * E] (tokens per expert as first / second
-// choice) or null, then the caller has zeroed `out`.
-FSB_API int fsb_moe_scatter_local(const void* x, int dtype, const int* flat, const float* w, long long S, int M, void* out, const int* counts, int E, int C,
-                                  cudaStream_t stream) {
-  if (S <= 0 || M <= 0) return 0;
-  if (dtype == FSB_F32) moe_scatter_t<float>(x, flat, w, S, M, out, counts, E, C, stream);
-  else if (dtype == FSB_F16) moe_scatter_t<__half>(x, flat, w, S, M, out, counts, E, C, stream);
-  else if (dtype == FSB_BF16) moe_scatter_t<__nv_bfloat16>(x, flat, w, S, M, out, counts, E, C, stream);
+// x [S, M], out [rows, M] (fp32 / fp16 / bf16); w fp32 [S, 2] or null; flat and claimed from fsb_moe_claim_rows.
+FSB_API int fsb_moe_scatter_local(const void* x, int dtype, const int* flat, const float* w, long long S, int M, void* out, const unsigned char* claimed,
+                                  long long rows, cudaStream_t stream) {
+  if (S + rows <= 0 || M <= 0) return 0;
+  if (dtype == FSB_F32) moe_scatter_t<float>(x, flat, w, S, M, out, claimed, rows, stream);
+  else if (dtype == FSB_F16) moe_scatter_t<__half>(x, flat, w, S, M, out, claimed, rows, stream);
+  else if (dtype == FSB_BF16) moe_scatter_t<__nv_bfloat16>(x, flat, w, S, M, out, claimed, rows, stream);
   else return -1;
   return static_cast<int>(cudaGetLastError());
 }

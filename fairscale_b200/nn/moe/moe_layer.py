@@ -108,27 +108,44 @@ def _local_rows(t: Tensor) -> bool:
     return t.is_cuda and t.dtype in (torch.float32, torch.float16, torch.bfloat16)
 
 
-def _flat_rows(route: Top2Route) -> Tensor:
-    """int32 ``[S, 2]``: row of the global ``[E * C, M]`` view that each choice claims, -1 if it was dropped."""
-    if getattr(route, "flat", None) is not None:
-        return route.flat
-    flat = route.expert * route.capacity + route.slot
-    return torch.where(route.keep, flat, torch.full_like(flat, -1)).to(torch.int32).contiguous()
+class _Claims:
+    """The rows of the global ``[E * C, M]`` view that a route's choices claim, for the row kernels: ``flat`` int32 ``[S, 2]`` (-1 if
+    not kept) and ``claimed`` uint8 ``[E * C]``.  Computed when the dispatch of a forward asks for it, shared with its combine."""
+
+    def __init__(self, route: Top2Route) -> None:
+        self.route = route
+        self._rows: Optional[Tuple[Tensor, Tensor]] = None
+
+    def rows(self) -> Tuple[Tensor, Tensor]:
+        if self._rows is None:
+            from ctypes import c_longlong, c_void_p
+
+            from ...ops import _bind
+
+            _bind._SIGNATURES.setdefault("fsb_moe_claim_rows", [c_void_p] * 3 + [c_longlong] * 3 + [c_void_p] * 3)
+            r, dev = self.route, self.route.expert.device
+            expert, slot = r.expert.long().contiguous(), r.slot.long().contiguous()
+            keep = r.keep.to(torch.bool).contiguous()
+            flat = torch.empty(tuple(expert.shape), dtype=torch.int32, device=dev)
+            claimed = torch.empty(r.num_experts * r.capacity, dtype=torch.uint8, device=dev)
+            _bind.call("fsb_moe_claim_rows", expert.data_ptr(), slot.data_ptr(), keep.data_ptr(), expert.shape[0], r.num_experts, r.capacity,
+                       flat.data_ptr(), claimed.data_ptr(), _bind.stream_ptr(dev))
+            self._rows = (flat, claimed)
+        return self._rows
 
 
-def _scatter_local(x: Tensor, flat: Tensor, w: Optional[Tensor], counts: Optional[Tensor], E: int, C: int) -> Tensor:
-    """``out[flat[s, k]] = x[s] (* w[s, k])`` as ``[E * C, M]``; rows nobody claimed are zero."""
+def _scatter_local(x: Tensor, flat: Tensor, claimed: Tensor, w: Optional[Tensor]) -> Tensor:
+    """``out[flat[s, k]] = x[s] (* w[s, k])`` with a row per entry of ``claimed``; rows nobody claimed are zero."""
     from ctypes import c_int, c_longlong, c_void_p
 
     from ...ops import _bind
 
-    _bind._SIGNATURES.setdefault("fsb_moe_scatter_local", [c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p])
+    _bind._SIGNATURES.setdefault("fsb_moe_scatter_local", [c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_longlong, c_void_p])
     x = x.contiguous()
     S, M = x.shape
-    # without per-expert counts the kernel cannot tell which rows stay unclaimed
-    out = x.new_empty((E * C, M)) if counts is not None else x.new_zeros((E * C, M))
+    out = x.new_empty((claimed.shape[0], M))
     _bind.call("fsb_moe_scatter_local", x.data_ptr(), _bind.dtype_code(x.dtype), flat.data_ptr(), _bind.ptr(w), S, M, out.data_ptr(),
-               _bind.ptr(counts), E, C, _bind.stream_ptr(x.device))
+               claimed.data_ptr(), claimed.shape[0], _bind.stream_ptr(x.device))
     return out
 
 
@@ -171,7 +188,8 @@ class _Dispatch(torch.autograd.Function):
     """tokens ``[S, M]`` -> expert inputs ``[n_local, world * C, M]`` on the owning ranks."""
 
     @staticmethod
-    def forward(ctx: Any, x: Tensor, route: Top2Route, group: Any, n_local: int, owner: Optional[_LayerBuffers] = None) -> Tensor:  # type: ignore[override]
+    def forward(ctx: Any, x: Tensor, route: Top2Route, group: Any, n_local: int, owner: Optional[_LayerBuffers] = None,
+                claims: Optional[_Claims] = None) -> Tensor:  # type: ignore[override]
         world, rank = comm.group_size(group), comm.group_rank(group)
         C, E, M = route.capacity, route.num_experts, x.shape[1]
         ctx.meta = (group, n_local, world, rank, C, E, M, x.dtype)
@@ -181,9 +199,9 @@ class _Dispatch(torch.autograd.Function):
             owner._mine = False
         ctx.local = ws is None and _local_rows(x)
         if ctx.local:
-            flat = _flat_rows(route)
+            flat, claimed = (claims or _Claims(route)).rows()
             ctx.save_for_backward(flat)
-            return _to_experts(_scatter_local(x, flat, None, route.counts, E, C), group, world, n_local, C)
+            return _to_experts(_scatter_local(x, flat, claimed, None), group, world, n_local, C)
         dst_rank, dst_row, flat = _routes(route, world, n_local, rank)
         ctx.save_for_backward(dst_rank, dst_row, flat, route.keep)
         if ws is not None:
@@ -210,7 +228,7 @@ class _Dispatch(torch.autograd.Function):
         group, n_local, world, rank, C, E, M, dtype = ctx.meta
         if ctx.local:
             (flat,) = ctx.saved_tensors
-            return _gather_local(_to_tokens(grad.contiguous(), group, world, n_local, C), flat, None), None, None, None, None
+            return _gather_local(_to_tokens(grad.contiguous(), group, world, n_local, C), flat, None), None, None, None, None, None
         dst_rank, dst_row, flat, keep = ctx.saved_tensors
         S = dst_rank.shape[0]
         if ctx.claimed:
@@ -221,7 +239,7 @@ class _Dispatch(torch.autograd.Function):
             buf.copy_(grad.reshape(-1, M))
             dx = torch.empty((S, M), dtype=grad.dtype, device=grad.device)
             ws.moe_gather_rows(buf, dx, dst_rank.view(-1), dst_row.view(-1), None, 2)
-            return dx, None, None, None, None
+            return dx, None, None, None, None, None
         g = grad.view(n_local, world, C, M).transpose(0, 1).contiguous().view(E * C, M)
         back = torch.empty_like(g)
         comm.all_to_all_single(back, g, group)
@@ -229,7 +247,7 @@ class _Dispatch(torch.autograd.Function):
         for k in range(2):
             kept = keep[:, k]
             dx[kept] += back[flat[kept, k]]
-        return dx, None, None, None, None
+        return dx, None, None, None, None, None
 
 
 class _Combine(torch.autograd.Function):
@@ -237,7 +255,7 @@ class _Combine(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx: Any, expert_out: Tensor, gate: Tensor, route: Top2Route, group: Any, n_local: int,
-                owner: Optional[_LayerBuffers] = None) -> Tensor:  # type: ignore[override]
+                owner: Optional[_LayerBuffers] = None, claims: Optional[_Claims] = None) -> Tensor:  # type: ignore[override]
         world, rank = comm.group_size(group), comm.group_rank(group)
         C, E, M = route.capacity, route.num_experts, expert_out.shape[-1]
         ctx.meta = (group, n_local, world, rank, C, E, M)
@@ -247,10 +265,10 @@ class _Combine(torch.autograd.Function):
         ctx.owner = owner
         ctx.local = ws is None and _local_rows(expert_out)
         if ctx.local:
-            flat = _flat_rows(route)
+            flat, claimed = (claims or _Claims(route)).rows()
             w = gate.to(torch.float32).contiguous()  # the kernels look at flat: a dropped choice's weight is not read
             home = _to_tokens(expert_out.contiguous(), group, world, n_local, C)
-            ctx.save_for_backward(flat, w, home)
+            ctx.save_for_backward(flat, claimed, w, home)
             return _gather_local(home, flat, w)
         dst_rank, dst_row, flat = _routes(route, world, n_local, rank)
         S = dst_rank.shape[0]
@@ -275,11 +293,10 @@ class _Combine(torch.autograd.Function):
     def backward(ctx: Any, dy: Tensor):  # type: ignore[override]
         group, n_local, world, rank, C, E, M = ctx.meta
         if ctx.local:
-            flat, w, home = ctx.saved_tensors
+            flat, claimed, w, home = ctx.saved_tensors
             dy = dy.to(home.dtype).contiguous()
-            counts = ctx.fill[0] if ctx.fill is not None else None
-            d_eo = _to_experts(_scatter_local(dy, flat, w, counts, E, C), group, world, n_local, C)
-            return d_eo, _gather_local(home, flat, None, grad=dy), None, None, None, None
+            d_eo = _to_experts(_scatter_local(dy, flat, claimed, w), group, world, n_local, C)
+            return d_eo, _gather_local(home, flat, None, grad=dy), None, None, None, None, None
         dst_rank, dst_row, flat, keep, w, saved = ctx.saved_tensors
         S = dst_rank.shape[0]
         dy = dy.contiguous()
@@ -302,7 +319,7 @@ class _Combine(torch.autograd.Function):
                 obuf.copy_(saved.reshape(-1, M))
             dots = torch.zeros((S, 2), dtype=torch.float32, device=dy.device)
             ws.moe_gather_rows(obuf, None, dst_rank.view(-1), dst_row.view(-1), None, 2, grad=dy, dots=dots.view(-1))
-            return d_eo, (dots * keep).to(w.dtype), None, None, None, None
+            return d_eo, (dots * keep).to(w.dtype), None, None, None, None, None
         rows = saved  # [S, 2, M]
         d_gate = (rows.float() * dy.float().unsqueeze(1)).sum(-1) * keep
         contrib = dy.float().unsqueeze(1) * w.unsqueeze(-1)  # [S, 2, M]
@@ -314,7 +331,7 @@ class _Combine(torch.autograd.Function):
         back = torch.empty_like(home)
         comm.all_to_all_single(back, home, group)
         d_eo = back.view(world, n_local, C, M).transpose(0, 1).reshape(n_local, world * C, M)
-        return d_eo, d_gate.to(w.dtype), None, None, None, None
+        return d_eo, d_gate.to(w.dtype), None, None, None, None, None
 
 
 class MOELayer(Base):
@@ -352,7 +369,8 @@ class MOELayer(Base):
             route: Top2Route = self.gate.route(tokens)
             self.l_aux = route.l_aux
             self._heap_buffers.expect_backward = torch.is_grad_enabled()
-            expert_in = _Dispatch.apply(tokens, route, self.group, self.num_local_experts, self._heap_buffers)  # [n_local, world*C, M]
+            claims = _Claims(route)
+            expert_in = _Dispatch.apply(tokens, route, self.group, self.num_local_experts, self._heap_buffers, claims)  # [n_local, world*C, M]
             if self._grouped:
                 expert_out = self.experts[0](expert_in)  # every local expert in one grouped launch
             else:
@@ -361,7 +379,7 @@ class MOELayer(Base):
                     chunk = expert_in[e].view(self.world_size, 1, route.capacity, d_model)
                     outs.append(expert(chunk).reshape(self.world_size * route.capacity, d_model))
                 expert_out = torch.stack(outs, dim=0)
-            combined = _Combine.apply(expert_out, route.gate, route, self.group, self.num_local_experts, self._heap_buffers)
+            combined = _Combine.apply(expert_out, route.gate, route, self.group, self.num_local_experts, self._heap_buffers, claims)
             return combined.reshape(x.shape)
 
         self.l_aux, combine_weights, dispatch_mask = self.gate(tokens)

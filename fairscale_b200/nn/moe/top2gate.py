@@ -55,7 +55,6 @@ class Top2Route(NamedTuple):
     capacity: int
     num_experts: int
     counts: Optional[Tensor] = None  # int32 [2 * E]: tokens per expert as first / second choice (CUDA index kernels only)
-    flat: Optional[Tensor] = None  # int32 [S, 2]: expert * C + slot, -1 for a dropped choice (CUDA index kernels only)
 
 
 def _route_indices_native(logits: Tensor, noise: Tensor) -> Optional[Tuple[Tensor, Tensor, Tensor, Tensor, Tensor]]:
@@ -79,21 +78,20 @@ def _route_indices_native(logits: Tensor, noise: Tensor) -> Optional[Tuple[Tenso
     return out, totals
 
 
-def _pack_route(route: Tensor, capacity: int) -> Tuple[Tensor, Tensor, Tensor, Tensor]:
-    """``expert``, ``slot`` (int64), ``keep`` (bool) and ``flat`` (int32), all ``[S, 2]``, from the index kernels' ``[4, S]``."""
+def _pack_route(route: Tensor, capacity: int) -> Tuple[Tensor, Tensor, Tensor]:
+    """``expert``, ``slot`` (int64) and ``keep`` (bool), all ``[S, 2]``, from the index kernels' ``[4, S]``."""
     from ctypes import c_int, c_void_p
 
     from ...ops import _bind
 
-    _bind._SIGNATURES.setdefault("fsb_moe_route_pack", [c_void_p, c_int, c_int] + [c_void_p] * 5)
+    _bind._SIGNATURES.setdefault("fsb_moe_route_pack", [c_void_p, c_int, c_int] + [c_void_p] * 4)
     S, dev = route.shape[1], route.device
     expert = torch.empty((S, 2), dtype=torch.int64, device=dev)
     slot = torch.empty((S, 2), dtype=torch.int64, device=dev)
     keep = torch.empty((S, 2), dtype=torch.bool, device=dev)
-    flat = torch.empty((S, 2), dtype=torch.int32, device=dev)
     _bind.call("fsb_moe_route_pack", route.data_ptr(), S, capacity, expert.data_ptr(), slot.data_ptr(), keep.data_ptr(),
-               flat.data_ptr(), _bind.stream_ptr(dev))
-    return expert, slot, keep, flat
+               _bind.stream_ptr(dev))
+    return expert, slot, keep
 
 
 class _GateValues(torch.autograd.Function):
@@ -158,8 +156,8 @@ def top2_route(logits: torch.Tensor, noise: Optional[Tensor] = None) -> Top2Rout
         route, counts2 = native
         count1 = counts2[:E]
         gate, l_aux = _GateValues.apply(logits, route, count1, capacity)
-        expert, slot, keep, flat = _pack_route(route, capacity)
-        return Top2Route(l_aux.to(logits.dtype), expert, slot, keep, gate, capacity, E, counts2, flat)
+        expert, slot, keep = _pack_route(route, capacity)
+        return Top2Route(l_aux.to(logits.dtype), expert, slot, keep, gate, capacity, E, counts2)
     gates = F.softmax(logits, dim=1, dtype=torch.float)
     idx1 = torch.argmax(gates, dim=1)
     noisy = (logits + noise).scatter(1, idx1.unsqueeze(1), float("-inf"))

@@ -134,6 +134,50 @@ def test_moe_rows_match_index_ops(S, E, M, dtype):
         torch.testing.assert_close(a.float(), b.float(), rtol=eps, atol=eps * b.float().abs().max().item())
 
 
+# a gate that changes what the routing kernels made: choices dropped out of place and in place, a smaller capacity
+@pytest.mark.parametrize("change", ["replace", "in_place", "capacity"])
+def test_moe_rows_follow_a_route_that_was_changed(change):
+    import torch.distributed as dist
+
+    from fairscale_b200.nn.moe import GroupedExperts, MOELayer, Top2Gate
+
+    if not dist.is_initialized():
+        dist.init_process_group("nccl", store=dist.HashStore(), rank=0, world_size=1)
+
+    class PickyGate(Top2Gate):
+        def route(self, x):
+            r = super().route(x)
+            if change == "capacity":
+                small = r.capacity // 2
+                return r._replace(capacity=small, keep=r.keep & (r.slot < small), slot=r.slot * (r.slot < small))
+            allowed = (torch.arange(r.keep.shape[0], device=r.keep.device) % 3 > 0).unsqueeze(1)
+            if change == "in_place":
+                r.keep.logical_and_(allowed)
+                return r
+            return r._replace(keep=r.keep & allowed)
+
+    torch.manual_seed(1)
+    S, E, M = 96, 4, 64
+    layer = MOELayer(PickyGate(M, E), GroupedExperts(E, M, 2 * M)).to(_dev()).to(torch.bfloat16)
+    seen = {}
+    layer.experts[0].register_forward_hook(lambda m, i, o: seen.update(rows=i[0].detach(), out=o))
+    x = torch.randn(1, S, M, device=_dev()).bfloat16().requires_grad_()
+    torch.full((64 << 20,), float("nan"), device=_dev())  # memory that the layer's buffers may be taken from
+    route = {}
+    inner = layer.gate.route
+    layer.gate.route = lambda t: route.setdefault("r", inner(t))
+    layer(x.view(E, S // E, M)).float().sum().backward()
+    r = route["r"]
+    want = torch.zeros(E * r.capacity, M, device=_dev(), dtype=torch.bfloat16)
+    for k in range(2):
+        kept = r.keep[:, k]
+        want[(r.expert * r.capacity + r.slot)[kept, k]] = x.detach().view(S, M)[kept]
+    assert torch.equal(seen["rows"].reshape(-1, M), want)
+    assert torch.isfinite(x.grad).all() and all(torch.isfinite(p.grad).all() for p in layer.parameters())
+    assert not r.keep.all()
+    _status_ok()
+
+
 # (M, N, K): below, at and above the 128 x 64 / 128 x 128 tiles, K of one block, K no multiple of a block, K with fewer
 # blocks than a cluster could split
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
