@@ -164,6 +164,11 @@ def _gather_local(buf: Tensor, flat: Tensor, w: Optional[Tensor], grad: Optional
     return out if dots is None else dots
 
 
+def _kept_rows(buf: Tensor, flat: Tensor) -> Tensor:
+    """``buf[flat[s, k]]`` as fp32 ``[S, 2, M]`` in torch operations, zero where ``flat`` is -1."""
+    return buf[flat.clamp(min=0).long()].float() * (flat >= 0).unsqueeze(-1)
+
+
 def _to_experts(rows: Tensor, group: Any, world: int, n_local: int, C: int) -> Tensor:
     """``[E * C, M]`` rows of this rank's tokens -> ``[n_local, world * C, M]`` rows of this rank's experts."""
     if world == 1:
@@ -228,6 +233,9 @@ class _Dispatch(torch.autograd.Function):
         group, n_local, world, rank, C, E, M, dtype = ctx.meta
         if ctx.local:
             (flat,) = ctx.saved_tensors
+            if torch.is_grad_enabled():  # create_graph: the gradient is linear in `grad`, and the graph has to know it
+                home = _to_tokens(grad.contiguous(), group, world, n_local, C)
+                return _kept_rows(home, flat).sum(1).to(grad.dtype), None, None, None, None, None
             return _gather_local(_to_tokens(grad.contiguous(), group, world, n_local, C), flat, None), None, None, None, None, None
         dst_rank, dst_row, flat, keep = ctx.saved_tensors
         S = dst_rank.shape[0]
@@ -295,6 +303,12 @@ class _Combine(torch.autograd.Function):
         if ctx.local:
             flat, claimed, w, home = ctx.saved_tensors
             dy = dy.to(home.dtype).contiguous()
+            if torch.is_grad_enabled():  # create_graph: as in the dispatch
+                dyf = dy.float().unsqueeze(1)
+                to = torch.where(flat >= 0, flat, E * C).long().view(-1)  # choices that were not kept go to a row that is cut off
+                d_rows = dyf.new_zeros((E * C + 1, M)).index_add(0, to, (dyf * w.unsqueeze(-1)).view(-1, M))[:-1].to(dy.dtype)
+                d_gate = (_kept_rows(home, flat) * dyf).sum(-1)
+                return _to_experts(d_rows, group, world, n_local, C), d_gate, None, None, None, None, None
             d_eo = _to_experts(_scatter_local(dy, flat, claimed, w), group, world, n_local, C)
             return d_eo, _gather_local(home, flat, None, grad=dy), None, None, None, None, None
         dst_rank, dst_row, flat, keep, w, saved = ctx.saved_tensors

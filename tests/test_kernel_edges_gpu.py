@@ -178,6 +178,34 @@ def test_moe_rows_follow_a_route_that_was_changed(change):
     _status_ok()
 
 
+def test_moe_row_gradients_can_be_differentiated():
+    """create_graph: what the CPU formulation offers (a gradient that is differentiable in the incoming one) holds on the GPU."""
+    import torch.distributed as dist
+
+    from fairscale_b200.nn.moe import top2gate
+    from fairscale_b200.nn.moe.moe_layer import _Combine, _Dispatch
+
+    if not dist.is_initialized():
+        dist.init_process_group("nccl", store=dist.HashStore(), rank=0, world_size=1)
+    torch.manual_seed(3)
+    S, E, M = 64, 4, 40
+    logits = torch.randn(S, E, device=_dev()) + torch.linspace(2, 0, E, device=_dev())
+    noise = top2gate.gumbel_rsample(logits.shape, logits.device)
+    x, dy = torch.randn(S, M, device=_dev()), torch.randn(S, M, device=_dev())
+    got = {}
+    for where, cast in (("gpu", lambda v: v.detach().clone()), ("cpu", lambda v: v.detach().cpu())):
+        xx, gg, dd = (cast(v).requires_grad_() for v in (x, logits, dy))
+        route = top2gate.top2_route(gg, cast(noise))
+        scale = cast(torch.arange(1.0, E + 1, device=_dev())).view(E, 1, 1)
+        out = _Combine.apply(_Dispatch.apply(xx, route, dist.group.WORLD, E) * scale, route.gate, route, dist.group.WORLD, E)
+        first = torch.autograd.grad(out, (xx, route.gate), dd, create_graph=True)
+        (second,) = torch.autograd.grad(sum(f.pow(2).sum() for f in first), dd)
+        got[where] = [v.detach().cpu() for v in (*first, second)]
+    _status_ok()
+    for a, b in zip(got["gpu"], got["cpu"]):
+        torch.testing.assert_close(a, b, rtol=1e-4, atol=1e-4 * b.abs().max().item())
+
+
 # (M, N, K): below, at and above the 128 x 64 / 128 x 128 tiles, K of one block, K no multiple of a block, K with fewer
 # blocks than a cluster could split
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
