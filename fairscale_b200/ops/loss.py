@@ -47,7 +47,9 @@ def ce_backward(logits: torch.Tensor, targets: torch.Tensor, lse: torch.Tensor, 
                 ignore_index: int = -100, vocab_start: int = 0, inplace: bool = True) -> torch.Tensor:
     """``(softmax - onehot) * grad_out * scale``; overwrites bf16 ``logits`` when ``inplace``."""
     rows, V = logits.shape
-    if not _native_takes(logits, targets):
+    # a caller that will differentiate the gradient again (create_graph) gets torch operations for fp32 logits
+    again = torch.is_grad_enabled() and logits.dtype == torch.float32 and (logits.requires_grad or grad_out.requires_grad)
+    if again or not _native_takes(logits, targets):
         p = torch.exp(logits.float() - lse.unsqueeze(1))
         local = targets - vocab_start
         inside = (local >= 0) & (local < V)

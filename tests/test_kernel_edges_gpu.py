@@ -495,3 +495,19 @@ def test_products_on_two_streams_and_in_a_graph_keep_their_tiles(M, N, K):
     for o in outs:
         assert torch.equal(o, want)
     _status_ok()
+
+
+def test_fp32_cross_entropy_gradient_can_be_differentiated():
+    """create_graph: fp32 logits, whose gradient is differentiable in the incoming one on the CPU, offer that on the GPU too."""
+    from fairscale_b200.ops.loss import ce_backward
+
+    torch.manual_seed(4)
+    x, t = torch.randn(64, 32, device=_dev()), torch.randint(0, 32, (64,), device=_dev())
+    lse, g = torch.logsumexp(x, -1), torch.rand(64, device=_dev())
+    got = {}
+    for where, cast in (("gpu", lambda v: v.detach().clone()), ("cpu", lambda v: v.detach().cpu())):
+        gg = cast(g).requires_grad_()
+        dx = ce_backward(cast(x), cast(t), cast(lse), gg, 1.0)
+        got[where] = [v.detach().cpu() for v in (dx, *torch.autograd.grad(dx.pow(2).sum(), gg))]
+    for a, b in zip(got["gpu"], got["cpu"]):
+        torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-6)
