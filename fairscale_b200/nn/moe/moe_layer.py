@@ -276,8 +276,15 @@ class _Combine(torch.autograd.Function):
             flat, claimed = (claims or _Claims(route)).rows()
             w = gate.to(torch.float32).contiguous()  # the kernels look at flat: a dropped choice's weight is not read
             home = _to_tokens(expert_out.contiguous(), group, world, n_local, C)
-            ctx.save_for_backward(flat, claimed, w, home)
-            return _gather_local(home, flat, w)
+            out = _gather_local(home, flat, w)
+            # the gates' gradient needs the rows once more; with one rank they are the experts' own output, which stays theirs to reuse
+            kept = home
+            if not ctx.needs_input_grad[1]:
+                kept = None
+            elif home.untyped_storage().data_ptr() == expert_out.untyped_storage().data_ptr():
+                kept = home.clone()
+            ctx.save_for_backward(flat, claimed, w, kept)
+            return out
         dst_rank, dst_row, flat = _routes(route, world, n_local, rank)
         S = dst_rank.shape[0]
         w = (gate * route.keep).to(torch.float32).contiguous()
@@ -302,15 +309,15 @@ class _Combine(torch.autograd.Function):
         group, n_local, world, rank, C, E, M = ctx.meta
         if ctx.local:
             flat, claimed, w, home = ctx.saved_tensors
-            dy = dy.to(home.dtype).contiguous()
+            dy = dy.contiguous()
             if torch.is_grad_enabled():  # create_graph: as in the dispatch
                 dyf = dy.float().unsqueeze(1)
                 to = torch.where(flat >= 0, flat, E * C).long().view(-1)  # choices that were not kept go to a row that is cut off
                 d_rows = dyf.new_zeros((E * C + 1, M)).index_add(0, to, (dyf * w.unsqueeze(-1)).view(-1, M))[:-1].to(dy.dtype)
-                d_gate = (_kept_rows(home, flat) * dyf).sum(-1)
+                d_gate = (_kept_rows(home, flat) * dyf).sum(-1) if home is not None else None
                 return _to_experts(d_rows, group, world, n_local, C), d_gate, None, None, None, None, None
             d_eo = _to_experts(_scatter_local(dy, flat, claimed, w), group, world, n_local, C)
-            return d_eo, _gather_local(home, flat, None, grad=dy), None, None, None, None, None
+            return d_eo, _gather_local(home, flat, None, grad=dy) if home is not None else None, None, None, None, None, None
         dst_rank, dst_row, flat, keep, w, saved = ctx.saved_tensors
         S = dst_rank.shape[0]
         dy = dy.contiguous()

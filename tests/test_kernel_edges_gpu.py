@@ -206,6 +206,58 @@ def test_moe_row_gradients_can_be_differentiated():
         torch.testing.assert_close(a, b, rtol=1e-4, atol=1e-4 * b.abs().max().item())
 
 
+def test_moe_experts_may_reuse_their_output_buffer():
+    """The layer keeps no hold on the experts' output: a second forward may overwrite it before the first one's backward."""
+    import torch.distributed as dist
+
+    from fairscale_b200.nn.moe import MOELayer, Top2Gate
+
+    if not dist.is_initialized():
+        dist.init_process_group("nccl", store=dist.HashStore(), rank=0, world_size=1)
+    S, E, M = 64, 4, 32
+
+    class Scale(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, x, scale, buf):
+            ctx.scale = scale
+            out = torch.empty_like(x) if buf is None else buf
+            return torch.mul(x, scale, out=out.view(x.shape)).view(x.shape)
+
+        @staticmethod
+        def backward(ctx, g):
+            return g * ctx.scale, None, None
+
+    class Experts(torch.nn.Module):
+        grouped = True
+
+        def __init__(self, buf):
+            super().__init__()
+            self.buf, self.scale = buf, torch.arange(1.0, E + 1, device=_dev()).view(E, 1, 1)
+
+        def __len__(self):
+            return E
+
+        def forward(self, x):
+            return Scale.apply(x, self.scale, self.buf)
+
+    torch.manual_seed(5)
+    x1, x2 = (torch.randn(E, S // E, M, device=_dev()) for _ in range(2))
+    gate = Top2Gate(M, E).to(_dev())
+    grads = []
+    for buf in (None, torch.empty(E, 2 * S // E, M, device=_dev())):
+        layer = MOELayer(gate, Experts(buf))
+        x = x1.clone().requires_grad_()
+        gate.zero_grad()
+        torch.manual_seed(6)  # the gate's noise
+        y = layer(x)
+        layer(x2)
+        y.pow(2).sum().backward()
+        grads.append((x.grad, gate.wg.weight.grad.clone()))
+    _status_ok()
+    for a, b in zip(*grads):
+        torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-5)
+
+
 # (M, N, K): below, at and above the 128 x 64 / 128 x 128 tiles, K of one block, K no multiple of a block, K with fewer
 # blocks than a cluster could split
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
