@@ -22,7 +22,7 @@ from ..ops.embedding import embedding
 from ..ops.gemm import linear
 from ..ops.loss import cross_entropy
 from ..ops.mlp import mlp
-from ..ops.norm import LayerNorm
+from ..ops.norm import LayerNorm, norm_and_residual
 
 
 @dataclass
@@ -92,11 +92,11 @@ class Block(nn.Module):
             nn.init.normal_(w, 0.0, cfg.init_std)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        h, x = self.ln1(x, with_residual=True)
+        h, x = norm_and_residual(self.ln1, x)
         qkv = linear(h, self.qkv_w, self.qkv_b)
         a = causal_attention(qkv, self.n_heads)
         x = linear(a, self.proj_w, self.proj_b, residual=x)
-        h, x = self.ln2(x, with_residual=True)
+        h, x = norm_and_residual(self.ln2, x)
         return mlp(h, self.fc1_w, self.fc1_b, self.fc2_w, self.fc2_b, residual=x)
 
 

@@ -29,7 +29,7 @@ from ..nn.model_parallel import (
 )
 from ..ops.activations import swiglu
 from ..ops.attention import causal_attention
-from ..ops.norm import RMSNorm
+from ..ops.norm import RMSNorm, norm_and_residual
 from ..ops.rope import rope_qkv
 from ..parallel import comm
 
@@ -110,13 +110,13 @@ class TPBlock(nn.Module):
 
     def forward(self, x: torch.Tensor, batch: int) -> torch.Tensor:  # x: [T / world, D], rows in (batch, seq) order
         cfg = self.cfg
-        h, x = self.norm1(x, with_residual=True)
+        h, x = norm_and_residual(self.norm1, x)
         qkv = self.qkv(h)  # [T, 3 * D / world]
         S = qkv.shape[0] // batch
         qkv = rope_qkv(qkv.view(batch, S, 3, self.local_heads, cfg.d_model // cfg.n_heads), cfg.rope_theta)
         o = causal_attention(qkv.reshape(batch, S, -1), self.local_heads)
         x = x + self.proj(o.reshape(batch * S, -1))
-        h, x = self.norm2(x, with_residual=True)
+        h, x = norm_and_residual(self.norm2, x)
         return x + self.down(swiglu(self.gate_up(h)))
 
 

@@ -6,6 +6,7 @@ from typing import Any, Optional, Tuple
 
 import torch
 from torch import nn
+from torch.nn.modules.module import _has_any_global_hook
 
 from . import _bind
 from .gemm import grad_slot_info, grad_window
@@ -120,14 +121,6 @@ class _NormResidualFn(torch.autograd.Function):
         return dx, dw, db, None, None
 
 
-def norm_and_residual(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], eps: float, rms: bool
-                      ) -> Tuple[torch.Tensor, torch.Tensor]:
-    """``norm(x)`` and ``x`` itself for the residual branch that goes past it."""
-    if _bind.no_graph():
-        return norm_forward(x, weight, bias, eps, rms)[0], x
-    return _NormResidualFn.apply(x, weight, bias, eps, rms)
-
-
 def layer_norm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], eps: float = 1e-5) -> torch.Tensor:
     if _bind.no_graph():
         return norm_forward(x, weight, bias, eps, False)[0]
@@ -149,10 +142,7 @@ class LayerNorm(nn.Module):
         self.bias = nn.Parameter(torch.zeros(hidden)) if bias else None
         self.eps = eps
 
-    def forward(self, x: torch.Tensor, with_residual: bool = False) -> Any:
-        """``with_residual``: also return ``x``, for the branch past the norm (see :func:`norm_and_residual`)."""
-        if with_residual:
-            return norm_and_residual(x, self.weight, self.bias, self.eps, False)
+    def forward(self, x: torch.Tensor) -> torch.Tensor:
         return layer_norm(x, self.weight, self.bias, self.eps)
 
 
@@ -162,7 +152,21 @@ class RMSNorm(nn.Module):
         self.weight = nn.Parameter(torch.ones(hidden))
         self.eps = eps
 
-    def forward(self, x: torch.Tensor, with_residual: bool = False) -> Any:
-        if with_residual:
-            return norm_and_residual(x, self.weight, None, self.eps, True)
+    def forward(self, x: torch.Tensor) -> torch.Tensor:
         return rms_norm(x, self.weight, self.eps)
+
+
+def _plain_call(module: nn.Module) -> bool:
+    """Would calling ``module`` do nothing but run the class's own ``forward``?"""
+    hooks = (module._forward_hooks, module._forward_pre_hooks, module._backward_hooks, module._backward_pre_hooks)
+    return not (any(hooks) or _has_any_global_hook() or "forward" in module.__dict__ or getattr(module, "_compiled_call_impl", None) is not None)
+
+
+def norm_and_residual(norm: nn.Module, x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+    """``norm(x)``, and ``x`` for the residual branch that goes past it.  The two are one autograd node where ``norm`` is one of
+    this file's and calling it would only run its ``forward``, and where ``x`` has a gradient to add up; any other module that
+    stands in a norm's place, or one with hooks, is simply called."""
+    if torch.is_grad_enabled() and x.requires_grad and type(norm) in (LayerNorm, RMSNorm) and _plain_call(norm):
+        rms = type(norm) is RMSNorm
+        return _NormResidualFn.apply(x, norm.weight, None if rms else norm.bias, norm.eps, rms)
+    return norm(x), x
