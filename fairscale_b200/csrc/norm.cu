@@ -457,8 +457,12 @@ FSB_API int fsb_norm_bwd_num_strips(long long rows) {
 FSB_API int fsb_norm_bwd_res(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd, const void* res, void* dx,
                              void* dgamma, void* dbeta, float* partials, long long rows, int H, int rms, cudaStream_t stream) {
   using namespace fsb;
-  if (rows <= 0) return 0;
   if (H % 8 != 0 || H > 8 * NORM_THREADS * NORM_MAX_VEC) return -1;
+  if (rows <= 0) {  // an empty sum is zero, and the outputs may be windows of a gradient that is used as it stands
+    cudaError_t e = cudaMemsetAsync(dgamma, 0, static_cast<size_t>(H) * 2, stream);
+    if (e == cudaSuccess && !rms && dbeta != nullptr) e = cudaMemsetAsync(dbeta, 0, static_cast<size_t>(H) * 2, stream);
+    return static_cast<int>(e);
+  }
   const bool fused = H <= NORM_ROWS_MAX_H;
   const int strips = fused ? norm_bwd_rows_ctas(rows) : norm_bwd_split_strips(rows);
   float* pg = partials;

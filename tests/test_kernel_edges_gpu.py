@@ -563,3 +563,26 @@ def test_fp32_cross_entropy_gradient_can_be_differentiated():
         got[where] = [v.detach().cpu() for v in (dx, *torch.autograd.grad(dx.pow(2).sum(), gg))]
     for a, b in zip(got["gpu"], got["cpu"]):
         torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("rms", [False, True])
+def test_norm_gradients_of_no_rows_are_zero(rms):
+    """Also where they are windows of a flat gradient, which is used as it stands."""
+    from fairscale_b200.nn.misc.flatten_params_wrapper import GradArena
+    from fairscale_b200.ops import norm
+
+    H = 64
+    x = torch.empty(0, H, device=_dev(), dtype=torch.bfloat16)
+    w = torch.ones(H, device=_dev(), dtype=torch.bfloat16)
+    b = None if rms else torch.zeros_like(w)
+    y, mean, rstd = norm.norm_forward(x, w, b, 1e-5, rms)
+    assert y.shape == x.shape
+    arena = GradArena(2 * H)
+    arena.buffer = torch.full((2 * H,), float("nan"), device=_dev(), dtype=torch.bfloat16)
+    windows = ((arena, 0, w.shape), (arena, H, w.shape))
+    for slots in ((None, None), windows):
+        torch.full((1 << 20,), float("nan"), device=_dev())  # memory that the results may be taken from
+        dx, dw, db = norm.norm_backward(x, x, w, mean, rstd, rms, not rms, slots)
+        assert dx.shape == x.shape and not dw.any() and (rms or not db.any())
+    assert not arena.buffer[: H if rms else 2 * H].any()
+    _status_ok()
