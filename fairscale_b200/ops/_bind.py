@@ -82,6 +82,13 @@ def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
 
+def dense16(t: torch.Tensor) -> torch.Tensor:
+    """``t`` contiguous and starting on a 16-byte boundary, as kernels with 16-byte accesses and TMA tensor maps need it (a view
+    may start at any element)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def _device_index(device: Any) -> int:
     index = device.index if isinstance(device, torch.device) else (device if isinstance(device, int) else None)
     if index is None:

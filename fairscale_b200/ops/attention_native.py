@@ -21,19 +21,13 @@ def _bind_sigs() -> None:
     _BOUND = True
 
 
-def _tma_operand(t: torch.Tensor) -> torch.Tensor:
-    """``t`` contiguous and starting on the 16-byte boundary that a TMA tensor map needs (a view may start anywhere)."""
-    t = t.contiguous()
-    return t if t.data_ptr() % 16 == 0 else t.clone()
-
-
 class _FlashAttnFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, qkv: torch.Tensor, n_heads: int, scale: float):  # type: ignore[override]
         _bind_sigs()
         B, S, three_hd = qkv.shape
         D = three_hd // (3 * n_heads)
-        qkv = _tma_operand(qkv)
+        qkv = _bind.dense16(qkv)
         o = torch.empty((B, S, n_heads * D), dtype=qkv.dtype, device=qkv.device)
         lse = torch.empty((B, n_heads, S), dtype=torch.float32, device=qkv.device)
         _bind.call("fsb_attn_fwd", qkv.data_ptr(), o.data_ptr(), lse.data_ptr(), B, S, n_heads, D, scale,
@@ -48,7 +42,7 @@ class _FlashAttnFn(torch.autograd.Function):
         B, S, three_hd = qkv.shape
         H = ctx.n_heads
         D = three_hd // (3 * H)
-        d_o = _tma_operand(d_o)
+        d_o = _bind.dense16(d_o)
         dqkv = torch.empty_like(qkv)
         S_pad = (S + 127) // 128 * 128
         delta = torch.empty((2, B, H, S_pad), dtype=torch.float32, device=lse.device)  # scale*delta, then base-2 lse

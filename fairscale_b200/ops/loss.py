@@ -10,13 +10,12 @@ from . import _bind
 
 
 def _native_takes(logits: torch.Tensor, targets: torch.Tensor) -> bool:
-    """bf16 or dense fp32 rows that start on 16-byte boundaries, int64 targets beside them."""
-    if not _bind.use_native(logits):
+    """Rows of bf16, or dense ones of fp32, that start on 16-byte boundaries; int64 targets beside them."""
+    if not _bind.use_native(logits, targets) or targets.dtype != torch.int64 or not targets.is_contiguous() or logits.data_ptr() % 16:
         return False
     if logits.dtype == torch.bfloat16:
-        return logits.stride(0) % 8 == 0
-    return (logits.dtype == torch.float32 and logits.is_contiguous() and logits.shape[1] % 4 == 0 and logits.data_ptr() % 16 == 0
-            and targets.is_cuda and targets.dtype == torch.int64 and targets.is_contiguous())
+        return logits.stride(0) % 8 == 0 and logits.stride(1) == 1
+    return logits.dtype == torch.float32 and logits.is_contiguous() and logits.shape[1] % 4 == 0
 
 
 def ce_forward(logits: torch.Tensor, targets: torch.Tensor, ignore_index: int = -100, vocab_start: int = 0,

@@ -33,7 +33,8 @@ def norm_forward(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Ten
             if bias is not None:
                 y = y + bias.float()
         return y.to(x.dtype), mean, rstd
-    x2 = x.contiguous().view(-1, H)
+    x2, weight = _bind.dense16(x).view(-1, H), _bind.dense16(weight)
+    bias = None if bias is None else _bind.dense16(bias)
     rows = x2.shape[0]
     y = torch.empty_like(x2)
     mean = None if rms else torch.empty(rows, dtype=torch.float32, device=x.device)
@@ -61,7 +62,7 @@ def norm_backward(dy: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, mean:
         if residual is not None:
             dx = dx + residual.float()
         return dx.to(x.dtype), dw.to(weight.dtype), None if db is None else db.to(weight.dtype)
-    x2, dy2 = x.contiguous().view(-1, H), dy.contiguous().view(-1, H)
+    x2, dy2, weight = _bind.dense16(x).view(-1, H), _bind.dense16(dy).view(-1, H), _bind.dense16(weight)
     rows = x2.shape[0]
     strips = _bind.fn("fsb_norm_bwd_num_strips")(rows)
     partials = torch.empty((2, strips, H), dtype=torch.float32, device=x.device)
@@ -74,7 +75,7 @@ def norm_backward(dy: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, mean:
         db = grad_window(slots[1], weight.dtype, x.device)
         if db is None:
             db = torch.empty(H, dtype=torch.bfloat16, device=x.device)
-    res2 = None if residual is None else residual.contiguous().view(-1, H)
+    res2 = None if residual is None else _bind.dense16(residual).view(-1, H)
     _bind.call("fsb_norm_bwd_res", dy2.data_ptr(), x2.data_ptr(), weight.data_ptr(), _bind.ptr(mean), rstd.data_ptr(), _bind.ptr(res2), dx.data_ptr(),
                dw.data_ptr(), _bind.ptr(db), partials.data_ptr(), rows, H, int(rms), _bind.stream_ptr(x.device),
                launches=2 if H <= 4096 else 3)

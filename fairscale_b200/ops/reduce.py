@@ -16,7 +16,7 @@ def column_sum(x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Ten
     rows, H = x2.shape
     if not _bind.use_native(x2) or x2.dtype != torch.bfloat16 or H % 8 or rows == 0:
         return x2.float().sum(0).to(x.dtype)
-    x2 = x2.contiguous()
+    x2 = _bind.dense16(x2)
     strips = _bind.fn("fsb_colsum_num_strips")(rows)
     partials = torch.empty((strips, H), dtype=torch.float32, device=x.device)
     if out is None:
@@ -30,9 +30,7 @@ def batched_column_sum(x: torch.Tensor) -> torch.Tensor:
     E, rows, H = x.shape
     if not _bind.use_native(x) or x.dtype != torch.bfloat16 or H % 8 or rows == 0:
         return x.float().sum(1).to(x.dtype)
-    x = x.contiguous()
-    if x.data_ptr() % 16:  # the kernel reads 16 bytes at a time
-        x = x.clone()
+    x = _bind.dense16(x)
     strips = _bind.fn("fsb_colsum_num_strips")(rows)
     partials = torch.empty((E, strips, H), dtype=torch.float32, device=x.device)
     out = torch.empty((E, H), dtype=torch.bfloat16, device=x.device)

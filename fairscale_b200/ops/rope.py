@@ -29,7 +29,7 @@ def _rope_apply(qkv: torch.Tensor, theta: float, backward: bool, pos_offset: int
     assert three == 3
     if not _bind.use_native(qkv) or qkv.dtype != torch.bfloat16 or D % 8:
         return rope_reference(qkv, theta, backward, pos_offset)
-    qkv = qkv.contiguous()
+    qkv = _bind.dense16(qkv)
     out = torch.empty_like(qkv)
     _bind.call("fsb_rope", qkv.data_ptr(), out.data_ptr(), B, S, H, D, float(theta), int(backward), int(pos_offset),
                _bind.stream_ptr(qkv.device))

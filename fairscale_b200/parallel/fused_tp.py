@@ -382,7 +382,7 @@ class _LinearReduceScatter(torch.autograd.Function):
             dx, gathered = ag_gemm(ws, dout, w, None, w_is_kn=True)  # dX = all_gather(dOut) @ W
         else:
             # with one rank the rows are all here (the forward's gather copies even then: its input stays the caller's to change)
-            gathered = dout if comm.group_size(ctx.group) == 1 else _all_gather_rows(dout, ctx.group)
+            gathered = _bind.dense16(dout) if comm.group_size(ctx.group) == 1 else _all_gather_rows(dout, ctx.group)
             dx = gathered @ w if ctx.needs_input_grad[0] else None
         if ctx.needs_input_grad[1]:
             dw = gemm_ops.linear_wgrad(gathered, x).to(w.dtype)

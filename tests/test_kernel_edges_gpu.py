@@ -586,3 +586,65 @@ def test_norm_gradients_of_no_rows_are_zero(rms):
         assert dx.shape == x.shape and not dw.any() and (rms or not db.any())
     assert not arena.buffer[: H if rms else 2 * H].any()
     _status_ok()
+
+
+def _off(t):
+    """The same values in a contiguous view that starts two bytes (fp32: four) after a 16-byte boundary."""
+    flat = torch.empty(t.numel() + 8, dtype=t.dtype, device=t.device)
+    view = flat[1 : 1 + t.numel()].view(t.shape)
+    view.copy_(t)
+    assert view.data_ptr() % 16 != 0 and view.is_contiguous()
+    return view
+
+
+def test_views_that_start_off_a_16_byte_boundary():
+    """The wrappers hand kernels with 16-byte accesses a copy; results are those of aligned tensors."""
+    import torch.distributed as dist
+
+    from fairscale_b200.ops import norm
+    from fairscale_b200.ops.attention import causal_attention
+    from fairscale_b200.ops.loss import ce_backward, ce_forward
+    from fairscale_b200.ops.reduce import batched_column_sum, column_sum
+    from fairscale_b200.ops.rope import rope_qkv
+    from fairscale_b200.parallel.fused_tp import _LinearReduceScatter
+
+    if not dist.is_initialized():
+        dist.init_process_group("nccl", store=dist.HashStore(), rank=0, world_size=1)
+    torch.manual_seed(7)
+
+    def randn(*shape):
+        return torch.randn(*shape, device=_dev()).bfloat16()
+
+    def both(f, *args):
+        want, got = f(*args), f(*(_off(a) for a in args))
+        for w, g in zip(want, got):
+            assert torch.equal(w, g)
+
+    def norms(x, dy, w, b, res):
+        out = []
+        for rms, bias in ((False, b), (True, None)):
+            y, mean, rstd = norm.norm_forward(x, w, bias, 1e-5, rms)
+            out += [y, *(t for t in norm.norm_backward(dy, x, w, mean, rstd, rms, not rms, residual=res) if t is not None)]
+        return out
+
+    for H in (256, 4104):
+        both(norms, randn(5, H), randn(5, H), randn(H), randn(H), randn(5, H))
+    both(lambda x: [column_sum(x)], randn(70, 264))
+    both(lambda x: [batched_column_sum(x)], randn(3, 70, 264))
+    both(lambda x: [rope_qkv(x)], randn(2, 5, 3, 2, 64))
+    both(lambda x: [causal_attention(x, 2)], randn(1, 128, 3 * 2 * 64))
+    x, w, g = randn(64, 128), randn(256, 128), randn(64, 256)
+
+    def row_parallel(gg):
+        xx, ww = x.clone().requires_grad_(), w.clone().requires_grad_()
+        return torch.autograd.grad(_LinearReduceScatter.apply(xx, ww, None, dist.group.WORLD), (xx, ww), gg)
+
+    both(row_parallel, g)
+    t = torch.randint(0, 512, (9,), device=_dev())
+    for dtype in (torch.bfloat16, torch.float32):
+        logits = torch.randn(9, 512, device=_dev()).to(dtype)
+        lse = ce_forward(logits, t)[1]
+        torch.testing.assert_close(ce_forward(_off(logits), t)[1], lse, rtol=1e-4, atol=1e-4)
+        up = torch.rand(9, device=_dev())
+        torch.testing.assert_close(ce_backward(_off(logits), t, lse, up, 1.0), ce_backward(logits.clone(), t, lse, up, 1.0), rtol=1e-2, atol=1e-4)
+    _status_ok()
