@@ -97,7 +97,8 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, 
 template <int BLOCK_N>
 __device__ __forceinline__ void epilogue_rows(uint32_t t_base, int row, int n0, const GemmParams& p) {
   const bool row_ok = row < p.M;
-  const bool vec_ok = (p.ldc % 8 == 0) && (p.ld_aux % 8 == 0);
+  const uintptr_t ptrs = reinterpret_cast<uintptr_t>(p.C) | reinterpret_cast<uintptr_t>(p.aux) | reinterpret_cast<uintptr_t>(p.aux_out);
+  const bool vec_ok = (p.ldc % 8 == 0) && (p.ld_aux % 8 == 0) && (ptrs & 15u) == 0;  // 16-byte accesses
 #pragma unroll 1
   for (int c = 0; c < BLOCK_N / 32; ++c) {
     uint32_t r[32];
@@ -158,7 +159,7 @@ __device__ __forceinline__ void epilogue_rows(uint32_t t_base, int row, int n0, 
       float* pc = reinterpret_cast<float*>(p.C) + static_cast<size_t>(row) * p.ldc + col0;
       if (p.accumulate_c) {
         for (int i = 0; i < 32 && col0 + i < p.N; ++i) pc[i] += v[i];
-      } else if (col0 + 32 <= p.N && (p.ldc % 4 == 0)) {
+      } else if (col0 + 32 <= p.N && (p.ldc % 4 == 0) && (reinterpret_cast<uintptr_t>(p.C) & 15u) == 0) {
 #pragma unroll
         for (int q = 0; q < 8; ++q)
           *reinterpret_cast<float4*>(pc + q * 4) = make_float4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);

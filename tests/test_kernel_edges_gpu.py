@@ -648,3 +648,25 @@ def test_views_that_start_off_a_16_byte_boundary():
         up = torch.rand(9, device=_dev())
         torch.testing.assert_close(ce_backward(_off(logits), t, lse, up, 1.0), ce_backward(logits.clone(), t, lse, up, 1.0), rtol=1e-2, atol=1e-4)
     _status_ok()
+
+
+# few tiles (split over K), one CTA per tile; CTA pairs share the code of the latter
+@pytest.mark.parametrize("M,N,K", [(136, 264, 512), (2600, 2056, 128)])
+def test_gemm_outputs_and_epilogue_operands_at_any_element(M, N, K):
+    from fairscale_b200.ops.gemm import EPI_BIAS_GELU, EPI_BIAS_RESIDUAL, EPI_DGELU, EPI_RESIDUAL, _launch
+
+    torch.manual_seed(M)
+    a, b, aux = (torch.randn(*s, device=_dev()).bfloat16() for s in ((M, K), (N, K), (M, N)))
+    bias = torch.randn(N, device=_dev()).bfloat16()
+
+    def run(place, epi=0, dtype=torch.bfloat16, use_aux=False, pre=False, accumulate=False):
+        c = place(torch.ones(M, N, device=_dev(), dtype=dtype))
+        out = place(torch.zeros(M, N, device=_dev(), dtype=torch.bfloat16)) if pre else None
+        _launch(a, b, c, M, N, K, False, False, epi, bias=place(bias), aux=place(aux) if use_aux else None, aux_out=out, accumulate=accumulate)
+        return [t for t in (c, out) if t is not None]
+
+    for kw in (dict(), dict(dtype=torch.float32), dict(dtype=torch.float32, accumulate=True), dict(epi=EPI_BIAS_GELU, pre=True),
+               dict(epi=EPI_BIAS_RESIDUAL, use_aux=True), dict(epi=EPI_DGELU, use_aux=True), dict(epi=EPI_RESIDUAL, use_aux=True)):
+        for want, got in zip(run(lambda t: t, **kw), run(_off, **kw)):
+            assert torch.equal(want, got), kw
+    _status_ok()
