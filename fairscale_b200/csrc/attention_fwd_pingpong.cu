@@ -43,6 +43,8 @@
 
 #include "sm100.cuh"
 
+#include <cfloat>
+
 namespace fsb {
 namespace pp {
 
@@ -325,6 +327,9 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
     const uint32_t tp = tmem_base + P_COL + t * P_STEP + lane_off;         // probabilities (columns [0, 64) of the scores unless SEP)
     const uint32_t to = tmem_base + O_COL + t * O_STEP + lane_off;         // output accumulator
     const float sl2 = p.scale * LOG2E;
+    // The running maximum starts at the lowest value that stays finite when scaled, not at -inf: a row whose keys so far all
+    // score -inf then has probabilities 2^(-inf) = 0, where -inf - -inf would be NaN.
+    const float m_low = sl2 > 1.f ? -FLT_MAX / sl2 : -FLT_MAX;
     uint32_t cs = 0;  // steps of this tile so far, over all items (phase of s_full / o_done)
     bool ok = true;
     for (int r = 0, item; ok && (item = snake_item(r)) < n_items; ++r) {
@@ -336,7 +341,7 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
       const int pos = q2 * 2 * BM + t * BM + row;  // this thread's position in the sequence
       const bool row_ok = pos < p.S;
       const bool traced = (item == static_cast<int>(blockIdx.x)) && quad == 2;
-      float m_run = -INFINITY, l_run = 0.f;
+      float m_run = m_low, l_run = 0.f;
       for (int j = 0; j < n_it && ok; ++j, ++cs) {
         if (!mbar_wait(&bars->s_full[t], cs & 1u, abort_flag)) { ok = false; break; }
         tc_fence_after_sync();
@@ -357,8 +362,8 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
         else       { mx = chunk_max<true>(r0, 64, row, mx);  mx = chunk_max<true>(r1, 96, row, mx); }
         // keep the old maximum while the new one is at most 2^8 above it: no rescaling of O, values stay in range
         float m_new = fmaxf(m_run, mx);
-        if (m_run != -INFINITY && (m_new - m_run) * sl2 <= 8.f) m_new = m_run;
-        const float alpha = (m_run == -INFINITY) ? 0.f : ex2_approx((m_run - m_new) * sl2);
+        if (j > 0 && (m_new - m_run) * sl2 <= 8.f) m_new = m_run;
+        const float alpha = j == 0 ? 0.f : ex2_approx((m_run - m_new) * sl2);
         const float mb = m_new * sl2;
         if (traced) { PP_TRACE(1 + t, j, 1); }
         const bool rescale = j > 0 && __any_sync(0xffffffffu, alpha != 1.f);

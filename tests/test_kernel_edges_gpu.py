@@ -101,6 +101,39 @@ def test_attention_ragged_infinities_stay_where_they_are():
     assert torch.equal(a[0, :140], causal_attention(y, 1)[0, :140])
 
 
+@pytest.mark.parametrize("S,D", [(300, 64), (300, 128), (512, 64), (512, 128)])
+def test_attention_rows_whose_first_keys_score_minus_infinity(S, D):
+    """A whole first key tile at -inf leaves the later keys as they are."""
+    from fairscale_b200.ops.attention import causal_attention
+
+    torch.manual_seed(S + D)
+    H = 2
+    x = torch.randn(2, S, 3, H, D, device=_dev()).bfloat16()
+    x[:, :, 0, :, 0] = 1.0
+    x[:, :128, 1, :, 0] = float("-inf")
+    x = x.view(2, S, 3 * H * D)
+    o, ref = causal_attention(x, H), _attention_ref(x.float(), H)
+    _status_ok()
+    assert torch.isfinite(ref[:, 128:]).all() and torch.isfinite(o[:, 128:]).all()
+    assert _rel_err(o[:, 128:], ref[:, 128:]) < 2e-2
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_attention_scales_of_either_sign(D):
+    """A scale that is zero or negative is taken at multiples of 128, as it always was."""
+    from fairscale_b200.ops.attention import causal_attention
+
+    torch.manual_seed(D)
+    H = 2
+    x = torch.randn(1, 384, 3, H, D, device=_dev()).bfloat16()
+    for scale in (-1.0, 0.0, 1.0):
+        y = x.clone()
+        y[:, :, 0] *= scale
+        want = _attention_ref(y.view(1, 384, -1).float(), H)
+        assert _rel_err(causal_attention(x.view(1, 384, -1), H, scale / math.sqrt(D)), want) < 2e-2
+    _status_ok()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("S,E,M", [(64, 4, 1024), (820, 4, 512), (48, 16, 33), (8, 2, 8)])
 def test_moe_rows_match_index_ops(S, E, M, dtype):
