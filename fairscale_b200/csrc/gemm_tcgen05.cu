@@ -755,7 +755,7 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* bia
                           int epilogue, int out_f32, int accumulate_c, int max_ctas, int* status, cudaStream_t stream,
                           const unsigned int* b_ready, unsigned int b_ready_epoch, long long b_piece_bytes, unsigned long long b_wait_ns,
                           const unsigned int* a_ready = nullptr, int a_shard_rows = 0, int a_piece_rows = 0, int a_first_shard = 0,
-                          int a_num_shards = 0, int b_first_piece = 0, int ck_block_n = 0, int ck_splits = 0);
+                          int a_num_shards = 0, int b_first_piece = 0, int ck_block_n = 0, int ck_splits = 0, int forced = 0);
 
 FSB_API int fsb_gemm_bf16(const void* A, const void* B, void* C, const void* bias, const void* aux, void* aux_out,
                           int M, int N, int K, int lda, int ldb, int ldc, int ld_aux, int a_mn_major, int b_mn_major,
@@ -772,6 +772,16 @@ FSB_API int fsb_gemm_bf16_cluster_k(const void* A, const void* B, void* C, const
   if (splits < 1) return -1;
   return gemm_bf16_impl(A, B, C, bias, aux, aux_out, M, N, K, lda, ldb, ldc, ld_aux, a_mn_major, b_mn_major, epilogue, out_f32,
                         accumulate_c, 0, status, stream, nullptr, 0u, 0, 0ull, nullptr, 0, 0, 0, 0, 0, block_n, splits);
+}
+
+// The same product by one of the persistent kernels whatever its size: plan 1 one CTA per tile, 2 CTA pairs (M and N at
+// least 256, -1 otherwise).  fsb_gemm_bf16 chooses these by itself.
+FSB_API int fsb_gemm_bf16_plan(const void* A, const void* B, void* C, const void* bias, const void* aux, void* aux_out,
+                               int M, int N, int K, int lda, int ldb, int ldc, int ld_aux, int a_mn_major, int b_mn_major,
+                               int epilogue, int out_f32, int accumulate_c, int plan, int* status, cudaStream_t stream) {
+  if (plan != 1 && !(plan == 2 && M >= 256 && N >= 256)) return -1;
+  return gemm_bf16_impl(A, B, C, bias, aux, aux_out, M, N, K, lda, ldb, ldc, ld_aux, a_mn_major, b_mn_major, epilogue, out_f32,
+                        accumulate_c, 0, status, stream, nullptr, 0u, 0, 0ull, nullptr, 0, 0, 0, 0, 0, 0, 0, plan);
 }
 
 // C[M, N] = epilogue(A[M, K] * B^T + bias) with B ([N, K], rows contiguous: ldb == K) arriving while the kernel runs:
@@ -808,7 +818,7 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* bia
                           int epilogue, int out_f32, int accumulate_c, int max_ctas, int* status, cudaStream_t stream,
                           const unsigned int* b_ready, unsigned int b_ready_epoch, long long b_piece_bytes, unsigned long long b_wait_ns,
                           const unsigned int* a_ready, int a_shard_rows, int a_piece_rows, int a_first_shard, int a_num_shards,
-                          int b_first_piece, int ck_block_n, int ck_splits) {
+                          int b_first_piece, int ck_block_n, int ck_splits, int forced) {
   using namespace fsb;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) % 16) || (reinterpret_cast<uintptr_t>(B) % 16)) return -1;
@@ -858,6 +868,7 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* bia
   const bool streamed = b_ready != nullptr || a_ready != nullptr;  // only the pair kernel waits for arriving operands
   GemmPlan plan = {GemmPlan::ONE_CTA, block_n, 1};
   if (streamed) plan.kind = GemmPlan::PAIR;
+  else if (forced != 0) plan.kind = forced == 2 ? GemmPlan::PAIR : GemmPlan::ONE_CTA;
   else if (max_ctas == 0) plan = choose_gemm_plan(M, N, K, num_sms, pair_enabled());
   if (plan.kind == GemmPlan::CLUSTER_K) return fsb_host::gemm_cluster_k(ta, B, ldb, p, plan.block_n, plan.splits, dev, stream);
   // Run-time tile hand-out for products large enough to share the device with a collective; small ones stride.
@@ -899,10 +910,10 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* bia
 // stride_*: elements between consecutive problems (stride_bias may be 0 for a shared bias).  Layout flags, leading
 // dimensions and epilogues as for fsb_gemm_bf16.  Rows of a problem never leak into the next one: the tensor maps are
 // three-dimensional, so a tile that overhangs M or N reads zeros.
-FSB_API int fsb_gemm_bf16_batched(const void* A, const void* B, void* C, const void* bias, const void* aux, void* aux_out, int batch,
+static int gemm_bf16_batched_impl(const void* A, const void* B, void* C, const void* bias, const void* aux, void* aux_out, int batch,
                                   int M, int N, int K, int lda, int ldb, int ldc, int ld_aux, long long stride_a, long long stride_b,
                                   long long stride_c, long long stride_aux, long long stride_bias, int a_mn_major, int b_mn_major,
-                                  int epilogue, int out_f32, int accumulate_c, int* status, cudaStream_t stream) {
+                                  int epilogue, int out_f32, int accumulate_c, int* status, cudaStream_t stream, int forced) {
   using namespace fsb;
   if (batch <= 0 || M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda % 8) || (ldb % 8) || (stride_a % 8) || (stride_b % 8) || (reinterpret_cast<uintptr_t>(A) % 16) || (reinterpret_cast<uintptr_t>(B) % 16)) return -1;
@@ -934,7 +945,7 @@ FSB_API int fsb_gemm_bf16_batched(const void* A, const void* B, void* C, const v
   cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
   const long long tiles = static_cast<long long>(batch) * ((M + BLOCK_M - 1) / BLOCK_M) * ((N + block_n - 1) / block_n);
   const int grid = tiles < num_sms ? static_cast<int>(tiles) : num_sms;
-  if (pair_enabled() && pair_pays(batch, M, N, K)) {
+  if (forced == 2 || (forced == 0 && pair_enabled() && pair_pays(batch, M, N, K))) {
     if (!b_mn_major && !fsb_host::encode_3d_16bit(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)batch, (uint64_t)ldb, (uint64_t)stride_b, BLOCK_K, PAIR_HALF_N, 1)) return -1;
     static bool pair_attr_set[64] = {false};
     if (!pair_attr_set[dev & 63]) {
@@ -963,4 +974,23 @@ FSB_API int fsb_gemm_bf16_batched(const void* A, const void* B, void* C, const v
     gemm_bf16_tcgen05_kernel<128, true><<<grid, GEMM_THREADS, SmemLayout<128>::TOTAL, stream>>>(ta, tb, p);
   }
   return static_cast<int>(cudaGetLastError());
+}
+
+FSB_API int fsb_gemm_bf16_batched(const void* A, const void* B, void* C, const void* bias, const void* aux, void* aux_out, int batch,
+                                  int M, int N, int K, int lda, int ldb, int ldc, int ld_aux, long long stride_a, long long stride_b,
+                                  long long stride_c, long long stride_aux, long long stride_bias, int a_mn_major, int b_mn_major,
+                                  int epilogue, int out_f32, int accumulate_c, int* status, cudaStream_t stream) {
+  return gemm_bf16_batched_impl(A, B, C, bias, aux, aux_out, batch, M, N, K, lda, ldb, ldc, ld_aux, stride_a, stride_b, stride_c, stride_aux, stride_bias, a_mn_major, b_mn_major,
+                           epilogue, out_f32, accumulate_c, status, stream, 0);
+}
+
+// The same products by one of the two kernels whatever their size: plan 1 one CTA per tile, 2 CTA pairs (M and N at least 256,
+// -1 otherwise).  fsb_gemm_bf16_batched chooses by itself.
+FSB_API int fsb_gemm_bf16_batched_plan(const void* A, const void* B, void* C, const void* bias, const void* aux, void* aux_out, int batch,
+                                  int M, int N, int K, int lda, int ldb, int ldc, int ld_aux, long long stride_a, long long stride_b,
+                                  long long stride_c, long long stride_aux, long long stride_bias, int a_mn_major, int b_mn_major,
+                                  int epilogue, int out_f32, int accumulate_c, int plan, int* status, cudaStream_t stream) {
+  if (plan != 1 && !(plan == 2 && M >= 256 && N >= 256)) return -1;
+  return gemm_bf16_batched_impl(A, B, C, bias, aux, aux_out, batch, M, N, K, lda, ldb, ldc, ld_aux, stride_a, stride_b, stride_c, stride_aux, stride_bias, a_mn_major, b_mn_major,
+                           epilogue, out_f32, accumulate_c, status, stream, plan);
 }

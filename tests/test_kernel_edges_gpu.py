@@ -337,24 +337,106 @@ def test_cluster_split_k_gemm(M, N, K, a_mn, b_mn, block_n, splits):
     _status_ok()
 
 
-@pytest.mark.parametrize("E,C,K,N", [(2, 256, 256, 256), (3, 257, 72, 264), (4, 410, 512, 2048), (1, 300, 64, 256)])
-def test_batched_pair_gemm_edges(E, C, K, N):
-    """Problems with whole 256 x 256 tiles run on CTA pairs; remainders must not leak into the next problem."""
-    from fairscale_b200.ops.gemm import batched_linear_dgrad, batched_linear_forward, batched_linear_wgrad
+# The persistent GEMM kernels by name, whatever the dispatch makes of the size: 1 one CTA per tile, 2 CTA pairs (256 x 256 tiles).
+# Whole tiles, remainders in M, N and K, fewer tiles than one wave of either kernel, more than one wave of both.
+@pytest.mark.parametrize("plan", [1, 2])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("M,N,K", [(256, 256, 64), (264, 328, 136), (520, 264, 1000), (1000, 264, 8192), (2600, 2056, 520), (8200, 1800, 264)])
+def test_persistent_gemm_kernels(M, N, K, a_mn, b_mn, plan):
+    from ctypes import c_int, c_void_p
 
+    from fairscale_b200.ops import _bind
+
+    _bind._SIGNATURES.setdefault("fsb_gemm_bf16_plan", [c_void_p] * 6 + [c_int] * 13 + [c_void_p] * 2)
+    torch.manual_seed(M + N + K)
+    a, b, aux = (torch.randn(*s, device=_dev()).bfloat16() for s in ((M, K), (N, K), (M, N)))
+    bias = torch.randn(N, device=_dev()).bfloat16()
+    sa, sb = (t.t().contiguous() if mn else t for t, mn in ((a, a_mn), (b, b_mn)))
+    ref = a.double() @ b.double().t()
+
+    def run(epi, dtype=torch.bfloat16, use_aux=False, pre=None, accumulate=0, into=None):
+        c = torch.full((M, N), float("nan"), device=_dev(), dtype=dtype) if into is None else into
+        _bind.call("fsb_gemm_bf16_plan", sa.data_ptr(), sb.data_ptr(), c.data_ptr(), bias.data_ptr() if epi in (1, 2, 3) else None,
+                   aux.data_ptr() if use_aux else None, _bind.ptr(pre), M, N, K, sa.stride(0), sb.stride(0), N, N, int(a_mn), int(b_mn),
+                   epi, int(dtype == torch.float32), accumulate, plan, _bind.status_ptr(_dev()), _bind.stream_ptr(_dev()))
+        return c
+
+    assert _rel_err(run(0), ref) < 1e-2
+    f32 = run(0, torch.float32)
+    assert _rel_err(f32, ref) < 1e-5
+    assert _rel_err(run(0, torch.float32, into=f32.clone(), accumulate=1), 2 * ref) < 1e-5
+    with_bias = ref + bias.double()
+    assert _rel_err(run(1), with_bias) < 1e-2
+    pre = torch.empty(M, N, device=_dev(), dtype=torch.bfloat16)
+    assert _rel_err(run(2, pre=pre), torch.nn.functional.gelu(with_bias)) < 1e-2
+    assert _rel_err(pre, with_bias) < 1e-2
+    assert _rel_err(run(3, use_aux=True), with_bias + aux.double()) < 1e-2
+    z = aux.double().requires_grad_()
+    torch.nn.functional.gelu(z).sum().backward()
+    assert _rel_err(run(4, use_aux=True), ref * z.grad) < 1e-2
+    assert _rel_err(run(5, use_aux=True), ref + aux.double()) < 1e-2
+    assert torch.equal(run(0, torch.float32), f32)
+    _status_ok()
+
+
+@pytest.mark.parametrize("plan", [0, 1, 2])
+@pytest.mark.parametrize("E,C,K,N", [(2, 256, 256, 256), (3, 257, 72, 264), (3, 257, 264, 264), (4, 410, 512, 2048), (1, 300, 64, 256), (17, 300, 264, 520)])
+def test_batched_gemm_edges(E, C, K, N, plan):
+    """Stacked problems on either kernel (0: the dispatch's choice); remainders must not leak into the next problem."""
+    from ctypes import c_int, c_longlong, c_void_p
+
+    from fairscale_b200.ops import _bind, gemm
+
+    _bind._SIGNATURES.setdefault("fsb_gemm_bf16_batched_plan", [c_void_p] * 6 + [c_int] * 8 + [c_longlong] * 5 + [c_int] * 6 + [c_void_p, c_void_p])
     torch.manual_seed(C)
     x = torch.randn(E, C, K, device=_dev()).bfloat16()
     w = torch.randn(E, N, K, device=_dev()).bfloat16()
     dy = torch.randn(E, C, N, device=_dev()).bfloat16()
     b = torch.randn(E, N, device=_dev()).bfloat16()
-    y, _ = batched_linear_forward(x, w, b)
-    want = torch.baddbmm(b.double().unsqueeze(1), x.double(), w.double().transpose(1, 2))
-    dx, dw = batched_linear_dgrad(dy, w), batched_linear_wgrad(dy, x)
+    call = _bind.call
+
+    def planned(name, *args, **kw):
+        if plan == 1 or (plan == 2 and min(args[7:9]) >= 256):  # the pairs take M and N from 256 on
+            name, args = name + "_plan", args[:-2] + (plan,) + args[-2:]
+        call(name, *args, **kw)
+
+    _bind.call = planned
+    try:
+        y, _ = gemm.batched_linear_forward(x, w, b)
+        act, pre = gemm.batched_linear_forward(x, w, b, gelu=True, save_pre_activation=True)
+        dx, dw = gemm.batched_linear_dgrad(dy, w), gemm.batched_linear_wgrad(dy, x)
+        dx_act = gemm.batched_linear_dgrad(dy, w, dgelu_pre=x)
+    finally:
+        _bind.call = call
     _status_ok()
+    want = torch.baddbmm(b.double().unsqueeze(1), x.double(), w.double().transpose(1, 2))
+    z = x.double().requires_grad_()
+    torch.nn.functional.gelu(z).sum().backward()
     for e in range(E):
-        assert _rel_err(y[e], want[e]) < 1e-2
-        assert _rel_err(dx[e], dy[e].double() @ w[e].double()) < 1e-2
+        assert _rel_err(y[e], want[e]) < 1e-2 and _rel_err(pre[e], want[e]) < 1e-2
+        assert _rel_err(act[e], torch.nn.functional.gelu(want[e])) < 1e-2
+        d = dy[e].double() @ w[e].double()
+        assert _rel_err(dx[e], d) < 1e-2 and _rel_err(dx_act[e], d * z.grad[e]) < 1e-2
         assert _rel_err(dw[e], dy[e].double().t() @ x[e].double()) < 1e-2
+
+
+def test_products_beyond_the_pair_threshold():
+    """The dispatch's own way onto CTA pairs: more than 2.56e11 operations, M and N no multiples of the 256 x 256 tiles."""
+    from fairscale_b200.ops.gemm import batched_linear_forward, linear_dgrad, linear_forward, linear_wgrad
+
+    torch.manual_seed(8)
+    M, N, K = 8200, 4360, 4096  # 2.9e11
+    x, w, dy = (torch.randn(*s, device=_dev()).bfloat16() for s in ((M, K), (N, K), (M, N)))
+    b, res = torch.randn(N, device=_dev()).bfloat16(), torch.randn(M, N, device=_dev()).bfloat16()
+    # fp32 oracle: its own sums differ by 1e-6, far below one rounding to bf16
+    assert _rel_err(linear_forward(x, w, b, residual=res)[0], x.float() @ w.float().t() + b.float() + res.float()) < 1e-2
+    assert _rel_err(linear_dgrad(dy, w), dy.float() @ w.float()) < 1e-2
+    assert _rel_err(linear_wgrad(dy, x), dy.float().t() @ x.float()) < 1e-2
+    xe, we, be = x[:8192].view(4, 2048, K), torch.randn(4, 4360, K, device=_dev()).bfloat16(), torch.randn(4, 4360, device=_dev()).bfloat16()
+    y, _ = batched_linear_forward(xe, we, be)
+    for e in range(4):
+        assert _rel_err(y[e], xe[e].float() @ we[e].float().t() + be[e].float()) < 1e-2
+    _status_ok()
 
 
 @pytest.mark.parametrize("E,rows,H", [(1, 1, 8), (3, 63, 256), (4, 410, 2048), (2, 5000, 264)])
