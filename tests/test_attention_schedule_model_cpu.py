@@ -1,180 +1,308 @@
-"""Exhaustive host-side model of the barrier schedule of the ping-pong attention forward
-(``csrc/attention_fwd_pingpong.cu``): one TMA producer, one MMA issuer, the in-order tensor pipe, and the softmax
-groups of the two query tiles A and B, synchronised by phase-parity mbarriers exactly as in the kernel.
+"""Exhaustive host-side models of the barrier schedules of the attention kernels: the ping-pong forward
+(``csrc/attention_fwd_pingpong.cu``) with either head size, and the two backward kernels (``csrc/attention.cu``).
 
-Every interleaving of the actors is explored (TMA loads land and tensor-pipe operations retire at arbitrary later
-times).  Checked in every reachable state: no deadlock; a K / V stage is never overwritten by a load while an issued
-product has yet to read it; S_t(j) is read by the softmax of step j only (not a stale or a later one); the
-probabilities P_t(j), which overwrite the score columns, are consumed by P V of step j before S_t(j+1) lands on them; a
-parity wait never passes on an older phase than the one the waiter means.
+A model is a set of actors (TMA producer, MMA issuer, groups of softmax warps) that run straight-line programs and are
+synchronised by phase-parity mbarriers exactly as in the kernel, plus TMA loads that land at arbitrary later times and the tensor
+pipe, which executes what was issued in order, at arbitrary later times.  Every interleaving is explored.  Each piece of memory -
+operand stages, score and probability columns, accumulators - carries the step that wrote it, and whoever reads one checks that
+it holds the step it means, so a stage or a buffer that is overwritten too early, or read too early, shows as a wrong step in
+some interleaving.  Checked besides: no deadlock, and no parity wait that passes on an older phase than the one the waiter means.
+
+The programs cover several work items of one persistent CTA (the barriers' phases run through all of them), among them items
+with a single query tile.
 """
-from collections import deque
-
 import pytest
 
 
-def _program_producer(n_kv):
-    steps = []
-    for j in range(n_kv):
-        st, par = j & 1, ((j >> 1) & 1) ^ 1
-        steps += [("wait", f"k_empty{st}", par, j), ("load", "K", st, j), ("wait", f"v_empty{st}", par, j), ("load", "V", st, j)]
-    return steps
+# Operations of a program:
+#   ("wait", barrier, parity, meant)      meant: number of completed phases the waiter relies on
+#   ("load", place, version, barrier)     a TMA load; completes a phase of the barrier when it lands
+#   ("mma", reads, place, version)        queued on the tensor pipe; reads: ((place, version), ...)
+#   ("commit", barrier)                   queued behind the products issued so far
+#   ("read", place, version), ("write", place, version), ("arrive", barrier)
+def forward_programs(items, sep, rescale, drop=()):
+    """items: (n_a, has_b) per item - key tiles of the first query tile, is there a second one (which sees one tile more)."""
+    producer, mma, softmax = [], [], ([], [])
 
+    def s_place(t):
+        return f"s{t}"
 
-def _program_mma(n_kv):
-    n_a = n_kv - 1
-    steps = []
+    def p_place(t):
+        return f"p{t}" if sep else f"s{t}"
 
-    def issue_s(t, j):
-        return [("wait", f"k_full{j & 1}", (j >> 1) & 1, j), ("mma", "S", t, j), ("commit", f"s_full{t}")]
+    kt = it_b = 0
+    cs, ss = [0, 0], [0, 0]
+    for it, (n_a, has_b) in enumerate(items):
+        n_kv = n_a + 1 if has_b else n_a
+        # ---- producer
+        producer += [("wait", "q_empty", (it & 1) ^ 1, it), ("load", "q", it, "q_full")]
+        for j in range(n_kv):
+            k = kt + j
+            st, par = k & 1, ((k >> 1) & 1) ^ 1
+            producer += [("wait", f"k_empty{st}", par, k >> 1), ("load", f"k{st}", k, f"k_full{st}"),
+                         ("wait", f"v_empty{st}", par, k >> 1), ("load", f"v{st}", k, f"v_full{st}")]
 
-    def issue_pv(t, j):
-        return [("wait", f"p_full{t}", j & 1, j), ("mma", "PV", t, j), ("commit", f"o_done{t}")]
+        # ---- MMA issuer
+        def issue_s(t, j):
+            k = kt + j
+            mma.append(("wait", f"k_full{k & 1}", (k >> 1) & 1, (k >> 1) + 1))
+            if sep and ss[t] > 0 and "s_read" not in drop:
+                mma.append(("wait", f"s_read{t}", (ss[t] - 1) & 1, ss[t]))
+            ss[t] += 1
+            mma.extend([("mma", (("q", it), (f"k{k & 1}", k)), s_place(t), ("S", it, j)), ("commit", f"s_full{t}")])
 
-    steps += issue_s(0, 0) + issue_s(1, 0) + [("commit", "k_empty0")]
-    for j in range(n_kv):
-        steps.append(("wait", f"v_full{j & 1}", (j >> 1) & 1, j))
-        if j < n_a:
-            steps += issue_pv(0, j)
-            if j + 1 < n_a:
-                steps += issue_s(0, j + 1)
-        steps += issue_pv(1, j) + [("commit", f"v_empty{j & 1}")]
-        if j + 1 < n_kv:
-            steps += issue_s(1, j + 1) + [("commit", f"k_empty{(j + 1) & 1}")]
-    return steps
+        def issue_pv(t, j):
+            k = kt + j
+            mma.extend([("wait", f"p_full{t}", cs[t] & 1, cs[t] + 1),
+                        ("mma", ((p_place(t), ("P", it, j)), (f"v{k & 1}", k)), f"o{t}", (it, j)), ("commit", f"o_done{t}")])
+            cs[t] += 1
 
+        mma.append(("wait", "q_full", it & 1, it + 1))
+        issue_s(0, 0)
+        if has_b:
+            issue_s(1, 0)
+        mma.append(("commit", f"k_empty{kt & 1}"))
+        if n_kv == 1:
+            mma.append(("commit", "q_empty"))
+        for j in range(n_kv):
+            k = kt + j
+            mma.append(("wait", f"v_full{k & 1}", (k >> 1) & 1, (k >> 1) + 1))
 
-def _program_softmax(t, n_kv, rescale):
-    n_it = n_kv - 1 if t == 0 else n_kv
-    steps = []
-    for j in range(n_it):
-        steps += [("wait", f"s_full{t}", j & 1, j), ("read_s", t, j)]
-        if rescale and j > 0:
-            steps += [("wait", f"o_done{t}", (j - 1) & 1, j - 1), ("touch_o", t, j - 1)]
-        steps += [("write_p", t, j), ("arrive", f"p_full{t}")]
-    steps += [("wait", f"o_done{t}", (n_it - 1) & 1, n_it - 1), ("touch_o", t, n_it - 1)]
-    return steps
+            def next_scores(t_list):
+                for t in t_list:
+                    if t == 0 and j + 1 < n_a or t == 1 and has_b and j + 1 < n_kv:
+                        issue_s(t, j + 1)
+                if 1 in t_list and j + 1 < n_kv:
+                    mma.append(("commit", f"k_empty{(k + 1) & 1}"))
+                    if j + 2 == n_kv:
+                        mma.append(("commit", "q_empty"))
 
-
-BARS = ["k_full0", "k_full1", "k_empty0", "k_empty1", "v_full0", "v_full1", "v_empty0", "v_empty1",
-        "s_full0", "s_full1", "p_full0", "p_full1", "o_done0", "o_done1"]
-
-
-def explore(n_kv, rescale, break_order=False):
-    progs = [_program_producer(n_kv), _program_mma(n_kv), _program_softmax(0, n_kv, rescale), _program_softmax(1, n_kv, rescale)]
-    if break_order:  # a wrong schedule: S_A(j+1) issued before P V_A(j) (the checker must notice)
-        mma = progs[1]
-        for i, s in enumerate(mma):
-            if s[:3] == ("mma", "PV", 0) and s[3] == 0:
-                k = next(x for x in range(i, len(mma)) if mma[x][:3] == ("mma", "S", 0) and mma[x][3] == 1)
-                mma[i - 1 : k + 2] = mma[k - 1 : k + 2] + mma[i - 1 : k - 1]  # move wait+S+commit ahead of wait+PV+commit
-                break
-    bar_idx = {b: i for i, b in enumerate(BARS)}
-    # state: pcs(4), completed phases per barrier, in-flight loads (frozenset), tensor queue (tuple), stage versions
-    # (K0,K1,V0,V1), score regions (kind, j) per tile, last P V retired per tile
-    start = ((0, 0, 0, 0), tuple([0] * len(BARS)), frozenset(), (), (-1, -1, -1, -1), (("free", -1), ("free", -1)), (-1, -1))
-    seen, queue = {start}, deque([start])
-    problems, deadlocks = [], 0
-
-    def passes(phases, name, parity, use):
-        c = phases[bar_idx[name]]
-        ok = parity != (c & 1)
-        return ok, c
-
-    while queue:
-        state = queue.popleft()
-        pcs, phases, loads, tq, stages, regions, pv_done = state
-        successors = []
-        # --- program steps of the four threads
-        for a in range(4):
-            if pcs[a] == len(progs[a]):
+            if sep:
+                next_scores((0, 1))
+            if j == 0:
+                mma.append(("wait", "o_free0", (it & 1) ^ 1, it))
+                if has_b:
+                    mma.append(("wait", "o_free1", (it_b & 1) ^ 1, it_b))
+            if "early_scores" in drop and not sep:  # in place, the next scores must not be issued ahead of the product
+                next_scores((0,))
+            if j < n_a:
+                issue_pv(0, j)
+                if not sep and "early_scores" not in drop:
+                    next_scores((0,))
+            if has_b:
+                issue_pv(1, j)
+            mma.append(("commit", f"v_empty{k & 1}"))
+            if not sep:
+                next_scores((1,))
+        kt += n_kv
+        it_b += has_b
+    # ---- softmax groups
+    for t in (0, 1):
+        c = 0
+        for it, (n_a, has_b) in enumerate(items):
+            if t == 1 and not has_b:
                 continue
-            op = progs[a][pcs[a]]
-            n_ph, n_loads, n_tq, n_stages, n_regions = phases, loads, tq, stages, regions
+            prog = softmax[t]
+            for j in range(n_a + t):
+                prog += [("wait", f"s_full{t}", c & 1, c + 1), ("read", s_place(t), ("S", it, j))]
+                if j > 0 and (sep or rescale):
+                    if "o_done" not in drop:
+                        prog.append(("wait", f"o_done{t}", (c - 1) & 1, c))
+                    if rescale:
+                        prog.append(("read", f"o{t}", (it, j - 1)))
+                if sep:
+                    prog += [("write", p_place(t), ("half", it, j)), ("read", s_place(t), ("S", it, j)), ("arrive", f"s_read{t}")]
+                prog += [("write", p_place(t), ("P", it, j)), ("arrive", f"p_full{t}")]
+                c += 1
+            prog += [("wait", f"o_done{t}", (c - 1) & 1, c), ("read", f"o{t}", (it, n_a + t - 1)), ("arrive", f"o_free{t}")]
+    return [producer, mma, *softmax], {}
+
+
+def backward_programs(items, nbuf, stages, steps_per_load, drop=()):
+    """items: steps per item (even).  ``steps_per_load`` 2: the dQ kernel (a K / V tile of 128 keys in two steps), 1: the dK / dV
+    kernel (a Q / dO sub-tile per step, whose statistics the softmax warps read from the same stage)."""
+    producer, mma, sets = [], [], ([], [])
+    jt0 = ut0 = 0
+    for it, n in enumerate(items):
+        producer += [("wait", "stat_empty", (it & 1) ^ 1, it), ("load", "stat", it, "stat_full")]
+        for j in range(n // steps_per_load):
+            jt = jt0 + j
+            st = jt % stages
+            producer += [("wait", f"str_empty{st}", ((jt // stages) & 1) ^ 1, jt // stages), ("load", f"str{st}", jt, f"str_full{st}")]
+
+        def stage(u):
+            jt = jt0 + u // steps_per_load
+            return jt, jt % stages
+
+        def issue_sp(u):
+            jt, st = stage(u)
+            buf = (ut0 + u) % nbuf
+            if u % steps_per_load == 0:
+                mma.append(("wait", f"str_full{st}", (jt // stages) & 1, jt // stages + 1))
+            mma.extend([("mma", (("stat", it), (f"str{st}", jt)), f"buf{buf}", ("S", ut0 + u)), ("commit", f"s_full{buf}")])
+            if u == n - 1:
+                mma.append(("commit", "stat_empty"))
+
+        mma.append(("wait", "stat_full", it & 1, it + 1))
+        for u in range(min(nbuf, n)):
+            issue_sp(u)
+        for u in range(n):
+            jt, st = stage(u)
+            ut = ut0 + u
+            buf = ut % nbuf
+            if "early_scores" in drop and u + nbuf < n:
+                issue_sp(u + nbuf)
+            if u == 0 and "acc_free" not in drop:
+                mma.append(("wait", "acc_free", (it & 1) ^ 1, it))
+            mma.extend([("wait", f"p_full{buf}", (ut // nbuf) & 1, ut // nbuf + 1),
+                        ("mma", ((f"buf{buf}", ("P", ut)), (f"str{st}", jt)), "acc", (it, u))])
+            if u % steps_per_load == steps_per_load - 1:
+                mma.append(("commit", f"str_empty{st}"))
+            if u == n - 1:
+                mma.append(("commit", "acc_done"))
+            if u + nbuf < n and "early_scores" not in drop:
+                issue_sp(u + nbuf)
+        for s in (0, 1):
+            for u in range(s, n, 2):
+                jt, st = stage(u)
+                ut = ut0 + u
+                buf = ut % nbuf
+                sets[s].extend([("wait", f"s_full{buf}", (ut // nbuf) & 1, ut // nbuf + 1), ("read", f"buf{buf}", ("S", ut))])
+                if steps_per_load == 1:
+                    sets[s].extend([("wait", f"str_full{st}", (jt // stages) & 1, jt // stages + 1), ("read", f"str{st}", jt)])
+                sets[s].extend([("write", f"buf{buf}", ("P", ut)), ("arrive", f"p_full{buf}")])
+            sets[s].extend([("wait", "acc_done", it & 1, it + 1), ("read", "acc", (it, n - 1)), ("arrive", "acc_free")])
+        jt0 += n // steps_per_load
+        ut0 += n
+    return [producer, mma, *sets], {"acc_free": 2}  # both sets read the accumulators
+
+
+def _commutes(progs):
+    """Per actor and position: a step that neither depends on nor is seen by another actor before the next one of its own kind may
+    be taken at once (queueing on the tensor pipe, starting a load after the wait for its stage)."""
+    return [[op[0] in ("mma", "commit", "load") for op in prog] for prog in progs]
+
+
+def explore(programs):
+    progs, counts = programs
+    names = sorted({op[1] for p in progs for op in p if op[0] in ("wait", "commit", "arrive")} | {op[3] for p in progs for op in p if op[0] == "load"})
+    bars = {b: i for i, b in enumerate(names)}
+    places = sorted({op[1] for p in progs for op in p if op[0] in ("load", "read", "write")} | {op[2] for p in progs for op in p if op[0] == "mma"})
+    slot = {p: i for i, p in enumerate(places)}
+    need = [counts.get(b, 1) for b in names]
+    at_once = _commutes(progs)
+    start = ((0,) * len(progs), (0,) * len(names), frozenset(), (), (None,) * len(places))
+    seen, stack = {start}, [start]
+    problems, deadlocks = set(), 0
+
+    def put(t, i, v):
+        return t[:i] + (v,) + t[i + 1:]
+
+    while stack and len(problems) < 20:
+        pcs, arrivals, loads, pipe, mem = stack.pop()
+        after = []
+        for a, prog in enumerate(progs):
+            pc = pcs[a]
+            if pc == len(prog):
+                continue
+            op = prog[pc]
+            n_arr, n_loads, n_pipe, n_mem = arrivals, loads, pipe, mem
             if op[0] == "wait":
-                ok, c = passes(phases, op[1], op[2], op[3])
-                if not ok:
+                i = bars[op[1]]
+                done = arrivals[i] // need[i]
+                if op[2] == (done & 1):
                     continue
-                # the waiter means use number `use_idx` of this barrier: stage barriers count every second step
-                name, use = op[1], op[3]
-                meant = use // 2 if name[0] in "kv" else use
-                if name.endswith("empty0") or name.endswith("empty1"):
-                    meant = use // 2 - 1  # the release of the previous occupant; -1 = never occupied
-                if meant >= 0 and c < meant + 1:
-                    problems.append(("wait passed on an older phase", a, op, c))
-            elif op[0] == "load":
-                n_loads = loads | {(op[1], op[2], op[3])}
-            elif op[0] == "mma":
-                n_tq = tq + (op,)
-            elif op[0] == "commit":
-                n_tq = tq + (op,)
+                if done < op[3]:
+                    problems.add(("a wait passed on an older phase", a, op, done))
             elif op[0] == "arrive":
-                i = bar_idx[op[1]]
-                n_ph = phases[:i] + (phases[i] + 1,) + phases[i + 1:]
-            elif op[0] == "read_s":
-                if regions[op[1]] != ("S", op[2]):
-                    problems.append(("softmax read a wrong score tile", op, regions[op[1]]))
-            elif op[0] == "write_p":
-                n_regions = tuple(("P", op[2]) if t == op[1] else r for t, r in enumerate(regions))
-            elif op[0] == "touch_o":
-                if pv_done[op[1]] < op[2]:
-                    problems.append(("output touched before its P V retired", op, pv_done))
-            n_pcs = pcs[:a] + (pcs[a] + 1,) + pcs[a + 1:]
-            successors.append((n_pcs, n_ph, n_loads, n_tq, n_stages, n_regions, pv_done))
-        # --- a TMA load lands
-        for ld in loads:
-            kind, st, j = ld
-            idx = st if kind == "K" else 2 + st
-            pending = [o for o in tq if o[0] == "mma" and ((kind == "K" and o[1] == "S") or (kind == "V" and o[1] == "PV")) and (o[3] & 1) == st and o[3] < j]
-            if pending:
-                problems.append(("stage overwritten before an issued product read it", ld, pending))
-            n_stages = stages[:idx] + (j,) + stages[idx + 1:]
-            i = bar_idx[("k_full" if kind == "K" else "v_full") + str(st)]
-            n_ph = phases[:i] + (phases[i] + 1,) + phases[i + 1:]
-            successors.append((pcs, n_ph, loads - {ld}, tq, n_stages, regions, pv_done))
-        # --- the tensor pipe retires its oldest entry
-        if tq:
-            op = tq[0]
-            n_ph, n_regions, n_pv = phases, regions, pv_done
-            if op[0] == "commit":
-                i = bar_idx[op[1]]
-                n_ph = phases[:i] + (phases[i] + 1,) + phases[i + 1:]
-            elif op[1] == "S":
-                _, _, t, j = op
-                if stages[j & 1] != j:
-                    problems.append(("S product read a K stage of another step", op, stages))
-                if regions[t][0] == "P":
-                    problems.append(("scores landed on unconsumed probabilities", op, regions[t]))
-                n_regions = tuple(("S", j) if x == t else r for x, r in enumerate(regions))
+                i = bars[op[1]]
+                n_arr = put(arrivals, i, arrivals[i] + 1)
+            elif op[0] == "read":
+                if mem[slot[op[1]]] != op[2]:
+                    problems.add(("read another step", a, op, mem[slot[op[1]]]))
+            elif op[0] == "write":
+                n_mem = put(mem, slot[op[1]], op[2])
+                if pc + 1 < len(prog) and prog[pc + 1][0] == "arrive":  # nobody looks at it before the arrival
+                    i = bars[prog[pc + 1][1]]
+                    n_arr = put(arrivals, i, arrivals[i] + 1)
+                    pc += 1
+            elif op[0] == "load":
+                n_loads = loads | {op[1:]}
             else:
-                _, _, t, j = op
-                if regions[t] != ("P", j):
-                    problems.append(("P V read wrong probabilities", op, regions[t]))
-                if stages[2 + (j & 1)] != j:
-                    problems.append(("P V read a V stage of another step", op, stages))
-                n_regions = tuple(("free", j) if x == t else r for x, r in enumerate(regions))
-                n_pv = tuple(j if x == t else d for x, d in enumerate(pv_done))
-            successors.append((pcs, n_ph, loads, tq[1:], stages, n_regions, n_pv))
-        done = all(pcs[a] == len(progs[a]) for a in range(4)) and not tq and not loads
-        if not successors and not done:
+                n_pipe = pipe + (op,)
+            pc += 1
+            while pc < len(prog) and at_once[a][pc]:
+                if prog[pc][0] == "load":
+                    n_loads = n_loads | {prog[pc][1:]}
+                else:
+                    n_pipe = n_pipe + (prog[pc],)
+                pc += 1
+            after.append((put(pcs, a, pc), n_arr, n_loads, n_pipe, n_mem))
+        for ld in loads:  # a TMA load lands
+            i = bars[ld[2]]
+            after.append((pcs, put(arrivals, i, arrivals[i] + 1), loads - {ld}, pipe, put(mem, slot[ld[0]], ld[1])))
+        if pipe:  # the tensor pipe completes its oldest entry
+            op = pipe[0]
+            if op[0] == "commit":
+                i = bars[op[1]]
+                after.append((pcs, put(arrivals, i, arrivals[i] + 1), loads, pipe[1:], mem))
+            else:
+                for place, version in op[1]:
+                    if mem[slot[place]] != version:
+                        problems.add(("a product read another step", op, place, mem[slot[place]]))
+                after.append((pcs, arrivals, loads, pipe[1:], put(mem, slot[op[2]], op[3])))
+        if not after and any(pc < len(p) for pc, p in zip(pcs, progs)):
             deadlocks += 1
-        for s in successors:
+        for s in after:
             if s not in seen:
                 seen.add(s)
-                queue.append(s)
-        if len(problems) > 50:
-            break
+                stack.append(s)
     return problems, deadlocks, len(seen)
+
+
+# (key tiles of the first query tile, is there a second one): a pair and a single tile in either order, three items
+FORWARD_ITEMS = [[(5, True)], [(1, True), (1, False)], [(1, False), (1, True)], [(3, False), (2, True)], [(3, True), (2, True), (1, False), (1, True)]]
 
 
 @pytest.mark.parametrize("n_kv", [2, 4])
 @pytest.mark.parametrize("rescale", [False, True])
 def test_pingpong_schedule_is_safe_and_live(n_kv, rescale):
-    problems, deadlocks, states = explore(n_kv, rescale)
-    assert states > 200
-    assert problems == [] and deadlocks == 0, (problems[:3], deadlocks)
+    problems, deadlocks, states = explore(forward_programs([(n_kv - 1, True)], False, rescale))
+    assert states > 50
+    assert not problems and deadlocks == 0, (sorted(map(str, problems))[:3], deadlocks)
 
 
 def test_checker_notices_scores_issued_ahead_of_the_product_that_reads_the_probabilities():
-    problems, deadlocks, _ = explore(4, False, break_order=True)
+    problems, deadlocks, _ = explore(forward_programs([(3, True)], False, False, drop=("early_scores",)))
+    assert problems or deadlocks
+
+
+@pytest.mark.parametrize("items", FORWARD_ITEMS, ids=str)
+@pytest.mark.parametrize("rescale", [False, True])
+@pytest.mark.parametrize("sep", [False, True], ids=["head128", "head64"])
+def test_forward_schedule_is_safe_and_live(items, rescale, sep):
+    problems, deadlocks, states = explore(forward_programs(items, sep, rescale))
+    assert states > 100
+    assert not problems and deadlocks == 0, (sorted(map(str, problems))[:3], deadlocks)
+
+
+# buffers, stages, steps per load of the four kernels; items long enough that buffers and stages come round
+@pytest.mark.parametrize("nbuf,stages,per_load,items", [(3, 4, 2, [8, 4, 2]), (2, 2, 2, [6, 4, 2]), (3, 6, 1, [8, 6, 2]), (2, 4, 1, [8, 4, 2])],
+                         ids=["dq64", "dq128", "dkv64", "dkv128"])
+def test_backward_schedule_is_safe_and_live(nbuf, stages, per_load, items):
+    problems, deadlocks, states = explore(backward_programs(items, nbuf, stages, per_load))
+    assert states > 100
+    assert not problems and deadlocks == 0, (sorted(map(str, problems))[:3], deadlocks)
+
+
+@pytest.mark.parametrize("mistake,sep", [("early_scores", False), ("s_read", True), ("o_done", True)])
+def test_checker_notices_a_wrong_forward(mistake, sep):
+    problems, deadlocks, _ = explore(forward_programs([(2, True), (1, True)], sep, True, drop=(mistake,)))
+    assert problems or deadlocks
+
+
+@pytest.mark.parametrize("mistake", ["early_scores", "acc_free"])
+@pytest.mark.parametrize("nbuf,stages,per_load", [(3, 4, 2), (2, 4, 1)])
+def test_checker_notices_a_wrong_backward(mistake, nbuf, stages, per_load):
+    problems, deadlocks, _ = explore(backward_programs([4, 4], nbuf, stages, per_load, drop=(mistake,)))
     assert problems or deadlocks
