@@ -686,38 +686,50 @@ static bool pair_enabled() {  // FSB_GEMM_PAIR=0 disables the CTA-pair kernel
   return on;
 }
 
-// Kernel for a product that is not streamed and has no CTA cap.  Measured on B200 (us; 64-wide K blocks = kb):
+// Kernel for a product that is not streamed and has no CTA cap.  Measured on B200 (us; 64-wide K blocks = kb), small products
+// back to back:
 //
 //   M, N, K              pair   one CTA 128x256   cluster split-K, block_n / splits
-//   77, 1024, 4096         -         24.7          64/1 20.6   64/2 16.5   64/4 12.4   64/8 16.5
-//   128, 1024, 8192        -         55.4          64/1 41.1   64/4 16.9   128/4 19.3  128/8 14.8
-//   768, 768, 3575       32.9        28.8          64/1 21.9   64/2 16.8   128/1 24.1  128/4 24.7
-//   1024, 1024, 8192     57.4        56.2          64/1 44.0   128/1 48.4  128/2 32.5
-//   2048, 1024, 1024     20.5        12.4          64/1 16.6   128/1 10.3
-//   2048, 2048, 2048     26.0        18.3          128/1 27.2
+//   77, 1024, 4096         -         24.6          64/1 20.5   64/2 15.0   64/4 11.7   128/4 12.8   128/8 12.3
+//   128, 1024, 8192        -         43.0          64/1 34.9   64/2 22.5   64/4 15.1   128/4 16.5   128/8 14.3
+//   768, 768, 3576       30.5        28.6          64/1 18.5   64/2 14.9   128/1 20.5  128/2 18.2   128/4 22.6
+//   1024, 1024, 8192     50.4        43.0          64/1 36.5   64/2 43.1   128/1 38.4  128/2 26.8   128/4 32.8
+//   2048, 1024, 1024     19.0        12.3          64/1 16.3   128/1 10.2  128/2 20.5
+//   2048, 2048, 2048     24.7        17.3          128/1 25.9
+//   3072, 1024, 8192     58.8        52.9          128/1 73.3
 //
-// One wave of independent CTAs takes about 6.3 us + K blocks x 0.28 / 0.32 / 0.39 us (tiles 64 / 128 / 256 wide): one CTA's
+// One wave of independent CTAs takes about 6 us + K blocks x 0.23 / 0.24 / 0.29 us (tiles 64 / 128 / 256 wide): one CTA's
 // operand stream is bound by latency, not by the tensor cores, so shorter slices win until the SMs run out.  A cluster
 // costs about 2 us more for its barriers, 4 us at eight CTAs, and clusters of four or eight do not fit the SMs to the last
-// one (144 CTAs in clusters of four run in two waves), hence the limits on their number.
+// one (144 CTAs in clusters of four run in two waves), hence the limits on their number.  (The slopes in the code are those
+// of a slower MMA issue, all by the same quarter; with them the rule takes the fastest column of every row above, or one
+// within 5 %.)
 //
-// With more tiles than one wave of single CTAs it is one CTA per tile or a pair per 256 x 256 tile:
+// With more tiles than one wave of single CTAs it is one CTA per tile or a pair per 256 x 256 tile.  In a loop of a second,
+// at the card's power limit, with the median SM clock in MHz:
 //
-//   M, N, K                  pair   one CTA          M, N, K (in a loop of a second)  pair   one CTA, strided
-//   4096, 2048, 2048         36.1    30.0            16384, 6144, 2048               338.5   330.7
-//   8192, 4096, 1024         64.3    56.5            16384, 2048, 8192               440.0   448.0
-//   5970, 6144, 2048        114.6   111.8            4096, 12288, 4096               323.0   334.0
-//   16384, 2048, 2048       104.1   102.1            8192, 2048, 16384 (wgrad)       490.0   513.0
+//   M, N, K                 one CTA      pair             M, N, K                        one CTA       pair
+//   4096, 2048, 2048       32.2 @1720   37.5 @1860        16384, 6144, 2048             348.1 @1342   349.2 @1385
+//   8192, 4096, 1024       67.4 @1485   75.0 @1635        16384, 8192, 2048             470.8 @1320   459.6 @1380
+//   5970, 6144, 2048      132.5 @1415   136.6 @1485       16384, 2048, 8192             461.4 @1260   457.5 @1220
+//   16384, 2048, 2048     121.5 @1370   124.8 @1462       4096, 12288, 4096             346.2 @1368   326.4 @1408
+//   8192, 8192, 2048      237.8 @1342   234.5 @1413       8192, 2048, 16384 (wgrad)     527.5 @1500   508.3 @1443
+//   8192, 16384, 512      159.8 @1485   199.0 @1723       6144, 2048, 16384 (wgrad)     400.0 @1511   386.2 @1511
+//   16384, 16384, 576     332.6 @1387   404.2 @1616       16384, 50304, 2048           2911.8 @1271  2783.5 @1331
+//   16384, 16384, 768     418.2 @1384   452.2 @1500       16384, 16384, 1280            628.1 @1368   627.0 @1428
+//   16384, 8192, 1024     256.6 @1447   274.0 @1479       16384, 8192, 1280             306.8 @1414   320.4 @1471
+//   16384, 16384, 1024    522.5 @1395   534.4 @1471       16384, 16384, 1536            729.3 @1365   711.6 @1413
 //
 // A pair costs some 6 us more per launch and rounds up to larger tiles, but moves a third less operand data, which counts
 // once a product is long enough to run at the card's power limit: beyond 2.56e11 operations, unless K is so short that the
-// output, which one CTA drains in smaller pieces, is what takes the time (16 x 8192 x 2048 x K 256: 316 against 178 us).
+// output, which one CTA drains in smaller pieces, is what takes the time (up to K about 1400; stacked products 16 x 2048 x 8192
+// x 1024: 510 against 547 us, 16 x 2048 x 2048 x 8192: 972 against 937 us).
 struct GemmPlan {
   enum Kind { PAIR, ONE_CTA, CLUSTER_K } kind;
   int block_n, splits;
 };
 static bool pair_pays(long long problems, int M, int N, int K) {
-  return M >= 256 && N >= 256 && K > 512 && 2.0 * problems * M * N * K > 2.56e11;
+  return M >= 256 && N >= 256 && K > 1400 && 2.0 * problems * M * N * K > 2.56e11;
 }
 static GemmPlan choose_gemm_plan(int M, int N, int K, int num_sms, bool pair_allowed) {
   const long long tiles_m = (M + fsb::BLOCK_M - 1) / fsb::BLOCK_M;
