@@ -35,8 +35,6 @@ struct AttnParams {
   int B, S, H, D;
   int S_pad;          // S rounded up to whole tiles of 128: row length of delta
   float scale;        // softmax scale (1/sqrt(D))
-  __nv_bfloat16* o;   // fwd out / bwd in   [B*S, H*D]
-  float* lse;         // [B, H, S]
   // [2, B, H, S_pad]: scale * rowsum(dO * O), then the base-2 lse, both written by attn_delta_kernel.  Rows past the end
   // hold 0 and +inf, so their probabilities 2^(0 - inf) and dS are exactly zero.
   const float* delta;
@@ -704,8 +702,7 @@ FSB_API int fsb_attn_bwd(const void* qkv, const void* o, const void* d_o, const 
   if (!fsb_host::encode_3d_16bit(&tm_do64, d_o, w_o, S, B, w_o, w_o * S, 64, KV_QSUB, 1)) return -5;
   AttnParams p{};
   p.B = B; p.S = S; p.S_pad = S_pad; p.H = H; p.D = D; p.scale = scale;
-  p.o = const_cast<__nv_bfloat16*>(static_cast<const __nv_bfloat16*>(o));
-  p.lse = const_cast<float*>(lse); p.delta = delta; p.dqkv = static_cast<__nv_bfloat16*>(dqkv); p.status = status;
+  p.delta = delta; p.dqkv = static_cast<__nv_bfloat16*>(dqkv); p.status = status;
   {
     const int threads = 256;
     long long blocks = (static_cast<long long>(B) * S + threads / 32 - 1) / (threads / 32);  // one token per warp at most ...

@@ -159,7 +159,7 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
   volatile int* abort_flag = &bars->abort_flag;
 
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // warp-uniform
-  // Work items (256 query rows of one head) ordered longest first and dealt round-robin to the persistent CTAs: every
+  // Work items (256 query rows of one head) ordered longest first and dealt to the persistent CTAs by snake_item: every
   // role of the CTA walks the same list.  item -> (q2, h, b): all heads of the longest rows come first.
   const int n_tiles = (p.S + BM - 1) / BM;  // 128-row tiles with at least one real row
   const int n_q2 = (n_tiles + 1) / 2;

@@ -148,15 +148,3 @@ FSB_API int fsb_ce_bwd_dtype(const void* logits, int dtype, const long long* tar
   else return -1;
   return static_cast<int>(cudaGetLastError());
 }
-
-// The same for bf16 logits.
-FSB_API int fsb_ce_fwd(const void* logits, const long long* targets, float* loss, float* lse, float* stats, long long rows,
-                       int V, long long ld, long long vocab_start, long long ignore_index, cudaStream_t stream) {
-  return fsb_ce_fwd_dtype(logits, FSB_BF16, targets, loss, lse, stats, rows, V, ld, vocab_start, ignore_index, stream);
-}
-
-FSB_API int fsb_ce_bwd(const void* logits, const long long* targets, const float* lse, const float* grad_out, int grad_is_scalar,
-                       float scale, void* dlogits, long long rows, int V, long long ld, long long vocab_start,
-                       long long ignore_index, cudaStream_t stream) {
-  return fsb_ce_bwd_dtype(logits, FSB_BF16, targets, lse, grad_out, grad_is_scalar, scale, dlogits, rows, V, ld, vocab_start, ignore_index, stream);
-}

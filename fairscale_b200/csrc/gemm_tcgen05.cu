@@ -11,7 +11,7 @@
 //
 // Structure: persistent kernel, one CTA per SM, 192 threads, tiles handed out at run time.
 //   warp 0      TMA producer: 128-byte-swizzled 64-wide K slabs of A and B into a 4-stage smem ring
-//   warp 1      allocates TMEM (2 x BLOCK_N fp32 columns) and issues tcgen05.mma (one elected lane)
+//   warp 1      allocates TMEM (2 x BLOCK_N fp32 columns) and issues tcgen05.mma (the whole warp, umma_f16_ss_warp)
 //   warps 2..5  epilogue: tcgen05.ld the finished accumulator (each warp its 32-lane quadrant),
 //               apply bias / GELU / GELU' / residual, convert and store; overlaps the next tile's
 //               main loop because the accumulator is double-buffered in TMEM.

@@ -77,12 +77,12 @@ __global__ void __launch_bounds__(NORM_WARPS * 32) norm_fwd_warp_kernel(const __
 }
 
 // ---- row-group backward (H <= 4096): a thread owns the same 8 columns of every row, so gamma and the dgamma / dbeta sums
-// stay in its registers; a CTA of H / 8 threads walks groups of R rows, one group after the other (persistent grid, 512
-// threads per SM: the 128 registers per thread hold two groups).  Bound by memory, and what counts is bytes in flight: the
-// next group's vectors are loaded before the current group's reductions, and R rows share one round of block reductions.
-// A warp per row, with all of a row's sums in one warp's registers, had room for one row only: 16384 x 2048 71 -> 53 us,
-// 8192 x 1024 31 -> 25 us, 4096 x 4096 (two kernels there) 43 -> 34 us.  (The forward has no sums to keep and is faster
-// with a warp per row: 35 against 41 us.)
+// stay in its registers; a CTA of H / 8 threads (in whole warps) walks groups of R rows, one group after the other.  At most
+// 2 x 148 CTAs: two fit an SM up to 2048 columns (128 registers per thread), one beyond, where the second half of the grid
+// runs after the first.  Bound by memory, and what counts is bytes in flight: the next group's vectors are loaded before the
+// current group's reductions, and R rows share one round of block reductions.  A warp per row, with all of a row's sums in
+// one warp's registers, had room for one row only: 16384 x 2048 71 -> 53 us, 8192 x 1024 31 -> 25 us, 4096 x 4096 (two kernels
+// there) 43 -> 34 us.  (The forward has no sums to keep and is faster with a warp per row: 35 against 41 us.)
 
 // Block-wide sums of N values per thread for blocks of whole warps; `red` holds 2 * 16 * N floats and is used in turn
 // (`turn` alternates), so one barrier per call is enough.
@@ -437,7 +437,7 @@ FSB_API int fsb_norm_fwd(const void* x, const void* gamma, const void* beta, voi
 }
 
 // Rows of fp32 partials the backward needs room for: the row-group kernel (H <= 4096) writes one row per CTA of its
-// persistent grid (two CTAs per SM, never more CTAs than groups of two rows), the two-kernel path at most 48.
+// grid (never more CTAs than groups of two rows), the two-kernel path at most 48.
 static int norm_bwd_rows_ctas(long long rows) {
   const long long want = (rows + 1) / 2;
   return static_cast<int>(want < 1 ? 1 : (want > fsb::NORM_ROWS_MAX_CTAS ? fsb::NORM_ROWS_MAX_CTAS : want));
@@ -498,11 +498,6 @@ FSB_API int fsb_norm_bwd_res(const void* dy, const void* x, const void* gamma, c
   column_reduce_kernel<<<dim3(blocks, want_beta ? 2 : 1), threads, 0, stream>>>(pg, strips, H, static_cast<__nv_bfloat16*>(dgamma),
                                                                                 want_beta ? static_cast<__nv_bfloat16*>(dbeta) : nullptr);
   return static_cast<int>(cudaGetLastError());
-}
-
-FSB_API int fsb_norm_bwd(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd, void* dx,
-                         void* dgamma, void* dbeta, float* partials, long long rows, int H, int rms, cudaStream_t stream) {
-  return fsb_norm_bwd_res(dy, x, gamma, mean, rstd, nullptr, dx, dgamma, dbeta, partials, rows, H, rms, stream);
 }
 
 FSB_API int fsb_colsum_num_strips(long long rows) {

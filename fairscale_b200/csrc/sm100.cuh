@@ -105,10 +105,9 @@ __device__ __forceinline__ void st_shared_cluster_u32(uint32_t cluster_addr, uin
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
 }
 
-// The warp that issues tcgen05.mma runs its control flow with all 32 lanes and elects one lane per instruction
-// group: loop counters, shared-memory addresses and descriptors then stay warp-uniform values, which keeps the cost
-// of issuing one MMA far below its execution time.  This is the all-lanes wait for that warp; the vote makes the
-// result (and every branch on it) uniform.
+// The warp that issues tcgen05.mma runs its control flow with all 32 lanes, and one elected lane issues (umma_f16_ss_warp; by
+// instruction group in gemm_comm_tcgen05.cu): loop counters, shared-memory addresses and descriptors then stay warp-uniform
+// values.  This is the all-lanes wait for that warp; the vote makes the result (and every branch on it) uniform.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int site = 1) {
   const bool ok = mbar_wait(bar, parity, abort_flag, site);
   return __all_sync(0xffffffffu, ok) != 0;
@@ -184,7 +183,8 @@ __device__ __forceinline__ void umma_f16_ss(uint32_t tmem_d, uint64_t adesc, uin
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Arrive on `bar` once every tcgen05 operation issued so far by this thread has completed.
+// Arrive on `bar` once every tcgen05 operation issued so far by this thread has completed.  (This form and umma_f16_ss, called
+// inside a one-lane branch, are used by the multi-GPU kernels of gemm_comm_tcgen05.cu only.)
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }

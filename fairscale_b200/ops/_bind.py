@@ -23,7 +23,6 @@ _SIGNATURES = {
     "fsb_norm_fwd": [c_void_p] * 6 + [c_longlong, c_int, c_float, c_int, c_void_p],
     "fsb_norm_bwd_res": [c_void_p] * 10 + [c_longlong, c_int, c_int, c_void_p],
     "fsb_norm_bwd_num_strips": [c_longlong],
-    "fsb_norm_bwd": [c_void_p] * 9 + [c_longlong, c_int, c_int, c_void_p],
     "fsb_colsum_num_strips": [c_longlong],
     "fsb_colsum": [c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p],
     "fsb_colsum_batched": [c_void_p, c_int, c_longlong, c_int, c_void_p, c_void_p, c_void_p],

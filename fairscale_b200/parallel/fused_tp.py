@@ -302,7 +302,7 @@ def _reduce_scatter_rows(x: torch.Tensor, group: Any) -> torch.Tensor:
     if world == 1:
         return x.contiguous()
     out = torch.empty((x.shape[0] // world,) + tuple(x.shape[1:]), dtype=x.dtype, device=x.device)
-    if world > 1 and dist.get_backend(group) == "gloo":  # gloo has no reduce-scatter
+    if dist.get_backend(group) == "gloo":  # gloo has no reduce-scatter
         full = x.contiguous().clone()
         dist.all_reduce(full, group=group)
         r = comm.group_rank(group)
