@@ -185,14 +185,15 @@ def linear_wgrad(dy: torch.Tensor, x: torch.Tensor, *, out: Optional[torch.Tenso
 
 
 def grad_slot_info(weight: torch.Tensor):
-    """Forward-time capture of a weight's flat-gradient window descriptor (None for ordinary tensors)."""
-    return getattr(weight, "_fsb_grad_slot", None)
+    """Forward-time capture of a weight's flat-gradient window descriptor (None for ordinary tensors, and for frozen ones: nobody
+    would take their window, and the flat gradient that it belongs to would be kept)."""
+    return getattr(weight, "_fsb_grad_slot", None) if weight.requires_grad else None
 
 
 def wgrad_into_slot(dy: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, slot_info=None) -> torch.Tensor:
     """``dw`` for ``weight``; written straight into the flat-gradient window of ``weight`` when it has one."""
     slot = None
-    info = slot_info if slot_info is not None else getattr(weight, "_fsb_grad_slot", None)
+    info = slot_info if slot_info is not None else grad_slot_info(weight)
     if info is not None and dy.is_cuda and weight.dtype == torch.bfloat16:
         arena, offset, shape = info
         if (offset * 2) % 16 == 0:

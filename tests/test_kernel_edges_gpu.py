@@ -785,3 +785,27 @@ def test_gemm_outputs_and_epilogue_operands_at_any_element(M, N, K):
         for want, got in zip(run(lambda t: t, **kw), run(_off, **kw)):
             assert torch.equal(want, got), kw
     _status_ok()
+
+
+def test_frozen_parameters_claim_no_window_of_a_flat_gradient():
+    """Their gradients go nowhere: a window would keep a whole flat gradient alive that no backward takes."""
+    from fairscale_b200.nn.misc.flatten_params_wrapper import GradArena
+    from fairscale_b200.ops import norm
+    from fairscale_b200.ops.gemm import linear
+    from fairscale_b200.ops.mlp import mlp
+
+    torch.manual_seed(9)
+    d = 64
+    arena = GradArena(5 * d * d)
+    shapes = dict(g=(d,), b=(d,), w=(d, d), wb=(d,), w1=(2 * d, d), b1=(2 * d,), w2=(d, 2 * d), b2=(d,))
+    p, off = {}, 0
+    for name, shape in shapes.items():
+        p[name] = torch.randn(shape, device=_dev()).bfloat16() * 0.1
+        p[name]._fsb_grad_slot = (arena, off, p[name].shape)
+        off += p[name].numel()
+    x = torch.randn(40, d, device=_dev()).bfloat16().requires_grad_()
+    y = linear(norm.layer_norm(x, p["g"], p["b"]), p["w"], p["wb"], residual=x)
+    mlp(y, p["w1"], p["b1"], p["w2"], p["b2"], residual=y).float().sum().backward()
+    assert torch.isfinite(x.grad).all()
+    assert arena.buffer is None and not arena.claimed
+    _status_ok()
