@@ -39,12 +39,14 @@ def _native_available() -> bool:
 def _native_takes(qkv: torch.Tensor, n_heads: int, D: int, scale: float) -> bool:
     """Does this call run the tcgen05 kernels?  bf16 and head size 64 or 128; whole tiles (a length that is a multiple of 128)
     always, any other length unless the call asks for what only torch's own operator offers: a functorch transform, forward-mode
-    differentiation, tracing, a softmax scale that is not positive, an empty tensor."""
+    differentiation, tracing, a softmax scale that is not positive, an empty tensor, autocast to another dtype."""
     if not (_bind.use_native(qkv) and qkv.dtype == torch.bfloat16 and D in (64, 128) and _native_available()):
         return False
     if qkv.shape[1] % 128 == 0:
         return True
     if qkv.numel() == 0 or qkv.shape[2] != 3 * n_heads * D or not (0.0 < scale < math.inf):
+        return False
+    if torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") != qkv.dtype:
         return False
     return not (torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0 or torch.compiler.is_compiling())
 

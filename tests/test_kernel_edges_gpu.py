@@ -118,6 +118,19 @@ def test_attention_rows_whose_first_keys_score_minus_infinity(S, D):
     assert _rel_err(o[:, 128:], ref[:, 128:]) < 2e-2
 
 
+def test_attention_of_ragged_lengths_under_autocast():
+    """Autocast to another 16-bit type casts what torch's operator takes; bf16 autocast leaves the kernels in place."""
+    from fairscale_b200.ops import attention
+
+    torch.manual_seed(0)
+    x = torch.randn(1, 77, 3 * 2 * 64, device=_dev()).bfloat16()
+    for dtype, backend in ((torch.float16, "torch-sdpa"), (torch.bfloat16, "tcgen05")):
+        with torch.autocast("cuda", dtype):
+            o = attention.causal_attention(x, 2)
+        assert o.dtype == dtype and attention.BACKEND == backend
+        assert _rel_err(o, _attention_ref(x.float(), 2)) < 2e-2
+
+
 @pytest.mark.parametrize("D", [64, 128])
 def test_attention_scales_of_either_sign(D):
     """A scale that is zero or negative is taken at multiples of 128, as it always was."""
