@@ -705,8 +705,8 @@ static bool pair_enabled() {  // FSB_GEMM_PAIR=0 disables the CTA-pair kernel
 // of a slower MMA issue, all by the same quarter; with them the rule takes the fastest column of every row above, or one
 // within 5 %.)
 //
-// With more tiles than one wave of single CTAs it is one CTA per tile or a pair per 256 x 256 tile.  In a loop of a second,
-// at the card's power limit, with the median SM clock in MHz:
+// From 90 tiles on it is one CTA per tile or a pair per 256 x 256 tile.  Aligned rows, in a loop of a second at the card's power
+// limit, with the median SM clock in MHz:
 //
 //   M, N, K                 one CTA      pair             M, N, K                        one CTA       pair
 //   4096, 2048, 2048       32.2 @1720   37.5 @1860        16384, 6144, 2048             348.1 @1342   349.2 @1385
@@ -720,27 +720,38 @@ static bool pair_enabled() {  // FSB_GEMM_PAIR=0 disables the CTA-pair kernel
 //   16384, 8192, 1024     256.6 @1447   274.0 @1479       16384, 8192, 1280             306.8 @1414   320.4 @1471
 //   16384, 16384, 1024    522.5 @1395   534.4 @1471       16384, 16384, 1536            729.3 @1365   711.6 @1413
 //
-// A pair costs some 6 us more per launch and rounds up to larger tiles, but moves a third less operand data, which counts
-// once a product is long enough to run at the card's power limit: beyond 2.56e11 operations, unless K is so short that the
-// output, which one CTA drains in smaller pieces, is what takes the time (up to K about 1400; stacked products 16 x 2048 x 8192
-// x 1024: 510 against 547 us, 16 x 2048 x 2048 x 8192: 972 against 937 us).
+// A pair costs some 6 us more per launch and rounds up to larger tiles, but moves a third less operand data.  That counts once
+// a product is long enough to run at the power limit, and much sooner where the operands' rows do not start on 128-byte lines
+// (a leading dimension that is no multiple of 64): every 128-byte row of a tile is then two lines.  Up to K about 1400 the
+// output, which one CTA drains in smaller pieces, is what takes the time.  (Stacked products, 16 x 2048 x 8192 x 1024: 510
+// against 547 us, 16 x 2048 x 2048 x 8192: 972 against 937 us.)  pair_pays puts that into two lines: us per K block and wave of
+// tiles, by the number of operands off the lines, and the pair's extra cost.  Over 197 products (M and N 256 .. 16384, K 512 ..
+// 16384, half of them with MN-major operands, most of odd sizes) the rule takes 0.6 % longer than the faster kernel would on
+// average, 12 % at worst; a single line at 2.56e11 operations took 4.7 %, and up to 44 % (2992 x 1976 x 13208 238 against 169 us,
+// 1936 x 5872 x 4360 139 against 110 us), always the pair 8 %, never 7 %.
 struct GemmPlan {
   enum Kind { PAIR, ONE_CTA, CLUSTER_K } kind;
   int block_n, splits;
 };
-static bool pair_pays(long long problems, int M, int N, int K) {
-  return M >= 256 && N >= 256 && K > 1400 && 2.0 * problems * M * N * K > 2.56e11;
+// Does the pair kernel pay for `problems` products of M x N x K with leading dimensions lda, ldb?
+static bool pair_pays(long long problems, int M, int N, int K, int lda, int ldb, int num_sms) {
+  const long long tiles = problems * ((M + fsb::BLOCK_M - 1) / fsb::BLOCK_M) * ((N + 255) / 256);
+  const long long pair_tiles = problems * ((M + 2 * fsb::BLOCK_M - 1) / (2 * fsb::BLOCK_M)) * ((N + fsb::PAIR_BLOCK_N - 1) / fsb::PAIR_BLOCK_N);
+  if (M < 256 || N < 256 || K <= 1400 || tiles < 90) return false;
+  static const float one_us[3] = {0.45f, 0.50f, 0.57f}, pair_us[3] = {0.435f, 0.44f, 0.49f};
+  const int off_line = (lda % 64 != 0) + (ldb % 64 != 0), num_kb = (K + fsb::BLOCK_K - 1) / fsb::BLOCK_K, pairs = num_sms / 2;
+  const float one = one_us[off_line] * num_kb * ((tiles + num_sms - 1) / num_sms);
+  const float pair = 8.f + pair_us[off_line] * num_kb * ((pair_tiles + pairs - 1) / pairs);
+  return pair < one;
 }
-static GemmPlan choose_gemm_plan(int M, int N, int K, int num_sms, bool pair_allowed) {
+static GemmPlan choose_gemm_plan(int M, int N, int K, int lda, int ldb, int num_sms, bool pair_allowed) {
   const long long tiles_m = (M + fsb::BLOCK_M - 1) / fsb::BLOCK_M;
   const int num_kb = (K + fsb::BLOCK_K - 1) / fsb::BLOCK_K;
   const int one_n = N <= 128 ? 128 : 256;  // tile width of the one-CTA kernel
   auto tiles = [&](int bn) -> long long { return tiles_m * ((N + bn - 1) / bn); };
   GemmPlan best = {GemmPlan::ONE_CTA, one_n, 1};
-  if (tiles(one_n) > num_sms) {
-    if (pair_allowed && pair_pays(1, M, N, K)) best.kind = GemmPlan::PAIR;
-    return best;
-  }
+  if (pair_allowed && pair_pays(1, M, N, K, lda, ldb, num_sms)) best.kind = GemmPlan::PAIR;
+  if (best.kind == GemmPlan::PAIR || tiles(one_n) > num_sms) return best;
   float cost = 6.5f + (one_n == 128 ? 0.32f : 0.39f) * num_kb;
   for (int bn = 64; bn <= 128; bn *= 2) {
     for (int c = 1; c <= 8 && c <= num_kb; c *= 2) {
@@ -756,6 +767,13 @@ static GemmPlan choose_gemm_plan(int M, int N, int K, int num_sms, bool pair_all
     }
   }
   return best;
+}
+
+// The kernel that a product (or `problems` stacked ones) would get on a device with `num_sms` SMs: 0 CTA pairs, 1 one CTA per
+// tile, 2 split-K over clusters (a single product only).
+FSB_API int fsb_gemm_plan_of(long long problems, int M, int N, int K, int lda, int ldb, int num_sms) {
+  if (problems > 1) return pair_enabled() && pair_pays(problems, M, N, K, lda, ldb, num_sms) ? 0 : 1;
+  return static_cast<int>(choose_gemm_plan(M, N, K, lda, ldb, num_sms, pair_enabled()).kind);
 }
 
 // C ABI ------------------------------------------------------------------------------------------
@@ -881,7 +899,7 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* bia
   GemmPlan plan = {GemmPlan::ONE_CTA, block_n, 1};
   if (streamed) plan.kind = GemmPlan::PAIR;
   else if (forced != 0) plan.kind = forced == 2 ? GemmPlan::PAIR : GemmPlan::ONE_CTA;
-  else if (max_ctas == 0) plan = choose_gemm_plan(M, N, K, num_sms, pair_enabled());
+  else if (max_ctas == 0) plan = choose_gemm_plan(M, N, K, lda, ldb, num_sms, pair_enabled());
   if (plan.kind == GemmPlan::CLUSTER_K) return fsb_host::gemm_cluster_k(ta, B, ldb, p, plan.block_n, plan.splits, dev, stream);
   // Run-time tile hand-out for products large enough to share the device with a collective; small ones stride.
   if (max_ctas == 0 && M >= 256 && N >= 256 && (plan.kind == GemmPlan::PAIR || tiles > num_sms)) {
@@ -957,7 +975,7 @@ static int gemm_bf16_batched_impl(const void* A, const void* B, void* C, const v
   cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
   const long long tiles = static_cast<long long>(batch) * ((M + BLOCK_M - 1) / BLOCK_M) * ((N + block_n - 1) / block_n);
   const int grid = tiles < num_sms ? static_cast<int>(tiles) : num_sms;
-  if (forced == 2 || (forced == 0 && pair_enabled() && pair_pays(batch, M, N, K))) {
+  if (forced == 2 || (forced == 0 && pair_enabled() && pair_pays(batch, M, N, K, lda, ldb, num_sms))) {
     if (!b_mn_major && !fsb_host::encode_3d_16bit(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)batch, (uint64_t)ldb, (uint64_t)stride_b, BLOCK_K, PAIR_HALF_N, 1)) return -1;
     static bool pair_attr_set[64] = {false};
     if (!pair_attr_set[dev & 63]) {

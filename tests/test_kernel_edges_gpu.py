@@ -434,18 +434,24 @@ def test_batched_gemm_edges(E, C, K, N, plan):
 
 
 def test_products_beyond_the_pair_threshold():
-    """The dispatch's own way onto CTA pairs: more than 2.56e11 operations, M and N no multiples of the 256 x 256 tiles."""
+    """The dispatch's own way onto CTA pairs; M, N and K no multiples of the tiles."""
+    from ctypes import c_int, c_longlong
+
+    from fairscale_b200.ops import _bind
     from fairscale_b200.ops.gemm import batched_linear_forward, linear_dgrad, linear_forward, linear_wgrad
 
+    _bind._SIGNATURES.setdefault("fsb_gemm_plan_of", [c_longlong] + [c_int] * 6)
+    plan_of, sms = _bind.fn("fsb_gemm_plan_of"), torch.cuda.get_device_properties(0).multi_processor_count
     torch.manual_seed(8)
-    M, N, K = 8200, 4360, 4096  # 2.9e11
+    M, N, K = 8200, 4360, 4360
+    assert plan_of(1, M, N, K, K, K, sms) == plan_of(1, M, K, N, N, K, sms) == plan_of(1, N, K, M, N, K, sms) == plan_of(4, 2048, N, K, K, K, sms) == 0
     x, w, dy = (torch.randn(*s, device=_dev()).bfloat16() for s in ((M, K), (N, K), (M, N)))
     b, res = torch.randn(N, device=_dev()).bfloat16(), torch.randn(M, N, device=_dev()).bfloat16()
     # fp32 oracle: its own sums differ by 1e-6, far below one rounding to bf16
     assert _rel_err(linear_forward(x, w, b, residual=res)[0], x.float() @ w.float().t() + b.float() + res.float()) < 1e-2
     assert _rel_err(linear_dgrad(dy, w), dy.float() @ w.float()) < 1e-2
     assert _rel_err(linear_wgrad(dy, x), dy.float().t() @ x.float()) < 1e-2
-    xe, we, be = x[:8192].view(4, 2048, K), torch.randn(4, 4360, K, device=_dev()).bfloat16(), torch.randn(4, 4360, device=_dev()).bfloat16()
+    xe, we, be = x[:8192].view(4, 2048, K), torch.randn(4, N, K, device=_dev()).bfloat16(), torch.randn(4, N, device=_dev()).bfloat16()
     y, _ = batched_linear_forward(xe, we, be)
     for e in range(4):
         assert _rel_err(y[e], xe[e].float() @ we[e].float().t() + be[e].float()) < 1e-2
@@ -630,7 +636,7 @@ def test_cross_entropy_keeps_nan_and_infinity(V, dtype):
 
 
 # one CTA per tile and CTA pairs, both with more tiles than one wave
-@pytest.mark.parametrize("M,N,K", [(4104, 2568, 512), (8200, 8200, 2048)])
+@pytest.mark.parametrize("M,N,K", [(4104, 2568, 512), (8200, 8200, 4096)])
 def test_products_on_two_streams_and_in_a_graph_keep_their_tiles(M, N, K):
     """The run-time tile hand-out belongs to a stream: a product that waits on one stream while many are enqueued on another,
     and one replayed from a graph, share no counter with them."""
