@@ -28,8 +28,9 @@
 // Any sequence length: the tensor map is three-dimensional (columns, positions, batch), so a tile that overhangs the
 // sequence reads zeros instead of the next sequence's rows; keys past the end lie above every real query's diagonal and
 // are masked with it; rows past the end are computed and not stored.  An item whose second query tile would lie wholly
-// past the end runs its first tile alone.  (Before, such lengths went through torch's operator, whose kernels are as fast
-// but need the packed tensor permuted, copied and concatenated: B4 S1543 H16 D128 forward + backward 539 us, now 330 us.)
+// past the end runs its first tile alone.  (torch's operator, which such lengths went through before, has the faster
+// forward but needs the packed tensor permuted and the gradients concatenated: B4 S1543 H16 D128 forward + backward 553 us there,
+// 296 us here.  ops/attention.py says which lengths come here.)
 //
 // The kernel is persistent: one CTA per SM walks a list of work items (256 query rows of one head), longest rows first,
 // dealt forwards and backwards in turn (snake_item; B2 S8192 H16 D64: 508 -> 471 us against plain round-robin).  TMEM,

@@ -36,15 +36,29 @@ def _native_available() -> bool:
         return False
 
 
+def _native_is_faster(B: int, S: int, H: int, inference: bool) -> bool:
+    """For a length that is no multiple of 128: the kernels here or torch's operator, which needs q, k and v permuted and their
+    gradients concatenated?  Forward + backward on B200 (us, torch / here): B4 S1543 H16 D128 553 / 296, B2 S4095 H16 D64 581 / 501,
+    B4 S5000 H16 D64 1553 / 1448, but B4 S7000 H16 D64 2579 / 2773 and B1 S8000 H2 D64 253 / 330 - the backward here makes the scores
+    twice, and few heads leave one long chain.  The forward alone is up to 30 % faster in torch's operator from S 500 on (B4 S1543
+    H16 D64 55 / 61, B2 S4095 H16 D64 98 / 124, short ones are bound by the host, B1 S77 33 / 27).  Only inference mode may go by that: a
+    forward without gradients may be the first pass of a checkpointed block, whose repetition has to compute the same."""
+    if inference:
+        return S <= 1024 and B * H * S <= 65536
+    return S <= 2048 or (S <= 5500 and B * H >= 8)
+
+
 def _native_takes(qkv: torch.Tensor, n_heads: int, D: int, scale: float) -> bool:
     """Does this call run the tcgen05 kernels?  bf16 and head size 64 or 128; whole tiles (a length that is a multiple of 128)
-    always, any other length unless the call asks for what only torch's own operator offers: a functorch transform, forward-mode
+    always, any other length where they are faster, unless the call asks for what only torch's own operator offers: a functorch transform, forward-mode
     differentiation, tracing, a softmax scale that is not positive, an empty tensor, autocast to another dtype."""
     if not (_bind.use_native(qkv) and qkv.dtype == torch.bfloat16 and D in (64, 128) and _native_available()):
         return False
     if qkv.shape[1] % 128 == 0:
         return True
     if qkv.numel() == 0 or qkv.shape[2] != 3 * n_heads * D or not (0.0 < scale < math.inf):
+        return False
+    if not _native_is_faster(qkv.shape[0], qkv.shape[1], n_heads, torch.is_inference_mode_enabled()):
         return False
     if torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") != qkv.dtype:
         return False
@@ -67,8 +81,8 @@ def causal_attention(qkv: torch.Tensor, n_heads: int, scale: Optional[float] = N
         if not _WARNED_LIBRARY_PATH:
             _WARNED_LIBRARY_PATH = True
             warnings.warn(
-                f"causal_attention: the tcgen05 kernels take bf16 with head size 64 or 128 (got {qkv.dtype}, head size {D}, length {S}); "
-                f"this call runs torch's scaled_dot_product_attention instead",
+                f"causal_attention: the tcgen05 kernels take bf16 with head size 64 or 128, and lengths that are no multiple of 128 where they "
+                f"are faster (got {qkv.dtype}, head size {D}, length {S}); this call runs torch's scaled_dot_product_attention instead",
                 stacklevel=2,
             )
         BACKEND = "torch-sdpa"

@@ -131,6 +131,26 @@ def test_attention_of_ragged_lengths_under_autocast():
         assert _rel_err(o, _attention_ref(x.float(), 2)) < 2e-2
 
 
+# (B, S, H): short, few heads and long, many heads and long, beyond the longest
+@pytest.mark.parametrize("B,S,H,trains,infers", [(1, 77, 2, True, True), (1, 2500, 2, False, False), (2, 2500, 4, True, False), (1, 5601, 8, False, False),
+                                                 (70, 100, 10, True, False)])
+def test_attention_of_ragged_lengths_runs_where_it_is_faster(B, S, H, trains, infers):
+    from fairscale_b200.ops import attention
+
+    torch.manual_seed(0)
+    x = torch.randn(B, S, 3 * H * 64, device=_dev()).bfloat16()
+    with torch.no_grad():
+        o = attention.causal_attention(x, H)
+    assert (attention.BACKEND == "tcgen05") == trains  # the same kernels with and without gradients
+    y = x.clone().requires_grad_()
+    assert torch.equal(attention.causal_attention(y, H), o) and (attention.BACKEND == "tcgen05") == trains
+    with torch.inference_mode():
+        i = attention.causal_attention(x, H)
+    assert (attention.BACKEND == "tcgen05") == infers
+    assert _rel_err(i.clone(), o) < 2e-2
+    _status_ok()
+
+
 @pytest.mark.parametrize("D", [64, 128])
 def test_attention_scales_of_either_sign(D):
     """A scale that is zero or negative is taken at multiples of 128, as it always was."""
