@@ -15,7 +15,6 @@ constexpr int NORM_THREADS = 256;
 constexpr int NORM_MAX_VEC = 4;  // block-per-row path: up to 4 x 8 bf16 per thread -> H <= 8192
 constexpr int NORM_WARPS = 4;    // warp-per-row forward: rows handled per CTA
 constexpr int NORM_ROWS_MAX_H = 4096;  // row-group backward: up to 512 threads of 8 columns
-constexpr int NORM_ROWS_MAX_CTAS = 2 * 148;
 
 // ---- warp-per-row forward (H <= 4096): a lane keeps VPL 16-byte vectors of the row in registers, all
 // reductions are warp shuffles, no shared memory and no block barriers.
@@ -76,94 +75,123 @@ __global__ void __launch_bounds__(NORM_WARPS * 32) norm_fwd_warp_kernel(const __
   }
 }
 
-// ---- row-group backward (H <= 4096): a thread owns the same 8 columns of every row, so gamma and the dgamma / dbeta sums
-// stay in its registers; a CTA of H / 8 threads (in whole warps) walks groups of R rows, one group after the other.  At most
-// 2 x 148 CTAs: two fit an SM up to 2048 columns (128 registers per thread), one beyond, where the second half of the grid
-// runs after the first.  Bound by memory, and what counts is bytes in flight: the next group's vectors are loaded before the
-// current group's reductions, and R rows share one round of block reductions.  A warp per row, with all of a row's sums in
-// one warp's registers, had room for one row only: 16384 x 2048 71 -> 53 us, 8192 x 1024 31 -> 25 us, 4096 x 4096 (two kernels
-// there) 43 -> 34 us.  (The forward has no sums to keep and is faster with a warp per row: 35 against 41 us.)
+// ---- row-group backward (H <= 4096): a thread owns the same 8 columns of every row it sees, so gamma and the dgamma / dbeta
+// sums stay in its registers.  A row takes H / 8 lanes: a power of two inside one warp up to 256 columns, whole warps beyond; a
+// CTA of about 256 threads holds as many such groups as fit (one from 1032 columns on), and each walks R rows at a time.
+// Persistent: two CTAs of up to 256 threads per SM (128 registers per thread), one of 288 to 512 for wider rows.  Bound by memory,
+// and what counts is bytes in flight: the next rows' vectors (x, dy and the residual's) are loaded before the current rows' sums,
+// and the narrower a row, the more of them are under way side by side.  One group per CTA whatever the width left a narrow row's
+// SM with a fraction of its 512 threads and took 65536 x 512 162 us (now 47 us), 16384 x 1024 51 (29), 16384 x 2048 66 (51),
+// 16384 x 4096, its grid in two waves, 138 (102); with a residual 16384 x 2048 75 (58).  A warp per row, with all of a row's sums
+// in one warp's registers and room for one row only, took 87, 41 and 67 us, two kernels for 4096 columns 188.  (All with the
+// reduction of the partial rows, ten calls in a graph.)  The forward has no sums to keep and is faster with a warp per row: 35
+// against 41 us.
+struct NormRowsShape {
+  int lanes;          // lanes of a warp that share a row
+  int warps_per_row;  // 1 unless lanes == 32
+  int groups;         // rows that the CTA works on side by side
+  int threads;
+};
+__host__ __device__ inline NormRowsShape norm_rows_shape(int H) {
+  NormRowsShape s;
+  const int need = H / 8;
+  s.lanes = 1;
+  while (s.lanes < 32 && s.lanes < need) s.lanes *= 2;
+  s.warps_per_row = (need + 31) / 32;
+  const int warp_groups = s.warps_per_row >= 8 ? 1 : 8 / s.warps_per_row;
+  s.groups = warp_groups * (32 / s.lanes);
+  s.threads = warp_groups * s.warps_per_row * 32;
+  return s;
+}
 
-// Block-wide sums of N values per thread for blocks of whole warps; `red` holds 2 * 16 * N floats and is used in turn
+// Sums of N values over the threads that share a row; `red` (per group of warps) holds 2 * 16 * N floats and is used in turn
 // (`turn` alternates), so one barrier per call is enough.
 template <int N>
-__device__ __forceinline__ void block_sums(float (&v)[N], float* red, int turn) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+__device__ __forceinline__ void row_sums(float (&v)[N], float* red, int turn, int lanes, int warps_per_row, int warp_group, int warp_in_row) {
+  for (int o = lanes >> 1; o > 0; o >>= 1) {
 #pragma unroll
-  for (int i = 0; i < N; ++i) v[i] = warp_sum(v[i]);
-  if (warps == 1) return;
-  float* buf = red + (turn & 1) * 16 * N;
-  if (lane == 0) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) buf[warp * N + i] = v[i];
+    for (int i = 0; i < N; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
   }
-  __syncthreads();
+  if (warps_per_row == 1) return;
+  float* buf = red + (turn & 1) * 16 * N;
+  if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) buf[warp_in_row * N + i] = v[i];
+  }
+  asm volatile("bar.sync %0, %1;" ::"r"(warp_group + 1), "r"(warps_per_row * 32) : "memory");
 #pragma unroll
   for (int i = 0; i < N; ++i) v[i] = 0.f;
-  for (int w = 0; w < warps; ++w) {
+  for (int w = 0; w < warps_per_row; ++w) {
 #pragma unroll
     for (int i = 0; i < N; ++i) v[i] += buf[w * N + i];
   }
 }
 
-// dx and the dgamma / dbeta partials in one pass over dy and x: dgamma_part / dbeta_part are [gridDim.x, H].  `res` (may be
-// null): a gradient of x from elsewhere - the residual branch around the norm - that is added before dx is rounded.
-template <bool RMS, int MAX_THREADS>
+// dx and the dgamma / dbeta partials in one pass over dy and x: dgamma_part / dbeta_part are [gridDim.x, H].  RES: `res` is a
+// gradient of x from elsewhere - the residual branch around the norm - that is added before dx is rounded.
+template <bool RMS, bool RES, int MAX_THREADS>
 __global__ void __launch_bounds__(MAX_THREADS, 512 / MAX_THREADS) norm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                                                const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
                                                                const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ res,
                                                                __nv_bfloat16* __restrict__ dx, float* __restrict__ dgamma_part,
                                                                float* __restrict__ dbeta_part, long long rows, int H) {
-  constexpr int R = 2;
-  __shared__ float red[2 * 16 * 2 * R];
-  const int col = threadIdx.x * 8;
+  constexpr int R = 2, N = 2 * R;
+  __shared__ float red[4][2 * 16 * N];  // per group of warps (more than one warp per row: at most four groups)
+  __shared__ __align__(16) float sums[MAX_THREADS <= 256 ? 256 * 8 : 4];  // one value per group and column, at the end
+  const NormRowsShape sh = norm_rows_shape(H);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int warp_group = warp / sh.warps_per_row, warp_in_row = warp - warp_group * sh.warps_per_row;
+  const int group = sh.warps_per_row == 1 ? static_cast<int>(threadIdx.x) / sh.lanes : warp_group;
+  const int col = sh.warps_per_row == 1 ? (lane & (sh.lanes - 1)) * 8 : (warp_in_row * 32 + lane) * 8;
   const bool mine = col < H;
+  float* my_red = red[sh.warps_per_row == 1 ? 0 : warp_group];
   float dg[8], db[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) dg[k] = db[k] = 0.f;
-  Vec16<__nv_bfloat16> tg, cx[R], cd[R], nx[R], nd[R], tr[R];
+  struct Rows {
+    Vec16<__nv_bfloat16> x[R], d[R], t[RES ? R : 1];
+    float m[R], r[R];
+  } cur, nxt;
+  Vec16<__nv_bfloat16> tg;
   tg.raw = make_uint4(0u, 0u, 0u, 0u);
   if (mine) tg = ld16(gamma + col);
-  float cm[R], cr[R], nm[R], nr[R];
-  auto load = [&](Vec16<__nv_bfloat16> (&tx)[R], Vec16<__nv_bfloat16> (&td)[R], float (&m)[R], float (&r)[R], long long row0) {
+  auto load = [&](Rows& v, long long row0) {
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-      tx[i].raw = td[i].raw = make_uint4(0u, 0u, 0u, 0u);
-      m[i] = r[i] = 0.f;
+      v.x[i].raw = v.d[i].raw = make_uint4(0u, 0u, 0u, 0u);
+      if (RES) v.t[i].raw = make_uint4(0u, 0u, 0u, 0u);
+      v.m[i] = v.r[i] = 0.f;
       if (row0 + i < rows) {
         if (mine) {
-          tx[i] = ld16(x + (row0 + i) * H + col);
-          td[i] = ld16(dy + (row0 + i) * H + col);
+          v.x[i] = ld16(x + (row0 + i) * H + col);
+          v.d[i] = ld16(dy + (row0 + i) * H + col);
+          if (RES) v.t[i] = ld16(res + (row0 + i) * H + col);
         }
-        if (!RMS) m[i] = mean_in[row0 + i];
-        r[i] = rstd_in[row0 + i];
+        if (!RMS) v.m[i] = mean_in[row0 + i];
+        v.r[i] = rstd_in[row0 + i];
       }
     }
   };
-  const long long step = static_cast<long long>(gridDim.x) * R;
-  long long row0 = static_cast<long long>(blockIdx.x) * R;
+  const long long step = static_cast<long long>(gridDim.x) * sh.groups * R;
+  long long base = static_cast<long long>(blockIdx.x) * sh.groups * R;  // the CTA's first row: the same trip count for all its lanes
+  long long row0 = base + group * R;
   int turn = 0;
-  load(cx, cd, cm, cr, row0);
-  for (; row0 < rows; row0 += step) {
-    load(nx, nd, nm, nr, row0 + step);
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      tr[i].raw = make_uint4(0u, 0u, 0u, 0u);
-      if (res != nullptr && mine && row0 + i < rows) tr[i] = ld16(res + (row0 + i) * H + col);
-    }
-    float s[2 * R];  // sum of w, sum of w * xhat, per row
+  load(cur, row0);
+  for (; base < rows; base += step, row0 += step) {
+    load(nxt, row0 + step);
+    float s[N];  // sum of w, sum of w * xhat, per row
 #pragma unroll
     for (int i = 0; i < R; ++i) {
       s[2 * i] = s[2 * i + 1] = 0.f;
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const float xh = (__bfloat162float(cx[i].v[k]) - cm[i]) * cr[i];
-        const float w = __bfloat162float(cd[i].v[k]) * __bfloat162float(tg.v[k]);
+        const float xh = (__bfloat162float(cur.x[i].v[k]) - cur.m[i]) * cur.r[i];
+        const float w = __bfloat162float(cur.d[i].v[k]) * __bfloat162float(tg.v[k]);
         s[2 * i] += w;
         s[2 * i + 1] = fmaf(w, xh, s[2 * i + 1]);
       }
     }
-    block_sums<2 * R>(s, red, turn++);
+    row_sums<N>(s, my_red, turn++, sh.lanes, sh.warps_per_row, warp_group, warp_in_row);
 #pragma unroll
     for (int i = 0; i < R; ++i) {
       if (row0 + i >= rows || !mine) break;
@@ -171,26 +199,36 @@ __global__ void __launch_bounds__(MAX_THREADS, 512 / MAX_THREADS) norm_bwd_rows_
       Vec16<__nv_bfloat16> o;
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const float xh = (__bfloat162float(cx[i].v[k]) - cm[i]) * cr[i];
-        const float d = __bfloat162float(cd[i].v[k]);
+        const float xh = (__bfloat162float(cur.x[i].v[k]) - cur.m[i]) * cur.r[i];
+        const float d = __bfloat162float(cur.d[i].v[k]);
         const float w = d * __bfloat162float(tg.v[k]);
-        o.v[k] = __float2bfloat16_rn(fmaf(cr[i], w - s1 - xh * s2, __bfloat162float(tr[i].v[k])));
+        o.v[k] = __float2bfloat16_rn(fmaf(cur.r[i], w - s1 - xh * s2, RES ? __bfloat162float(cur.t[RES ? i : 0].v[k]) : 0.f));
         dg[k] = fmaf(d, xh, dg[k]);
         if (!RMS) db[k] += d;
       }
       st16(dx + (row0 + i) * H + col, o);
     }
-#pragma unroll
-    for (int i = 0; i < R; ++i) { cx[i] = nx[i]; cd[i] = nd[i]; cm[i] = nm[i]; cr[i] = nr[i]; }
+    cur = nxt;
   }
-  if (mine) {
-    float* pg = dgamma_part + static_cast<long long>(blockIdx.x) * H + col;
-    *reinterpret_cast<float4*>(pg) = make_float4(dg[0], dg[1], dg[2], dg[3]);
-    *reinterpret_cast<float4*>(pg + 4) = make_float4(dg[4], dg[5], dg[6], dg[7]);
-    if (!RMS && dbeta_part != nullptr) {
-      float* pb = dbeta_part + static_cast<long long>(blockIdx.x) * H + col;
-      *reinterpret_cast<float4*>(pb) = make_float4(db[0], db[1], db[2], db[3]);
-      *reinterpret_cast<float4*>(pb + 4) = make_float4(db[4], db[5], db[6], db[7]);
+  // the CTA's partial row: its groups in order, dgamma first and dbeta second through the same buffer
+#pragma unroll
+  for (int which = 0; which < (RMS ? 1 : 2); ++which) {
+    float* out = which == 0 ? dgamma_part : dbeta_part;
+    if (out == nullptr) break;  // uniform
+    out += static_cast<long long>(blockIdx.x) * H;
+    const float (&v)[8] = which == 0 ? dg : db;
+    float* to = sh.groups == 1 ? out + col : sums + group * H + col;
+    if (which == 1 && sh.groups > 1) __syncthreads();
+    if (mine) {
+      *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]);
+      *reinterpret_cast<float4*>(to + 4) = make_float4(v[4], v[5], v[6], v[7]);
+    }
+    if (sh.groups == 1) continue;
+    __syncthreads();
+    for (int c = threadIdx.x; c < H; c += blockDim.x) {
+      float acc = 0.f;
+      for (int g = 0; g < sh.groups; ++g) acc += sums[g * H + c];
+      out[c] = acc;
     }
   }
 }
@@ -407,8 +445,6 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16
 
 // H must be a multiple of 8 and <= 8192. mean/rstd are fp32 [rows]. rms != 0 selects RMSNorm
 // (beta and mean ignored).
-static int norm_rows_threads(int H) { return (H / 8 + 31) / 32 * 32; }
-
 template <bool RMS>
 static void launch_norm_fwd(const __nv_bfloat16* x, const __nv_bfloat16* g, const __nv_bfloat16* b, __nv_bfloat16* y, float* mean,
                             float* rstd, long long rows, int H, float eps, cudaStream_t stream) {
@@ -436,11 +472,12 @@ FSB_API int fsb_norm_fwd(const void* x, const void* gamma, const void* beta, voi
   return static_cast<int>(cudaGetLastError());
 }
 
-// Rows of fp32 partials the backward needs room for: the row-group kernel (H <= 4096) writes one row per CTA of its
-// grid (never more CTAs than groups of two rows), the two-kernel path at most 48.
-static int norm_bwd_rows_ctas(long long rows) {
-  const long long want = (rows + 1) / 2;
-  return static_cast<int>(want < 1 ? 1 : (want > fsb::NORM_ROWS_MAX_CTAS ? fsb::NORM_ROWS_MAX_CTAS : want));
+// Rows of fp32 partials the backward needs room for: the row-group kernel (H <= 4096) writes one row per CTA of its persistent
+// grid - two CTAs of up to 256 threads or one larger one per SM, never more than there are groups of rows - the two-kernel path
+// at most 48.
+static int norm_bwd_rows_ctas(long long rows, int groups, int ctas_per_sm) {
+  const long long per_cta = 2ll * groups, want = (rows + per_cta - 1) / per_cta, most = 148ll * ctas_per_sm;
+  return static_cast<int>(want < 1 ? 1 : (want > most ? most : want));
 }
 static int norm_bwd_split_strips(long long rows) {
   const long long want = (rows + 7) / 8;
@@ -448,7 +485,7 @@ static int norm_bwd_split_strips(long long rows) {
 }
 
 FSB_API int fsb_norm_bwd_num_strips(long long rows) {
-  const int a = norm_bwd_rows_ctas(rows), b = norm_bwd_split_strips(rows);
+  const int a = norm_bwd_rows_ctas(rows, 1, 2), b = norm_bwd_split_strips(rows);
   return a > b ? a : b;
 }
 
@@ -464,7 +501,8 @@ FSB_API int fsb_norm_bwd_res(const void* dy, const void* x, const void* gamma, c
     return static_cast<int>(e);
   }
   const bool fused = H <= NORM_ROWS_MAX_H;
-  const int strips = fused ? norm_bwd_rows_ctas(rows) : norm_bwd_split_strips(rows);
+  const NormRowsShape sh = norm_rows_shape(H);
+  const int strips = fused ? norm_bwd_rows_ctas(rows, sh.groups, sh.threads <= 256 ? 2 : 1) : norm_bwd_split_strips(rows);
   float* pg = partials;
   float* pb = partials + static_cast<long long>(strips) * H;
   auto* d = static_cast<const __nv_bfloat16*>(dy);
@@ -474,13 +512,13 @@ FSB_API int fsb_norm_bwd_res(const void* dy, const void* x, const void* gamma, c
   auto* o = static_cast<__nv_bfloat16*>(dx);
   const bool want_beta = !rms && dbeta != nullptr;
   if (fused) {
-    const int threads = norm_rows_threads(H);
-    if (threads <= 256) {
-      if (rms) norm_bwd_rows_kernel<true, 256><<<strips, threads, 0, stream>>>(d, xx, gg, mean, rstd, rr, o, pg, nullptr, rows, H);
-      else     norm_bwd_rows_kernel<false, 256><<<strips, threads, 0, stream>>>(d, xx, gg, mean, rstd, rr, o, pg, want_beta ? pb : nullptr, rows, H);
+    auto launch = [&](auto kernel) { kernel<<<strips, sh.threads, 0, stream>>>(d, xx, gg, mean, rstd, rr, o, pg, want_beta ? pb : nullptr, rows, H); };
+    if (sh.threads <= 256) {
+      if (rms) rr != nullptr ? launch(norm_bwd_rows_kernel<true, true, 256>) : launch(norm_bwd_rows_kernel<true, false, 256>);
+      else     rr != nullptr ? launch(norm_bwd_rows_kernel<false, true, 256>) : launch(norm_bwd_rows_kernel<false, false, 256>);
     } else {
-      if (rms) norm_bwd_rows_kernel<true, 512><<<strips, threads, 0, stream>>>(d, xx, gg, mean, rstd, rr, o, pg, nullptr, rows, H);
-      else     norm_bwd_rows_kernel<false, 512><<<strips, threads, 0, stream>>>(d, xx, gg, mean, rstd, rr, o, pg, want_beta ? pb : nullptr, rows, H);
+      if (rms) rr != nullptr ? launch(norm_bwd_rows_kernel<true, true, 512>) : launch(norm_bwd_rows_kernel<true, false, 512>);
+      else     rr != nullptr ? launch(norm_bwd_rows_kernel<false, true, 512>) : launch(norm_bwd_rows_kernel<false, false, 512>);
     }
   } else {
     dim3 block(32, 8), grid((H / 8 + 31) / 32, strips);

@@ -490,10 +490,12 @@ def test_batched_column_sum(E, rows, H):
     assert torch.equal(batched_column_sum(x)[-1], batched_column_sum(x[-1:])[0])
 
 
-# one column group per thread up to 4096 columns (whole and partial warps), one CTA per row beyond; row counts that are no
-# multiple of the rows a CTA takes at a time, and more rows than the persistent grid takes in one round
+# one column group per thread up to 4096 columns (part of a warp, one, two to eight warps with one to four rows side by side, nine
+# to sixteen), one CTA per row beyond; row counts that are no multiple of the rows a CTA takes at a time, and more rows than the
+# persistent grid takes in one round
 @pytest.mark.parametrize("rms", [False, True])
-@pytest.mark.parametrize("rows,H", [(1, 8), (3, 264), (5, 2048), (7, 2056), (2, 4096), (3, 4104), (1801, 768)])
+@pytest.mark.parametrize("rows,H", [(1, 8), (3, 264), (5, 2048), (7, 2056), (2, 4096), (3, 4104), (1801, 768),
+                                    (9, 24), (37, 64), (40001, 128), (10007, 256), (5003, 264), (5003, 520), (601, 1032), (903, 2304)])
 def test_norm_backward_edges(rows, H, rms):
     from fairscale_b200.ops import norm
 
