@@ -4,15 +4,16 @@
 //   claim   : expert, slot, keep -> flat (int32 [S, 2]) = expert * C + slot, or -1 for a choice that is not kept, and one
 //             byte per row of the [E * C, M] buffer: does a token claim it?
 //   scatter : out[flat[s, k], :] = x[s, :] (* w[s, k]);   rows of out that no token claimed are zeroed
-//   gather  : out[s, :] = sum_k w[s, k] * buf[flat[s, k], :];   dots[s, k] = <buf[flat[s, k], :], g[s, :]>
+//   gather  : out[s, :] = sum_k w[s, k] * buf[flat[s, k], :];   dots[s, k] = <buf[flat[s, k], :], g[s, :]>;
+//             kept[s, k, :] = buf[flat[s, k], :] on the way (zero for a choice that is not kept), for a later gather without flat
 //
 // All three are bound by memory traffic: a warp moves one row with 16-byte accesses (four in flight per lane), scatter
 // reads a token once for both of its slots, gather sums both choices in fp32 registers.  A choice is known to be dropped
 // from its flat index alone, so nothing on the host depends on how many tokens were kept (the index_copy formulation
 // compacts the kept rows first, which makes the host wait for the device twice per direction).  Both come from the route as
 // the layer gets it - a gate may have changed what the routing kernels made - and never from counts taken before that.
-// Layer forward + backward, 8192 tokens of 1024 bf16, 8 experts of 4096: 3722 us with index ops, 1278 us with these kernels
-// and the expert products on CTA pairs; 820 tokens of 512, 4 experts of 2048: 2481 -> 1192 us.
+// Layer forward + backward, 8192 tokens of 1024 bf16, 8 experts of 4096: 3740 us with index ops, 1224 us now (866 us of them the
+// expert products); 820 tokens of 512, 4 experts of 2048: 2606 -> 1036 us.
 //
 // Replaces the dense einsum dispatch / combine of the reference (fairscale/nn/moe/moe_layer.py:77,88).
 
@@ -105,11 +106,11 @@ __global__ void __launch_bounds__(MR_THREADS) moe_scatter_local_kernel(const T* 
 template <typename T, int VEC>
 __global__ void __launch_bounds__(MR_THREADS) moe_gather_local_kernel(const T* __restrict__ buf, const int* __restrict__ flat, const float* __restrict__ w,
                                                                       long long S, int M, T* __restrict__ out, const T* __restrict__ g,
-                                                                      float* __restrict__ dots) {
+                                                                      float* __restrict__ dots, T* __restrict__ kept) {
   const int lane = threadIdx.x & 31;
   const long long warps = static_cast<long long>(gridDim.x) * MR_WARPS;
   for (long long s = static_cast<long long>(blockIdx.x) * MR_WARPS + (threadIdx.x >> 5); s < S; s += warps) {
-    const int r0 = flat[2 * s], r1 = flat[2 * s + 1];
+    const int r0 = flat != nullptr ? flat[2 * s] : static_cast<int>(2 * s), r1 = flat != nullptr ? flat[2 * s + 1] : static_cast<int>(2 * s + 1);
     const float w0 = w != nullptr ? w[2 * s] : 1.f, w1 = w != nullptr ? w[2 * s + 1] : 1.f;
     const T* b0 = buf + static_cast<long long>(r0) * M;
     const T* b1 = buf + static_cast<long long>(r1) * M;
@@ -121,6 +122,10 @@ __global__ void __launch_bounds__(MR_THREADS) moe_gather_local_kernel(const T* _
       for (int k = 0; k < VEC; ++k) a.v[k] = b.v[k] = gv.v[k] = from_f32<T>(0.f);
       if (r0 >= 0) a = row_ld<T, VEC>(b0 + j);
       if (r1 >= 0) b = row_ld<T, VEC>(b1 + j);
+      if (kept != nullptr) {
+        row_st<T, VEC>(kept + 2 * s * M + j, a);
+        row_st<T, VEC>(kept + (2 * s + 1) * M + j, b);
+      }
       if (dots != nullptr) {
         gv = row_ld<T, VEC>(g + s * M + j);
 #pragma unroll
@@ -210,25 +215,27 @@ FSB_API int fsb_moe_scatter_local(const void* x, int dtype, const int* flat, con
 }
 
 template <typename T>
-static void moe_gather_t(const void* buf, const int* flat, const float* w, long long S, int M, void* out, const void* g, float* dots, cudaStream_t stream) {
+static void moe_gather_t(const void* buf, const int* flat, const float* w, long long S, int M, void* out, const void* g, float* dots, void* kept,
+                         cudaStream_t stream) {
   using namespace fsb;
   const int grid = mr_grid(S);
-  if (mr_vec(M, sizeof(T), buf, out, g))
-    moe_gather_local_kernel<T, 16 / sizeof(T)><<<grid, MR_THREADS, 0, stream>>>(static_cast<const T*>(buf), flat, w, S, M, static_cast<T*>(out),
-                                                                              static_cast<const T*>(g), dots);
-  else
-    moe_gather_local_kernel<T, 1><<<grid, MR_THREADS, 0, stream>>>(static_cast<const T*>(buf), flat, w, S, M, static_cast<T*>(out),
-                                                                 static_cast<const T*>(g), dots);
+  auto launch = [&](auto kernel) {
+    kernel<<<grid, MR_THREADS, 0, stream>>>(static_cast<const T*>(buf), flat, w, S, M, static_cast<T*>(out), static_cast<const T*>(g), dots,
+                                            static_cast<T*>(kept));
+  };
+  if (mr_vec(M, sizeof(T), buf, out, g) && mr_vec(M, sizeof(T), kept, nullptr, nullptr)) launch(moe_gather_local_kernel<T, 16 / sizeof(T)>);
+  else launch(moe_gather_local_kernel<T, 1>);
 }
 
-// buf [rows, M]; out [S, M] or null; g [S, M] and dots fp32 [S, 2], or both null.
+// buf [rows, M] with flat from fsb_moe_claim_rows, or [2 * S, M] with flat null: the rows of choice (s, k) are row 2 * s + k.  out
+// [S, M] or null; g [S, M] and dots fp32 [S, 2], or both null; kept [2 * S, M] or null.
 FSB_API int fsb_moe_gather_local(const void* buf, int dtype, const int* flat, const float* w, long long S, int M, void* out, const void* g, float* dots,
-                                 cudaStream_t stream) {
+                                 void* kept, cudaStream_t stream) {
   if (S <= 0) return 0;
-  if ((g == nullptr) != (dots == nullptr)) return -1;
-  if (dtype == FSB_F32) moe_gather_t<float>(buf, flat, w, S, M, out, g, dots, stream);
-  else if (dtype == FSB_F16) moe_gather_t<__half>(buf, flat, w, S, M, out, g, dots, stream);
-  else if (dtype == FSB_BF16) moe_gather_t<__nv_bfloat16>(buf, flat, w, S, M, out, g, dots, stream);
+  if ((g == nullptr) != (dots == nullptr) || 2 * S > 0x7fffffffll) return -1;
+  if (dtype == FSB_F32) moe_gather_t<float>(buf, flat, w, S, M, out, g, dots, kept, stream);
+  else if (dtype == FSB_F16) moe_gather_t<__half>(buf, flat, w, S, M, out, g, dots, kept, stream);
+  else if (dtype == FSB_BF16) moe_gather_t<__nv_bfloat16>(buf, flat, w, S, M, out, g, dots, kept, stream);
   else return -1;
   return static_cast<int>(cudaGetLastError());
 }

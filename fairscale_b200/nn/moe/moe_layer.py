@@ -23,6 +23,7 @@ import torch.distributed as dist
 from torch import Tensor
 from torch.nn import Module, ModuleList
 
+from ...ops import _bind
 from ...parallel import comm, symm
 from .top2gate import Top2Route
 
@@ -109,64 +110,60 @@ def _local_rows(t: Tensor) -> bool:
 
 
 class _Claims:
-    """The rows of the global ``[E * C, M]`` view that a route's choices claim, for the row kernels: ``flat`` int32 ``[S, 2]`` (-1 if
-    not kept) and ``claimed`` uint8 ``[E * C]``.  Computed when the dispatch of a forward asks for it, shared with its combine."""
+    """The rows of the global ``[E * C, M]`` view that a route's choices claim, for the row kernels.  One buffer: ``flat`` int32
+    ``[S, 2]`` (-1 if not kept), then ``claimed`` uint8 ``[E * C]``.  Computed when the dispatch of a forward asks for it, shared
+    with its combine."""
 
     def __init__(self, route: Top2Route) -> None:
         self.route = route
-        self._rows: Optional[Tuple[Tensor, Tensor]] = None
+        self._buffer: Optional[Tensor] = None
 
-    def rows(self) -> Tuple[Tensor, Tensor]:
-        if self._rows is None:
-            from ctypes import c_longlong, c_void_p
-
-            from ...ops import _bind
-
-            _bind._SIGNATURES.setdefault("fsb_moe_claim_rows", [c_void_p] * 3 + [c_longlong] * 3 + [c_void_p] * 3)
-            r, dev = self.route, self.route.expert.device
-            expert, slot = r.expert.long().contiguous(), r.slot.long().contiguous()
-            keep = r.keep.to(torch.bool).contiguous()
-            flat = torch.empty(tuple(expert.shape), dtype=torch.int32, device=dev)
-            claimed = torch.empty(r.num_experts * r.capacity, dtype=torch.uint8, device=dev)
-            _bind.call("fsb_moe_claim_rows", expert.data_ptr(), slot.data_ptr(), keep.data_ptr(), expert.shape[0], r.num_experts, r.capacity,
-                       flat.data_ptr(), claimed.data_ptr(), _bind.stream_ptr(dev))
-            self._rows = (flat, claimed)
-        return self._rows
+    def buffer(self) -> Tensor:
+        if self._buffer is None:
+            r = self.route
+            expert, slot, keep = r.expert, r.slot, r.keep
+            if not (expert.dtype == slot.dtype == torch.int64 and expert.is_contiguous() and slot.is_contiguous()):
+                expert, slot = expert.long().contiguous(), slot.long().contiguous()
+            if keep.dtype != torch.bool or not keep.is_contiguous():
+                keep = keep.to(torch.bool).contiguous()
+            S, E, C = expert.shape[0], r.num_experts, r.capacity
+            self._buffer = torch.empty(8 * S + E * C, dtype=torch.uint8, device=expert.device)
+            flat = self._buffer.data_ptr()
+            _bind.call("fsb_moe_claim_rows", expert.data_ptr(), slot.data_ptr(), keep.data_ptr(), S, E, C, flat, flat + 8 * S,
+                       _bind.stream_ptr(expert.device))
+        return self._buffer
 
 
-def _scatter_local(x: Tensor, flat: Tensor, claimed: Tensor, w: Optional[Tensor]) -> Tensor:
+def _flat_rows(claims: Tensor, S: int) -> Tensor:
+    return claims[: 8 * S].view(torch.int32).view(S, 2)
+
+
+def _scatter_local(x: Tensor, claims: Tensor, w: Optional[Tensor]) -> Tensor:
     """``out[flat[s, k]] = x[s] (* w[s, k])`` with a row per entry of ``claimed``; rows nobody claimed are zero."""
-    from ctypes import c_int, c_longlong, c_void_p
-
-    from ...ops import _bind
-
-    _bind._SIGNATURES.setdefault("fsb_moe_scatter_local", [c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_longlong, c_void_p])
     x = x.contiguous()
     S, M = x.shape
-    out = x.new_empty((claimed.shape[0], M))
-    _bind.call("fsb_moe_scatter_local", x.data_ptr(), _bind.dtype_code(x.dtype), flat.data_ptr(), _bind.ptr(w), S, M, out.data_ptr(),
-               claimed.data_ptr(), claimed.shape[0], _bind.stream_ptr(x.device))
+    rows, flat = claims.shape[0] - 8 * S, claims.data_ptr()
+    out = x.new_empty((rows, M))
+    _bind.call("fsb_moe_scatter_local", x.data_ptr(), _bind.dtype_code(x.dtype), flat, _bind.ptr(w), S, M, out.data_ptr(), flat + 8 * S, rows,
+               _bind.stream_ptr(x.device))
     return out
 
 
-def _gather_local(buf: Tensor, flat: Tensor, w: Optional[Tensor], grad: Optional[Tensor] = None) -> Tensor:
-    """``sum_k w[s, k] * buf[flat[s, k]]`` as ``[S, M]``, or with ``grad`` the fp32 dots ``<buf[flat[s, k]], grad[s]>`` ``[S, 2]``."""
-    from ctypes import c_int, c_longlong, c_void_p
-
-    from ...ops import _bind
-
-    _bind._SIGNATURES.setdefault("fsb_moe_gather_local", [c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_void_p])
-    S, M = flat.shape[0], buf.shape[1]
-    out = None if grad is not None else buf.new_empty((S, M))
-    dots = buf.new_empty((S, 2), dtype=torch.float32) if grad is not None else None
-    _bind.call("fsb_moe_gather_local", buf.data_ptr(), _bind.dtype_code(buf.dtype), flat.data_ptr(), _bind.ptr(w), S, M, _bind.ptr(out),
-               _bind.ptr(grad), _bind.ptr(dots), _bind.stream_ptr(buf.device))
-    return out if dots is None else dots
+def _gather_local(buf: Tensor, claims: Tensor, S: int, w: Optional[Tensor], kept: Optional[Tensor] = None) -> Tensor:
+    """``sum_k w[s, k] * buf[flat[s, k]]`` as ``[S, M]``; ``kept`` ``[S, 2, M]`` also receives the rows themselves."""
+    out = buf.new_empty((S, buf.shape[1]))
+    _bind.call("fsb_moe_gather_local", buf.data_ptr(), _bind.dtype_code(buf.dtype), claims.data_ptr(), _bind.ptr(w), S, buf.shape[1], out.data_ptr(),
+               None, None, _bind.ptr(kept), _bind.stream_ptr(buf.device))
+    return out
 
 
-def _kept_rows(buf: Tensor, flat: Tensor) -> Tensor:
-    """``buf[flat[s, k]]`` as fp32 ``[S, 2, M]`` in torch operations, zero where ``flat`` is -1."""
-    return buf[flat.clamp(min=0).long()].float() * (flat >= 0).unsqueeze(-1)
+def _row_dots(kept: Tensor, grad: Tensor) -> Tensor:
+    """fp32 ``<kept[s, k], grad[s]>`` as ``[S, 2]``."""
+    S, _, M = kept.shape
+    dots = kept.new_empty((S, 2), dtype=torch.float32)
+    _bind.call("fsb_moe_gather_local", kept.data_ptr(), _bind.dtype_code(kept.dtype), None, None, S, M, None, grad.data_ptr(), dots.data_ptr(), None,
+               _bind.stream_ptr(kept.device))
+    return dots
 
 
 def _to_experts(rows: Tensor, group: Any, world: int, n_local: int, C: int) -> Tensor:
@@ -204,9 +201,10 @@ class _Dispatch(torch.autograd.Function):
             owner._mine = False
         ctx.local = ws is None and _local_rows(x)
         if ctx.local:
-            flat, claimed = (claims or _Claims(route)).rows()
-            ctx.save_for_backward(flat)
-            return _to_experts(_scatter_local(x, flat, claimed, None), group, world, n_local, C)
+            rows = (claims or _Claims(route)).buffer()
+            ctx.save_for_backward(rows)
+            ctx.tokens = x.shape[0]
+            return _to_experts(_scatter_local(x, rows, None), group, world, n_local, C)
         dst_rank, dst_row, flat = _routes(route, world, n_local, rank)
         ctx.save_for_backward(dst_rank, dst_row, flat, route.keep)
         if ws is not None:
@@ -232,11 +230,14 @@ class _Dispatch(torch.autograd.Function):
     def backward(ctx: Any, grad: Tensor):  # type: ignore[override]
         group, n_local, world, rank, C, E, M, dtype = ctx.meta
         if ctx.local:
-            (flat,) = ctx.saved_tensors
+            (rows,) = ctx.saved_tensors
+            home = _to_tokens(grad.contiguous(), group, world, n_local, C)
             if torch.is_grad_enabled():  # create_graph: the gradient is linear in `grad`, and the graph has to know it
-                home = _to_tokens(grad.contiguous(), group, world, n_local, C)
-                return _kept_rows(home, flat).sum(1).to(grad.dtype), None, None, None, None, None
-            return _gather_local(_to_tokens(grad.contiguous(), group, world, n_local, C), flat, None), None, None, None, None, None
+                flat = _flat_rows(rows, ctx.tokens)
+                dx = (home[flat.clamp(min=0).long()].float() * (flat >= 0).unsqueeze(-1)).sum(1).to(grad.dtype)
+            else:
+                dx = _gather_local(home, rows, ctx.tokens, None)
+            return dx, None, None, None, None, None
         dst_rank, dst_row, flat, keep = ctx.saved_tensors
         S = dst_rank.shape[0]
         if ctx.claimed:
@@ -273,18 +274,13 @@ class _Combine(torch.autograd.Function):
         ctx.owner = owner
         ctx.local = ws is None and _local_rows(expert_out)
         if ctx.local:
-            flat, claimed = (claims or _Claims(route)).rows()
+            rows = (claims or _Claims(route)).buffer()
             w = gate.to(torch.float32).contiguous()  # the kernels look at flat: a dropped choice's weight is not read
             home = _to_tokens(expert_out.contiguous(), group, world, n_local, C)
-            out = _gather_local(home, flat, w)
-            # the gates' gradient needs the rows once more; with one rank they are the experts' own output, which stays theirs to reuse
-            kept = home
-            if not ctx.needs_input_grad[1]:
-                kept = None
-            elif home.untyped_storage().data_ptr() == expert_out.untyped_storage().data_ptr():
-                kept = home.clone()
-            ctx.save_for_backward(flat, claimed, w, kept)
-            return out
+            # the gates' gradient needs the rows once more, and the experts' output stays theirs to reuse: the gather keeps them
+            kept = home.new_empty((gate.shape[0], 2, M)) if ctx.needs_input_grad[1] else None
+            ctx.save_for_backward(rows, w, kept)
+            return _gather_local(home, rows, gate.shape[0], w, kept)
         dst_rank, dst_row, flat = _routes(route, world, n_local, rank)
         S = dst_rank.shape[0]
         w = (gate * route.keep).to(torch.float32).contiguous()
@@ -308,16 +304,17 @@ class _Combine(torch.autograd.Function):
     def backward(ctx: Any, dy: Tensor):  # type: ignore[override]
         group, n_local, world, rank, C, E, M = ctx.meta
         if ctx.local:
-            flat, claimed, w, home = ctx.saved_tensors
+            rows, w, kept = ctx.saved_tensors
             dy = dy.contiguous()
             if torch.is_grad_enabled():  # create_graph: as in the dispatch
-                dyf = dy.float().unsqueeze(1)
+                dyf, flat = dy.float().unsqueeze(1), _flat_rows(rows, dy.shape[0])
                 to = torch.where(flat >= 0, flat, E * C).long().view(-1)  # choices that were not kept go to a row that is cut off
                 d_rows = dyf.new_zeros((E * C + 1, M)).index_add(0, to, (dyf * w.unsqueeze(-1)).view(-1, M))[:-1].to(dy.dtype)
-                d_gate = (_kept_rows(home, flat) * dyf).sum(-1) if home is not None else None
-                return _to_experts(d_rows, group, world, n_local, C), d_gate, None, None, None, None, None
-            d_eo = _to_experts(_scatter_local(dy, flat, claimed, w), group, world, n_local, C)
-            return d_eo, _gather_local(home, flat, None, grad=dy) if home is not None else None, None, None, None, None, None
+                d_gate = (kept.float() * dyf).sum(-1) if kept is not None else None
+            else:
+                d_rows = _scatter_local(dy, rows, w)
+                d_gate = _row_dots(kept, dy) if kept is not None else None
+            return _to_experts(d_rows, group, world, n_local, C), d_gate, None, None, None, None, None
         dst_rank, dst_row, flat, keep, w, saved = ctx.saved_tensors
         S = dst_rank.shape[0]
         dy = dy.contiguous()

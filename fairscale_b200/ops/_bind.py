@@ -28,6 +28,9 @@ _SIGNATURES = {
     "fsb_colsum_batched": [c_void_p, c_int, c_longlong, c_int, c_void_p, c_void_p, c_void_p],
     "fsb_ce_fwd_dtype": [c_void_p, c_int] + [c_void_p] * 4 + [c_longlong, c_int, c_longlong, c_longlong, c_longlong, c_void_p],
     "fsb_ce_bwd_dtype": [c_void_p, c_int] + [c_void_p] * 3 + [c_int, c_float, c_void_p, c_longlong, c_int, c_longlong, c_longlong, c_longlong, c_void_p],
+    "fsb_moe_claim_rows": [c_void_p] * 3 + [c_longlong] * 3 + [c_void_p] * 3,
+    "fsb_moe_scatter_local": [c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_longlong, c_void_p],
+    "fsb_moe_gather_local": [c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_int] + [c_void_p] * 5,
     "fsb_embedding_fwd": [c_void_p] * 4 + [c_longlong, c_int, c_int, c_longlong, c_longlong, c_float, c_void_p],
     "fsb_embedding_bwd": [c_void_p] * 4 + [c_longlong, c_int, c_int, c_longlong, c_longlong, c_float, c_void_p],
     "fsb_cast": [c_void_p, c_int, c_void_p, c_int, c_longlong, c_float, c_void_p],
