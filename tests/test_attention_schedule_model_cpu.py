@@ -296,13 +296,13 @@ def test_backward_schedule_is_safe_and_live(nbuf, stages, per_load, items):
 
 
 @pytest.mark.parametrize("mistake,sep", [("early_scores", False), ("s_read", True), ("o_done", True)])
-def test_checker_notices_a_wrong_forward(mistake, sep):
+def test_model_notices_a_wrong_forward(mistake, sep):
     problems, deadlocks, _ = explore(forward_programs([(2, True), (1, True)], sep, True, drop=(mistake,)))
     assert problems or deadlocks
 
 
 @pytest.mark.parametrize("mistake", ["early_scores", "acc_free"])
 @pytest.mark.parametrize("nbuf,stages,per_load", [(3, 4, 2), (2, 4, 1)])
-def test_checker_notices_a_wrong_backward(mistake, nbuf, stages, per_load):
+def test_model_notices_a_wrong_backward(mistake, nbuf, stages, per_load):
     problems, deadlocks, _ = explore(backward_programs([4, 4], nbuf, stages, per_load, drop=(mistake,)))
     assert problems or deadlocks
