@@ -9,8 +9,12 @@
 //   softmax A   :          [ softmax A(j) ............ ]              [ softmax A(j+1) ............ ]
 //   softmax B   :                    [ softmax B(j) ............ ]              [ softmax B(j+1) ..... ]
 //
-// Roles (320 threads): warp 0 TMA producer, warp 1 MMA issuer and TMEM owner, warps 2-5 softmax of tile A, warps 6-9
-// softmax of tile B; one thread per query row (TMEM lane), so the row maximum and row sum need no exchange.
+// Roles (576 threads): warp 0 TMA producer, warp 1 MMA issuer and TMEM owner, warps 2-9 softmax of tile A, warps 10-17
+// softmax of tile B.  Two threads share a query row (TMEM lane), 64 of a step's 128 keys each: they read their scores once and
+// keep them in registers, pass each other the row maximum through shared memory, and with four warps per scheduler one warp's
+// loads and waits hide behind the exponentials of others.  (One thread per row read the scores twice, once for the maximum,
+// and left the exponential unit, which bounds head size 64, idle 46 % of the time: B2 S8192 H16 D64 433 -> 398 us,
+// B8 S1024 H16 D64 53.8 -> 45.8 us; head size 128, where the products bound the step, 168.8 -> 168.3 us at B8 S2048 H16.)
 // TMEM (512 columns): S_A [0,128)  S_B [128,256)  O_A [256,256+D)  O_B [384,384+D).  With head size 128 the bf16 probabilities overwrite
 // the first 64 columns of their own score tile (two values per 32-bit column) and feed P V as the TMEM A operand of
 // tcgen05.mma, so they never pass through shared memory.  The tensor pipe executes in issue order: S_t(j+1) is issued
@@ -18,8 +22,8 @@
 // Tile A skips the last key tile of the item (it lies wholly above A's diagonal).  Every mbarrier wait is bounded.
 //
 // Head size 64 leaves 128 TMEM columns free, and the probabilities get them (P_A [384,448)  P_B [448,512), O_B [320,384)).
-// Then S_t(j+1) need not wait for PV_t(j): it is issued as soon as the softmax warps have read the last scores of step j,
-// half-way through their exponentials, and is ready when they come back for it:
+// Then S_t(j+1) need not wait for PV_t(j): it is issued as soon as the softmax warps have read the scores of step j, before
+// their exponentials, and is ready when they come back for it:
 //
 //   tensor pipe :  S_A(j+1)  S_B(j+1)  PV_A(j)  PV_B(j)  S_A(j+2) ...
 //
@@ -49,7 +53,7 @@
 namespace fsb {
 namespace pp {
 
-constexpr int THREADS = 320;
+constexpr int THREADS = 576;
 constexpr int BM = 128;          // rows of a query tile == TMEM lanes
 constexpr int BN = 128;          // keys per step
 constexpr float LOG2E = 1.4426950408889634f;
@@ -61,24 +65,19 @@ struct Params {
   __nv_bfloat16* o;
   float* lse;
   int* status;
-  unsigned long long* trace;  // optional timeline of CTA (0,0,0): [role][step][4] nanosecond stamps
 };
-
-// role 0: MMA issuer, 1: softmax of tile A (warp 2, lane 0), 2: softmax of tile B (warp 6, lane 0)
-#define PP_TRACE(role, j, k)                                                                              \
-  if (p.trace != nullptr && blockIdx.x == 0 && (j) < 32 && (threadIdx.x & 31) == 0)                            \
-    p.trace[((role) * 32 + (j)) * 4 + (k)] = globaltimer_ns();
 
 struct Bars {
   uint64_t q_full;
   uint64_t k_full[2], k_empty[2];
   uint64_t v_full[2], v_empty[2];
   uint64_t s_full[2];   // per query tile: scores of the current step are in TMEM
-  uint64_t p_full[2];   // per query tile: probabilities written (4 warp arrivals)
+  uint64_t p_full[2];   // per query tile: probabilities written (8 warp arrivals)
   uint64_t o_done[2];   // per query tile: P V of the current step has completed
-  uint64_t s_read[2];   // per query tile, head size 64: the softmax warps hold all scores of the step (4 warp arrivals)
+  uint64_t s_read[2];   // per query tile, head size 64: the softmax warps hold all scores of the step (8 warp arrivals)
   uint64_t q_empty;     // the item's last Q K^T products have completed: the query tiles may be replaced
-  uint64_t o_free[2];   // per query tile: the softmax warps have read the item's output accumulator (4 warp arrivals)
+  uint64_t o_free[2];   // per query tile: the softmax warps have read the item's output accumulator (8 warp arrivals)
+  uint64_t pair[2][4];  // per query tile and lane quadrant: both warps of the rows have left a value for each other (2 warp arrivals)
   uint32_t tmem_slot;
   int abort_flag;
 };
@@ -90,7 +89,8 @@ struct Smem {
   static constexpr int K_OFF = 2 * TILE;     // two stages
   static constexpr int V_OFF = 4 * TILE;     // two stages
   static constexpr int BAR_OFF = 6 * TILE;
-  static constexpr int TOTAL = BAR_OFF + 256 + 1024;
+  static constexpr int XCH_OFF = BAR_OFF + 512;  // [2 parities][2 tiles][2 halves][BM] values passed between the two threads of a row
+  static constexpr int TOTAL = XCH_OFF + 2 * 2 * 2 * BM * 4 + 1024;
 };
 
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -117,31 +117,55 @@ __device__ __forceinline__ constexpr uint32_t kstep_kmajor(int ks, uint32_t slab
 }
 __device__ __forceinline__ constexpr uint32_t kstep_mnmajor(int ks) { return static_cast<uint32_t>(ks) * 2048u; }
 
+// Two fp32 values per instruction: half the issue slots of the scaling and of the row sum.
+__device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// Largest of 32 scores of a row and `m`; DIAG: of those of keys col0 + i <= row only.
 template <bool DIAG>
 __device__ __forceinline__ float chunk_max(const uint32_t (&r)[32], int col0, int row, float m) {
   float a[4] = {m, m, m, m};
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    if (!DIAG || (col0 + i) <= row) a[i & 3] = fmaxf(a[i & 3], __uint_as_float(r[i]));
+  for (int i = 0; i < 32; i += 2) {
+    float x = __uint_as_float(r[i]), y = __uint_as_float(r[i + 1]);
+    if (DIAG) {
+      if (col0 + i > row) x = m;
+      if (col0 + i + 1 > row) y = m;
+    }
+    a[(i >> 1) & 3] = fmaxf(fmaxf(a[(i >> 1) & 3], x), y);
   }
   return fmaxf(fmaxf(a[0], a[1]), fmaxf(a[2], a[3]));
 }
 
+// Probabilities of 32 scores, packed to bf16; their sum is added to `acc`.
 template <bool DIAG>
-__device__ __forceinline__ float chunk_exp(const uint32_t (&r)[32], int col0, int row, float sl2, float mb, uint32_t (&pk)[16]) {
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+__device__ __forceinline__ void chunk_exp(const uint32_t (&r)[32], int col0, int row, uint64_t sl2, uint64_t neg_mb, uint64_t (&acc)[2], uint32_t (&pk)[16]) {
 #pragma unroll
   for (int i = 0; i < 32; i += 2) {
-    float p0 = ex2_approx(fmaf(__uint_as_float(r[i]), sl2, -mb));
-    float p1 = ex2_approx(fmaf(__uint_as_float(r[i + 1]), sl2, -mb));
+    float x, y;
+    unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), sl2, neg_mb), x, y);
+    float p0 = ex2_approx(x), p1 = ex2_approx(y);
     if (DIAG) {
       if (col0 + i > row) p0 = 0.f;
       if (col0 + i + 1 > row) p1 = 0.f;
     }
-    acc[(i >> 1) & 3] += p0 + p1;
+    acc[(i >> 1) & 1] = add_f32x2(acc[(i >> 1) & 1], pack_f32x2(p0, p1));
     pk[i >> 1] = pack_bf16(p0, p1);
   }
-  return (acc[0] + acc[1]) + (acc[2] + acc[3]);
 }
 
 template <int D>
@@ -177,10 +201,11 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
       mbar_init(&bars->v_full[i], 1);
       mbar_init(&bars->v_empty[i], 1);
       mbar_init(&bars->s_full[i], 1);
-      mbar_init(&bars->p_full[i], 4);
+      mbar_init(&bars->p_full[i], 8);
       mbar_init(&bars->o_done[i], 1);
-      mbar_init(&bars->o_free[i], 4);
-      mbar_init(&bars->s_read[i], 4);
+      mbar_init(&bars->o_free[i], 8);
+      mbar_init(&bars->s_read[i], 8);
+      for (int q = 0; q < 4; ++q) mbar_init(&bars->pair[i][q], 2);
     }
     bars->abort_flag = 0;
     fence_barrier_init();
@@ -284,10 +309,8 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
         const uint32_t kt = kt0 + j;
         const int st = kt & 1;
         if (!mbar_wait_warp(&bars->v_full[st], (kt >> 1) & 1u, abort_flag)) { ok = false; break; }
-        if (item == static_cast<int>(blockIdx.x)) { PP_TRACE(0, j, 0); }
-        if (p.trace != nullptr && item == 0 && j < 32 && lane == 0) p.trace[384 + j] = clock64();
         if (SEP) {
-          // the next step's scores first: they wait for reads half-way through the exponentials of this one
+          // the next step's scores first: they wait for reads that come before the exponentials of this one
           if (j + 1 < n_a && !issue_s(0, kt + 1)) { ok = false; break; }
           if (j + 1 < n_kv) {
             if (has_b && !issue_s(1, kt + 1)) { ok = false; break; }
@@ -302,12 +325,9 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
         }
         if (j < n_a) {
           if (!issue_pv(0, kt, j == 0)) { ok = false; break; }
-          if (item == static_cast<int>(blockIdx.x)) { PP_TRACE(0, j, 1); }
           if (!SEP && j + 1 < n_a && !issue_s(0, kt + 1)) { ok = false; break; }
         }
-        if (item == static_cast<int>(blockIdx.x)) { PP_TRACE(0, j, 2); }
         if (has_b && !issue_pv(1, kt, j == 0)) { ok = false; break; }
-        if (item == static_cast<int>(blockIdx.x)) { PP_TRACE(0, j, 3); }
         commit(&bars->v_empty[st]);
         if (!SEP && j + 1 < n_kv) {
           if (has_b && !issue_s(1, kt + 1)) { ok = false; break; }
@@ -319,15 +339,33 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
       it_b += has_b ? 1u : 0u;
     }
   } else {
-    // ------------------------------------------------------------------ softmax warps: one thread per query row
-    const int t = (warp - 2) >> 2;
+    // ------------------------------------------------------------------ softmax warps: two threads per query row
+    const int t = (warp - 2) >> 3;           // query tile
+    const int half = ((warp - 2) >> 2) & 1;  // which 64 of a step's 128 keys, which D / 2 output columns
     const int quad = warp & 3;
     const int row = quad * 32 + lane;
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
-    const uint32_t ts = tmem_base + t * 128 + lane_off;                   // scores
-    const uint32_t tp = tmem_base + P_COL + t * P_STEP + lane_off;         // probabilities (columns [0, 64) of the scores unless SEP)
-    const uint32_t to = tmem_base + O_COL + t * O_STEP + lane_off;         // output accumulator
+    const uint32_t ts = tmem_base + t * 128 + half * 64 + lane_off;                  // this thread's scores
+    const uint32_t tp = tmem_base + P_COL + t * P_STEP + half * 32 + lane_off;        // its probabilities (in columns [0, 64) of the tile's scores unless SEP)
+    const uint32_t to = tmem_base + O_COL + t * O_STEP + half * (D / 2) + lane_off;  // its output columns
+    const int col0 = half * 64;
+    float* const xch = reinterpret_cast<float*>(smem + L::XCH_OFF) + t * 2 * BM + row;  // + parity * 4 BM + half * BM
+    uint64_t* const pair_bar = &bars->pair[t][quad];
+    uint32_t xs = 0;  // exchanges so far (parity of the buffer, phase of pair_bar)
+    // The value that the other thread of this row passes in the same exchange.  The buffers alternate: a thread writes one
+    // again only after the partner has arrived at the exchange in between, i.e. has read it.
+    auto exchange = [&](float v, float& other) -> bool {
+      float* const x = xch + (xs & 1u) * 4 * BM;
+      x[half * BM] = v;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(pair_bar);
+      if (!mbar_wait(pair_bar, xs & 1u, abort_flag)) return false;
+      other = x[(half ^ 1) * BM];
+      ++xs;
+      return true;
+    };
     const float sl2 = p.scale * LOG2E;
+    const uint64_t sl2x2 = pack_f32x2(sl2, sl2);
     // The running maximum starts at the lowest value that stays finite when scaled, not at -inf: a row whose keys so far all
     // score -inf then has probabilities 2^(-inf) = 0, where -inf - -inf would be NaN.
     const float m_low = sl2 > 1.f ? -FLT_MAX / sl2 : -FLT_MAX;
@@ -341,32 +379,36 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
       const int n_it = 2 * q2 + 1 + t;
       const int pos = q2 * 2 * BM + t * BM + row;  // this thread's position in the sequence
       const bool row_ok = pos < p.S;
-      const bool traced = (item == static_cast<int>(blockIdx.x)) && quad == 2;
-      float m_run = m_low, l_run = 0.f;
+      float m_run = m_low, l_run = 0.f;  // l_run: over this thread's keys
       for (int j = 0; j < n_it && ok; ++j, ++cs) {
         if (!mbar_wait(&bars->s_full[t], cs & 1u, abort_flag)) { ok = false; break; }
         tc_fence_after_sync();
-        if (traced) { PP_TRACE(1 + t, j, 0); }
         const bool diag = (j == n_it - 1);
         uint32_t r0[32], r1[32];
-        // pass 1: row maximum
-        float mx = -INFINITY;
         tmem_ld_32x32(ts, r0);
         tmem_ld_32x32(ts + 32, r1);
         tmem_ld_wait();
-        if (!diag) { mx = chunk_max<false>(r0, 0, row, mx); mx = chunk_max<false>(r1, 32, row, mx); }
-        else       { mx = chunk_max<true>(r0, 0, row, mx);  mx = chunk_max<true>(r1, 32, row, mx); }
-        tmem_ld_32x32(ts + 64, r0);
-        tmem_ld_32x32(ts + 96, r1);
-        tmem_ld_wait();
-        if (!diag) { mx = chunk_max<false>(r0, 64, row, mx); mx = chunk_max<false>(r1, 96, row, mx); }
-        else       { mx = chunk_max<true>(r0, 64, row, mx);  mx = chunk_max<true>(r1, 96, row, mx); }
+        if (SEP) {  // all scores of the step are in registers: the next products may overwrite them
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->s_read[t]);
+        }
+        float mx = -INFINITY, mo;
+        if (!diag) { mx = chunk_max<false>(r0, col0, row, mx); mx = chunk_max<false>(r1, col0 + 32, row, mx); }
+        else       { mx = chunk_max<true>(r0, col0, row, mx);  mx = chunk_max<true>(r1, col0 + 32, row, mx); }
+        // (in place, the exchange also keeps this thread's probabilities behind the partner's reads of the same columns)
+        tc_fence_before_sync();
+        if (!exchange(mx, mo)) { ok = false; break; }
+        tc_fence_after_sync();
         // keep the old maximum while the new one is at most 2^8 above it: no rescaling of O, values stay in range
-        float m_new = fmaxf(m_run, mx);
+        float m_new = fmaxf(m_run, fmaxf(mx, mo));
         if (j > 0 && (m_new - m_run) * sl2 <= 8.f) m_new = m_run;
         const float alpha = j == 0 ? 0.f : ex2_approx((m_run - m_new) * sl2);
         const float mb = m_new * sl2;
-        if (traced) { PP_TRACE(1 + t, j, 1); }
+        const uint64_t neg_mb = pack_f32x2(-mb, -mb);
+        uint64_t acc[2] = {0ull, 0ull};
+        uint32_t pk[16];
+        if (!diag) chunk_exp<false>(r0, col0, row, sl2x2, neg_mb, acc, pk); else chunk_exp<true>(r0, col0, row, sl2x2, neg_mb, acc, pk);
         const bool rescale = j > 0 && __any_sync(0xffffffffu, alpha != 1.f);
         if (j > 0 && (SEP || rescale)) {
           // O_t (and P_t, where it has columns of its own) belongs to P V of step j-1 until that has completed; in place it
@@ -374,78 +416,62 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
           if (!mbar_wait(&bars->o_done[t], (cs - 1u) & 1u, abort_flag)) { ok = false; break; }
           tc_fence_after_sync();
         }
+        tmem_st_32x16(tp, pk);
+        if (!diag) chunk_exp<false>(r1, col0 + 32, row, sl2x2, neg_mb, acc, pk); else chunk_exp<true>(r1, col0 + 32, row, sl2x2, neg_mb, acc, pk);
+        tmem_st_32x16(tp + 16, pk);
         if (rescale) {
 #pragma unroll 1
-          for (int c = 0; c < D / 32; ++c) {
-            uint32_t r[32];
-            tmem_ld_32x32(to + c * 32, r);
+          for (int c = 0; c < D / 64; ++c) {
+            uint32_t o[32];
+            tmem_ld_32x32(to + c * 32, o);
             tmem_ld_wait();
             uint32_t lo[16], hi[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
-              lo[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-              hi[i] = __float_as_uint(__uint_as_float(r[16 + i]) * alpha);
+              lo[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+              hi[i] = __float_as_uint(__uint_as_float(o[16 + i]) * alpha);
             }
             tmem_st_32x16(to + c * 32, lo);
             tmem_st_32x16(to + c * 32 + 16, hi);
           }
         }
-        if (traced) { PP_TRACE(1 + t, j, 2); }
-        // pass 2: exponentials; chunk c of 32 keys becomes 16 packed columns at [16 c, 16 c + 16), in place always behind the reads
-        float rs = 0.f;
-        uint32_t pk[16];
-        tmem_ld_32x32(ts, r0);
-        tmem_ld_32x32(ts + 32, r1);
-        tmem_ld_wait();
-        if (!diag) rs += chunk_exp<false>(r0, 0, row, sl2, mb, pk); else rs += chunk_exp<true>(r0, 0, row, sl2, mb, pk);
-        tmem_ld_32x32(ts + 64, r0);  // in flight during the next exponentials
-        tmem_st_32x16(tp, pk);
-        if (!diag) rs += chunk_exp<false>(r1, 32, row, sl2, mb, pk); else rs += chunk_exp<true>(r1, 32, row, sl2, mb, pk);
-        tmem_ld_32x32(ts + 96, r1);
-        tmem_st_32x16(tp + 16, pk);
-        tmem_ld_wait();
-        if (SEP) {
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bars->s_read[t]);
-        }
-        if (!diag) rs += chunk_exp<false>(r0, 64, row, sl2, mb, pk); else rs += chunk_exp<true>(r0, 64, row, sl2, mb, pk);
-        tmem_st_32x16(tp + 32, pk);
-        if (!diag) rs += chunk_exp<false>(r1, 96, row, sl2, mb, pk); else rs += chunk_exp<true>(r1, 96, row, sl2, mb, pk);
-        tmem_st_32x16(tp + 48, pk);
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->p_full[t]);
-        if (traced) { PP_TRACE(1 + t, j, 3); }
-        l_run = l_run * alpha + rs;
+        float a0, a1;
+        unpack_f32x2(add_f32x2(acc[0], acc[1]), a0, a1);
+        l_run = l_run * alpha + (a0 + a1);
         m_run = m_new;
       }
       if (!ok) break;
-      // epilogue of the item: normalise and store this thread's output row, then hand the accumulator back
+      // epilogue of the item: normalise and store this thread's half of the output row, then hand the accumulator back
+      float l_other;
+      if (!exchange(l_run, l_other)) { ok = false; break; }
+      l_run += l_other;
       if (!mbar_wait(&bars->o_done[t], (cs - 1u) & 1u, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
       const float inv = 1.f / l_run;
-      __nv_bfloat16* orow = p.o + (static_cast<size_t>(b) * p.S + pos) * HD + h * D;
+      __nv_bfloat16* orow = p.o + (static_cast<size_t>(b) * p.S + pos) * HD + h * D + half * (D / 2);
 #pragma unroll 1
-      for (int c = 0; c < D / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32(to + c * 32, r);
+      for (int c = 0; c < D / 64; ++c) {
+        uint32_t o[32];
+        tmem_ld_32x32(to + c * 32, o);
         tmem_ld_wait();
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           uint4 v;
-          v.x = pack_bf16(__uint_as_float(r[q * 8 + 0]) * inv, __uint_as_float(r[q * 8 + 1]) * inv);
-          v.y = pack_bf16(__uint_as_float(r[q * 8 + 2]) * inv, __uint_as_float(r[q * 8 + 3]) * inv);
-          v.z = pack_bf16(__uint_as_float(r[q * 8 + 4]) * inv, __uint_as_float(r[q * 8 + 5]) * inv);
-          v.w = pack_bf16(__uint_as_float(r[q * 8 + 6]) * inv, __uint_as_float(r[q * 8 + 7]) * inv);
+          v.x = pack_bf16(__uint_as_float(o[q * 8 + 0]) * inv, __uint_as_float(o[q * 8 + 1]) * inv);
+          v.y = pack_bf16(__uint_as_float(o[q * 8 + 2]) * inv, __uint_as_float(o[q * 8 + 3]) * inv);
+          v.z = pack_bf16(__uint_as_float(o[q * 8 + 4]) * inv, __uint_as_float(o[q * 8 + 5]) * inv);
+          v.w = pack_bf16(__uint_as_float(o[q * 8 + 6]) * inv, __uint_as_float(o[q * 8 + 7]) * inv);
           if (row_ok) *reinterpret_cast<uint4*>(orow + c * 32 + q * 8) = v;
         }
       }
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->o_free[t]);
-      if (p.lse != nullptr && row_ok)
+      if (half == 0 && p.lse != nullptr && row_ok)
         p.lse[(static_cast<size_t>(b) * p.H + h) * p.S + pos] = (m_run * sl2 + log2f(l_run)) * LN2;
     }
   }
@@ -470,14 +496,6 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
 }  // namespace fsb
 
 // C ABI.  Any S >= 1, D in {64, 128}; returns -1 otherwise.  Tensors are contiguous and 16-byte aligned.
-// Debug aid: a device buffer of 416 uint64 receives nanosecond stamps [role][step][4] of the first item of CTA 0 and, from
-// entry 384, the issuer's clock64 per step; nullptr switches it off.
-static unsigned long long* g_pp_trace = nullptr;
-FSB_API int fsb_attn_pp_set_trace(void* buf) {
-  g_pp_trace = static_cast<unsigned long long*>(buf);
-  return 0;
-}
-
 FSB_API int fsb_attn_fwd_pingpong(const void* qkv, void* o, float* lse, int B, int S, int H, int D, float scale, int* status,
                                   cudaStream_t stream) {
   using namespace fsb;
@@ -487,7 +505,7 @@ FSB_API int fsb_attn_fwd_pingpong(const void* qkv, void* o, float* lse, int B, i
   if (!fsb_host::encode_3d_16bit(&tm, qkv, (uint64_t)3 * H * D, (uint64_t)S, (uint64_t)B, (uint64_t)3 * H * D, (uint64_t)3 * H * D * S, 64, BM, 1)) return -1;
   Params p{};
   p.B = B; p.S = S; p.H = H; p.D = D; p.scale = scale;
-  p.o = static_cast<__nv_bfloat16*>(o); p.lse = lse; p.status = status; p.trace = g_pp_trace;
+  p.o = static_cast<__nv_bfloat16*>(o); p.lse = lse; p.status = status;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
