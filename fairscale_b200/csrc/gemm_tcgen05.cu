@@ -63,9 +63,9 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   const int tiles_per_problem = tiles_m * tiles_n;
   const int num_tiles = tiles_per_problem * (BATCHED ? p.batch : 1);
   const int num_kb = (p.K + BLOCK_K - 1) / BLOCK_K;
-  auto load_tile = [&](void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
-    if (BATCHED) tma_load_3d(dst, map, bar, x, y, z);
-    else         tma_load_2d(dst, map, bar, x, y);
+  auto load_tile = [&](uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
+    if (BATCHED) tma_load_3d_warp(dst, map, bar, x, y, z);
+    else         tma_load_2d_warp(dst, map, bar, x, y);
   };
 
   if (threadIdx.x == 0) {
@@ -116,56 +116,58 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   };
 
   if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      auto fetch = [&](int before) -> int {  // `before`: the last index this CTA was given
-        return static_cast<int>(gridDim.x) + (counted ? static_cast<int>(atomicAdd(&sched[0], 1u)) : before);
-      };
-      int nxt = fetch(static_cast<int>(blockIdx.x));  // needed when the first tile's loads are all on their way
-      for (int tile = blockIdx.x, next_tile = -1; tile >= 0 && ok; tile = next_tile) {
-        const int pb = BATCHED ? tile / tiles_per_problem : 0;
-        int tm, tn;
-        tile_coords(tile - pb * tiles_per_problem, tiles_m, tiles_n, tm, tn);
-        const int m0 = tm * BLOCK_M, n0 = tn * BLOCK_N;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
-          uint8_t* sa = smem + stage * L::STAGE_BYTES;
-          uint8_t* sb = sa + L::A_BYTES;
-          mbar_expect_tx(&full_bar[stage], L::STAGE_BYTES);
-          const int k0 = kb * BLOCK_K;
-          if (!p.a_mn_major) {
-            load_tile(sa, &tmap_a, &full_bar[stage], k0, m0, pb);
-          } else {
+    // ------------------------------------------------------------------ TMA producer (the whole warp, as in the CTA-pair kernel below and for the same reason)
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    auto fetch = [&](int before) -> int {  // `before`: the last index this CTA was given; lane 0 holds the result
+      return static_cast<int>(gridDim.x) + (counted ? (lane == 0 ? static_cast<int>(atomicAdd(&sched[0], 1u)) : 0) : before);
+    };
+    const uint32_t smem0 = smem_u32(smem), full0 = smem_u32(full_bar);
+    int nxt = fetch(static_cast<int>(blockIdx.x));  // needed when the first tile's loads are all on their way
+    for (int tile = blockIdx.x, next_tile = -1; tile >= 0 && ok; tile = next_tile) {
+      const int pb = BATCHED ? tile / tiles_per_problem : 0;
+      int tm, tn;
+      tile_coords(tile - pb * tiles_per_problem, tiles_m, tiles_n, tm, tn);
+      const int m0 = tm * BLOCK_M, n0 = tn * BLOCK_N;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
+        const uint32_t sa = smem0 + stage * L::STAGE_BYTES, sb = sa + L::A_BYTES, bar = full0 + stage * 8;
+        mbar_expect_tx_warp(bar, L::STAGE_BYTES);
+        const int k0 = kb * BLOCK_K;
+        if (!p.a_mn_major) {
+          load_tile(sa, &tmap_a, bar, k0, m0, pb);
+        } else {
 #pragma unroll
-            for (int j = 0; j < BLOCK_M / 64; ++j) load_tile(sa + j * 8192, &tmap_a, &full_bar[stage], m0 + j * 64, k0, pb);
-          }
-          if (!p.b_mn_major) {
-            load_tile(sb, &tmap_b, &full_bar[stage], k0, n0, pb);
-          } else {
-#pragma unroll
-            for (int j = 0; j < BLOCK_N / 64; ++j) load_tile(sb + j * 8192, &tmap_b, &full_bar[stage], n0 + j * 64, k0, pb);
-          }
-          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          for (int j = 0; j < BLOCK_M / 64; ++j) load_tile(sa + j * 8192, &tmap_a, bar, m0 + j * 64, k0, pb);
         }
-        if (!ok) break;
-        // the other roles are a ring of loads behind and look for the next index after this
-        next_tile = nxt < num_tiles ? nxt : -1;
-        if (!mbar_wait(&sched_empty[q], qphase ^ 1u, abort_flag)) break;
+        if (!p.b_mn_major) {
+          load_tile(sb, &tmap_b, bar, k0, n0, pb);
+        } else {
+#pragma unroll
+          for (int j = 0; j < BLOCK_N / 64; ++j) load_tile(sb + j * 8192, &tmap_b, bar, n0 + j * 64, k0, pb);
+        }
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+      }
+      if (!ok) break;
+      // the other roles are a ring of loads behind and look for the next index after this
+      nxt = __shfl_sync(0xffffffffu, nxt, 0);
+      next_tile = nxt < num_tiles ? nxt : -1;
+      if (!mbar_wait_warp(&sched_empty[q], qphase ^ 1u, abort_flag)) break;
+      if (lane == 0) {
         sched_tile[q] = next_tile;
         mbar_arrive(&sched_full[q]);
-        if (++q == SCHED_DEPTH) { q = 0; qphase ^= 1u; }
-        if (next_tile >= 0) nxt = fetch(next_tile);  // used one tile from now
       }
-      if (counted) {
-        // The last CTA to get here has seen every CTA's final fetch (each adds to sched[1] after the value of its last fetch
-        // came back, so no fence is needed): put the counters back for the next launch.
-        if (atomicAdd(&sched[1], 1u) == gridDim.x - 1u) {
-          sched[0] = 0u;
-          sched[1] = 0u;
-        }
+      __syncwarp();
+      if (++q == SCHED_DEPTH) { q = 0; qphase ^= 1u; }
+      if (next_tile >= 0) nxt = fetch(next_tile);  // used one tile from now
+    }
+    if (counted && lane == 0) {
+      // The last CTA to get here has seen every CTA's final fetch (each adds to sched[1] after the value of its last fetch
+      // came back, so no fence is needed): put the counters back for the next launch.
+      if (atomicAdd(&sched[1], 1u) == gridDim.x - 1u) {
+        sched[0] = 0u;
+        sched[1] = 0u;
       }
     }
   } else if (warp == 1) {
@@ -253,20 +255,23 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
 // shared-memory traffic per MMA drops by a third and 6 stages fit. CTA 0 (the leader) issues the MMAs;
 // both CTAs load with their own per-CTA TMA (nothing is broadcast), and both drain their half of the
 // accumulator. Barriers: full[] lives in the leader and counts both CTAs' bytes; empty[] and tmem_full[]
-// exist in both CTAs and are signalled by two commits (local + peer); tmem_empty[] lives in the leader
+// exist in both CTAs and are signalled by one commit to both; tmem_empty[] lives in the leader
 // and collects the 8 epilogue warps of the pair.
 // ------------------------------------------------------------------------------------------------
 constexpr int PAIR_BLOCK_N = 256;
 constexpr int PAIR_HALF_N = 128;
-constexpr int PAIR_STAGES = 6;
 constexpr int PAIR_EPI_WARPS = 8;                        // two per TMEM lane quadrant, 128 columns each
 constexpr int PAIR_THREADS = 64 + 32 * PAIR_EPI_WARPS;   // producer warp + MMA warp + epilogue warps
 
+// MH: blocks of 128 rows that each CTA of the pair owns.  1: tiles of 256 x 256, two accumulators in TMEM; 2: tiles of
+// 512 x 256, whose two row blocks fill TMEM (see the kernel).
+template <int MH>
 struct PairSmem {
-  static constexpr int A_BYTES = BLOCK_M * BLOCK_K * 2;      // 16 KB: this CTA's 128 rows
-  static constexpr int B_BYTES = PAIR_HALF_N * BLOCK_K * 2;  // 16 KB: this CTA's 128 columns
+  static constexpr int STAGES = MH == 1 ? 6 : 4;
+  static constexpr int A_BYTES = MH * BLOCK_M * BLOCK_K * 2;  // 16 KB per row block
+  static constexpr int B_BYTES = PAIR_HALF_N * BLOCK_K * 2;   // 16 KB: this CTA's 128 columns
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int EPI_OFFSET = PAIR_STAGES * STAGE_BYTES;           // 4 KB of staging per epilogue warp
+  static constexpr int EPI_OFFSET = STAGES * STAGE_BYTES;           // 4 KB of staging per epilogue warp
   static constexpr int BAR_OFFSET = EPI_OFFSET + PAIR_EPI_WARPS * 4096;
   // No slack for re-aligning the base: the kernel has no static shared memory, so its dynamic window starts 1024-byte
   // aligned (checked at run time).  With the 1 KB the hardware reserves per CTA this leaves 2816 bytes of the SM's
@@ -275,7 +280,12 @@ struct PairSmem {
   static constexpr int TOTAL = BAR_OFFSET + 256;
 };
 
+template <int MH>
 __device__ __forceinline__ void pair_tile_coords(const GemmParams& p, int tile, int tiles_m, int tiles_n, int& tm, int& tn) {
+  if (MH == 2) {
+    tile_coords<8>(tile, tiles_m, tiles_n, tm, tn);
+    return;
+  }
   if (p.b_ready != nullptr) {  // N-major in sending order of the pieces of B: every M tile of the rows that arrive first
     const int lin = tile / tiles_m;
     tm = tile - lin * tiles_m;
@@ -359,10 +369,19 @@ __device__ __forceinline__ bool wait_a_rows(const GemmParams& p, int r0, int r1,
   return true;
 }
 
-template <bool BATCHED>
+// MH 2, tiles of 512 x 256: the operands of a 64-wide K block are 48 KB per CTA for twice the products (64 KB in two 256 x 256
+// tiles), and a stage's barriers are paid half as often.  What bounds a long product is the power limit, and the operand stream
+// out of L2 is what can be saved there: 8192 x 2048 x 16384 (weight gradient) 486 -> 435 us, 16384 x 50304 x 2048 2696 -> 2518 us,
+// 22016 x 4096 x 4096 (weight gradient) 611 -> 555 us (cuBLAS 428, 2594, 550).  The two row blocks fill TMEM, so instead of a second pair of
+// accumulators each block is handed back as soon as the epilogue warps hold it in registers, packed to bf16: the last products
+// of a tile's second block run while the first block is read, the next tile's first ones while the second is.  Only epilogues
+// whose result is final in registers can do that; those that read another operand or write two results stay with MH 1.
+template <bool BATCHED, int MH>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, GemmParams p) {
-  using L = PairSmem;
+  using L = PairSmem<MH>;
+  constexpr int PAIR_STAGES = L::STAGES;
+  constexpr int CTA_ROWS = MH * BLOCK_M;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   if ((smem_u32(smem_raw) & 1023u) != 0u) {  // same for every thread of the pair: nothing has been set up yet
@@ -386,15 +405,23 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
   const bool leader = rank == 0;
   const int num_pairs = gridDim.x >> 1;
 
-  const int tiles_m = (p.M + 2 * BLOCK_M - 1) / (2 * BLOCK_M);
+  const int tiles_m = (p.M + 2 * CTA_ROWS - 1) / (2 * CTA_ROWS);
   const int tiles_n = (p.N + PAIR_BLOCK_N - 1) / PAIR_BLOCK_N;
   const int tiles_per_problem = tiles_m * tiles_n;
   const int num_tiles = tiles_per_problem * (BATCHED ? p.batch : 1);
   const int num_kb = (p.K + BLOCK_K - 1) / BLOCK_K;
-  auto load_tile = [&](void* dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
-    if (BATCHED) tma_load_3d_pair(dst, map, bar, x, y, z);
-    else         tma_load_2d_pair(dst, map, bar, x, y);
+  auto load_tile = [&](uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
+    if (BATCHED) tma_load_3d_pair_warp(dst, map, bar, x, y, z);
+    else         tma_load_2d_pair_warp(dst, map, bar, x, y);
   };
+  // Index of this pair's first tile (lane 0 of the leader's producer warp): on its way while the pair sets itself up.
+  unsigned int* const sched = g_sched_counters + 2 * p.sched_slot;
+  const bool counted = p.sched_slot != 0;
+  auto fetch = [&](int before) -> int {  // `before`: the last index this pair was given
+    return counted ? static_cast<int>(atomicAdd(&sched[0], 1u)) : before + num_pairs;
+  };
+  int first = 0;
+  if (leader && threadIdx.x == 0) first = fetch(static_cast<int>(blockIdx.x >> 1) - num_pairs);
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -434,88 +461,88 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
   // Tiles are handed out at run time: the leader's producer takes the next index from a counter in global memory and
   // publishes it (or -1 at the end) to both CTAs through a small ring; every role reads the ring in order.  An SM that
   // is slowed down or taken by a kernel of another stream (a collective) then simply works off fewer tiles, instead of
-  // holding back the tiles a static schedule would have given it.  A launch without a counter strides through the tiles.
-  unsigned int* const sched = g_sched_counters + 2 * p.sched_slot;
-  const bool counted = p.sched_slot != 0;
+  // holding back the ones a static schedule would have given it.  A launch without a counter strides through the tiles.
+  // No fence of cluster scope is on the way of an index: it is a remote store that completes on the reader's barrier, and a
+  // slot is handed back by a CTA-scope arrive.  (With plain stores, release and acquire at cluster scope the MMA warp stood
+  // still for 2 400 cycles a tile of 20 400, 8192 x 8192 x 2048, and the producers for about as long.)
   // Reader side: wait for slot q, take the index, hand the slot back to the leader.
   auto take_tile = [&](int q, uint32_t qphase, int site) -> int {
-    if (!mbar_wait_cluster(&sched_full[q], qphase, abort_flag, site)) return -2;
+    if (!mbar_wait(&sched_full[q], qphase, abort_flag, site)) return -2;
     const int t = sched_tile[q];
-    mbar_arrive_cluster(map_to_cta(smem_u32(&sched_empty[q]), 0));
+    mbar_arrive_remote(map_to_cta(smem_u32(&sched_empty[q]), 0));
     return t;
   };
 
   if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      int q = 0;
-      uint32_t qphase = 0;
-      bool ok = true;
-      // Leader: `cur` is the tile to load now (already published), `nxt` the one after it.  Indices are published one
-      // tile ahead, so the other roles find theirs without waiting, and fetched one more tile ahead, so the atomic's
-      // round trip hides behind a whole tile of loads.
-      auto publish = [&](int t) -> bool {
-        if (!mbar_wait(&sched_empty[q], qphase ^ 1u, abort_flag, 2)) return false;
-        sched_tile[q] = t;
-        st_shared_cluster_u32(map_to_cta(smem_u32(const_cast<int*>(&sched_tile[q])), 1), static_cast<uint32_t>(t));
-        mbar_arrive_cluster(map_to_cta(smem_u32(&sched_full[q]), 0));
-        mbar_arrive_cluster(map_to_cta(smem_u32(&sched_full[q]), 1));
-        if (++q == SCHED_DEPTH) { q = 0; qphase ^= 1u; }
-        return true;
-      };
-      auto fetch = [&](int before) -> int {  // `before`: the last index this pair was given
-        return counted ? static_cast<int>(atomicAdd(&sched[0], 1u)) : before + num_pairs;
-      };
-      int cur = -1, nxt = -1;
-      int b_upto = -1;  // highest B piece known to have arrived
-      if (leader) {
-        cur = fetch(static_cast<int>(blockIdx.x >> 1) - num_pairs);
-        if (cur >= num_tiles) cur = -1;
-        ok = publish(cur);
-        if (cur >= 0) nxt = fetch(cur);
+    // ------------------------------------------------------------------ TMA producer (both CTAs, the whole warp)
+    // Like the MMAs, the loads are issued from uniform control flow by an elected lane: inside a one-lane branch every
+    // operand of a load has to be moved to a uniform register first, and the four loads that a K block of MN-major operands
+    // takes cost more than its 512 cycles of tensor time (weight gradient 8192 x 2048 x 16384: 631 -> 543 cycles per block).
+    int stage = 0;
+    uint32_t phase = 0;
+    int q = 0;
+    uint32_t qphase = 0;
+    bool ok = true;
+    auto publish = [&](int t) -> bool {
+      if (!mbar_wait_warp(&sched_empty[q], qphase ^ 1u, abort_flag, 2)) return false;
+      if (lane == 0) {
+#pragma unroll
+        for (uint32_t c = 0; c < 2; ++c) {
+          const uint32_t fb = map_to_cta(smem_u32(&sched_full[q]), c);
+          mbar_expect_tx_remote(fb, 4);
+          st_async_u32(map_to_cta(smem_u32(const_cast<int*>(&sched_tile[q])), c), static_cast<uint32_t>(t), fb);
+        }
       }
-      while (ok) {
-        int tile;
-        if (leader) {
-          tile = cur;
-          if (tile >= 0) {
-            const int nt = nxt < num_tiles ? nxt : -1;
-            if (!publish(nt)) break;
-            cur = nt;
-            if (nt >= 0) nxt = fetch(nt);  // used one tile from now
-          }
-        } else {
-          tile = take_tile(q, qphase, 3);
-          if (++q == SCHED_DEPTH) { q = 0; qphase ^= 1u; }
-        }
-        if (tile < 0) break;
-        const int pb = BATCHED ? tile / tiles_per_problem : 0;
-        int tm, tn;
-        pair_tile_coords(p, tile - pb * tiles_per_problem, tiles_m, tiles_n, tm, tn);
-        const int m0 = tm * 2 * BLOCK_M + static_cast<int>(rank) * BLOCK_M;
-        const int n0 = tn * PAIR_BLOCK_N + static_cast<int>(rank) * PAIR_HALF_N;
-        if (p.b_ready != nullptr && n0 < p.N) {
-          const long long row_bytes = static_cast<long long>(p.K) * 2;
-          const int n1 = n0 + PAIR_HALF_N < p.N ? n0 + PAIR_HALF_N : p.N;
-          if (!wait_b_pieces(p, n0 * row_bytes, n1 * row_bytes, b_upto, abort_flag)) break;
-        }
-        if (p.a_ready != nullptr && m0 < p.M) {
-          if (!wait_a_rows(p, m0, m0 + BLOCK_M < p.M ? m0 + BLOCK_M : p.M, b_upto, abort_flag)) break;
-        }
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, 4)) { ok = false; break; }
-          uint8_t* sa = smem + stage * L::STAGE_BYTES;
-          uint8_t* sb = sa + L::A_BYTES;
-          if (leader) mbar_expect_tx(&full_bar[stage], 2 * L::STAGE_BYTES);
-          const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0);
+      __syncwarp();
+      if (++q == SCHED_DEPTH) { q = 0; qphase ^= 1u; }
+      return true;
+    };
+    auto take = [&]() -> int {  // the peer's side of the ring
+      int t = 0;
+      if (lane == 0) t = take_tile(q, qphase, 3);
+      if (++q == SCHED_DEPTH) { q = 0; qphase ^= 1u; }
+      return __shfl_sync(0xffffffffu, t, 0);
+    };
+    // The next index is fetched before the loads of the current tile and published behind the first of them: the atomic's
+    // round trip hides, the readers find theirs without waiting, and neither holds up a tile's first loads.
+    const int publish_kb = num_kb < PAIR_STAGES ? num_kb : PAIR_STAGES;
+    int b_upto = -1;  // highest B piece known to have arrived
+    int tile;
+    if (leader) {
+      tile = __shfl_sync(0xffffffffu, first, 0);
+      if (tile >= num_tiles) tile = -1;
+      ok = publish(tile);
+    } else {
+      tile = take();
+    }
+    const uint32_t smem0 = smem_u32(smem), full_local = smem_u32(full_bar), full0 = map_to_cta(full_local, 0);
+    while (ok && tile >= 0) {
+      const int pb = BATCHED ? tile / tiles_per_problem : 0;
+      int tm, tn;
+      pair_tile_coords<MH>(p, tile - pb * tiles_per_problem, tiles_m, tiles_n, tm, tn);
+      const int m0 = (tm * 2 + static_cast<int>(rank)) * CTA_ROWS;
+      const int n0 = tn * PAIR_BLOCK_N + static_cast<int>(rank) * PAIR_HALF_N;
+      // (every lane waits and fences: any of them may be the one that issues the loads)
+      if (MH == 1 && p.b_ready != nullptr && n0 < p.N) {
+        const long long row_bytes = static_cast<long long>(p.K) * 2;
+        const int n1 = n0 + PAIR_HALF_N < p.N ? n0 + PAIR_HALF_N : p.N;
+        if (!__all_sync(0xffffffffu, wait_b_pieces(p, n0 * row_bytes, n1 * row_bytes, b_upto, abort_flag))) break;
+      }
+      if (MH == 1 && p.a_ready != nullptr && m0 < p.M) {
+        if (!__all_sync(0xffffffffu, wait_a_rows(p, m0, m0 + BLOCK_M < p.M ? m0 + BLOCK_M : p.M, b_upto, abort_flag))) break;
+      }
+      auto load_blocks = [&](int kb0, int kb1) -> bool {
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag, 4)) return false;
+          const uint32_t sa = smem0 + stage * L::STAGE_BYTES, sb = sa + L::A_BYTES, bar = full0 + stage * 8;
+          if (leader) mbar_expect_tx_warp(full_local + stage * 8, 2 * L::STAGE_BYTES);
           const int k0 = kb * BLOCK_K;
           if (!p.a_mn_major) {
-            load_tile(sa, &tmap_a, bar, k0, m0, pb);
+#pragma unroll
+            for (int h = 0; h < MH; ++h) load_tile(sa + h * 16384, &tmap_a, bar, k0, m0 + h * BLOCK_M, pb);
           } else {
 #pragma unroll
-            for (int j = 0; j < BLOCK_M / 64; ++j) load_tile(sa + j * 8192, &tmap_a, bar, m0 + j * 64, k0, pb);
+            for (int j = 0; j < CTA_ROWS / 64; ++j) load_tile(sa + j * 8192, &tmap_a, bar, m0 + j * 64, k0, pb);
           }
           if (!p.b_mn_major) {
             load_tile(sb, &tmap_b, bar, k0, n0, pb);
@@ -525,15 +552,27 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
           }
           if (++stage == PAIR_STAGES) { stage = 0; phase ^= 1u; }
         }
+        return true;
+      };
+      int next = -1, nxt = 0;
+      if (leader && (lane == 0 || !counted)) nxt = fetch(tile);
+      if (!load_blocks(0, publish_kb)) break;
+      if (leader) {
+        const int nt = __shfl_sync(0xffffffffu, nxt, 0);
+        next = nt < num_tiles ? nt : -1;
+        if (!publish(next)) break;
       }
-      if (leader && counted) {
-        // the last pair to get here has seen every pair's final fetch: put the counters back for the next launch
+      if (!load_blocks(publish_kb, num_kb)) break;
+      if (!leader) next = take();
+      tile = next;
+    }
+    if (leader && counted && lane == 0) {
+      // the last pair to get here has seen every pair's final fetch: put the counters back for the next launch
+      __threadfence();
+      if (atomicAdd(&sched[1], 1u) == static_cast<unsigned int>(num_pairs - 1)) {
+        sched[0] = 0u;
+        sched[1] = 0u;
         __threadfence();
-        if (atomicAdd(&sched[1], 1u) == static_cast<unsigned int>(num_pairs - 1)) {
-          sched[0] = 0u;
-          sched[1] = 0u;
-          __threadfence();
-        }
       }
     }
   } else if (warp == 1) {
@@ -543,7 +582,6 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
       const uint32_t a_lbo = p.a_mn_major ? 8192u : 16u, b_lbo = p.b_mn_major ? 8192u : 16u;
       const uint32_t a_kstep = p.a_mn_major ? 2048u : 32u, b_kstep = p.b_mn_major ? 2048u : 32u;
       const uint64_t adesc0 = make_smem_desc(smem_u32(smem), a_lbo, 1024u), bdesc0 = make_smem_desc(smem_u32(smem) + L::A_BYTES, b_lbo, 1024u);
-      const uint32_t empty0 = map_to_cta(smem_u32(empty_bar), 0), empty1 = map_to_cta(smem_u32(empty_bar), 1);
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -557,26 +595,38 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
         tile = __shfl_sync(0xffffffffu, tile, 0);
         if (++q == SCHED_DEPTH) { q = 0; qphase ^= 1u; }
         if (tile < 0) break;
-        if (!mbar_wait_warp(&tmem_empty_bar[acc], acc_phase ^ 1u, abort_flag, 6)) { ok = false; break; }
-        tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * PAIR_BLOCK_N);
+        if (MH == 1) {
+          if (!mbar_wait_warp(&tmem_empty_bar[acc], acc_phase ^ 1u, abort_flag, 6)) { ok = false; break; }
+          tc_fence_after_sync();
+        }
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag, 7)) { ok = false; break; }
           tc_fence_after_sync();
           const uint64_t ad = desc_offset(adesc0, stage * L::STAGE_BYTES), bd = desc_offset(bdesc0, stage * L::STAGE_BYTES);
 #pragma unroll
-          for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
-            umma_f16_ss_pair_warp(d_tmem, desc_offset(ad, k * a_kstep), desc_offset(bd, k * b_kstep), idesc, (kb | k) != 0 ? 1u : 0u);
-          umma_commit_pair_warp(empty0 + stage * 8);
-          umma_commit_pair_warp(empty1 + stage * 8);
+          for (int h = 0; h < MH; ++h) {
+            if (MH == 2 && kb == 0) {
+              if (!mbar_wait_warp(&tmem_empty_bar[h], acc_phase ^ 1u, abort_flag, 6)) { ok = false; break; }
+              tc_fence_after_sync();
+            }
+            const uint32_t d_tmem = tmem_base + static_cast<uint32_t>((MH == 1 ? acc : h) * PAIR_BLOCK_N);
+#pragma unroll
+            for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
+              umma_f16_ss_pair_warp(d_tmem, desc_offset(ad, h * 16384 + k * a_kstep), desc_offset(bd, k * b_kstep), idesc, (kb | k) != 0 ? 1u : 0u);
+            if (MH == 2 && kb == num_kb - 1) umma_commit_pair_warp(&tmem_full_bar[h]);
+          }
+          if (!ok) break;
+          umma_commit_pair_warp(&empty_bar[stage]);
           if (++stage == PAIR_STAGES) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
-        const uint32_t fb = smem_u32(&tmem_full_bar[acc]);
-        umma_commit_pair_warp(map_to_cta(fb, 0));
-        umma_commit_pair_warp(map_to_cta(fb, 1));
-        acc ^= 1;
-        if (acc == 0) acc_phase ^= 1u;
+        if (MH == 1) {
+          umma_commit_pair_warp(&tmem_full_bar[acc]);
+          acc ^= 1;
+          if (acc == 0) acc_phase ^= 1u;
+        } else {
+          acc_phase ^= 1u;
+        }
       }
     }
   } else {
@@ -599,23 +649,60 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
       if (tile < 0) break;
       const int pb = BATCHED ? tile / tiles_per_problem : 0;
       int tm, tn;
-      pair_tile_coords(p, tile - pb * tiles_per_problem, tiles_m, tiles_n, tm, tn);
+      pair_tile_coords<MH>(p, tile - pb * tiles_per_problem, tiles_m, tiles_n, tm, tn);
       const GemmParams pt = BATCHED ? gemm_params_of_batch(p, pb) : p;
-      const int row0 = tm * 2 * BLOCK_M + static_cast<int>(rank) * BLOCK_M + quad * 32;
+      const int row0 = (tm * 2 + static_cast<int>(rank)) * CTA_ROWS + quad * 32;
       const int n0 = tn * PAIR_BLOCK_N + half * (PAIR_BLOCK_N / 2);
-      uint4 pre[8];
-      if (coalesce && epilogue_needs_aux(p.epilogue) && n0 < p.N) epi_slab_prefetch(pre, pt.aux, pt.ld_aux, row0, n0, pt.M, pt.N, lane);
-      if (!mbar_wait(&tmem_full_bar[acc], acc_phase, abort_flag, 9)) { ok = false; break; }
-      tc_fence_after_sync();
-      const uint32_t t_base = tmem_base + static_cast<uint32_t>(acc * PAIR_BLOCK_N + half * (PAIR_BLOCK_N / 2)) +
-                              (static_cast<uint32_t>(quad * 32) << 16);
-      if (coalesce) epilogue_rows_coalesced(t_base, row0, n0, PAIR_BLOCK_N / 2, pt, stage, lane, pre);
-      else          epilogue_rows<PAIR_BLOCK_N / 2>(t_base, row0 + lane, n0, pt);
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty_bar[acc]), 0));
-      acc ^= 1;
-      if (acc == 0) acc_phase ^= 1u;
+      const uint32_t t_base = tmem_base + static_cast<uint32_t>(half * (PAIR_BLOCK_N / 2)) + (static_cast<uint32_t>(quad * 32) << 16);
+      if (MH == 1) {
+        uint4 pre[8];
+        if (coalesce && epilogue_needs_aux(p.epilogue) && n0 < p.N) epi_slab_prefetch(pre, pt.aux, pt.ld_aux, row0, n0, pt.M, pt.N, lane);
+        if (!mbar_wait(&tmem_full_bar[acc], acc_phase, abort_flag, 9)) { ok = false; break; }
+        tc_fence_after_sync();
+        const uint32_t t_acc = t_base + static_cast<uint32_t>(acc * PAIR_BLOCK_N);
+        if (coalesce) epilogue_rows_coalesced(t_acc, row0, n0, PAIR_BLOCK_N / 2, pt, stage, lane, pre);
+        else          epilogue_rows<PAIR_BLOCK_N / 2>(t_acc, row0 + lane, n0, pt);
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_remote(map_to_cta(smem_u32(&tmem_empty_bar[acc]), 0));
+        acc ^= 1;
+        if (acc == 0) acc_phase ^= 1u;
+      } else {
+        // Both row blocks to registers first, each handed back at once: the next tile's products wait for nothing else.  So the
+        // bias waits in the staging buffer already (read from global memory it cost an L2 round trip per 64 columns there).
+        uint32_t pk[2][64];
+        __nv_bfloat16* const bias = pt.epilogue == EPI_BIAS ? reinterpret_cast<__nv_bfloat16*>(stage) : nullptr;
+        if (bias != nullptr) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) bias[lane * 4 + i] = n0 + lane * 4 + i < pt.N ? pt.bias[n0 + lane * 4 + i] : __float2bfloat16_rn(0.f);
+          __syncwarp();
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (!mbar_wait(&tmem_full_bar[h], acc_phase, abort_flag, 9)) { ok = false; break; }
+          tc_fence_after_sync();
+#pragma unroll
+          for (int c = 0; c < 2; ++c) epi_pack64(t_base + static_cast<uint32_t>(h * PAIR_BLOCK_N + c * 64), bias == nullptr ? nullptr : bias + c * 64, &pk[h][c * 32]);
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_remote(map_to_cta(smem_u32(&tmem_empty_bar[h]), 0));
+        }
+        if (!ok) break;
+        acc_phase ^= 1u;
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              *reinterpret_cast<uint4*>(stage + epi_swz(lane, k)) = make_uint4(pk[h][c * 32 + k * 4], pk[h][c * 32 + k * 4 + 1], pk[h][c * 32 + k * 4 + 2], pk[h][c * 32 + k * 4 + 3]);
+            __syncwarp();
+            epi_slab_store(stage, reinterpret_cast<__nv_bfloat16*>(pt.C), pt.ldc, row0 + h * BLOCK_M, n0 + c * 64, pt.M, pt.N, lane);
+            __syncwarp();
+          }
+        }
+      }
     }
   }
 
@@ -642,6 +729,26 @@ namespace fsb_host {
 // gemm_cluster_k.cu
 int gemm_cluster_k(const CUtensorMap& ta, const void* B, int ldb, const fsb::GemmParams& p, int block_n, int splits, int dev, cudaStream_t stream);
 }  // namespace fsb_host
+
+// Products that the 512 x 256 pair kernel takes: bf16 rows that its epilogue can store in 16-byte pieces, no operand besides a bias.
+static bool wide_takes(const fsb::GemmParams& p) {
+  return p.M >= 512 && p.N >= 256 && !p.out_f32 && (p.epilogue == fsb::EPI_NONE || p.epilogue == fsb::EPI_BIAS) && p.ldc % 8 == 0 && p.N % 8 == 0 &&
+         p.stride_c % 8 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15u) == 0 && p.b_ready == nullptr && p.a_ready == nullptr;
+}
+
+template <bool BATCHED, int MH>
+static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const fsb::GemmParams& p, int num_sms, int di, cudaStream_t stream) {
+  using namespace fsb;
+  static bool attr_set[64] = {false};  // the attribute is per device
+  if (!attr_set[di]) {
+    cudaFuncSetAttribute(gemm_bf16_tcgen05_pair_kernel<BATCHED, MH>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem<MH>::TOTAL);
+    attr_set[di] = true;
+  }
+  const long long tiles = static_cast<long long>(p.batch) * ((p.M + 2 * MH * BLOCK_M - 1) / (2 * MH * BLOCK_M)) * ((p.N + PAIR_BLOCK_N - 1) / PAIR_BLOCK_N);
+  const int pairs = tiles < num_sms / 2 ? static_cast<int>(tiles) : num_sms / 2;
+  gemm_bf16_tcgen05_pair_kernel<BATCHED, MH><<<2 * pairs, PAIR_THREADS, PairSmem<MH>::TOTAL, stream>>>(ta, tb, p);
+  return static_cast<int>(cudaGetLastError());
+}
 
 // Slot of the tile counters for a launch on `stream`: every stream keeps one of its own for the life of the process, so two
 // launches that use the same counters are ordered by their stream, however far the host runs ahead.  Streams are told apart
@@ -686,7 +793,7 @@ static bool pair_enabled() {  // FSB_GEMM_PAIR=0 disables the CTA-pair kernel
   return on;
 }
 
-// Kernel for a product that is not streamed and has no CTA cap.  Measured on B200 (us; 64-wide K blocks = kb), small products
+// Kernel for a product that is not streamed and has no CTA cap (choose_with_wide goes on from here).  Measured on B200 (us; 64-wide K blocks = kb), small products
 // back to back:
 //
 //   M, N, K              pair   one CTA 128x256   cluster split-K, block_n / splits
@@ -730,7 +837,7 @@ static bool pair_enabled() {  // FSB_GEMM_PAIR=0 disables the CTA-pair kernel
 // average, 12 % at worst; a single line at 2.56e11 operations took 4.7 %, and up to 44 % (2992 x 1976 x 13208 238 against 169 us,
 // 1936 x 5872 x 4360 139 against 110 us), always the pair 8 %, never 7 %.
 struct GemmPlan {
-  enum Kind { PAIR, ONE_CTA, CLUSTER_K } kind;
+  enum Kind { PAIR, ONE_CTA, CLUSTER_K, WIDE_PAIR } kind;
   int block_n, splits;
 };
 // Does the pair kernel pay for `problems` products of M x N x K with leading dimensions lda, ldb?
@@ -743,6 +850,28 @@ static bool pair_pays(long long problems, int M, int N, int K, int lda, int ldb,
   const float one = one_us[off_line] * num_kb * ((tiles + num_sms - 1) / num_sms);
   const float pair = 8.f + pair_us[off_line] * num_kb * ((pair_tiles + pairs - 1) / pairs);
   return pair < one;
+}
+// Which of the three persistent kernels for `problems` products that the 512 x 256 tiles can take (wide_takes), in estimated us:
+// a launch, and per wave of tiles its start and its K blocks; the share that goes with the tiles per SM instead of whole waves is
+// what the card's power limit gives back when a wave is partly empty.  Fitted to 90 products (M and N 256 .. 16384, K 256 .. 32000,
+// one or 4 to 16 stacked, all operand layouts, a third with rows off the 128-byte lines): taking the lowest estimate costs 0.8 %
+// over the fastest kernel on average, taking pair_pays' choice between the other two 9.6 %.  Measured (us, wide / pair / one CTA):
+//   16384 x 6144 x 2048 287 / 313 / 326       8192 x 2048 x 16384 (wgrad) 435 / 486 / 486     50304 x 2048 x 16384 (wgrad) 2576 / 3055 / 2847
+//   4096 x 12288 x 4096 317 / 306 / 342        2048 x 2048 x 16384 (wgrad) 167 / 120 / 124     16384 x 50304 x 2048 2518 / 2696 / 2898
+//   8 x 2048 x 1024 x 4096 115 / 125 / 139     8192 x 3072 x 1024 53.3 / 53.6 / 51.1           2792 x 3968 x 256 16.4 / 20.2 / 14.4
+static GemmPlan::Kind choose_with_wide(long long problems, int M, int N, int K, int lda, int ldb, int num_sms) {
+  const long long tiles_n = (N + 255) / 256;
+  auto tiles = [&](int rows) -> long long { return problems * ((M + rows - 1) / rows) * tiles_n; };
+  const int off_line = (lda % 64 != 0) + (ldb % 64 != 0);
+  const float num_kb = static_cast<float>((K + fsb::BLOCK_K - 1) / fsb::BLOCK_K);
+  auto cost = [&](long long n, int units, float launch, float start, float per_wave, float per_share) -> float {
+    const float waves = static_cast<float>((n + units - 1) / units), share = static_cast<float>(n) / units;
+    return launch + waves * (start + num_kb * per_wave) + num_kb * share * per_share;
+  };
+  const float wide = cost(tiles(512), num_sms / 2, 7.2f, 2.0f, 0.52f, 0.25f);
+  const float pair = cost(tiles(256), num_sms / 2, 7.2f, 2.2f, 0.262f + 0.017f * off_line, 0.16f);
+  const float one = cost(tiles(128), num_sms, 5.0f, 1.1f, 0.229f + 0.064f * off_line, 0.25f);
+  return wide <= pair && wide <= one ? GemmPlan::WIDE_PAIR : pair < one ? GemmPlan::PAIR : GemmPlan::ONE_CTA;
 }
 static GemmPlan choose_gemm_plan(int M, int N, int K, int lda, int ldb, int num_sms, bool pair_allowed) {
   const long long tiles_m = (M + fsb::BLOCK_M - 1) / fsb::BLOCK_M;
@@ -769,8 +898,8 @@ static GemmPlan choose_gemm_plan(int M, int N, int K, int lda, int ldb, int num_
   return best;
 }
 
-// The kernel that a product (or `problems` stacked ones) would get on a device with `num_sms` SMs: 0 CTA pairs, 1 one CTA per
-// tile, 2 split-K over clusters (a single product only).
+// The kernel that a product (or `problems` stacked ones) whose epilogue the wide tiles do not take would get on a device with
+// `num_sms` SMs: 0 CTA pairs, 1 one CTA per tile, 2 split-K over clusters (a single product only).
 FSB_API int fsb_gemm_plan_of(long long problems, int M, int N, int K, int lda, int ldb, int num_sms) {
   if (problems > 1) return pair_enabled() && pair_pays(problems, M, N, K, lda, ldb, num_sms) ? 0 : 1;
   return static_cast<int>(choose_gemm_plan(M, N, K, lda, ldb, num_sms, pair_enabled()).kind);
@@ -805,11 +934,11 @@ FSB_API int fsb_gemm_bf16_cluster_k(const void* A, const void* B, void* C, const
 }
 
 // The same product by one of the persistent kernels whatever its size: plan 1 one CTA per tile, 2 CTA pairs (M and N at
-// least 256, -1 otherwise).  fsb_gemm_bf16 chooses these by itself.
+// least 256, -1 otherwise), 3 CTA pairs with tiles of 512 rows (what wide_takes, -1 otherwise).  fsb_gemm_bf16 chooses these by itself.
 FSB_API int fsb_gemm_bf16_plan(const void* A, const void* B, void* C, const void* bias, const void* aux, void* aux_out,
                                int M, int N, int K, int lda, int ldb, int ldc, int ld_aux, int a_mn_major, int b_mn_major,
                                int epilogue, int out_f32, int accumulate_c, int plan, int* status, cudaStream_t stream) {
-  if (plan != 1 && !(plan == 2 && M >= 256 && N >= 256)) return -1;
+  if (plan != 1 && !((plan == 2 || plan == 3) && M >= 256 && N >= 256)) return -1;
   return gemm_bf16_impl(A, B, C, bias, aux, aux_out, M, N, K, lda, ldb, ldc, ld_aux, a_mn_major, b_mn_major, epilogue, out_f32,
                         accumulate_c, 0, status, stream, nullptr, 0u, 0, 0ull, nullptr, 0, 0, 0, 0, 0, 0, 0, plan);
 }
@@ -898,26 +1027,22 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* bia
   const bool streamed = b_ready != nullptr || a_ready != nullptr;  // only the pair kernel waits for arriving operands
   GemmPlan plan = {GemmPlan::ONE_CTA, block_n, 1};
   if (streamed) plan.kind = GemmPlan::PAIR;
-  else if (forced != 0) plan.kind = forced == 2 ? GemmPlan::PAIR : GemmPlan::ONE_CTA;
-  else if (max_ctas == 0) plan = choose_gemm_plan(M, N, K, lda, ldb, num_sms, pair_enabled());
+  else if (forced == 3 && !wide_takes(p)) return -1;
+  else if (forced != 0) plan.kind = forced == 3 ? GemmPlan::WIDE_PAIR : forced == 2 ? GemmPlan::PAIR : GemmPlan::ONE_CTA;
+  else if (max_ctas == 0) {
+    plan = choose_gemm_plan(M, N, K, lda, ldb, num_sms, pair_enabled());
+    // more tiles than one wave of single CTAs (below, the wide tiles leave most SMs without one) and K as far as it was measured
+    if (tiles > num_sms && K >= 256 && pair_enabled() && wide_takes(p)) plan.kind = choose_with_wide(1, M, N, K, lda, ldb, num_sms);
+  }
   if (plan.kind == GemmPlan::CLUSTER_K) return fsb_host::gemm_cluster_k(ta, B, ldb, p, plan.block_n, plan.splits, dev, stream);
   // Run-time tile hand-out for products large enough to share the device with a collective; small ones stride.
-  if (max_ctas == 0 && M >= 256 && N >= 256 && (plan.kind == GemmPlan::PAIR || tiles > num_sms)) {
+  if (max_ctas == 0 && M >= 256 && N >= 256 && (plan.kind == GemmPlan::PAIR || plan.kind == GemmPlan::WIDE_PAIR || tiles > num_sms)) {
     p.sched_slot = sched_slot_of(di, stream);
   }
-  if (plan.kind == GemmPlan::PAIR) {
+  if (plan.kind == GemmPlan::PAIR || plan.kind == GemmPlan::WIDE_PAIR) {
     // the B map's box is this CTA's 128 columns (K-major) / 64 (MN-major, unchanged)
     if (!b_mn_major && !fsb_host::encode_2d_16bit(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BLOCK_K, PAIR_HALF_N)) return -1;
-    static bool pair_attr_set[64] = {false};
-    if (!pair_attr_set[di]) {
-      cudaFuncSetAttribute(gemm_bf16_tcgen05_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem::TOTAL);
-      pair_attr_set[di] = true;
-    }
-    const int pair_tiles = ((M + 2 * BLOCK_M - 1) / (2 * BLOCK_M)) * ((N + PAIR_BLOCK_N - 1) / PAIR_BLOCK_N);
-    const int max_pairs = num_sms / 2;
-    const int pairs = pair_tiles < max_pairs ? pair_tiles : max_pairs;
-    gemm_bf16_tcgen05_pair_kernel<false><<<2 * pairs, PAIR_THREADS, PairSmem::TOTAL, stream>>>(ta, tb, p);
-    return static_cast<int>(cudaGetLastError());
+    return plan.kind == GemmPlan::PAIR ? launch_pair<false, 1>(ta, tb, p, num_sms, di, stream) : launch_pair<false, 2>(ta, tb, p, num_sms, di, stream);
   }
   if (block_n == 256) {
     if (!attr_set[di][0]) {
@@ -975,18 +1100,16 @@ static int gemm_bf16_batched_impl(const void* A, const void* B, void* C, const v
   cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
   const long long tiles = static_cast<long long>(batch) * ((M + BLOCK_M - 1) / BLOCK_M) * ((N + block_n - 1) / block_n);
   const int grid = tiles < num_sms ? static_cast<int>(tiles) : num_sms;
-  if (forced == 2 || (forced == 0 && pair_enabled() && pair_pays(batch, M, N, K, lda, ldb, num_sms))) {
+  if (forced == 3 && !wide_takes(p)) return -1;
+  GemmPlan::Kind kind = forced == 3 ? GemmPlan::WIDE_PAIR : forced == 2 ? GemmPlan::PAIR : GemmPlan::ONE_CTA;
+  if (forced == 0 && pair_enabled()) {
+    if (pair_pays(batch, M, N, K, lda, ldb, num_sms)) kind = GemmPlan::PAIR;
+    if (tiles > num_sms && K >= 256 && wide_takes(p)) kind = choose_with_wide(batch, M, N, K, lda, ldb, num_sms);
+  }
+  if (kind != GemmPlan::ONE_CTA) {
     if (!b_mn_major && !fsb_host::encode_3d_16bit(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)batch, (uint64_t)ldb, (uint64_t)stride_b, BLOCK_K, PAIR_HALF_N, 1)) return -1;
-    static bool pair_attr_set[64] = {false};
-    if (!pair_attr_set[dev & 63]) {
-      cudaFuncSetAttribute(gemm_bf16_tcgen05_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem::TOTAL);
-      pair_attr_set[dev & 63] = true;
-    }
-    const long long pair_tiles = static_cast<long long>(batch) * ((M + 2 * BLOCK_M - 1) / (2 * BLOCK_M)) * ((N + PAIR_BLOCK_N - 1) / PAIR_BLOCK_N);
-    const int pairs = pair_tiles < num_sms / 2 ? static_cast<int>(pair_tiles) : num_sms / 2;
     p.sched_slot = sched_slot_of(dev & 63, stream);
-    gemm_bf16_tcgen05_pair_kernel<true><<<2 * pairs, PAIR_THREADS, PairSmem::TOTAL, stream>>>(ta, tb, p);
-    return static_cast<int>(cudaGetLastError());
+    return kind == GemmPlan::WIDE_PAIR ? launch_pair<true, 2>(ta, tb, p, num_sms, dev & 63, stream) : launch_pair<true, 1>(ta, tb, p, num_sms, dev & 63, stream);
   }
   static bool attr_set_dev[64][2] = {{false}};  // the attribute is per device
   bool* attr_set = attr_set_dev[dev & 63];
@@ -1020,7 +1143,7 @@ FSB_API int fsb_gemm_bf16_batched_plan(const void* A, const void* B, void* C, co
                                   int M, int N, int K, int lda, int ldb, int ldc, int ld_aux, long long stride_a, long long stride_b,
                                   long long stride_c, long long stride_aux, long long stride_bias, int a_mn_major, int b_mn_major,
                                   int epilogue, int out_f32, int accumulate_c, int plan, int* status, cudaStream_t stream) {
-  if (plan != 1 && !(plan == 2 && M >= 256 && N >= 256)) return -1;
+  if (plan != 1 && !((plan == 2 || plan == 3) && M >= 256 && N >= 256)) return -1;
   return gemm_bf16_batched_impl(A, B, C, bias, aux, aux_out, batch, M, N, K, lda, ldb, ldc, ld_aux, stride_a, stride_b, stride_c, stride_aux, stride_bias, a_mn_major, b_mn_major,
                            epilogue, out_f32, accumulate_c, status, stream, plan);
 }

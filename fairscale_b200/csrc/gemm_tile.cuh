@@ -80,9 +80,9 @@ struct SmemLayout {
   static constexpr int TOTAL = EPI_OFFSET + 4 * 4096 + 1024;  // + slack for 1024-byte alignment
 };
 
+template <int GROUP_M = 16>
 __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, int& tm, int& tn) {
-  // Groups of 16 M-tiles walk N together, so concurrently running CTAs share A and B slabs in L2.
-  constexpr int GROUP_M = 16;
+  // Groups of GROUP_M M-tiles walk N together, so concurrently running CTAs share A and B slabs in L2.
   const int per_group = GROUP_M * tiles_n;
   const int g = tile / per_group;
   const int first_m = g * GROUP_M;
@@ -242,6 +242,30 @@ __device__ __forceinline__ void epi_row_to_stage(uint8_t* stage, const float (&v
 #pragma unroll
     for (int i = 0; i < 8; ++i) o.v[i] = __float2bfloat16_rn(v[c * 8 + i]);
     *reinterpret_cast<uint4*>(stage + epi_swz(lane, c)) = o.raw;
+  }
+}
+
+// This thread's row of 64 accumulator columns packed to bf16, after adding the 64 values at `bias` (shared memory, or none).
+__device__ __forceinline__ void epi_pack64(uint32_t taddr, const __nv_bfloat16* bias, uint32_t* pk) {
+  uint32_t r0[32], r1[32];
+  tmem_ld_32x32(taddr, r0);
+  tmem_ld_32x32(taddr + 32, r1);
+  tmem_ld_wait();
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(c < 4 ? r0[(c & 3) * 8 + i] : r1[(c & 3) * 8 + i]);
+    if (bias != nullptr) {
+      const Vec16<__nv_bfloat16> b = ld16(bias + c * 8);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] += __bfloat162float(b.v[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+      pk[c * 4 + i] = *reinterpret_cast<const uint32_t*>(&b);
+    }
   }
 }
 

@@ -412,6 +412,40 @@ def test_persistent_gemm_kernels(M, N, K, a_mn, b_mn, plan):
     _status_ok()
 
 
+# The CTA-pair kernel with tiles of 512 x 256 (plan 3): one tile, remainders in M, N and K, more tiles than pairs, stacked problems, a
+# bias that starts off a 16-byte boundary.  It sums K in the order of the 256 x 256 tiles: every result is the same to the bit.
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("E,M,N,K", [(1, 512, 256, 64), (1, 520, 264, 8), (1, 776, 1000, 264), (1, 5128, 4360, 520), (3, 1032, 264, 200), (5, 2056, 2056, 136)])
+def test_wide_pair_gemm(E, M, N, K, a_mn, b_mn):
+    from ctypes import c_int, c_longlong, c_void_p
+
+    from fairscale_b200.ops import _bind
+
+    _bind._SIGNATURES.setdefault("fsb_gemm_bf16_plan", [c_void_p] * 6 + [c_int] * 13 + [c_void_p] * 2)
+    _bind._SIGNATURES.setdefault("fsb_gemm_bf16_batched_plan", [c_void_p] * 6 + [c_int] * 8 + [c_longlong] * 5 + [c_int] * 6 + [c_void_p, c_void_p])
+    torch.manual_seed(M + N + K)
+    a, b = (torch.randn(*s, device=_dev()).bfloat16() for s in ((E, M, K), (E, N, K)))
+    bias = torch.randn(E * N + 1, device=_dev()).bfloat16()[1:].view(E, N)
+    sa, sb = (t.transpose(1, 2).contiguous() if mn else t for t, mn in ((a, a_mn), (b, b_mn)))
+    ref = a.double() @ b.double().transpose(1, 2)
+
+    def run(epi, plan):
+        c = torch.full((E, M, N), float("nan"), device=_dev(), dtype=torch.bfloat16)
+        ptrs = (sa.data_ptr(), sb.data_ptr(), c.data_ptr(), bias.data_ptr() if epi else None, None, None)
+        tail = (int(a_mn), int(b_mn), epi, 0, 0, plan, _bind.status_ptr(_dev()), _bind.stream_ptr(_dev()))
+        if E == 1:
+            _bind.call("fsb_gemm_bf16_plan", *ptrs, M, N, K, sa.stride(1), sb.stride(1), N, 0, *tail)
+        else:
+            _bind.call("fsb_gemm_bf16_batched_plan", *ptrs, E, M, N, K, sa.stride(1), sb.stride(1), N, 0, sa.stride(0), sb.stride(0), M * N, 0, N, *tail)
+        return c
+
+    for epi, want in ((0, ref), (1, ref + bias.double().unsqueeze(1))):
+        got = run(epi, 3)
+        assert _rel_err(got, want) < 1e-2
+        assert torch.equal(got, run(epi, 2))
+    _status_ok()
+
+
 @pytest.mark.parametrize("plan", [0, 1, 2])
 @pytest.mark.parametrize("E,C,K,N", [(2, 256, 256, 256), (3, 257, 72, 264), (3, 257, 264, 264), (4, 410, 512, 2048), (1, 300, 64, 256), (17, 300, 264, 520)])
 def test_batched_gemm_edges(E, C, K, N, plan):
