@@ -10,9 +10,12 @@
 //   backward dQ (items of 128 query rows)      S = Q K^T, dP = dO V^T -> dS -> dQ += dS K
 //   backward dK/dV (items of 128 key rows)     S^T = K Q^T, dP^T = V dO^T -> P^T, dS^T -> dV += P^T dO, dK += dS^T Q
 //
-// This file holds the backward.  Thread roles per CTA (576 threads): warp 0 TMA producer, warp 1 MMA issuer (+TMEM
-// allocation), warps 2..17 four groups of four "softmax" warps, one thread per accumulator row (TMEM lane == row), which do
-// the exponentials in registers and hand the bf16 results back to the tensor cores through TMEM.
+// This file holds the backward.  Thread roles per CTA (608 threads): warp 0 TMA producer, warp 1 issuer of the score products
+// (+TMEM allocation), warps 2..17 four groups of four "softmax" warps, one thread per accumulator row (TMEM lane == row), which
+// do the exponentials in registers and hand the bf16 results back to the tensor cores through TMEM, warp 18 issuer of the
+// accumulating products.  An issuing warp is held until the tensor pipe takes its products, and a wait that does not block
+// costs it 100 - 200 cycles all the same; one warp for all products left the pipe idle behind its waits (B2 S8192 H16 D64: of
+// 1 290 cycles a step of 64 queries or keys, 650 of products, while the probabilities of the step lay ready for 1 500).
 // A K-major tile [rows, 64] and an MN-major tile of the same bytes differ only in the MMA descriptor, so each
 // streamed tile is loaded once and used both as a "transposed" and a "plain" operand.
 // Any sequence length: the tensor maps are three-dimensional (columns, positions, batch), so a tile that overhangs the
@@ -27,7 +30,8 @@
 
 namespace fsb {
 
-constexpr int ATT_THREADS = 576;  // TMA warp + MMA warp + 16 compute warps (four per TMEM lane quadrant)
+constexpr int ATT_THREADS = 608;  // TMA warp, MMA warp, 16 compute warps (four per TMEM lane quadrant), second MMA warp
+constexpr int ATT_ACC_WARP = 18;  // the second MMA warp: accumulating products
 constexpr int ATT_BM = 128;  // rows owned by a CTA (TMEM lanes)
 constexpr float LOG2E = 1.4426950408889634f;
 
@@ -76,6 +80,7 @@ struct AttnBars {
   uint64_t str_empty[6];  // streamed stage free again
   uint64_t s_full[3];     // scores and dP of a step are in buffer b
   uint64_t p_full[3];     // the 8 warps of the step have written dS (dQ kernel) / P^T and dS^T (dK/dV kernel) over them
+  uint64_t buf_free[3];   // the accumulating products that read buffer b have completed
   uint64_t acc_done;      // the item's accumulating products have completed
   uint64_t acc_free;      // the 16 compute warps have read the item's output accumulators
   uint32_t tmem_slot;
@@ -94,6 +99,7 @@ __device__ __forceinline__ void attn_init_bars(AttnBars* b) {
   for (int i = 0; i < 3; ++i) {
     mbar_init(&b->s_full[i], 1);
     mbar_init(&b->p_full[i], 8);
+    mbar_init(&b->buf_free[i], 1);
   }
   mbar_init(&b->acc_done, 1);
   mbar_init(&b->acc_free, 16);
@@ -144,9 +150,8 @@ __device__ __forceinline__ void dq_cols16(const uint32_t (&rs)[16], const uint32
 // Backward of B2 S8192 H16 D64: 1870 us with eight warps that all worked on the same step and passed dS through shared
 // memory, 1447 us with the two sets (B8 S2048 H16 D128 750 -> 690 us).
 // dS overwrites scores that the same thread has read (32 keys become the first 16 of their 32 columns) and feeds dS K as
-// the TMEM A operand, so it does not pass through shared memory.  The tensor pipe executes in issue order,
-//   S,dP(0) .. S,dP(n-1) | dQ(0)  S,dP(n)  dQ(1)  S,dP(n+1) ...        with n score buffers, step u in buffer u mod n,
-// so S(u+n), issued behind dQ(u), cannot overwrite dS(u) early and the buffers need no "empty" barriers.  Head size 64
+// the TMEM A operand, so it does not pass through shared memory.  Step u uses buffer u mod n; one warp issues S and dP of
+// step u + n as soon as dQ(u), issued by another warp, has read the buffer (buf_free).  Head size 64
 // leaves TMEM for three buffers: a set that has finished step u then finds the scores of step u + 2 ready, where with two
 // it waits for dQ(u) and those products (backward of B2 S8192 H16 D64 1447 -> 1315 us).
 // =================================================================================================
@@ -229,54 +234,61 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    // MMA issuer: the whole warp, see umma_f16_ss_warp
+    // Issuer of S and dP: the whole warp, see umma_f16_ss_warp.  Step u = key tile u / 2, keys [64 (u & 1), +64) of it; stages
+    // and buffers go round over the steps of all items.
     const uint32_t idesc_s = make_idesc_f16(ATT_BM, 64, true, false, false);
-    const uint32_t idesc_q = make_idesc_f16(ATT_BM, D, true, false, true);  // dS K : dS from TMEM, K tile read MN-major
     const uint64_t dq = desc_kmajor(smem_u32(smem + L::Q_OFF)), ddo = desc_kmajor(smem_u32(smem + L::DO_OFF));
     const uint64_t dk0 = desc_kmajor(smem_u32(smem + L::K_OFF)), dv0 = desc_kmajor(smem_u32(smem + L::V_OFF));
-    const uint64_t dkt0 = desc_mnmajor(smem_u32(smem + L::K_OFF), SLAB);
-    uint32_t jt0 = 0, ut0 = 0, it = 0;  // key tiles / steps of earlier items, items so far
+    uint32_t st = 0, st_phase = 0, buf = 0, buf_phase = 0, it = 0;
     bool ok = true;
-    // step u = key tile u / 2, keys [64 (u & 1), +64) of it; buffers go round over the steps of all items
-    auto issue_sp = [&](int u, int n_steps) -> bool {
-      const uint32_t jt = jt0 + (u >> 1);
-      const int hh = u & 1, st = jt % L::STAGES, buf = (ut0 + u) % NBUF;
-      if (hh == 0 && !mbar_wait_warp(&bars->str_full[st], (jt / L::STAGES) & 1u, abort_flag, 35)) return false;
-      tc_fence_after_sync();
-      const uint32_t off = st * L::TILE + hh * 8192u;  // rows 64 hh .. of every slab
-      const uint64_t dk = desc_offset(dk0, off), dv = desc_offset(dv0, off);
-#pragma unroll
-      for (int ks = 0; ks < D / 16; ++ks)
-        umma_f16_ss_warp(tmem_base + buf * 128, desc_offset(dq, kstep_kmajor(ks, SLAB)), desc_offset(dk, kstep_kmajor(ks, SLAB)), idesc_s, ks != 0);
-#pragma unroll
-      for (int ks = 0; ks < D / 16; ++ks)
-        umma_f16_ss_warp(tmem_base + buf * 128 + 64, desc_offset(ddo, kstep_kmajor(ks, SLAB)), desc_offset(dv, kstep_kmajor(ks, SLAB)), idesc_s, ks != 0);
-      umma_commit_warp(&bars->s_full[buf]);
-      if (u == n_steps - 1) umma_commit_warp(&bars->stat_empty);  // the item's last use of Q and dO
-      return true;
-    };
     for (int item; ok && (item = snake_item(static_cast<int>(it))) < n_items; ++it) {
       const int qt = n_qt - 1 - item / HB;
       const int n_steps = 2 * (qt + 1);
       if (!mbar_wait_warp(&bars->stat_full, it & 1u, abort_flag, 37)) { ok = false; break; }
-      for (int u = 0; u < NBUF && u < n_steps && ok; ++u) ok = issue_sp(u, n_steps);
-      for (int u = 0; u < n_steps && ok; ++u) {
-        const uint32_t jt = jt0 + (u >> 1), ut = ut0 + u;
-        const int hh = u & 1, st = jt % L::STAGES, buf = ut % NBUF;
-        // the dQ accumulator still belongs to the previous item until its threads have read it
-        if (u == 0 && !mbar_wait_warp(&bars->acc_free, (it & 1u) ^ 1u, abort_flag, 38)) { ok = false; break; }
-        if (!mbar_wait_warp(&bars->p_full[buf], (ut / NBUF) & 1u, abort_flag, 39)) { ok = false; break; }
+      for (int u = 0; u < n_steps; ++u) {
+        if ((u & 1) == 0 && !mbar_wait_warp(&bars->str_full[st], st_phase, abort_flag, 35)) { ok = false; break; }
+        if (!mbar_wait_warp(&bars->buf_free[buf], buf_phase ^ 1u, abort_flag, 36)) { ok = false; break; }
         tc_fence_after_sync();
-        const uint64_t dkt = desc_offset(dkt0, st * L::TILE + hh * 4 * 2048u);
+        const uint32_t off = st * L::TILE + (u & 1) * 8192u;  // rows 64 (u & 1) .. of every slab
+        const uint64_t dk = desc_offset(dk0, off), dv = desc_offset(dv0, off);
+        const uint32_t t_s = tmem_base + buf * 128;
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks)
+          umma_f16_ss_warp(t_s, desc_offset(dq, kstep_kmajor(ks, SLAB)), desc_offset(dk, kstep_kmajor(ks, SLAB)), idesc_s, ks != 0);
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks)
+          umma_f16_ss_warp(t_s + 64, desc_offset(ddo, kstep_kmajor(ks, SLAB)), desc_offset(dv, kstep_kmajor(ks, SLAB)), idesc_s, ks != 0);
+        umma_commit_warp(&bars->s_full[buf]);
+        if (u == n_steps - 1) umma_commit_warp(&bars->stat_empty);  // the item's last use of Q and dO
+        if (++buf == NBUF) { buf = 0; buf_phase ^= 1u; }
+        if ((u & 1) != 0 && ++st == L::STAGES) { st = 0; st_phase ^= 1u; }
+      }
+    }
+  } else if (warp == ATT_ACC_WARP) {
+    // Issuer of dQ += dS K: dS from TMEM, K tile read MN-major.  (Its stage is full: S of the step was made of it.)
+    const uint32_t idesc_q = make_idesc_f16(ATT_BM, D, true, false, true);
+    const uint64_t dkt0 = desc_mnmajor(smem_u32(smem + L::K_OFF), SLAB);
+    uint32_t st = 0, buf = 0, buf_phase = 0, it = 0;
+    bool ok = true;
+    for (int item; ok && (item = snake_item(static_cast<int>(it))) < n_items; ++it) {
+      const int qt = n_qt - 1 - item / HB;
+      const int n_steps = 2 * (qt + 1);
+      // the dQ accumulator still belongs to the previous item until its threads have read it
+      if (!mbar_wait_warp(&bars->acc_free, (it & 1u) ^ 1u, abort_flag, 38)) { ok = false; break; }
+      for (int u = 0; u < n_steps; ++u) {
+        if (!mbar_wait_warp(&bars->p_full[buf], buf_phase, abort_flag, 39)) { ok = false; break; }
+        tc_fence_after_sync();
+        const uint64_t dkt = desc_offset(dkt0, st * L::TILE + (u & 1) * 4 * 2048u);
+        const uint32_t t_s = tmem_base + buf * 128;
 #pragma unroll
         for (int ks = 0; ks < 64 / 16; ++ks)
-          umma_f16_ts_warp(tmem_base + DQ_COL, tmem_base + buf * 128 + (ks >> 1) * 32 + (ks & 1) * 8, desc_offset(dkt, kstep_mnmajor(ks)), idesc_q, (u | ks) != 0);
-        if (hh == 1) umma_commit_warp(&bars->str_empty[st]);
+          umma_f16_ts_warp(tmem_base + DQ_COL, t_s + (ks >> 1) * 32 + (ks & 1) * 8, desc_offset(dkt, kstep_mnmajor(ks)), idesc_q, (u | ks) != 0);
+        umma_commit_warp(&bars->buf_free[buf]);
+        if ((u & 1) != 0) umma_commit_warp(&bars->str_empty[st]);
         if (u == n_steps - 1) umma_commit_warp(&bars->acc_done);
-        if (u + NBUF < n_steps && !issue_sp(u + NBUF, n_steps)) { ok = false; break; }
+        if (++buf == NBUF) { buf = 0; buf_phase ^= 1u; }
+        if ((u & 1) != 0 && ++st == L::STAGES) st = 0;
       }
-      jt0 += static_cast<uint32_t>(n_steps >> 1);
-      ut0 += static_cast<uint32_t>(n_steps);
     }
   } else {
     const int quad = warp & 3;
@@ -380,8 +392,8 @@ __device__ __forceinline__ void dkv_cols16(const uint32_t (&rs)[16], const uint3
 // Backward, dK / dV: one CTA per 128 key rows; streams 64-row Q / dO sub-tiles with their statistics (copied to shared
 // memory with the tiles: read from global memory where they are used, each first touch cost an L2 round trip inside the
 // softmax chain).  The same scheme as the dQ kernel: two sets of eight warps take alternate sub-tiles, P^T and dS^T overwrite
-// their own scores in TMEM and are the A operands of the accumulating products, and head size 64 has three score buffers;
-// the tensor pipe runs  S,dP(0) .. S,dP(n-1) | dV,dK(0)  S,dP(n)  dV,dK(1)  S,dP(n+1) ...
+// their own scores in TMEM and are the A operands of the accumulating products, head size 64 has three score buffers, and two
+// warps issue, one the score products, one the accumulating ones.
 // =================================================================================================
 constexpr int KV_QSUB = 64;
 
@@ -478,46 +490,50 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    // MMA issuer: the whole warp, see umma_f16_ss_warp
-    const uint32_t idesc_s = make_idesc_f16(ATT_BM, KV_QSUB, true, false, false);  // K Q^T, V dO^T
-    const uint32_t idesc_a = make_idesc_f16(ATT_BM, D, true, false, true);         // P^T dO, dS^T Q (A in TMEM, B MN-major)
+    // Issuer of S^T(t) = K Q_t^T and dP^T(t) = V dO_t^T: the whole warp, see umma_f16_ss_warp.  Stages and buffers go round over
+    // the sub-tiles of all items.
+    const uint32_t idesc_s = make_idesc_f16(ATT_BM, KV_QSUB, true, false, false);
     const uint64_t dk = desc_kmajor(smem_u32(smem + L::K_OFF)), dv = desc_kmajor(smem_u32(smem + L::V_OFF));
     const uint64_t dq0 = desc_kmajor(smem_u32(smem + L::Q_OFF)), ddo0 = desc_kmajor(smem_u32(smem + L::DO_OFF));
-    const uint64_t dqt0 = desc_mnmajor(smem_u32(smem + L::Q_OFF), QSLAB), ddot0 = desc_mnmajor(smem_u32(smem + L::DO_OFF), QSLAB);
-    uint32_t tt0 = 0, it = 0;
+    uint32_t st = 0, st_phase = 0, buf = 0, buf_phase = 0, it = 0;
     bool ok = true;
-    // S^T(t) = K Q_t^T and dP^T(t) = V dO_t^T; buffers go round over the sub-tiles of all items
-    auto issue_sp = [&](int t, int n_sub) -> bool {
-      const uint32_t tt = tt0 + t;
-      const int st = tt % L::STAGES, buf = tt % NBUF;
-      if (!mbar_wait_warp(&bars->str_full[st], (tt / L::STAGES) & 1u, abort_flag, 67)) return false;
-      tc_fence_after_sync();
-      const uint64_t dq = desc_offset(dq0, st * L::QTILE), ddo = desc_offset(ddo0, st * L::QTILE);
-      const uint32_t t_s = tmem_base + buf * BUF_STEP;
-#pragma unroll
-      for (int ks = 0; ks < D / 16; ++ks)
-        umma_f16_ss_warp(t_s, desc_offset(dk, kstep_kmajor(ks, SLAB)), desc_offset(dq, kstep_kmajor(ks, QSLAB)), idesc_s, ks != 0);
-#pragma unroll
-      for (int ks = 0; ks < D / 16; ++ks)
-        umma_f16_ss_warp(t_s + 64, desc_offset(dv, kstep_kmajor(ks, SLAB)), desc_offset(ddo, kstep_kmajor(ks, QSLAB)), idesc_s, ks != 0);
-      umma_commit_warp(&bars->s_full[buf]);
-      if (t == n_sub - 1) umma_commit_warp(&bars->stat_empty);  // the item's last use of the K and V tiles
-      return true;
-    };
     for (int item; ok && (item = snake_item(static_cast<int>(it))) < n_items; ++it) {
       const int kt = item / HB;
       const int n_sub = p.S_pad / KV_QSUB - kt * (ATT_BM / KV_QSUB);
       if (!mbar_wait_warp(&bars->stat_full, it & 1u, abort_flag, 69)) { ok = false; break; }
-      for (int t = 0; t < NBUF && t < n_sub && ok; ++t) ok = issue_sp(t, n_sub);
-      for (int t = 0; t < n_sub && ok; ++t) {
-        const uint32_t tt = tt0 + t;
-        const int st = tt % L::STAGES;
-        const uint64_t dqt = desc_offset(dqt0, st * L::QTILE), ddot = desc_offset(ddot0, st * L::QTILE);
-        // dK / dV still belong to the previous item until its threads have read them
-        if (t == 0 && !mbar_wait_warp(&bars->acc_free, (it & 1u) ^ 1u, abort_flag, 70)) { ok = false; break; }
-        const int buf = tt % NBUF;
-        if (!mbar_wait_warp(&bars->p_full[buf], (tt / NBUF) & 1u, abort_flag, 71)) { ok = false; break; }
+      for (int t = 0; t < n_sub; ++t) {
+        if (!mbar_wait_warp(&bars->str_full[st], st_phase, abort_flag, 67)) { ok = false; break; }
+        if (!mbar_wait_warp(&bars->buf_free[buf], buf_phase ^ 1u, abort_flag, 68)) { ok = false; break; }
         tc_fence_after_sync();
+        const uint64_t dq = desc_offset(dq0, st * L::QTILE), ddo = desc_offset(ddo0, st * L::QTILE);
+        const uint32_t t_s = tmem_base + buf * BUF_STEP;
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks)
+          umma_f16_ss_warp(t_s, desc_offset(dk, kstep_kmajor(ks, SLAB)), desc_offset(dq, kstep_kmajor(ks, QSLAB)), idesc_s, ks != 0);
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks)
+          umma_f16_ss_warp(t_s + 64, desc_offset(dv, kstep_kmajor(ks, SLAB)), desc_offset(ddo, kstep_kmajor(ks, QSLAB)), idesc_s, ks != 0);
+        umma_commit_warp(&bars->s_full[buf]);
+        if (t == n_sub - 1) umma_commit_warp(&bars->stat_empty);  // the item's last use of the K and V tiles
+        if (++buf == NBUF) { buf = 0; buf_phase ^= 1u; }
+        if (++st == L::STAGES) { st = 0; st_phase ^= 1u; }
+      }
+    }
+  } else if (warp == ATT_ACC_WARP) {
+    // Issuer of dV += P^T dO and dK += dS^T Q (A in TMEM, B MN-major)
+    const uint32_t idesc_a = make_idesc_f16(ATT_BM, D, true, false, true);
+    const uint64_t dqt0 = desc_mnmajor(smem_u32(smem + L::Q_OFF), QSLAB), ddot0 = desc_mnmajor(smem_u32(smem + L::DO_OFF), QSLAB);
+    uint32_t st = 0, buf = 0, buf_phase = 0, it = 0;
+    bool ok = true;
+    for (int item; ok && (item = snake_item(static_cast<int>(it))) < n_items; ++it) {
+      const int kt = item / HB;
+      const int n_sub = p.S_pad / KV_QSUB - kt * (ATT_BM / KV_QSUB);
+      // dK / dV still belong to the previous item until its threads have read them
+      if (!mbar_wait_warp(&bars->acc_free, (it & 1u) ^ 1u, abort_flag, 70)) { ok = false; break; }
+      for (int t = 0; t < n_sub; ++t) {
+        if (!mbar_wait_warp(&bars->p_full[buf], buf_phase, abort_flag, 71)) { ok = false; break; }
+        tc_fence_after_sync();
+        const uint64_t dqt = desc_offset(dqt0, st * L::QTILE), ddot = desc_offset(ddot0, st * L::QTILE);
         const uint32_t t_s = tmem_base + buf * BUF_STEP;
 #pragma unroll
         for (int ks = 0; ks < KV_QSUB / 16; ++ks)
@@ -525,11 +541,12 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_cons
 #pragma unroll
         for (int ks = 0; ks < KV_QSUB / 16; ++ks)
           umma_f16_ts_warp(tmem_base + DK_COL, t_s + 64 + (ks >> 1) * 32 + (ks & 1) * 8, desc_offset(dqt, kstep_mnmajor(ks)), idesc_a, (t | ks) != 0);
+        umma_commit_warp(&bars->buf_free[buf]);
         umma_commit_warp(&bars->str_empty[st]);
         if (t == n_sub - 1) umma_commit_warp(&bars->acc_done);
-        if (t + NBUF < n_sub && !issue_sp(t + NBUF, n_sub)) { ok = false; break; }
+        if (++buf == NBUF) { buf = 0; buf_phase ^= 1u; }
+        if (++st == L::STAGES) st = 0;
       }
-      tt0 += static_cast<uint32_t>(n_sub);
     }
   } else {
     const int quad = warp & 3;

@@ -9,8 +9,8 @@
 //   softmax A   :          [ softmax A(j) ............ ]              [ softmax A(j+1) ............ ]
 //   softmax B   :                    [ softmax B(j) ............ ]              [ softmax B(j+1) ..... ]
 //
-// Roles (576 threads): warp 0 TMA producer, warp 1 MMA issuer and TMEM owner, warps 2-9 softmax of tile A, warps 10-17
-// softmax of tile B.  Two threads share a query row (TMEM lane), 64 of a step's 128 keys each: they read their scores once and
+// Roles (608 threads): warp 0 TMA producer, warp 1 MMA issuer and TMEM owner, warps 2-9 softmax of tile A, warps 10-17
+// softmax of tile B, warp 18 MMA issuer of tile B with head size 64 (below).  Two threads share a query row (TMEM lane), 64 of a step's 128 keys each: they read their scores once and
 // keep them in registers, pass each other the row maximum through shared memory, and with four warps per scheduler one warp's
 // loads and waits hide behind the exponentials of others.  (One thread per row read the scores twice, once for the maximum,
 // and left the exponential unit, which bounds head size 64, idle 46 % of the time: B2 S8192 H16 D64 433 -> 398 us,
@@ -27,6 +27,9 @@
 //
 //   tensor pipe :  S_A(j+1)  S_B(j+1)  PV_A(j)  PV_B(j)  S_A(j+2) ...
 //
+// and each tile has an issuer of its own: one for both held up the products of one tile behind its waits for the other
+// (B2 S8192 H16 D64 398 -> 381 us, B16 S512 H16 D64 44 -> 33 us together with the two threads a row).  With head size 128, in
+// place and bound by the products, strict turns are the faster order (B8 S2048 H16 D128 168 us, 177 with two issuers).
 // (In place, the chain exponentials -> PV -> S -> maximum kept the exponential unit, which bounds this head size, at 57 %.)
 //
 // Any sequence length: the tensor map is three-dimensional (columns, positions, batch), so a tile that overhangs the
@@ -53,7 +56,7 @@
 namespace fsb {
 namespace pp {
 
-constexpr int THREADS = 576;
+constexpr int THREADS = 608;
 constexpr int BM = 128;          // rows of a query tile == TMEM lanes
 constexpr int BN = 128;          // keys per step
 constexpr float LOG2E = 1.4426950408889634f;
@@ -69,13 +72,13 @@ struct Params {
 
 struct Bars {
   uint64_t q_full;
-  uint64_t k_full[2], k_empty[2];
+  uint64_t k_full[2], k_empty[2];  // empty: a commit of every issuer
   uint64_t v_full[2], v_empty[2];
   uint64_t s_full[2];   // per query tile: scores of the current step are in TMEM
   uint64_t p_full[2];   // per query tile: probabilities written (8 warp arrivals)
   uint64_t o_done[2];   // per query tile: P V of the current step has completed
   uint64_t s_read[2];   // per query tile, head size 64: the softmax warps hold all scores of the step (8 warp arrivals)
-  uint64_t q_empty;     // the item's last Q K^T products have completed: the query tiles may be replaced
+  uint64_t q_empty;     // the item's last Q K^T products of either tile have completed: the query tiles may be replaced
   uint64_t o_free[2];   // per query tile: the softmax warps have read the item's output accumulator (8 warp arrivals)
   uint64_t pair[2][4];  // per query tile and lane quadrant: both warps of the rows have left a value for each other (2 warp arrivals)
   uint32_t tmem_slot;
@@ -194,12 +197,13 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
 
   if (threadIdx.x == 0) {
     mbar_init(&bars->q_full, 1);
-    mbar_init(&bars->q_empty, 1);
+    constexpr int ISSUERS = SEP ? 2 : 1;
+    mbar_init(&bars->q_empty, ISSUERS);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars->k_full[i], 1);
-      mbar_init(&bars->k_empty[i], 1);
+      mbar_init(&bars->k_empty[i], ISSUERS);
       mbar_init(&bars->v_full[i], 1);
-      mbar_init(&bars->v_empty[i], 1);
+      mbar_init(&bars->v_empty[i], ISSUERS);
       mbar_init(&bars->s_full[i], 1);
       mbar_init(&bars->p_full[i], 8);
       mbar_init(&bars->o_done[i], 1);
@@ -257,23 +261,25 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
         }
       }
     }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer (the whole warp, see umma_f16_ss_warp)
+  } else if (warp == 1 || warp == 18) {
+    // ------------------------------------------------------------------ MMA issuers (whole warps, see umma_f16_ss_warp)
     const uint32_t idesc_s = make_idesc_f16(BM, BN, true, false, false);  // Q K^T: both K-major
     const uint32_t idesc_o = make_idesc_f16(BM, D, true, false, true);    // P V: P from TMEM, V MN-major
     const uint64_t dq0 = desc_kmajor(smem_u32(smem + L::Q_OFF)), dk0 = desc_kmajor(smem_u32(smem + L::K_OFF));
     const uint64_t dv0 = desc_mnmajor(smem_u32(smem + L::V_OFF), SLAB);
-    uint32_t kt0 = 0;          // key tiles consumed by earlier items
-    uint32_t cs[2] = {0, 0};   // steps issued so far per query tile (phase of p_full)
+    uint32_t kt0 = 0;           // key tiles of earlier items
+    // Counted per query tile this warp issues for (i_of), over all items:
+    uint32_t cs[2] = {0, 0};    // steps (phase of p_full)
+    uint32_t ss[2] = {0, 0};    // score products (phase of s_read)
+    uint32_t its[2] = {0, 0};   // items with that tile (phase of o_free)
+    auto i_of = [](int t) { return SEP ? 0 : t; };
     uint32_t it = 0;
-    uint32_t it_b = 0;         // items with a second query tile so far (phase of o_free[1])
-    uint32_t ss[2] = {0, 0};   // score products issued so far per query tile (phase of s_read)
     bool ok = true;
     auto issue_s = [&](int t, uint32_t kt) -> bool {
       const int st = kt & 1;
       if (!mbar_wait_warp(&bars->k_full[st], (kt >> 1) & 1u, abort_flag)) return false;
-      if (SEP && ss[t] > 0 && !mbar_wait_warp(&bars->s_read[t], (ss[t] - 1u) & 1u, abort_flag)) return false;
-      ++ss[t];
+      if (SEP && ss[i_of(t)] > 0 && !mbar_wait_warp(&bars->s_read[t], (ss[i_of(t)] - 1u) & 1u, abort_flag)) return false;
+      ++ss[i_of(t)];
       tc_fence_after_sync();
       const uint64_t dq = desc_offset(dq0, t * L::TILE), dk = desc_offset(dk0, st * L::TILE);
 #pragma unroll
@@ -283,7 +289,9 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
       return true;
     };
     auto issue_pv = [&](int t, uint32_t kt, bool first) -> bool {
-      if (!mbar_wait_warp(&bars->p_full[t], cs[t] & 1u, abort_flag)) return false;
+      // the output accumulator still belongs to the previous item until its softmax warps have read it
+      if (first && !mbar_wait_warp(&bars->o_free[t], (its[i_of(t)] & 1u) ^ 1u, abort_flag)) return false;
+      if (!mbar_wait_warp(&bars->p_full[t], cs[i_of(t)] & 1u, abort_flag)) return false;
       tc_fence_after_sync();
       const uint64_t dv = desc_offset(dv0, (kt & 1) * L::TILE);
 #pragma unroll
@@ -291,52 +299,70 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
         umma_f16_ts_warp(tmem_base + O_COL + t * O_STEP, tmem_base + P_COL + t * P_STEP + ks * 8, desc_offset(dv, kstep_mnmajor(ks)), idesc_o,
                          (!first || ks != 0) ? 1u : 0u);
       umma_commit_warp(&bars->o_done[t]);
-      ++cs[t];
+      ++cs[i_of(t)];
       return true;
     };
-    auto commit = [&](uint64_t* bar) { umma_commit_warp(bar); };
+    auto wait_k = [&](uint32_t kt) -> bool { return mbar_wait_warp(&bars->k_full[kt & 1], (kt >> 1) & 1u, abort_flag); };
+    auto wait_v = [&](uint32_t kt) -> bool { return mbar_wait_warp(&bars->v_full[kt & 1], (kt >> 1) & 1u, abort_flag); };
     for (int item; ok && (item = snake_item(static_cast<int>(it))) < n_items; ++it) {
       const int q2 = n_q2 - 1 - item / HB;
       const bool has_b = 2 * q2 + 1 < n_tiles;
       const int n_a = 2 * q2 + 1;               // key tiles seen by tile A; tile B sees one more
       const int n_kv = has_b ? n_a + 1 : n_a;
-      if (!mbar_wait_warp(&bars->q_full, it & 1u, abort_flag)) { ok = false; break; }
-      ok = issue_s(0, kt0);
-      if (ok && has_b) ok = issue_s(1, kt0);
-      if (ok) commit(&bars->k_empty[kt0 & 1]);
-      if (ok && n_kv == 1) commit(&bars->q_empty);
-      for (int j = 0; j < n_kv && ok; ++j) {
-        const uint32_t kt = kt0 + j;
-        const int st = kt & 1;
-        if (!mbar_wait_warp(&bars->v_full[st], (kt >> 1) & 1u, abort_flag)) { ok = false; break; }
-        if (SEP) {
-          // the next step's scores first: they wait for reads that come before the exponentials of this one
-          if (j + 1 < n_a && !issue_s(0, kt + 1)) { ok = false; break; }
-          if (j + 1 < n_kv) {
-            if (has_b && !issue_s(1, kt + 1)) { ok = false; break; }
-            commit(&bars->k_empty[(kt + 1) & 1]);
-            if (j + 2 == n_kv) commit(&bars->q_empty);  // that was the item's last use of the query tiles
+      if (SEP) {
+        // an issuer for each tile: neither is held up behind its waits for the other
+        const int t = warp == 1 ? 0 : 1;
+        const int n_own = t == 0 ? n_a : (has_b ? n_kv : 0);
+        if (!mbar_wait_warp(&bars->q_full, it & 1u, abort_flag)) { ok = false; break; }
+        for (int j = -1; j < n_own && ok && n_own > 0; ++j) {
+          const uint32_t kt = kt0 + j;
+          if (j + 1 < n_own) {  // the next step's scores first: they wait for reads that come before the exponentials of this one
+            if (!issue_s(t, kt + 1)) { ok = false; break; }
+            umma_commit_warp(&bars->k_empty[(kt + 1) & 1]);
+            if (j + 2 == n_own) umma_commit_warp(&bars->q_empty);  // that was the tile's last use of its queries
+          }
+          if (j >= 0) {
+            if (!wait_v(kt) || !issue_pv(t, kt, j == 0)) { ok = false; break; }
+            umma_commit_warp(&bars->v_empty[kt & 1]);
           }
         }
-        if (j == 0) {
-          // the output accumulators still belong to the previous item until its softmax warps have read them
-          if (!mbar_wait_warp(&bars->o_free[0], (it & 1u) ^ 1u, abort_flag)) { ok = false; break; }
-          if (has_b && !mbar_wait_warp(&bars->o_free[1], (it_b & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+        if (ok && n_own == 0) umma_commit_warp(&bars->q_empty);
+        its[0] += n_own > 0 ? 1u : 0u;
+        // key tiles that only the other query tile sees pass by (once they have landed: until then an earlier phase may be open)
+        for (int j = n_own; j < n_kv && ok; ++j) {
+          const uint32_t kt = kt0 + j;
+          if (!wait_k(kt)) { ok = false; break; }
+          umma_commit_warp(&bars->k_empty[kt & 1]);
+          if (!wait_v(kt)) { ok = false; break; }
+          umma_commit_warp(&bars->v_empty[kt & 1]);
         }
-        if (j < n_a) {
-          if (!issue_pv(0, kt, j == 0)) { ok = false; break; }
-          if (!SEP && j + 1 < n_a && !issue_s(0, kt + 1)) { ok = false; break; }
+      } else {
+        // one issuer: the products of the two tiles in turn
+        if (warp != 1) break;
+        if (!mbar_wait_warp(&bars->q_full, it & 1u, abort_flag)) { ok = false; break; }
+        ok = issue_s(0, kt0);
+        if (ok && has_b) ok = issue_s(1, kt0);
+        if (ok) umma_commit_warp(&bars->k_empty[kt0 & 1]);
+        if (ok && n_kv == 1) umma_commit_warp(&bars->q_empty);
+        for (int j = 0; j < n_kv && ok; ++j) {
+          const uint32_t kt = kt0 + j;
+          if (!wait_v(kt)) { ok = false; break; }
+          if (j < n_a) {
+            if (!issue_pv(0, kt, j == 0)) { ok = false; break; }
+            if (j + 1 < n_a && !issue_s(0, kt + 1)) { ok = false; break; }
+          }
+          if (has_b && !issue_pv(1, kt, j == 0)) { ok = false; break; }
+          umma_commit_warp(&bars->v_empty[kt & 1]);
+          if (j + 1 < n_kv) {
+            if (has_b && !issue_s(1, kt + 1)) { ok = false; break; }
+            umma_commit_warp(&bars->k_empty[(kt + 1) & 1]);
+            if (j + 2 == n_kv) umma_commit_warp(&bars->q_empty);  // that was the item's last use of the query tiles
+          }
         }
-        if (has_b && !issue_pv(1, kt, j == 0)) { ok = false; break; }
-        commit(&bars->v_empty[st]);
-        if (!SEP && j + 1 < n_kv) {
-          if (has_b && !issue_s(1, kt + 1)) { ok = false; break; }
-          commit(&bars->k_empty[(kt + 1) & 1]);
-          if (j + 2 == n_kv) commit(&bars->q_empty);  // that was the item's last use of the query tiles
-        }
+        ++its[0];
+        its[1] += has_b ? 1u : 0u;
       }
       kt0 += n_kv;
-      it_b += has_b ? 1u : 0u;
     }
   } else {
     // ------------------------------------------------------------------ softmax warps: two threads per query row
