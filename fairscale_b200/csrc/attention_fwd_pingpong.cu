@@ -120,24 +120,6 @@ __device__ __forceinline__ constexpr uint32_t kstep_kmajor(int ks, uint32_t slab
 }
 __device__ __forceinline__ constexpr uint32_t kstep_mnmajor(int ks) { return static_cast<uint32_t>(ks) * 2048u; }
 
-// Two fp32 values per instruction: half the issue slots of the scaling and of the row sum.
-__device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
 // Largest of 32 scores of a row and `m`; DIAG: of those of keys col0 + i <= row only.
 template <bool DIAG>
 __device__ __forceinline__ float chunk_max(const uint32_t (&r)[32], int col0, int row, float m) {

@@ -100,6 +100,29 @@ template <typename T> __device__ __forceinline__ void st16(T* p, const Vec16<T>&
   *reinterpret_cast<uint4*>(p) = x.raw;
 }
 
+// ---- two fp32 values per instruction (each rounded as the scalar instruction rounds it): half the issue slots --------------
+__device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
 // erf(x) as an odd polynomial x * P(x^2) of degree 17 on |x| <= 3.5 (least-squares fit on Chebyshev nodes, max error
 // 2.1e-4 in fp32), constant beyond.  The GEMM epilogues evaluate it per element: with the libdevice routine, or with
 // any formula built on a reciprocal and an exponential, they were bound by the special-function pipe; this one runs
@@ -121,10 +144,43 @@ __device__ __forceinline__ float fast_erf(float x) {
 __device__ __forceinline__ float gelu_erf(float x) {
   return 0.5f * x * (1.f + fast_erf(x * 0.70710678118654752f));
 }
+// Two at once, to the bit the values of gelu_erf and (below) gelu_erf_grad: the GEMM epilogues are bound by their issue slots.
+__device__ __forceinline__ uint64_t fast_erf_x2(uint64_t x) {
+  auto both = [](float v) { return pack_f32x2(v, v); };
+  float x0, x1, q0, q1;
+  unpack_f32x2(x, x0, x1);
+  const uint64_t ax = pack_f32x2(fminf(fabsf(x0), 3.5f), fminf(fabsf(x1), 3.5f));
+  const uint64_t t = mul_f32x2(ax, ax);
+  uint64_t p = both(1.7347794642241373e-08f);
+  p = fma_f32x2(p, t, both(-1.0356023911367276e-06f));
+  p = fma_f32x2(p, t, both(2.671026157385393e-05f));
+  p = fma_f32x2(p, t, both(-0.0003934614440707046f));
+  p = fma_f32x2(p, t, both(0.0037059609711284783f));
+  p = fma_f32x2(p, t, both(-0.02383114556013128f));
+  p = fma_f32x2(p, t, both(0.10964519147478315f));
+  p = fma_f32x2(p, t, both(-0.37479130195833465f));
+  p = fma_f32x2(p, t, both(1.1282852575734723f));
+  unpack_f32x2(mul_f32x2(ax, p), q0, q1);
+  return pack_f32x2(copysignf(fminf(q0, 1.f), x0), copysignf(fminf(q1, 1.f), x1));
+}
+__device__ __forceinline__ void gelu_erf_x2(float& a, float& b) {
+  const uint64_t x = pack_f32x2(a, b);
+  const uint64_t e = fast_erf_x2(mul_f32x2(x, pack_f32x2(0.70710678118654752f, 0.70710678118654752f)));
+  unpack_f32x2(mul_f32x2(mul_f32x2(pack_f32x2(0.5f, 0.5f), x), add_f32x2(pack_f32x2(1.f, 1.f), e)), a, b);
+}
 // d/dx gelu(x) = Phi(x) + x phi(x): the polynomial erf plus one exponential.
 __device__ __forceinline__ float gelu_erf_grad(float x) {
   const float cdf = fmaf(0.5f, fast_erf(x * 0.70710678118654752f), 0.5f);
   return fmaf(x * 0.3989422804014327f, __expf(-0.5f * x * x), cdf);
+}
+// (a, b) times gelu' of (x0, x1)
+__device__ __forceinline__ void mul_gelu_erf_grad_x2(float& a, float& b, float x0, float x1) {
+  const uint64_t x = pack_f32x2(x0, x1), half = pack_f32x2(0.5f, 0.5f);
+  const uint64_t cdf = fma_f32x2(half, fast_erf_x2(mul_f32x2(x, pack_f32x2(0.70710678118654752f, 0.70710678118654752f))), half);
+  float y0, y1;
+  unpack_f32x2(mul_f32x2(mul_f32x2(pack_f32x2(-0.5f, -0.5f), x), x), y0, y1);
+  const uint64_t g = fma_f32x2(mul_f32x2(x, pack_f32x2(0.3989422804014327f, 0.3989422804014327f)), pack_f32x2(__expf(y0), __expf(y1)), cdf);
+  unpack_f32x2(mul_f32x2(pack_f32x2(a, b), g), a, b);
 }
 
 }  // namespace fsb

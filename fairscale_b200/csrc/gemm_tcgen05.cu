@@ -730,12 +730,6 @@ namespace fsb_host {
 int gemm_cluster_k(const CUtensorMap& ta, const void* B, int ldb, const fsb::GemmParams& p, int block_n, int splits, int dev, cudaStream_t stream);
 }  // namespace fsb_host
 
-// Products that the 512 x 256 pair kernel takes: bf16 rows that its epilogue can store in 16-byte pieces, no operand besides a bias.
-static bool wide_takes(const fsb::GemmParams& p) {
-  return p.M >= 512 && p.N >= 256 && !p.out_f32 && (p.epilogue == fsb::EPI_NONE || p.epilogue == fsb::EPI_BIAS) && p.ldc % 8 == 0 && p.N % 8 == 0 &&
-         p.stride_c % 8 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15u) == 0 && p.b_ready == nullptr && p.a_ready == nullptr;
-}
-
 template <bool BATCHED, int MH>
 static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const fsb::GemmParams& p, int num_sms, int di, cudaStream_t stream) {
   using namespace fsb;
@@ -793,7 +787,7 @@ static bool pair_enabled() {  // FSB_GEMM_PAIR=0 disables the CTA-pair kernel
   return on;
 }
 
-// Kernel for a product that is not streamed and has no CTA cap (choose_with_wide goes on from here).  Measured on B200 (us; 64-wide K blocks = kb), small products
+// Kernel for a product that is not streamed and has no CTA cap (choose_persistent goes on from here).  Measured on B200 (us; 64-wide K blocks = kb), small products
 // back to back:
 //
 //   M, N, K              pair   one CTA 128x256   cluster split-K, block_n / splits
@@ -851,27 +845,46 @@ static bool pair_pays(long long problems, int M, int N, int K, int lda, int ldb,
   const float pair = 8.f + pair_us[off_line] * num_kb * ((pair_tiles + pairs - 1) / pairs);
   return pair < one;
 }
-// Which of the three persistent kernels for `problems` products that the 512 x 256 tiles can take (wide_takes), in estimated us:
-// a launch, and per wave of tiles its start and its K blocks; the share that goes with the tiles per SM instead of whole waves is
-// what the card's power limit gives back when a wave is partly empty.  Fitted to 90 products (M and N 256 .. 16384, K 256 .. 32000,
-// one or 4 to 16 stacked, all operand layouts, a third with rows off the 128-byte lines): taking the lowest estimate costs 0.8 %
-// over the fastest kernel on average, taking pair_pays' choice between the other two 9.6 %.  Measured (us, wide / pair / one CTA):
+// Which of the three persistent kernels for `problems` products with bf16 rows in 16-byte pieces (row_pieces), in estimated us: a
+// launch, and per wave of tiles its start and its K blocks, or its epilogue where that takes longer; the share that goes with the
+// tiles per SM instead of whole waves is what the card's power limit gives back when a wave is partly empty.
+// Plain and bias products: fitted to 90 of them (M and N 256 .. 16384, K 256 .. 32000, one or 4 to 16 stacked, all operand layouts,
+// a third with rows off the 128-byte lines): taking the lowest estimate costs 0.8 % over the fastest kernel on average, taking
+// pair_pays' choice between the other two 9.6 %.  Measured (us, wide / pair / one CTA):
 //   16384 x 6144 x 2048 287 / 313 / 326       8192 x 2048 x 16384 (wgrad) 435 / 486 / 486     50304 x 2048 x 16384 (wgrad) 2576 / 3055 / 2847
 //   4096 x 12288 x 4096 317 / 306 / 342        2048 x 2048 x 16384 (wgrad) 167 / 120 / 124     16384 x 50304 x 2048 2518 / 2696 / 2898
 //   8 x 2048 x 1024 x 4096 115 / 125 / 139     8192 x 3072 x 1024 53.3 / 53.6 / 51.1           2792 x 3968 x 256 16.4 / 20.2 / 14.4
-static GemmPlan::Kind choose_with_wide(long long problems, int M, int N, int K, int lda, int ldb, int num_sms) {
-  const long long tiles_n = (N + 255) / 256;
-  auto tiles = [&](int rows) -> long long { return problems * ((M + rows - 1) / rows) * tiles_n; };
+// The other epilogues take time of their own, and the pair drains a tile with eight warps per CTA instead of four (us, pair / one CTA):
+//   GELU      16384 x 8192 x 2048 457 / 480    8192 x 4096 x 1024 72 / 81    3575 x 3072 x 768 (and its input stored) 31 / 37
+//   GELU'     16384 x 8192 x 2048 498 / 538    8192 x 4096 x 1024 88 / 106   3575 x 3072 x 768 35 / 39
+//   residual  16384 x 2048 x 8192 455 / 474    8192 x 1024 x 4096 68 / 71    8192 x 1024 x 1024 24.6 / 26.4
+static bool row_pieces(const fsb::GemmParams& p) {
+  const uintptr_t ptrs = reinterpret_cast<uintptr_t>(p.C) | reinterpret_cast<uintptr_t>(p.aux) | reinterpret_cast<uintptr_t>(p.aux_out);
+  return !p.out_f32 && p.N % 8 == 0 && p.ldc % 8 == 0 && p.ld_aux % 8 == 0 && p.stride_c % 8 == 0 && p.stride_aux % 8 == 0 && (ptrs & 15u) == 0;
+}
+// ... of those, what the 512 x 256 tiles take: no operand besides a bias, one result
+static bool wide_takes(const fsb::GemmParams& p) {
+  return p.M >= 512 && p.N >= 256 && (p.epilogue == fsb::EPI_NONE || p.epilogue == fsb::EPI_BIAS) && row_pieces(p) && p.b_ready == nullptr && p.a_ready == nullptr;
+}
+static GemmPlan::Kind choose_persistent(const fsb::GemmParams& p, int lda, int ldb, int num_sms) {
+  const long long tiles_n = (p.N + 255) / 256;
+  auto tiles = [&](int rows) -> long long { return p.batch * ((p.M + rows - 1) / rows) * tiles_n; };
   const int off_line = (lda % 64 != 0) + (ldb % 64 != 0);
-  const float num_kb = static_cast<float>((K + fsb::BLOCK_K - 1) / fsb::BLOCK_K);
-  auto cost = [&](long long n, int units, float launch, float start, float per_wave, float per_share) -> float {
+  const float num_kb = static_cast<float>((p.K + fsb::BLOCK_K - 1) / fsb::BLOCK_K);
+  auto cost = [&](long long n, int units, float launch, float start, float per_wave, float per_share, float epilogue) -> float {
     const float waves = static_cast<float>((n + units - 1) / units), share = static_cast<float>(n) / units;
-    return launch + waves * (start + num_kb * per_wave) + num_kb * share * per_share;
+    const float main_loops = waves * (start + num_kb * per_wave) + num_kb * share * per_share;
+    return launch + (main_loops > waves * epilogue ? main_loops : waves * epilogue);
   };
-  const float wide = cost(tiles(512), num_sms / 2, 7.2f, 2.0f, 0.52f, 0.25f);
-  const float pair = cost(tiles(256), num_sms / 2, 7.2f, 2.2f, 0.262f + 0.017f * off_line, 0.16f);
-  const float one = cost(tiles(128), num_sms, 5.0f, 1.1f, 0.229f + 0.064f * off_line, 0.25f);
-  return wide <= pair && wide <= one ? GemmPlan::WIDE_PAIR : pair < one ? GemmPlan::PAIR : GemmPlan::ONE_CTA;
+  const bool gelu = p.epilogue == fsb::EPI_BIAS_GELU, dgelu = p.epilogue == fsb::EPI_DGELU;
+  const bool residual = p.epilogue == fsb::EPI_BIAS_RESIDUAL || p.epilogue == fsb::EPI_RESIDUAL;
+  const float pair = cost(tiles(256), num_sms / 2, 7.2f, residual ? 3.f : 2.2f, 0.262f + 0.017f * off_line, 0.16f, gelu ? 9.5f : dgelu ? 11.4f : 0.f);
+  const float one = cost(tiles(128), num_sms, 5.0f, residual ? 3.6f : 1.1f, 0.229f + 0.064f * off_line, 0.25f, gelu ? 12.f : dgelu ? 14.2f : 0.f);
+  if (wide_takes(p)) {
+    const float wide = cost(tiles(512), num_sms / 2, 7.2f, 2.0f, 0.52f, 0.25f, 0.f);
+    if (wide <= pair && wide <= one) return GemmPlan::WIDE_PAIR;
+  }
+  return pair < one ? GemmPlan::PAIR : GemmPlan::ONE_CTA;
 }
 static GemmPlan choose_gemm_plan(int M, int N, int K, int lda, int ldb, int num_sms, bool pair_allowed) {
   const long long tiles_m = (M + fsb::BLOCK_M - 1) / fsb::BLOCK_M;
@@ -898,8 +911,9 @@ static GemmPlan choose_gemm_plan(int M, int N, int K, int lda, int ldb, int num_
   return best;
 }
 
-// The kernel that a product (or `problems` stacked ones) whose epilogue the wide tiles do not take would get on a device with
-// `num_sms` SMs: 0 CTA pairs, 1 one CTA per tile, 2 split-K over clusters (a single product only).
+// The kernel that a product (or `problems` stacked ones) would get on a device with `num_sms` SMs where choose_persistent does not
+// come in (fp32 or unaligned results, K below 256, one wave or less): 0 CTA pairs, 1 one CTA per tile, 2 split-K over clusters
+// (a single product only).
 FSB_API int fsb_gemm_plan_of(long long problems, int M, int N, int K, int lda, int ldb, int num_sms) {
   if (problems > 1) return pair_enabled() && pair_pays(problems, M, N, K, lda, ldb, num_sms) ? 0 : 1;
   return static_cast<int>(choose_gemm_plan(M, N, K, lda, ldb, num_sms, pair_enabled()).kind);
@@ -1032,7 +1046,7 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* bia
   else if (max_ctas == 0) {
     plan = choose_gemm_plan(M, N, K, lda, ldb, num_sms, pair_enabled());
     // more tiles than one wave of single CTAs (below, the wide tiles leave most SMs without one) and K as far as it was measured
-    if (tiles > num_sms && K >= 256 && pair_enabled() && wide_takes(p)) plan.kind = choose_with_wide(1, M, N, K, lda, ldb, num_sms);
+    if (tiles > num_sms && M >= 256 && N >= 256 && K >= 256 && pair_enabled() && row_pieces(p)) plan.kind = choose_persistent(p, lda, ldb, num_sms);
   }
   if (plan.kind == GemmPlan::CLUSTER_K) return fsb_host::gemm_cluster_k(ta, B, ldb, p, plan.block_n, plan.splits, dev, stream);
   // Run-time tile hand-out for products large enough to share the device with a collective; small ones stride.
@@ -1104,7 +1118,7 @@ static int gemm_bf16_batched_impl(const void* A, const void* B, void* C, const v
   GemmPlan::Kind kind = forced == 3 ? GemmPlan::WIDE_PAIR : forced == 2 ? GemmPlan::PAIR : GemmPlan::ONE_CTA;
   if (forced == 0 && pair_enabled()) {
     if (pair_pays(batch, M, N, K, lda, ldb, num_sms)) kind = GemmPlan::PAIR;
-    if (tiles > num_sms && K >= 256 && wide_takes(p)) kind = choose_with_wide(batch, M, N, K, lda, ldb, num_sms);
+    if (tiles > num_sms && M >= 256 && N >= 256 && K >= 256 && row_pieces(p)) kind = choose_persistent(p, lda, ldb, num_sms);
   }
   if (kind != GemmPlan::ONE_CTA) {
     if (!b_mn_major && !fsb_host::encode_3d_16bit(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)batch, (uint64_t)ldb, (uint64_t)stride_b, BLOCK_K, PAIR_HALF_N, 1)) return -1;

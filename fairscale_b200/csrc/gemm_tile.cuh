@@ -310,7 +310,7 @@ __device__ __forceinline__ void epilogue_rows_coalesced(uint32_t t_base, int row
         a.raw = *reinterpret_cast<const uint4*>(stage + epi_swz(lane, c));
         if (epi == EPI_DGELU) {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) v[c * 8 + i] *= gelu_erf_grad(__bfloat162float(a.v[i]));
+          for (int i = 0; i < 8; i += 2) mul_gelu_erf_grad_x2(v[c * 8 + i], v[c * 8 + i + 1], __bfloat162float(a.v[i]), __bfloat162float(a.v[i + 1]));
         } else {
 #pragma unroll
           for (int i = 0; i < 8; ++i) v[c * 8 + i] += __bfloat162float(a.v[i]);
@@ -327,7 +327,7 @@ __device__ __forceinline__ void epilogue_rows_coalesced(uint32_t t_base, int row
         __syncwarp();
       }
 #pragma unroll
-      for (int i = 0; i < 64; ++i) v[i] = gelu_erf(v[i]);
+      for (int i = 0; i < 64; i += 2) gelu_erf_x2(v[i], v[i + 1]);
     }
     epi_row_to_stage(stage, v, lane);
     __syncwarp();
