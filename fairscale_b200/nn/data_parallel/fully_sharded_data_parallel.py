@@ -137,16 +137,56 @@ class _NullStream:
 _NULL_STREAM = _NullStream()
 
 
+# The helpers below run ten to twenty times per unit and pass, and a small model's step is bound by such host work: they call what
+# torch.cuda.current_stream, torch.cuda.stream and torch.no_grad come down to once their arguments are known.
 def _current_stream(device: torch.device) -> Any:
     if device.type == "cuda":
-        return torch.cuda.current_stream(device)
+        index = torch.cuda.current_device() if device.index is None else device.index
+        stream_id, device_index, device_type = torch._C._cuda_getCurrentStream(index)
+        return torch.cuda.Stream(stream_id=stream_id, device_index=device_index, device_type=device_type)
     return _NULL_STREAM
+
+
+class _StreamScope:
+    """``torch.cuda.stream`` for a stream of the current device."""
+
+    __slots__ = ("stream", "before")
+
+    def __init__(self, stream: Any) -> None:
+        self.stream = stream
+
+    def __enter__(self) -> None:
+        s = self.stream
+        self.before = torch._C._cuda_getCurrentStream(s.device_index)
+        torch._C._cuda_setStream(stream_id=s.stream_id, device_index=s.device_index, device_type=s.device_type)
+
+    def __exit__(self, *exc: Any) -> None:
+        stream_id, device_index, device_type = self.before
+        torch._C._cuda_setStream(stream_id=stream_id, device_index=device_index, device_type=device_type)
 
 
 def _on_stream(stream: Any) -> Any:
     if isinstance(stream, _NullStream) or stream is None:
         return contextlib.nullcontext()
+    if torch._C._cuda_getDevice() == stream.device_index:
+        return _StreamScope(stream)
     return torch.cuda.stream(stream)
+
+
+def _no_grad(fn: Any) -> Any:
+    """``torch.no_grad()`` around a plain function or method."""
+
+    @functools.wraps(fn)
+    def run(*args: Any, **kwargs: Any) -> Any:
+        if not torch.is_grad_enabled():
+            return fn(*args, **kwargs)
+        torch._C._set_grad_enabled(False)
+        try:
+            return fn(*args, **kwargs)
+        finally:
+            torch._C._set_grad_enabled(True)
+
+    return run
 
 
 def _record_stream(t: torch.Tensor, stream: Any) -> None:
@@ -528,6 +568,15 @@ class FullyShardedDataParallel(nn.Module):
                 f"clear_autocast_cache={self.clear_autocast_cache}, force_input_to_fp32={self.force_input_to_fp32}, "
             )
         return text
+
+    # State that changes several times per unit and pass; always plain values, never parameters, buffers or modules.
+    _PLAIN_STATE = frozenset(("training_state", "has_full_params", "_allow_deferred_gather", "_post_backward_callback_queued", "_pre_backward_hook_has_run"))
+
+    def __setattr__(self, name: str, value: Any) -> None:
+        if name in FullyShardedDataParallel._PLAIN_STATE:
+            self.__dict__[name] = value
+        else:
+            super().__setattr__(name, value)
 
     def __getattr__(self, name: str) -> Any:
         try:
@@ -1071,7 +1120,7 @@ class FullyShardedDataParallel(nn.Module):
                 p._shard_bwd_hook = (self, handle)  # type: ignore[attr-defined]
 
     # ------------------------------------------------------------------ backward
-    @torch.no_grad()
+    @_no_grad
     def _post_backward_hook(self, param: Parameter, *unused: Any) -> None:
         """Runs when ``param``'s gradient for this backward is complete: free the full parameter, then
         (on the reduction stream) pre-divide, reduce-scatter and hand the shard to
@@ -1224,7 +1273,7 @@ class FullyShardedDataParallel(nn.Module):
             self._post_backward_callback_queued = True
             Variable._execution_engine.queue_callback(self._wait_for_post_backward)
 
-    @torch.no_grad()
+    @_no_grad
     def _wait_for_post_backward(self) -> None:
         """End of backward (root): flush the reducer, join the reduction stream, publish ``p.grad`` shards
         and return every instance to IDLE."""
@@ -1310,7 +1359,7 @@ class FullyShardedDataParallel(nn.Module):
                 self._output_pre_backward_hook_registered.clear()
 
     # ------------------------------------------------------------------ parameter (re)materialisation
-    @torch.no_grad()
+    @_no_grad
     def _rebuild_full_params(
         self, force_full_precision: bool = False, wait: bool = True
     ) -> Optional[List[Tuple[torch.Tensor, bool]]]:
@@ -1436,7 +1485,7 @@ class FullyShardedDataParallel(nn.Module):
         self._pending_gathers.append(gemm_ops.defer_gather(gemm_ops.PendingGather(ws, shard, landing, self._streams["all_gather"])))
         return True
 
-    @torch.no_grad()
+    @_no_grad
     def _use_full_params(self) -> None:
         """Re-point ``p.data`` at full parameters that are still resident (``reshard_after_forward=False``)."""
         assert self.has_full_params
@@ -1450,7 +1499,7 @@ class FullyShardedDataParallel(nn.Module):
                 assert not _storage_is_free(p._full_param_padded), f"{p._orig_size} {id(self)}"  # type: ignore[attr-defined]
                 p.data = p._full_param_padded[: p._orig_size.numel()].view(p._orig_size)  # type: ignore[attr-defined]
 
-    @torch.no_grad()
+    @_no_grad
     def _prep_grads_for_backward(self) -> None:
         """Sort out what a leftover ``p.grad`` is: a full-size gradient from ``no_sync`` (keep
         accumulating), or a reduced shard from a previous backward (stash; summed after this reduction)."""
@@ -1470,7 +1519,7 @@ class FullyShardedDataParallel(nn.Module):
             else:
                 raise AssertionError(f"unexpected grad shape: {p.grad.size()}")
 
-    @torch.no_grad()
+    @_no_grad
     def _free_full_params(self, params: Optional[List[Parameter]] = None) -> None:
         params = self.params if params is None else params
         self.has_full_params = False
@@ -1565,12 +1614,12 @@ class FullyShardedDataParallel(nn.Module):
         return full
 
     # ------------------------------------------------------------------ shard bookkeeping
-    @torch.no_grad()
+    @_no_grad
     def _use_fp32_param_shard(self, params: Optional[List[Parameter]] = None) -> None:
         for p in self.params if params is None else params:
             p.data = p._fp32_shard  # type: ignore[attr-defined]
 
-    @torch.no_grad()
+    @_no_grad
     def _cast_fp32_param_shards_to_fp16(self, params: Optional[List[Parameter]] = None) -> None:
         """Master shard → compute-dtype shard (and host → device when offloading) on the cast stream."""
         cast_stream = self._streams["fp32_to_fp16"]
@@ -1586,7 +1635,7 @@ class FullyShardedDataParallel(nn.Module):
                 p.data = p._fp16_shard  # type: ignore[attr-defined]
         _current_stream(self.compute_device).wait_stream(cast_stream)
 
-    @torch.no_grad()
+    @_no_grad
     def _free_fp16_param_shard(self, params: Optional[List[Parameter]] = None) -> None:
         if self.persistent_compute_shards:
             return

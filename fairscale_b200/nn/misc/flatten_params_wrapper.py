@@ -369,7 +369,13 @@ class FlattenParamsWrapper(nn.Module):
         views: List[Tensor] = []
         fwd_views = chain.from_iterable(p.get_param_views_for_forward() for p in self.flat_params)  # type: ignore[attr-defined]
         for (_, mod, attr), v in zip(self._param_infos, fwd_views):
-            setattr(mod, attr, v)  # plain attribute: the view is not an nn.Parameter
+            # Plain attribute: the view is not an nn.Parameter.  Once it is one, nn.Module's own __setattr__, which looks through
+            # parameters, buffers and modules first, would only replace the entry.
+            d = mod.__dict__
+            if attr in d and type(mod).__setattr__ is nn.Module.__setattr__:
+                d[attr] = v
+            else:
+                setattr(mod, attr, v)
             views.append(v)
         # checkpoint_wrapper consults this to decide whether outputs need grad
         setattr(self._fpw_module, "_unflattened_param_views", views)

@@ -226,3 +226,53 @@ def test_a_flat_parameter_is_not_flattened_again():
     for k, v in want_state.items():
         torch.testing.assert_close(got_state[k], v)
     assert sorted(p.numel() for p in outer.parameters()) == [4 * 2 + 2, 4 * 4 + 4]
+
+
+@pytest.mark.parametrize("own_setattr", [False, True])
+def test_views_of_later_passes_reach_the_module(own_setattr):
+    """From the second pass on a view replaces the module's attribute directly, unless the module looks at assignments itself; an
+    attribute that was made a buffer in between goes through the module's own rules."""
+    seen = []
+
+    class Scale(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.w = torch.nn.Parameter(torch.tensor([2.0, 3.0]))
+
+        def forward(self, x):
+            return x * self.w
+
+        if own_setattr:
+            def __setattr__(self, name, value):
+                seen.append(name)
+                super().__setattr__(name, value)
+
+    m = FlattenParamsWrapper(Scale())
+    x = torch.ones(2)
+    for k in range(3):
+        seen.clear()
+        with torch.no_grad():
+            m.flat_param_0.copy_(torch.tensor([k, k + 1.0]))
+        assert torch.equal(m(x), torch.tensor([k, k + 1.0]))
+        assert not own_setattr or "w" in seen
+    del m.module.w
+    m.module.register_buffer("w", torch.zeros(2))
+    assert torch.equal(m(x), torch.tensor([2.0, 3.0])) and "w" in m.module._buffers
+
+
+def test_no_grad_helper_restores_the_mode():
+    from fairscale_b200.nn.data_parallel import fully_sharded_data_parallel as fsdp
+
+    @fsdp._no_grad
+    def f(fail=False):
+        assert not torch.is_grad_enabled()
+        if fail:
+            raise ValueError
+        return 1
+
+    for mode in (True, False):
+        with torch.set_grad_enabled(mode):
+            assert f() == 1
+            with pytest.raises(ValueError):
+                f(fail=True)
+            assert torch.is_grad_enabled() == mode
