@@ -229,28 +229,28 @@ def explore(programs):
             elif op[0] == "load":
                 n_loads = loads | {op[1:]}
             else:
-                n_pipe = pipe + (op,)
+                n_pipe = pipe + ((a, op),)
             pc += 1
             while pc < len(prog) and at_once[a][pc]:
                 if prog[pc][0] == "load":
                     n_loads = n_loads | {prog[pc][1:]}
                 else:
-                    n_pipe = n_pipe + (prog[pc],)
+                    n_pipe = n_pipe + ((a, prog[pc]),)
                 pc += 1
             after.append((put(pcs, a, pc), n_arr, n_loads, n_pipe, n_mem))
         for ld in loads:  # a TMA load lands
             i = bars[ld[2]]
             after.append((pcs, put(arrivals, i, arrivals[i] + 1), loads - {ld}, pipe, put(mem, slot[ld[0]], ld[1])))
-        if pipe:  # the tensor pipe completes its oldest entry
-            op = pipe[0]
+        for at in {a: k for k, (a, _) in reversed(list(enumerate(pipe)))}.values():  # the tensor pipe completes the oldest entry of an issuer
+            op, rest = pipe[at][1], pipe[:at] + pipe[at + 1:]
             if op[0] == "commit":
                 i = bars[op[1]]
-                after.append((pcs, put(arrivals, i, arrivals[i] + 1), loads, pipe[1:], mem))
+                after.append((pcs, put(arrivals, i, arrivals[i] + 1), loads, rest, mem))
             else:
                 for place, version in op[1]:
                     if mem[slot[place]] != version:
                         problems.add(("a product read another step", op, place, mem[slot[place]]))
-                after.append((pcs, arrivals, loads, pipe[1:], put(mem, slot[op[2]], op[3])))
+                after.append((pcs, arrivals, loads, rest, put(mem, slot[op[2]], op[3])))
         if not after and any(pc < len(p) for pc, p in zip(pcs, progs)):
             deadlocks += 1
         for s in after:
@@ -306,3 +306,106 @@ def test_model_notices_a_wrong_forward(mistake, sep):
 def test_model_notices_a_wrong_backward(mistake, nbuf, stages, per_load):
     problems, deadlocks, _ = explore(backward_programs([4, 4], nbuf, stages, per_load, drop=(mistake,)))
     assert problems or deadlocks
+
+
+# ---- two issuers: nothing orders the products of one behind those of the other but barriers
+def split_backward_programs(items, nbuf, stages, steps_per_load, drop=()):
+    """The backward kernels as they issue: score products by one warp, accumulating products by another."""
+    (producer, _, *sets), counts = backward_programs(items, nbuf, stages, steps_per_load)
+    scores, sums = [], []
+    jt0 = ut0 = 0
+    for it, n in enumerate(items):
+        scores.append(("wait", "stat_full", it & 1, it + 1))
+        sums.append(("wait", "acc_free", (it & 1) ^ 1, it))
+        for u in range(n):
+            jt, ut = jt0 + u // steps_per_load, ut0 + u
+            st, buf, last = jt % stages, ut % nbuf, u == n - 1
+            if u % steps_per_load == 0:
+                scores.append(("wait", f"str_full{st}", (jt // stages) & 1, jt // stages + 1))
+            if "buf_free" not in drop:
+                scores.append(("wait", f"buf_free{buf}", ((ut // nbuf) & 1) ^ 1, ut // nbuf))
+            scores.extend([("mma", (("stat", it), (f"str{st}", jt)), f"buf{buf}", ("S", ut)), ("commit", f"s_full{buf}")])
+            sums.extend([("wait", f"p_full{buf}", (ut // nbuf) & 1, ut // nbuf + 1),
+                         ("mma", ((f"buf{buf}", ("P", ut)), (f"str{st}", jt)), "acc", (it, u)), ("commit", f"buf_free{buf}")])
+            if u % steps_per_load == steps_per_load - 1:
+                sums.append(("commit", f"str_empty{st}"))
+            if last:
+                scores.append(("commit", "stat_empty"))
+                sums.append(("commit", "acc_done"))
+        jt0 += n // steps_per_load
+        ut0 += n
+    return [producer, scores, sums, *sets], counts
+
+
+def split_forward_programs(items, drop=()):
+    """The forward with head size 64 as it issues: a warp for each query tile."""
+    producer, _, *_ = forward_programs(items, True, False)[0]
+    issuers, softmax = ([], []), ([], [])
+    for t in (0, 1):
+        prog, soft = issuers[t], softmax[t]
+        kt0 = c = own = 0
+        for it, (n_a, has_b) in enumerate(items):
+            n_kv = n_a + 1 if has_b else n_a
+            n_own = n_a if t == 0 else (n_kv if has_b else 0)
+
+            def wait_tile(kind, j):
+                k = kt0 + j
+                return ("wait", f"{kind}_full{k & 1}", (k >> 1) & 1, (k >> 1) + 1)
+
+            prog.append(("wait", "q_full", it & 1, it + 1))
+            for j in range(-1, n_own if n_own else -1):
+                k = kt0 + j
+                if j + 1 < n_own:
+                    prog.append(wait_tile("k", j + 1))
+                    if c + j + 1 > 0:
+                        prog.append(("wait", f"s_read{t}", (c + j) & 1, c + j + 1))
+                    prog.extend([("mma", (("q", it), (f"k{(k + 1) & 1}", k + 1)), f"s{t}", ("S", it, j + 1)), ("commit", f"s_full{t}"),
+                                 ("commit", f"k_empty{(k + 1) & 1}")])
+                    if j + 2 == n_own:
+                        prog.append(("commit", "q_empty"))
+                if j >= 0:
+                    prog.append(wait_tile("v", j))
+                    if j == 0:
+                        prog.append(("wait", f"o_free{t}", (own & 1) ^ 1, own))
+                    prog.extend([("wait", f"p_full{t}", (c + j) & 1, c + j + 1), ("mma", ((f"p{t}", ("P", it, j)), (f"v{k & 1}", k)), f"o{t}", (it, j)),
+                                 ("commit", f"o_done{t}"), ("commit", f"v_empty{k & 1}")])
+            if n_own == 0:
+                prog.append(("commit", "q_empty"))
+            for j in range(n_own, n_kv):
+                k = kt0 + j
+                for kind in "kv":
+                    if "pass_wait" not in drop:
+                        prog.append(wait_tile(kind, j))
+                    prog.append(("commit", f"{kind}_empty{k & 1}"))
+            for j in range(n_own):
+                soft.extend([("wait", f"s_full{t}", (c + j) & 1, c + j + 1), ("read", f"s{t}", ("S", it, j)), ("arrive", f"s_read{t}")])
+                if j > 0:
+                    soft.append(("wait", f"o_done{t}", (c + j - 1) & 1, c + j))
+                soft.extend([("write", f"p{t}", ("P", it, j)), ("arrive", f"p_full{t}")])
+            if n_own:
+                c += n_own
+                own += 1
+                soft.extend([("wait", f"o_done{t}", (c - 1) & 1, c), ("read", f"o{t}", (it, n_own - 1)), ("arrive", f"o_free{t}")])
+            kt0 += n_kv
+    counts = {"q_empty": 2, "k_empty0": 2, "k_empty1": 2, "v_empty0": 2, "v_empty1": 2}
+    return [producer, *issuers, *softmax], counts
+
+
+@pytest.mark.parametrize("nbuf,stages,per_load,items", [(3, 4, 2, [6, 2, 2]), (2, 2, 2, [4, 2, 2]), (3, 6, 1, [6, 2]), (2, 4, 1, [6, 2])],
+                         ids=["dq64", "dq128", "dkv64", "dkv128"])
+def test_backward_with_two_issuers_is_safe_and_live(nbuf, stages, per_load, items):
+    problems, deadlocks, states = explore(split_backward_programs(items, nbuf, stages, per_load))
+    assert states > 100
+    assert not problems and deadlocks == 0, (sorted(map(str, problems))[:3], deadlocks)
+
+
+@pytest.mark.parametrize("items", [[(2, True)], [(1, True), (1, False)], [(1, False), (1, True)], [(2, False), (1, True)]], ids=str)
+def test_forward_with_two_issuers_is_safe_and_live(items):
+    problems, deadlocks, states = explore(split_forward_programs(items))
+    assert states > 100
+    assert not problems and deadlocks == 0, (sorted(map(str, problems))[:3], deadlocks)
+
+
+def test_model_notices_two_issuers_without_their_barriers():
+    assert any(explore(split_backward_programs([4, 4], 2, 4, 1, drop=("buf_free",)))[:2])
+    assert any(explore(split_forward_programs([(2, True), (1, True)], drop=("pass_wait",)))[:2])
