@@ -18,6 +18,9 @@ constexpr int NORM_ROWS_MAX_H = 4096;  // row-group backward: up to 512 threads 
 
 // ---- warp-per-row forward (H <= 4096): a lane keeps VPL 16-byte vectors of the row in registers, all
 // reductions are warp shuffles, no shared memory and no block barriers.
+// Bound by memory, and by how many rows are in flight: kept as bf16 a row takes 64 registers a thread at 2048 columns (95 as fp32)
+// and 96 at 4096 (164): 16384 x 2048 35.2 -> 28.9 us (20.5 at the copy rate), 4096 x 4096 20.0 -> 18.0; up to 1024 columns, where
+// registers were no limit, the same (8192 x 1024 10.3 us).
 template <bool RMS, int VPL>
 __global__ void __launch_bounds__(NORM_WARPS * 32) norm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
                                                                         const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
@@ -28,15 +31,19 @@ __global__ void __launch_bounds__(NORM_WARPS * 32) norm_fwd_warp_kernel(const __
   if (row >= rows) return;
   const int nvec = H / 8;
   const __nv_bfloat16* xr = x + row * H;
-  float v[VPL][8];
+  Vec16<__nv_bfloat16> v[VPL];  // as they came: in fp32 they took twice the registers and half the warps in flight
   float sum = 0.f;
 #pragma unroll
   for (int it = 0; it < VPL; ++it) {
     const int j = lane + it * 32;
-    if (j < nvec) {
-      const Vec16<__nv_bfloat16> t = ld16(xr + j * 8);
+    if (j < nvec) v[it] = ld16(xr + j * 8);
+  }
 #pragma unroll
-      for (int k = 0; k < 8; ++k) { v[it][k] = __bfloat162float(t.v[k]); sum += v[it][k]; }
+  for (int it = 0; it < VPL; ++it) {
+    const int j = lane + it * 32;
+    if (j < nvec) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) sum += __bfloat162float(v[it].v[k]);
     }
   }
   const float mean = RMS ? 0.f : warp_sum(sum) / H;
@@ -46,7 +53,7 @@ __global__ void __launch_bounds__(NORM_WARPS * 32) norm_fwd_warp_kernel(const __
     const int j = lane + it * 32;
     if (j < nvec) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) { const float d = v[it][k] - mean; sq += d * d; }
+      for (int k = 0; k < 8; ++k) { const float d = __bfloat162float(v[it].v[k]) - mean; sq += d * d; }
     }
   }
   const float rstd = rsqrtf(warp_sum(sq) / H + eps);
@@ -65,10 +72,10 @@ __global__ void __launch_bounds__(NORM_WARPS * 32) norm_fwd_warp_kernel(const __
         const Vec16<__nv_bfloat16> b = ld16(beta + j * 8);
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-          o.v[k] = __float2bfloat16_rn((v[it][k] - mean) * rstd * __bfloat162float(g.v[k]) + __bfloat162float(b.v[k]));
+          o.v[k] = __float2bfloat16_rn((__bfloat162float(v[it].v[k]) - mean) * rstd * __bfloat162float(g.v[k]) + __bfloat162float(b.v[k]));
       } else {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) o.v[k] = __float2bfloat16_rn((v[it][k] - mean) * rstd * __bfloat162float(g.v[k]));
+        for (int k = 0; k < 8; ++k) o.v[k] = __float2bfloat16_rn((__bfloat162float(v[it].v[k]) - mean) * rstd * __bfloat162float(g.v[k]));
       }
       st16(yr + j * 8, o);
     }
@@ -84,7 +91,7 @@ __global__ void __launch_bounds__(NORM_WARPS * 32) norm_fwd_warp_kernel(const __
 // SM with a fraction of its 512 threads and took 65536 x 512 162 us (now 47 us), 16384 x 1024 51 (29), 16384 x 2048 66 (51),
 // 16384 x 4096, its grid in two waves, 138 (102); with a residual 16384 x 2048 75 (58).  A warp per row, with all of a row's sums
 // in one warp's registers and room for one row only, took 87, 41 and 67 us, two kernels for 4096 columns 188.  (All with the
-// reduction of the partial rows, ten calls in a graph.)  The forward has no sums to keep and is faster with a warp per row: 35
+// reduction of the partial rows, ten calls in a graph.)  The forward has no sums to keep and is faster with a warp per row: 29
 // against 41 us.
 struct NormRowsShape {
   int lanes;          // lanes of a warp that share a row
