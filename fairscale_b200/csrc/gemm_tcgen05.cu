@@ -278,6 +278,7 @@ struct PairSmem {
   // 228 KB, enough for two of the 128-thread communication CTAs (1 KB reserve + 8 bytes each) to stay resident beside
   // a GEMM CTA; a third would keep the next GEMM CTA off the SM.
   static constexpr int TOTAL = BAR_OFFSET + 256;
+  static_assert(8 * (2 * STAGES + 4 + 2 * SCHED_DEPTH + 2) + 4 * (SCHED_DEPTH + 3) <= 256, "barriers, tile indices, TMEM address, abort flag");
 };
 
 template <int MH>
@@ -393,10 +394,13 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
   uint64_t* empty_bar = full_bar + PAIR_STAGES;
   uint64_t* tmem_full_bar = empty_bar + PAIR_STAGES;
   uint64_t* tmem_empty_bar = tmem_full_bar + 2;
-  uint64_t* sched_full = tmem_empty_bar + 2;           // [SCHED_DEPTH] in every CTA: the slot holds a tile index
-  uint64_t* sched_empty = sched_full + SCHED_DEPTH;  // [SCHED_DEPTH] in the leader: every reader has taken it
-  volatile int* sched_tile = reinterpret_cast<volatile int*>(sched_empty + SCHED_DEPTH);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(const_cast<int*>(sched_tile) + SCHED_DEPTH);
+  uint64_t* sched_full = tmem_empty_bar + 2;         // [SCHED_DEPTH] the slot holds a tile index
+  uint64_t* sched_empty = sched_full + SCHED_DEPTH;  // [SCHED_DEPTH] every reader in this CTA has taken it
+  uint64_t* mail_full = sched_empty + SCHED_DEPTH;   // in the peer: mail_tile holds the next index
+  uint64_t* mail_empty = mail_full + 1;              // in the leader: the peer has taken it
+  volatile int* sched_tile = reinterpret_cast<volatile int*>(mail_empty + 1);
+  volatile int* mail_tile = sched_tile + SCHED_DEPTH;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(const_cast<int*>(mail_tile) + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // warp-uniform
@@ -435,8 +439,10 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
     }
     for (int q = 0; q < SCHED_DEPTH; ++q) {
       mbar_init(&sched_full[q], 1);
-      mbar_init(&sched_empty[q], 2 + 2 * PAIR_EPI_WARPS);  // the peer's producer, the MMA warp, all epilogue warps of the pair
+      mbar_init(&sched_empty[q], (leader ? 1 : 0) + PAIR_EPI_WARPS);  // the MMA warp, the epilogue warps
     }
+    mbar_init(mail_full, 1);
+    mbar_init(mail_empty, 1);
     fence_barrier_init();
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
@@ -458,18 +464,19 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
   tc_fence_after_sync();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
-  // Tiles are handed out at run time: the leader's producer takes the next index from a counter in global memory and
-  // publishes it (or -1 at the end) to both CTAs through a small ring; every role reads the ring in order.  An SM that
-  // is slowed down or taken by a kernel of another stream (a collective) then simply works off fewer tiles, instead of
-  // holding back the ones a static schedule would have given it.  A launch without a counter strides through the tiles.
-  // No fence of cluster scope is on the way of an index: it is a remote store that completes on the reader's barrier, and a
-  // slot is handed back by a CTA-scope arrive.  (With plain stores, release and acquire at cluster scope the MMA warp stood
-  // still for 2 400 cycles a tile of 20 400, 8192 x 8192 x 2048, and the producers for about as long.)
-  // Reader side: wait for slot q, take the index, hand the slot back to the leader.
+  // Tiles are handed out at run time: the leader's producer takes the next index from a counter in global memory and sends it
+  // (or -1 at the end) to the peer's producer; each of the two publishes it to its own CTA through a small ring that every role
+  // reads in order.  An SM that is slowed down or taken by a kernel of another stream (a collective) then simply works off fewer
+  // tiles, instead of holding back the ones a static schedule would have given it.  A launch without a counter strides through the tiles.
+  // One thread of each CTA takes part in what crosses the pair, and only there is cluster scope needed: the index is a remote
+  // store that completes on the peer's barrier, and the peer's producer, which has nothing but loads in flight, hands the word
+  // back with a release of cluster scope while its ring of loads is full.  (With every role of both CTAs releasing and acquiring at
+  // cluster scope the MMA warp stood still for 2 400 cycles a tile of 20 400, 8192 x 8192 x 2048, and the producers for about as long.)
+  // Reader side: wait for slot q of this CTA's ring, take the index, hand the slot back.
   auto take_tile = [&](int q, uint32_t qphase, int site) -> int {
     if (!mbar_wait(&sched_full[q], qphase, abort_flag, site)) return -2;
     const int t = sched_tile[q];
-    mbar_arrive_remote(map_to_cta(smem_u32(&sched_empty[q]), 0));
+    mbar_arrive(&sched_empty[q]);
     return t;
   };
 
@@ -483,37 +490,50 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
     int q = 0;
     uint32_t qphase = 0;
     bool ok = true;
-    auto publish = [&](int t) -> bool {
+    auto publish = [&](int t) -> bool {  // to the roles of this CTA
       if (!mbar_wait_warp(&sched_empty[q], qphase ^ 1u, abort_flag, 2)) return false;
       if (lane == 0) {
-#pragma unroll
-        for (uint32_t c = 0; c < 2; ++c) {
-          const uint32_t fb = map_to_cta(smem_u32(&sched_full[q]), c);
-          mbar_expect_tx_remote(fb, 4);
-          st_async_u32(map_to_cta(smem_u32(const_cast<int*>(&sched_tile[q])), c), static_cast<uint32_t>(t), fb);
-        }
+        sched_tile[q] = t;
+        mbar_arrive(&sched_full[q]);
       }
       __syncwarp();
       if (++q == SCHED_DEPTH) { q = 0; qphase ^= 1u; }
       return true;
     };
-    auto take = [&]() -> int {  // the peer's side of the ring
-      int t = 0;
-      if (lane == 0) t = take_tile(q, qphase, 3);
-      if (++q == SCHED_DEPTH) { q = 0; qphase ^= 1u; }
+    uint32_t mail_phase = 0;
+    auto send = [&](int t) -> bool {  // leader: to the peer's producer
+      if (!mbar_wait_warp<WaitScope::CLUSTER>(mail_empty, mail_phase ^ 1u, abort_flag, 12)) return false;
+      if (lane == 0) {
+        const uint32_t bar = map_to_cta(smem_u32(mail_full), 1);
+        mbar_expect_tx_remote(bar, 4);
+        st_async_u32(map_to_cta(smem_u32(const_cast<int*>(mail_tile)), 1), static_cast<uint32_t>(t), bar);
+      }
+      __syncwarp();
+      mail_phase ^= 1u;
+      return true;
+    };
+    auto receive = [&]() -> int {  // peer: what the leader sent, -2 if the wait ran out
+      int t = -2;
+      if (lane == 0 && mbar_wait<WaitScope::CLUSTER>(mail_full, mail_phase, abort_flag, 3)) {
+        t = *mail_tile;
+        mbar_arrive_release_cluster(map_to_cta(smem_u32(mail_empty), 0));
+      }
+      mail_phase ^= 1u;
       return __shfl_sync(0xffffffffu, t, 0);
     };
-    // The next index is fetched before the loads of the current tile and published behind the first of them: the atomic's
-    // round trip hides, the readers find theirs without waiting, and neither holds up a tile's first loads.
+    // The next index is fetched before the loads of the current tile and handed on behind the first of them, when the ring of
+    // loads is full: the atomic's round trip and the way to the peer hide, the readers find theirs without waiting, and neither
+    // holds up a tile's first loads.
     const int publish_kb = num_kb < PAIR_STAGES ? num_kb : PAIR_STAGES;
     int b_upto = -1;  // highest B piece known to have arrived
     int tile;
     if (leader) {
       tile = __shfl_sync(0xffffffffu, first, 0);
       if (tile >= num_tiles) tile = -1;
-      ok = publish(tile);
+      ok = publish(tile) && send(tile);
     } else {
-      tile = take();
+      tile = receive();
+      ok = tile != -2 && publish(tile);
     }
     const uint32_t smem0 = smem_u32(smem), full_local = smem_u32(full_bar), full0 = map_to_cta(full_local, 0);
     while (ok && tile >= 0) {
@@ -560,10 +580,12 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
       if (leader) {
         const int nt = __shfl_sync(0xffffffffu, nxt, 0);
         next = nt < num_tiles ? nt : -1;
-        if (!publish(next)) break;
+        if (!publish(next) || !send(next)) break;
+      } else {
+        next = receive();
+        if (next == -2 || !publish(next)) break;
       }
       if (!load_blocks(publish_kb, num_kb)) break;
-      if (!leader) next = take();
       tile = next;
     }
     if (leader && counted && lane == 0) {
@@ -596,7 +618,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
         if (++q == SCHED_DEPTH) { q = 0; qphase ^= 1u; }
         if (tile < 0) break;
         if (MH == 1) {
-          if (!mbar_wait_warp(&tmem_empty_bar[acc], acc_phase ^ 1u, abort_flag, 6)) { ok = false; break; }
+          if (!mbar_wait_warp<WaitScope::CLUSTER_RELAXED>(&tmem_empty_bar[acc], acc_phase ^ 1u, abort_flag, 6)) { ok = false; break; }
           tc_fence_after_sync();
         }
         for (int kb = 0; kb < num_kb; ++kb) {
@@ -606,7 +628,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
 #pragma unroll
           for (int h = 0; h < MH; ++h) {
             if (MH == 2 && kb == 0) {
-              if (!mbar_wait_warp(&tmem_empty_bar[h], acc_phase ^ 1u, abort_flag, 6)) { ok = false; break; }
+              if (!mbar_wait_warp<WaitScope::CLUSTER_RELAXED>(&tmem_empty_bar[h], acc_phase ^ 1u, abort_flag, 6)) { ok = false; break; }
               tc_fence_after_sync();
             }
             const uint32_t d_tmem = tmem_base + static_cast<uint32_t>((MH == 1 ? acc : h) * PAIR_BLOCK_N);
@@ -664,7 +686,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
         else          epilogue_rows<PAIR_BLOCK_N / 2>(t_acc, row0 + lane, n0, pt);
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive_remote(map_to_cta(smem_u32(&tmem_empty_bar[acc]), 0));
+        if (lane == 0) mbar_arrive_relaxed_cluster(map_to_cta(smem_u32(&tmem_empty_bar[acc]), 0));
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1u;
       } else {
@@ -685,7 +707,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
           for (int c = 0; c < 2; ++c) epi_pack64(t_base + static_cast<uint32_t>(h * PAIR_BLOCK_N + c * 64), bias == nullptr ? nullptr : bias + c * 64, &pk[h][c * 32]);
           tc_fence_before_sync();
           __syncwarp();
-          if (lane == 0) mbar_arrive_remote(map_to_cta(smem_u32(&tmem_empty_bar[h]), 0));
+          if (lane == 0) mbar_arrive_relaxed_cluster(map_to_cta(smem_u32(&tmem_empty_bar[h]), 0));
         }
         if (!ok) break;
         acc_phase ^= 1u;

@@ -33,15 +33,38 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// What a wait orders.  CTA: the accesses behind it come after those that threads of this CTA made before they arrived.  CLUSTER:
+// also those of the cluster's other CTAs, if they arrived with a release of cluster scope or their st.async completed the phase.
+// CLUSTER_RELAXED: the phase itself, of whichever CTA, and nothing in memory; with tcgen05.fence on both sides it orders accesses to
+// TMEM, which need no more.
+enum class WaitScope { CTA, CLUSTER, CLUSTER_RELAXED };
+template <WaitScope SCOPE = WaitScope::CTA>
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
+  if (SCOPE == WaitScope::CTA)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+  else if (SCOPE == WaitScope::CLUSTER)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
   return ok != 0;
 }
 
@@ -53,11 +76,12 @@ static __device__ unsigned int g_blocked_wait_sites[8];
 
 // `site` (1..255) identifies the wait in the kernel's source; the first wait that runs out leaves it in the abort flag and
 // the kernel reports it in bits 8..15 of the status word.
+template <WaitScope SCOPE = WaitScope::CTA>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int site = 1) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (mbar_try_wait<SCOPE>(bar, parity)) return true;
   const long long t0 = clock64();
   uint32_t spins = 0;
-  while (!mbar_try_wait(bar, parity)) {
+  while (!mbar_try_wait<SCOPE>(bar, parity)) {
     if (((++spins) & 63u) == 0u) {
       if (*abort_flag) {
         atomicOr(&g_blocked_wait_sites[(site >> 5) & 7], 1u << (site & 31));
@@ -76,8 +100,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 // The warp that issues tcgen05.mma runs its control flow with all 32 lanes, and one elected lane issues (umma_f16_ss_warp; by
 // instruction group in gemm_comm_tcgen05.cu): loop counters, shared-memory addresses and descriptors then stay warp-uniform
 // values.  This is the all-lanes wait for that warp; the vote makes the result (and every branch on it) uniform.
+template <WaitScope SCOPE = WaitScope::CTA>
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int site = 1) {
-  const bool ok = mbar_wait(bar, parity, abort_flag, site);
+  const bool ok = mbar_wait<SCOPE>(bar, parity, abort_flag, site);
   return __all_sync(0xffffffffu, ok) != 0;
 }
 
@@ -294,13 +319,17 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t local_smem_addr, uint32_
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_smem_addr), "r"(rank));
   return r;
 }
-// Arrive on a barrier of either CTA with the default (CTA-scope) release: for a slot that the arriving thread only read, or an
-// accumulator that it read with tcgen05.ld (ordered by tcgen05.fence::before_thread_sync).  A cluster-scope release makes the
-// thread wait until all its earlier stores to global memory are visible, 1000 cycles and more behind an epilogue's stores.
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+// Arrive on a barrier of either CTA of the cluster.  Release: what this thread did before is done for whoever waits with cluster
+// scope.  That costs until all its earlier stores to global memory are visible, 1000 cycles and more behind an epilogue's stores,
+// so a thread that only hands back an accumulator (read with tcgen05.ld, ordered by tcgen05.fence::before_thread_sync) arrives relaxed.
+__device__ __forceinline__ void mbar_arrive_release_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// A word for a CTA of the cluster: the store completes its bytes on that CTA's barrier, so data and signal need no fence.
+__device__ __forceinline__ void mbar_arrive_relaxed_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// A word for a CTA of the cluster: the store completes its bytes on that CTA's barrier (a release of cluster scope), so the sender
+// needs no fence.
 __device__ __forceinline__ void mbar_expect_tx_remote(uint32_t bar_cluster_addr, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(bar_cluster_addr), "r"(bytes) : "memory");
 }
