@@ -10,11 +10,14 @@
 //   softmax B   :                    [ softmax B(j) ............ ]              [ softmax B(j+1) ..... ]
 //
 // Roles (608 threads): warp 0 TMA producer, warp 1 MMA issuer and TMEM owner, warps 2-9 softmax of tile A, warps 10-17
-// softmax of tile B, warp 18 MMA issuer of tile B with head size 64 (below).  Two threads share a query row (TMEM lane), 64 of a step's 128 keys each: they read their scores once and
-// keep them in registers, pass each other the row maximum through shared memory, and with four warps per scheduler one warp's
-// loads and waits hide behind the exponentials of others.  (One thread per row read the scores twice, once for the maximum,
-// and left the exponential unit, which bounds head size 64, idle 46 % of the time: B2 S8192 H16 D64 433 -> 398 us,
-// B8 S1024 H16 D64 53.8 -> 45.8 us; head size 128, where the products bound the step, 168.8 -> 168.3 us at B8 S2048 H16.)
+// softmax of tile B, warp 18 MMA issuer of tile B with head size 64 (below).  Two threads share a query row (TMEM lane), 64 of a
+// step's 128 keys each: they read their scores once and keep them in registers, pass each other the row maximum and their sums
+// through shared memory, and with four warps per scheduler one warp's loads and waits hide behind the exponentials of others.
+// (One thread per row read the scores twice, once for the maximum, and left the exponential unit, which bounds head size 64, idle
+// 46 % of the time.  Against that, and with an issuer for each tile: B2 S8192 H16 D64 428 -> 395 us, B8 S1024 H16 D64 53.3 -> 45.1,
+// B16 S512 H16 D64 41.7 -> 32.6; head size 128, where the products bound the step, 47.1 -> 45.3 us at B2 S2048 H16.  The output and
+// the normaliser are to the bit those of one thread per row: a running sum for each thread would take 383 us at B2 S8192 H16 D64,
+// and make the result depend on how a row is divided.)
 // TMEM (512 columns): S_A [0,128)  S_B [128,256)  O_A [256,256+D)  O_B [384,384+D).  With head size 128 the bf16 probabilities overwrite
 // the first 64 columns of their own score tile (two values per 32-bit column) and feed P V as the TMEM A operand of
 // tcgen05.mma, so they never pass through shared memory.  The tensor pipe executes in issue order: S_t(j+1) is issued
@@ -27,10 +30,10 @@
 //
 //   tensor pipe :  S_A(j+1)  S_B(j+1)  PV_A(j)  PV_B(j)  S_A(j+2) ...
 //
-// and each tile has an issuer of its own: one for both held up the products of one tile behind its waits for the other
-// (B2 S8192 H16 D64 398 -> 381 us, B16 S512 H16 D64 44 -> 33 us together with the two threads a row).  With head size 128, in
-// place and bound by the products, strict turns are the faster order (B8 S2048 H16 D128 168 us, 177 with two issuers).
-// (In place, the chain exponentials -> PV -> S -> maximum kept the exponential unit, which bounds this head size, at 57 %.)
+// (In place, the chain exponentials -> PV -> S -> maximum kept the exponential unit, which bounds this head size, at 57 %.)  Each
+// tile has an issuer of its own: one for both held up the products of one tile behind its waits for the other (B16 S512 H16 D64
+// 44 -> 33 us together with the two threads a row).  With head size 128, in place and bound by the products, strict turns are the
+// faster order (B8 S2048 H16 D128 162 us, 177 with two issuers).
 //
 // Any sequence length: the tensor map is three-dimensional (columns, positions, batch), so a tile that overhangs the
 // sequence reads zeros instead of the next sequence's rows; keys past the end lie above every real query's diagonal and
@@ -92,10 +95,16 @@ struct Smem {
   static constexpr int K_OFF = 2 * TILE;     // two stages
   static constexpr int V_OFF = 4 * TILE;     // two stages
   static constexpr int BAR_OFF = 6 * TILE;
-  static constexpr int XCH_OFF = BAR_OFF + 512;  // [2 parities][2 tiles][2 halves][BM] values passed between the two threads of a row
-  static constexpr int TOTAL = XCH_OFF + 2 * 2 * 2 * BM * 4 + 1024;
+  static constexpr int XCH_OFF = BAR_OFF + 512;  // [2 parities][2 tiles][2 halves][3][BM] values passed between the two threads of a row
+  static constexpr int TOTAL = XCH_OFF + 2 * 2 * 2 * 3 * BM * 4 + 1024;
 };
 
+__device__ __forceinline__ void st_shared_f32(uint32_t addr, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
+__device__ __forceinline__ float ld_shared_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -136,9 +145,12 @@ __device__ __forceinline__ float chunk_max(const uint32_t (&r)[32], int col0, in
   return fmaxf(fmaxf(a[0], a[1]), fmaxf(a[2], a[3]));
 }
 
-// Probabilities of 32 scores, packed to bf16; their sum is added to `acc`.
+// Probabilities of 32 scores, packed to bf16; returns their sum: pairs of keys into four partial sums in turn.  (Packed additions
+// would be half as many, but take their operands from neighbouring registers, where the conversion to bf16 wants other
+// neighbours: B2 S8192 H16 D64 401 us, 412 with them, B4 S1543 H16 D128 67.7 us, 71.5.)
 template <bool DIAG>
-__device__ __forceinline__ void chunk_exp(const uint32_t (&r)[32], int col0, int row, uint64_t sl2, uint64_t neg_mb, uint64_t (&acc)[2], uint32_t (&pk)[16]) {
+__device__ __forceinline__ float chunk_exp(const uint32_t (&r)[32], int col0, int row, uint64_t sl2, uint64_t neg_mb, uint32_t (&pk)[16]) {
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
   for (int i = 0; i < 32; i += 2) {
     float x, y;
@@ -148,9 +160,10 @@ __device__ __forceinline__ void chunk_exp(const uint32_t (&r)[32], int col0, int
       if (col0 + i > row) p0 = 0.f;
       if (col0 + i + 1 > row) p1 = 0.f;
     }
-    acc[(i >> 1) & 1] = add_f32x2(acc[(i >> 1) & 1], pack_f32x2(p0, p1));
+    acc[(i >> 1) & 3] += p0 + p1;
     pk[i >> 1] = pack_bf16(p0, p1);
   }
+  return (acc[0] + acc[1]) + (acc[2] + acc[3]);
 }
 
 template <int D>
@@ -357,20 +370,28 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
     const uint32_t tp = tmem_base + P_COL + t * P_STEP + half * 32 + lane_off;        // its probabilities (in columns [0, 64) of the tile's scores unless SEP)
     const uint32_t to = tmem_base + O_COL + t * O_STEP + half * (D / 2) + lane_off;  // its output columns
     const int col0 = half * 64;
-    float* const xch = reinterpret_cast<float*>(smem + L::XCH_OFF) + t * 2 * BM + row;  // + parity * 4 BM + half * BM
+    const uint32_t xch = smem_u32(smem + L::XCH_OFF) + (t * 6 * BM + row) * 4;  // + parity * XCH_PARITY + half * XCH_HALF + value * 4 BM
+    constexpr uint32_t XCH_PARITY = 12 * BM * 4, XCH_HALF = 3 * BM * 4;
     uint64_t* const pair_bar = &bars->pair[t][quad];
     uint32_t xs = 0;  // exchanges so far (parity of the buffer, phase of pair_bar)
-    // The value that the other thread of this row passes in the same exchange.  The buffers alternate: a thread writes one
-    // again only after the partner has arrived at the exchange in between, i.e. has read it.
-    auto exchange = [&](float v, float& other) -> bool {
-      float* const x = xch + (xs & 1u) * 4 * BM;
-      x[half * BM] = v;
+    // What the two threads of a row pass each other at a step: their maxima, and the sums of their probabilities of the step before
+    // (leave_sum, per 32 keys).  Both then add up the row in the order of its keys: the four sums of a step one after the other,
+    // then on to the running sum.  (With a running sum for each thread the result would depend on how a row is divided.)  The
+    // buffers alternate: a thread writes one again only after the partner has arrived at the exchange in between, i.e. has read it.
+    auto leave_sum = [&](int k, float v) { st_shared_f32(xch + (xs & 1u) * XCH_PARITY + half * XCH_HALF + (1 + k) * 4 * BM, v); };  // for the next exchange
+    auto exchange = [&](float mx, float& other) -> bool {
+      const uint32_t x = xch + (xs & 1u) * XCH_PARITY;
+      st_shared_f32(x + half * XCH_HALF, mx);
       __syncwarp();
       if (lane == 0) mbar_arrive(pair_bar);
       if (!mbar_wait(pair_bar, xs & 1u, abort_flag)) return false;
-      other = x[(half ^ 1) * BM];
+      other = ld_shared_f32(x + (half ^ 1) * XCH_HALF);
       ++xs;
       return true;
+    };
+    auto sums = [&]() -> float {  // of the row at the step before, after this step's exchange and before the next
+      const uint32_t x = xch + ((xs & 1u) ^ 1u) * XCH_PARITY;
+      return ((ld_shared_f32(x + 4 * BM) + ld_shared_f32(x + 8 * BM)) + ld_shared_f32(x + XCH_HALF + 4 * BM)) + ld_shared_f32(x + XCH_HALF + 8 * BM);
     };
     const float sl2 = p.scale * LOG2E;
     const uint64_t sl2x2 = pack_f32x2(sl2, sl2);
@@ -387,7 +408,8 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
       const int n_it = 2 * q2 + 1 + t;
       const int pos = q2 * 2 * BM + t * BM + row;  // this thread's position in the sequence
       const bool row_ok = pos < p.S;
-      float m_run = m_low, l_run = 0.f;  // l_run: over this thread's keys
+      float m_run = m_low, mo;
+      float l_run = 0.f, alpha_run = 0.f;  // sum of the row up to the step before, scaling of that step
       for (int j = 0; j < n_it && ok; ++j, ++cs) {
         if (!mbar_wait(&bars->s_full[t], cs & 1u, abort_flag)) { ok = false; break; }
         tc_fence_after_sync();
@@ -401,7 +423,7 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars->s_read[t]);
         }
-        float mx = -INFINITY, mo;
+        float mx = -INFINITY;
         if (!diag) { mx = chunk_max<false>(r0, col0, row, mx); mx = chunk_max<false>(r1, col0 + 32, row, mx); }
         else       { mx = chunk_max<true>(r0, col0, row, mx);  mx = chunk_max<true>(r1, col0 + 32, row, mx); }
         // (in place, the exchange also keeps this thread's probabilities behind the partner's reads of the same columns)
@@ -414,9 +436,8 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
         const float alpha = j == 0 ? 0.f : ex2_approx((m_run - m_new) * sl2);
         const float mb = m_new * sl2;
         const uint64_t neg_mb = pack_f32x2(-mb, -mb);
-        uint64_t acc[2] = {0ull, 0ull};
         uint32_t pk[16];
-        if (!diag) chunk_exp<false>(r0, col0, row, sl2x2, neg_mb, acc, pk); else chunk_exp<true>(r0, col0, row, sl2x2, neg_mb, acc, pk);
+        const float c0 = !diag ? chunk_exp<false>(r0, col0, row, sl2x2, neg_mb, pk) : chunk_exp<true>(r0, col0, row, sl2x2, neg_mb, pk);
         const bool rescale = j > 0 && __any_sync(0xffffffffu, alpha != 1.f);
         if (j > 0 && (SEP || rescale)) {
           // O_t (and P_t, where it has columns of its own) belongs to P V of step j-1 until that has completed; in place it
@@ -425,7 +446,7 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
           tc_fence_after_sync();
         }
         tmem_st_32x16(tp, pk);
-        if (!diag) chunk_exp<false>(r1, col0 + 32, row, sl2x2, neg_mb, acc, pk); else chunk_exp<true>(r1, col0 + 32, row, sl2x2, neg_mb, acc, pk);
+        const float c1 = !diag ? chunk_exp<false>(r1, col0 + 32, row, sl2x2, neg_mb, pk) : chunk_exp<true>(r1, col0 + 32, row, sl2x2, neg_mb, pk);
         tmem_st_32x16(tp + 16, pk);
         if (rescale) {
 #pragma unroll 1
@@ -447,16 +468,17 @@ attn_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tm_qkv, Params p) {
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->p_full[t]);
-        float a0, a1;
-        unpack_f32x2(add_f32x2(acc[0], acc[1]), a0, a1);
-        l_run = l_run * alpha + (a0 + a1);
+        // the sums have time: the products wait for nothing below
+        leave_sum(0, c0);
+        leave_sum(1, c1);
+        if (j > 0) l_run = l_run * alpha_run + sums();
         m_run = m_new;
+        alpha_run = alpha;
       }
       if (!ok) break;
       // epilogue of the item: normalise and store this thread's half of the output row, then hand the accumulator back
-      float l_other;
-      if (!exchange(l_run, l_other)) { ok = false; break; }
-      l_run += l_other;
+      if (!exchange(0.f, mo)) { ok = false; break; }
+      l_run = l_run * alpha_run + sums();
       if (!mbar_wait(&bars->o_done[t], (cs - 1u) & 1u, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
       const float inv = 1.f / l_run;

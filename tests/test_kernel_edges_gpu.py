@@ -884,3 +884,57 @@ def test_frozen_parameters_claim_no_window_of_a_flat_gradient():
     assert torch.isfinite(x.grad).all()
     assert arena.buffer is None and not arena.claimed
     _status_ok()
+
+
+def _row_sums(p, four_by_four):
+    """fp32 sums over the keys of a row, ``p [rows, keys]``, steps of 128 keys: in the order of the keys (per 32 keys four partial
+    sums of pairs, the four sums of a step one after the other), or with a running sum for each half of a step."""
+    import numpy as np
+
+    p = np.pad(p, ((0, 0), (0, -p.shape[1] % 128))).astype(np.float32)
+    run = np.zeros((2, p.shape[0]), np.float32)
+    for j in range(0, p.shape[1], 128):
+        step = p[:, j:j + 128]
+        if four_by_four:
+            rs = np.zeros(p.shape[0], np.float32)
+            for c in range(0, 128, 32):
+                acc = [np.zeros(p.shape[0], np.float32) for _ in range(4)]
+                for i in range(0, 32, 2):
+                    acc[(i >> 1) & 3] = acc[(i >> 1) & 3] + (step[:, c + i] + step[:, c + i + 1])
+                rs = rs + ((acc[0] + acc[1]) + (acc[2] + acc[3]))
+            run[0] = run[0] + rs
+        else:
+            for h in (0, 1):
+                acc = [np.zeros(p.shape[0], np.float32) for _ in range(4)]
+                for i in range(0, 64, 2):
+                    for k in (0, 1):
+                        acc[2 * ((i >> 1) & 1) + k] = acc[2 * ((i >> 1) & 1) + k] + step[:, 64 * h + i + k]
+                run[h] = run[h] + ((acc[0] + acc[2]) + (acc[1] + acc[3]))
+    return run[0] + run[1]
+
+
+@pytest.mark.parametrize("S,D", [(128, 64), (128, 128), (715, 64), (715, 128), (1543, 128)])
+def test_attention_adds_a_row_up_in_the_order_of_its_keys(S, D):
+    """The normaliser of a row to the last bit.  Every score is a small integer and the scale makes the exponentials powers of two,
+    so all that is rounded is the sum.  Bound: a last bit of the sum (1 to 1.02) is 1.2e-7 of its logarithm; the logarithm, below
+    0.02, is itself good to 2 ulp of its value, 4e-9."""
+    import numpy as np
+
+    from fairscale_b200.ops import _bind, attention_native
+
+    attention_native._bind_sigs()
+    scale = float(np.float32(1) / np.float32(1.4426950408889634))  # times log2(e) in fp32: 1
+    rng = np.random.default_rng(S + D)
+    scores = rng.integers(-26, -13, S).astype(np.float32)
+    scores[0] = 0.0  # the maximum of every row, met at its first key
+    qkv = torch.zeros(1, S, 3, 1, D, dtype=torch.bfloat16, device=_dev())
+    qkv[0, :, 0, 0, 0] = 1.0
+    qkv[0, :, 1, 0, 0] = torch.from_numpy(scores).to(_dev())
+    o = torch.empty(1, S, D, dtype=torch.bfloat16, device=_dev())
+    lse = torch.empty(1, 1, S, dtype=torch.float32, device=_dev())
+    _bind.call("fsb_attn_fwd", qkv.data_ptr(), o.data_ptr(), lse.data_ptr(), 1, S, 1, D, scale, _bind.status_ptr(_dev()), _bind.stream_ptr(_dev()))
+    _status_ok()
+    p = np.where(np.tril(np.ones((S, S), bool)), np.exp2(scores)[None], 0.0).astype(np.float32)
+    want, divided = _row_sums(p, True).astype(np.float64), _row_sums(p, False).astype(np.float64)
+    assert want.max() < 1.02 and (want != divided).mean() > 0.1  # the two orders can be told apart
+    assert np.abs(lse.cpu().numpy()[0, 0].astype(np.float64) - np.log(want)).max() < 1e-8
