@@ -87,6 +87,7 @@ struct Bars {
   uint32_t tmem_slot;
   int abort_flag;
 };
+static_assert(sizeof(Bars) <= 512, "the values that the threads of a row exchange start behind the barriers (Smem::XCH_OFF)");
 
 template <int D>
 struct Smem {
