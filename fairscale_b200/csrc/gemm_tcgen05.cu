@@ -933,9 +933,29 @@ static GemmPlan choose_gemm_plan(int M, int N, int K, int lda, int ldb, int num_
   return best;
 }
 
-// The kernel that a product (or `problems` stacked ones) would get on a device with `num_sms` SMs where choose_persistent does not
-// come in (fp32 or unaligned results, K below 256, one wave or less): 0 CTA pairs, 1 one CTA per tile, 2 split-K over clusters
-// (a single product only).
+// The kernel of a product, or of `p.batch` stacked ones, that is neither streamed nor capped: what fsb_gemm_bf16 and
+// fsb_gemm_bf16_batched launch and fsb_gemm_kernel_of reports.
+static GemmPlan plan_product(const fsb::GemmParams& p, bool stacked, int lda, int ldb, int num_sms) {
+  const bool pairs = pair_enabled();
+  const int block_n = p.N <= 128 ? 128 : 256;
+  const long long tiles = static_cast<long long>(p.batch) * ((p.M + fsb::BLOCK_M - 1) / fsb::BLOCK_M) * ((p.N + block_n - 1) / block_n);
+  // more tiles than one wave of single CTAs (below, the wide tiles leave most SMs without one) and K as far as it was measured
+  if (pairs && tiles > num_sms && p.M >= 256 && p.N >= 256 && p.K >= 256 && row_pieces(p))
+    return {choose_persistent(p, lda, ldb, num_sms), block_n, 1};
+  if (!stacked) return choose_gemm_plan(p.M, p.N, p.K, lda, ldb, num_sms, pairs);
+  return {pairs && pair_pays(p.batch, p.M, p.N, p.K, lda, ldb, num_sms) ? GemmPlan::PAIR : GemmPlan::ONE_CTA, block_n, 1};
+}
+
+// What plan_product makes of a product (or of `problems` stacked ones) on a device with `num_sms` SMs, all pointers 16-byte aligned:
+// 0 CTA pairs, 1 one CTA per tile, 2 split-K over clusters (a single product only), 3 CTA pairs with tiles of 512 rows.
+FSB_API int fsb_gemm_kernel_of(int problems, int M, int N, int K, int lda, int ldb, int ldc, int ld_aux, int epilogue, int out_f32, int num_sms) {
+  fsb::GemmParams p{};
+  p.M = M; p.N = N; p.K = K;
+  p.ldc = ldc; p.ld_aux = ld_aux > 0 ? ld_aux : ldc;
+  p.epilogue = epilogue; p.out_f32 = out_f32; p.batch = problems;
+  return static_cast<int>(plan_product(p, problems > 1, lda, ldb, num_sms).kind);
+}
+// The same where choose_persistent does not come in (fp32 or unaligned results, K below 256, one wave or less).
 FSB_API int fsb_gemm_plan_of(long long problems, int M, int N, int K, int lda, int ldb, int num_sms) {
   if (problems > 1) return pair_enabled() && pair_pays(problems, M, N, K, lda, ldb, num_sms) ? 0 : 1;
   return static_cast<int>(choose_gemm_plan(M, N, K, lda, ldb, num_sms, pair_enabled()).kind);
@@ -1065,11 +1085,7 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, const void* bia
   if (streamed) plan.kind = GemmPlan::PAIR;
   else if (forced == 3 && !wide_takes(p)) return -1;
   else if (forced != 0) plan.kind = forced == 3 ? GemmPlan::WIDE_PAIR : forced == 2 ? GemmPlan::PAIR : GemmPlan::ONE_CTA;
-  else if (max_ctas == 0) {
-    plan = choose_gemm_plan(M, N, K, lda, ldb, num_sms, pair_enabled());
-    // more tiles than one wave of single CTAs (below, the wide tiles leave most SMs without one) and K as far as it was measured
-    if (tiles > num_sms && M >= 256 && N >= 256 && K >= 256 && pair_enabled() && row_pieces(p)) plan.kind = choose_persistent(p, lda, ldb, num_sms);
-  }
+  else if (max_ctas == 0) plan = plan_product(p, false, lda, ldb, num_sms);
   if (plan.kind == GemmPlan::CLUSTER_K) return fsb_host::gemm_cluster_k(ta, B, ldb, p, plan.block_n, plan.splits, dev, stream);
   // Run-time tile hand-out for products large enough to share the device with a collective; small ones stride.
   if (max_ctas == 0 && M >= 256 && N >= 256 && (plan.kind == GemmPlan::PAIR || plan.kind == GemmPlan::WIDE_PAIR || tiles > num_sms)) {
@@ -1138,10 +1154,7 @@ static int gemm_bf16_batched_impl(const void* A, const void* B, void* C, const v
   const int grid = tiles < num_sms ? static_cast<int>(tiles) : num_sms;
   if (forced == 3 && !wide_takes(p)) return -1;
   GemmPlan::Kind kind = forced == 3 ? GemmPlan::WIDE_PAIR : forced == 2 ? GemmPlan::PAIR : GemmPlan::ONE_CTA;
-  if (forced == 0 && pair_enabled()) {
-    if (pair_pays(batch, M, N, K, lda, ldb, num_sms)) kind = GemmPlan::PAIR;
-    if (tiles > num_sms && M >= 256 && N >= 256 && K >= 256 && row_pieces(p)) kind = choose_persistent(p, lda, ldb, num_sms);
-  }
+  if (forced == 0) kind = plan_product(p, true, lda, ldb, num_sms).kind;
   if (kind != GemmPlan::ONE_CTA) {
     if (!b_mn_major && !fsb_host::encode_3d_16bit(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)batch, (uint64_t)ldb, (uint64_t)stride_b, BLOCK_K, PAIR_HALF_N, 1)) return -1;
     p.sched_slot = sched_slot_of(dev & 63, stream);
@@ -1173,8 +1186,8 @@ FSB_API int fsb_gemm_bf16_batched(const void* A, const void* B, void* C, const v
                            epilogue, out_f32, accumulate_c, status, stream, 0);
 }
 
-// The same products by one of the two kernels whatever their size: plan 1 one CTA per tile, 2 CTA pairs (M and N at least 256,
-// -1 otherwise).  fsb_gemm_bf16_batched chooses by itself.
+// The same products by one of the persistent kernels whatever their size: plan 1, 2 or 3 as for fsb_gemm_bf16_plan.
+// fsb_gemm_bf16_batched chooses by itself.
 FSB_API int fsb_gemm_bf16_batched_plan(const void* A, const void* B, void* C, const void* bias, const void* aux, void* aux_out, int batch,
                                   int M, int N, int K, int lda, int ldb, int ldc, int ld_aux, long long stride_a, long long stride_b,
                                   long long stride_c, long long stride_aux, long long stride_bias, int a_mn_major, int b_mn_major,
