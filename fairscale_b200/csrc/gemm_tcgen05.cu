@@ -871,15 +871,19 @@ static bool pair_pays(long long problems, int M, int N, int K, int lda, int ldb,
 // launch, and per wave of tiles its start and its K blocks, or its epilogue where that takes longer; the share that goes with the
 // tiles per SM instead of whole waves is what the card's power limit gives back when a wave is partly empty.
 // Plain and bias products: fitted to 90 of them (M and N 256 .. 16384, K 256 .. 32000, one or 4 to 16 stacked, all operand layouts,
-// a third with rows off the 128-byte lines): taking the lowest estimate costs 0.8 % over the fastest kernel on average, taking
-// pair_pays' choice between the other two 9.6 %.  Measured (us, wide / pair / one CTA):
-//   16384 x 6144 x 2048 287 / 313 / 326       8192 x 2048 x 16384 (wgrad) 435 / 486 / 486     50304 x 2048 x 16384 (wgrad) 2576 / 3055 / 2847
-//   4096 x 12288 x 4096 317 / 306 / 342        2048 x 2048 x 16384 (wgrad) 167 / 120 / 124     16384 x 50304 x 2048 2518 / 2696 / 2898
-//   8 x 2048 x 1024 x 4096 115 / 125 / 139     8192 x 3072 x 1024 53.3 / 53.6 / 51.1           2792 x 3968 x 256 16.4 / 20.2 / 14.4
-// The other epilogues take time of their own, and the pair drains a tile with eight warps per CTA instead of four (us, pair / one CTA):
-//   GELU      16384 x 8192 x 2048 457 / 480    8192 x 4096 x 1024 72 / 81    3575 x 3072 x 768 (and its input stored) 31 / 37
-//   GELU'     16384 x 8192 x 2048 498 / 538    8192 x 4096 x 1024 88 / 106   3575 x 3072 x 768 35 / 39
-//   residual  16384 x 2048 x 8192 455 / 474    8192 x 1024 x 4096 68 / 71    8192 x 1024 x 1024 24.6 / 26.4
+// a third with rows off the 128-byte lines).  Over 40 others the choice costs 0.3 % on average and 9 % at worst (2208 x 2640 x 2240,
+// wide 32.7, one CTA 30.0); pair_pays' choice between the other two costs 7 %.  Measured (us, wide / pair / one CTA, a quarter of a second each):
+//   16384 x 6144 x 2048 323 / 352 / 345       8192 x 2048 x 16384 (wgrad) 435 / 476 / 482     50304 x 2048 x 16384 (wgrad) 2552 / 2837 / 2798
+//   4096 x 12288 x 4096 322 / 323 / 345       8192 x 3072 x 1024 50.8 / 55.2 / 52.0           16384 x 50304 x 2048 2527 / 2784 / 2853
+//   8 x 2048 x 1024 x 4096 123 / 127 / 133    2792 x 3968 x 256 16.5 / 16.4 / 14.3            16384 x 16384 x 1400 641 / 791 / 895
+// The other epilogues take time of their own, and the pair drains a tile with eight warps per CTA instead of four.  Fitted for each
+// to 68 products (M 1024 .. 16384, N 256 .. 8192, K 256 .. 12288, half of them off the lines), the mean of bursts of 3 ms and of
+// stretches of 0.2 s at the power limit: the choice costs 0.1 % on average and 2.8 % at worst.  (With the residual's constants of a
+// plain product but for its start it cost 1 % and 7.3 %.)  Measured (us at the power limit, pair / one CTA):
+//   GELU           16384 x 8192 x 2048 482 / 462    16384 x 2048 x 2048 127 / 119    8192 x 2048 x 512 32.4 / 36.8    14724 x 1144 x 2680 106 / 129
+//   GELU'          16384 x 8192 x 2048 512 / 523    16384 x 2048 x 2048 134 / 135    8192 x 2048 x 512 45.6 / 48.9    14724 x 1144 x 2680 115 / 136
+//   bias+residual  16384 x 8192 x 2048 505 / 482    16384 x 2048 x 2048 133 / 123    8192 x 2048 x 512 35.2 / 39.6    14724 x 1144 x 2680 111 / 134
+//   residual       16384 x 8192 x 2048 501 / 479    16384 x 2048 x 2048 131 / 122    8192 x 2048 x 512 31.2 / 34.3    14724 x 1144 x 2680 110 / 133
 static bool row_pieces(const fsb::GemmParams& p) {
   const uintptr_t ptrs = reinterpret_cast<uintptr_t>(p.C) | reinterpret_cast<uintptr_t>(p.aux) | reinterpret_cast<uintptr_t>(p.aux_out);
   return !p.out_f32 && p.N % 8 == 0 && p.ldc % 8 == 0 && p.ld_aux % 8 == 0 && p.stride_c % 8 == 0 && p.stride_aux % 8 == 0 && (ptrs & 15u) == 0;
@@ -898,10 +902,17 @@ static GemmPlan::Kind choose_persistent(const fsb::GemmParams& p, int lda, int l
     const float main_loops = waves * (start + num_kb * per_wave) + num_kb * share * per_share;
     return launch + (main_loops > waves * epilogue ? main_loops : waves * epilogue);
   };
-  const bool gelu = p.epilogue == fsb::EPI_BIAS_GELU, dgelu = p.epilogue == fsb::EPI_DGELU;
-  const bool residual = p.epilogue == fsb::EPI_BIAS_RESIDUAL || p.epilogue == fsb::EPI_RESIDUAL;
-  const float pair = cost(tiles(256), num_sms / 2, 7.2f, residual ? 3.f : 2.2f, 0.262f + 0.017f * off_line, 0.16f, gelu ? 9.5f : dgelu ? 11.4f : 0.f);
-  const float one = cost(tiles(128), num_sms, 5.0f, residual ? 3.6f : 1.1f, 0.229f + 0.064f * off_line, 0.25f, gelu ? 12.f : dgelu ? 14.2f : 0.f);
+  struct Wave { float start, per_wave, per_off_line, per_share, epilogue; };
+  // by EPI_*: none, bias, bias + GELU, bias + residual, GELU', residual
+  static const Wave pair_wave[] = {{2.2f, 0.262f, 0.017f, 0.16f, 0.f},   {2.2f, 0.262f, 0.017f, 0.16f, 0.f},   {1.06f, 0.243f, 0.021f, 0.194f, 6.952f},
+                                   {2.108f, 0.209f, 0.029f, 0.217f, 7.733f}, {3.58f, 0.194f, 0.025f, 0.228f, 10.249f}, {2.181f, 0.171f, 0.029f, 0.256f, 6.407f}};
+  static const Wave one_wave[] = {{1.1f, 0.229f, 0.064f, 0.25f, 0.f},    {1.1f, 0.229f, 0.064f, 0.25f, 0.f},    {0.693f, 0.376f, 0.059f, 0.066f, 8.515f},
+                                  {2.111f, 0.349f, 0.068f, 0.074f, 9.57f},  {3.949f, 0.299f, 0.059f, 0.129f, 11.766f}, {2.247f, 0.281f, 0.068f, 0.144f, 7.904f}};
+  auto wave_cost = [&](int rows, int units, float launch, const Wave& w) -> float {
+    return cost(tiles(rows), units, launch, w.start, w.per_wave + w.per_off_line * off_line, w.per_share, w.epilogue);
+  };
+  const int epi = p.epilogue >= fsb::EPI_NONE && p.epilogue <= fsb::EPI_RESIDUAL ? p.epilogue : fsb::EPI_NONE;
+  const float pair = wave_cost(256, num_sms / 2, 7.2f, pair_wave[epi]), one = wave_cost(128, num_sms, 5.0f, one_wave[epi]);
   if (wide_takes(p)) {
     const float wide = cost(tiles(512), num_sms / 2, 7.2f, 2.0f, 0.52f, 0.25f, 0.f);
     if (wide <= pair && wide <= one) return GemmPlan::WIDE_PAIR;
