@@ -9,6 +9,8 @@
 
 #include "common.cuh"
 
+#include <atomic>
+
 namespace fsb {
 
 constexpr int NORM_THREADS = 256;
@@ -16,12 +18,29 @@ constexpr int NORM_MAX_VEC = 4;  // block-per-row path: up to 4 x 8 bf16 per thr
 constexpr int NORM_WARPS = 4;    // warp-per-row forward: rows handled per CTA
 constexpr int NORM_ROWS_MAX_H = 4096;  // row-group backward: up to 512 threads of 8 columns
 
-// ---- warp-per-row forward (H <= 4096): a lane keeps VPL 16-byte vectors of the row in registers, all
+// Eight columns of a row in a lane's registers, as fp32 or as they came.
+template <bool F32> struct RowPiece {
+  float v[8];
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) {
+    const Vec16<__nv_bfloat16> t = ld16(p);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = __bfloat162float(t.v[k]);
+  }
+  __device__ __forceinline__ float operator[](int k) const { return v[k]; }
+};
+template <> struct RowPiece<false> {
+  Vec16<__nv_bfloat16> v;
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = ld16(p); }
+  __device__ __forceinline__ float operator[](int k) const { return __bfloat162float(v.v[k]); }
+};
+
+// ---- warp-per-row forward (H <= 4096): a lane keeps VPL pieces of eight columns of the row in registers, all
 // reductions are warp shuffles, no shared memory and no block barriers.
-// Bound by memory, and by how many rows are in flight: kept as bf16 a row takes 64 registers a thread at 2048 columns (95 as fp32)
-// and 96 at 4096 (164): 16384 x 2048 35.2 -> 28.9 us (20.5 at the copy rate), 4096 x 4096 20.0 -> 18.0; up to 1024 columns, where
-// registers were no limit, the same (8192 x 1024 10.3 us).
-template <bool RMS, int VPL>
+// Bound by memory, and by how many rows are in flight: as bf16 a row takes 64 registers a thread at 2048 columns (95 as fp32)
+// and 96 at 4096 (164): 16384 x 2048 31.8 -> 25.9 us (20.5 at the copy rate), 16384 x 4096 71 -> 58.  But each value is then
+// converted three times, and where registers are no limit that is what takes the time: 65536 x 328 22.9 us as fp32, 25.8 as
+// bf16, 16384 x 1024 11.3 and 12.3, 300 x 3072 6.1 and 7.0.  launch_norm_fwd has the line.
+template <bool RMS, int VPL, bool F32>
 __global__ void __launch_bounds__(NORM_WARPS * 32) norm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
                                                                         const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y,
                                                                         float* __restrict__ mean_out, float* __restrict__ rstd_out,
@@ -31,19 +50,19 @@ __global__ void __launch_bounds__(NORM_WARPS * 32) norm_fwd_warp_kernel(const __
   if (row >= rows) return;
   const int nvec = H / 8;
   const __nv_bfloat16* xr = x + row * H;
-  Vec16<__nv_bfloat16> v[VPL];  // as they came: in fp32 they took twice the registers and half the warps in flight
+  RowPiece<F32> v[VPL];
   float sum = 0.f;
 #pragma unroll
   for (int it = 0; it < VPL; ++it) {
     const int j = lane + it * 32;
-    if (j < nvec) v[it] = ld16(xr + j * 8);
+    if (j < nvec) v[it].load(xr + j * 8);
   }
 #pragma unroll
   for (int it = 0; it < VPL; ++it) {
     const int j = lane + it * 32;
     if (j < nvec) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) sum += __bfloat162float(v[it].v[k]);
+      for (int k = 0; k < 8; ++k) sum += v[it][k];
     }
   }
   const float mean = RMS ? 0.f : warp_sum(sum) / H;
@@ -53,7 +72,7 @@ __global__ void __launch_bounds__(NORM_WARPS * 32) norm_fwd_warp_kernel(const __
     const int j = lane + it * 32;
     if (j < nvec) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) { const float d = __bfloat162float(v[it].v[k]) - mean; sq += d * d; }
+      for (int k = 0; k < 8; ++k) { const float d = v[it][k] - mean; sq += d * d; }
     }
   }
   const float rstd = rsqrtf(warp_sum(sq) / H + eps);
@@ -72,10 +91,10 @@ __global__ void __launch_bounds__(NORM_WARPS * 32) norm_fwd_warp_kernel(const __
         const Vec16<__nv_bfloat16> b = ld16(beta + j * 8);
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-          o.v[k] = __float2bfloat16_rn((__bfloat162float(v[it].v[k]) - mean) * rstd * __bfloat162float(g.v[k]) + __bfloat162float(b.v[k]));
+          o.v[k] = __float2bfloat16_rn((v[it][k] - mean) * rstd * __bfloat162float(g.v[k]) + __bfloat162float(b.v[k]));
       } else {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) o.v[k] = __float2bfloat16_rn((__bfloat162float(v[it].v[k]) - mean) * rstd * __bfloat162float(g.v[k]));
+        for (int k = 0; k < 8; ++k) o.v[k] = __float2bfloat16_rn((v[it][k] - mean) * rstd * __bfloat162float(g.v[k]));
       }
       st16(yr + j * 8, o);
     }
@@ -450,21 +469,48 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16
 
 }  // namespace fsb
 
-// H must be a multiple of 8 and <= 8192. mean/rstd are fp32 [rows]. rms != 0 selects RMSNorm
-// (beta and mean ignored).
+// Rows of the widest warp-per-row forward that the device holds at a time.
+template <bool RMS, bool F32>
+static long long norm_rows_in_flight() {
+  using namespace fsb;
+  static std::atomic<int> cache[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  int rows = cache[dev & 63].load(std::memory_order_relaxed);
+  if (rows == 0) {
+    int ctas = 1, sms = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, norm_fwd_warp_kernel<RMS, 16, F32>, NORM_WARPS * 32, 0);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    rows = ctas * sms * NORM_WARPS;
+    if (rows < 1) rows = 1;
+    cache[dev & 63].store(rows, std::memory_order_relaxed);
+  }
+  return rows;
+}
+
+// Rows in fp32 up to 1024 columns, where they are all in flight either way; as bf16 beyond, up to 2048 columns at any number of
+// rows (fewer than one wave: within 5 % of one another); beyond that by the number of waves, of which fp32 takes more (1776 rows
+// each, bf16 2960) but shorter ones (us, fp32 / bf16, 4096 columns: 1200 rows 8.6 / 9.0, 2048 13.3 / 9.4, 3200 13.7 / 15.1).
 template <bool RMS>
 static void launch_norm_fwd(const __nv_bfloat16* x, const __nv_bfloat16* g, const __nv_bfloat16* b, __nv_bfloat16* y, float* mean,
                             float* rstd, long long rows, int H, float eps, cudaStream_t stream) {
   using namespace fsb;
   const unsigned grid = static_cast<unsigned>((rows + NORM_WARPS - 1) / NORM_WARPS);
   const int vpl = (H / 8 + 31) / 32;
-  if (vpl <= 2)       norm_fwd_warp_kernel<RMS, 2><<<grid, NORM_WARPS * 32, 0, stream>>>(x, g, b, y, mean, rstd, rows, H, eps);
-  else if (vpl <= 4)  norm_fwd_warp_kernel<RMS, 4><<<grid, NORM_WARPS * 32, 0, stream>>>(x, g, b, y, mean, rstd, rows, H, eps);
-  else if (vpl <= 8)  norm_fwd_warp_kernel<RMS, 8><<<grid, NORM_WARPS * 32, 0, stream>>>(x, g, b, y, mean, rstd, rows, H, eps);
-  else if (vpl <= 16) norm_fwd_warp_kernel<RMS, 16><<<grid, NORM_WARPS * 32, 0, stream>>>(x, g, b, y, mean, rstd, rows, H, eps);
+  auto warp_rows = [&](auto kernel) { kernel<<<grid, NORM_WARPS * 32, 0, stream>>>(x, g, b, y, mean, rstd, rows, H, eps); };
+  if (vpl <= 2)       warp_rows(norm_fwd_warp_kernel<RMS, 2, true>);
+  else if (vpl <= 4)  warp_rows(norm_fwd_warp_kernel<RMS, 4, true>);
+  else if (vpl <= 8)  warp_rows(norm_fwd_warp_kernel<RMS, 8, false>);
+  else if (vpl <= 16) {
+    const long long in_f32 = norm_rows_in_flight<RMS, true>(), in_bf16 = norm_rows_in_flight<RMS, false>();
+    if ((rows + in_f32 - 1) / in_f32 <= (rows + in_bf16 - 1) / in_bf16) warp_rows(norm_fwd_warp_kernel<RMS, 16, true>);
+    else                                                                warp_rows(norm_fwd_warp_kernel<RMS, 16, false>);
+  }
   else norm_fwd_kernel<RMS><<<static_cast<unsigned>(rows), NORM_THREADS, 0, stream>>>(x, g, b, y, mean, rstd, H, eps);
 }
 
+// H must be a multiple of 8 and <= 8192. mean/rstd are fp32 [rows]. rms != 0 selects RMSNorm
+// (beta and mean ignored).
 FSB_API int fsb_norm_fwd(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd,
                          long long rows, int H, float eps, int rms, cudaStream_t stream) {
   using namespace fsb;

@@ -938,3 +938,24 @@ def test_attention_adds_a_row_up_in_the_order_of_its_keys(S, D):
     want, divided = _row_sums(p, True).astype(np.float64), _row_sums(p, False).astype(np.float64)
     assert want.max() < 1.02 and (want != divided).mean() > 0.1  # the two orders can be told apart
     assert np.abs(lse.cpu().numpy()[0, 0].astype(np.float64) - np.log(want)).max() < 1e-8
+
+
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("H", [8, 264, 1024, 2048, 2056, 3000, 4096])
+def test_a_row_is_normalised_alike_however_many_there_are(H, rms):
+    """Rows of more than 2048 columns are kept as fp32 or as bf16 by their number (300 and 2048 lie on either side): to the bit the same."""
+    from fairscale_b200.ops import norm
+
+    torch.manual_seed(H)
+    x = (torch.randn(2048, H, device=_dev()) * 3 + 1).bfloat16()
+    w, b = torch.randn(H, device=_dev()).bfloat16(), None if rms else torch.randn(H, device=_dev()).bfloat16()
+    many, few, one = (norm.norm_forward(x[:n], w, b, 1e-5, rms) for n in (2048, 300, 1))
+    _status_ok()
+    for m, f, o in zip(many, few, one):
+        assert (m is None) == (f is None) == (o is None)
+        if m is not None:
+            assert torch.equal(m[:300], f) and torch.equal(m[:1], o)
+    xd = x.double()
+    want = xd if rms else xd - xd.mean(1, keepdim=True)
+    want = want * torch.rsqrt((want * want).mean(1, keepdim=True) + 1e-5) * w.double() + (0 if rms else b.double())
+    assert _rel_err(many[0], want) < 1e-2
