@@ -16,6 +16,10 @@
 // accumulating products.  An issuing warp is held until the tensor pipe takes its products, and a wait that does not block
 // costs it 100 - 200 cycles all the same; one warp for all products left the pipe idle behind its waits (B2 S8192 H16 D64: of
 // 1 290 cycles a step of 64 queries or keys, 650 of products, while the probabilities of the step lay ready for 1 500).
+// The score products of an item are issued behind the accumulating ones of the item before (acc_issued): ahead of the last of
+// those, whose result the compute warps wait for, they held up items of few steps (HB sequences of all heads, us without / with: S16
+// HB1760 D128 85.9 / 83.2, S77 HB640 D64 46.0 / 45.1, S268 HB640 D128 223.6 / 221.1; long ones alike).  What an issuer more still
+// costs the shortest sequences is 2 to 4 % (78.6, 43.3 and 221.1 us with one).
 // A K-major tile [rows, 64] and an MN-major tile of the same bytes differ only in the MMA descriptor, so each
 // streamed tile is loaded once and used both as a "transposed" and a "plain" operand.
 // Any sequence length: the tensor maps are three-dimensional (columns, positions, batch), so a tile that overhangs the
@@ -81,6 +85,7 @@ struct AttnBars {
   uint64_t s_full[3];     // scores and dP of a step are in buffer b
   uint64_t p_full[3];     // the 8 warps of the step have written dS (dQ kernel) / P^T and dS^T (dK/dV kernel) over them
   uint64_t buf_free[3];   // the accumulating products that read buffer b have completed
+  uint64_t acc_issued;    // the item's accumulating products are on their way: the next item's score products may follow
   uint64_t acc_done;      // the item's accumulating products have completed
   uint64_t acc_free;      // the 16 compute warps have read the item's output accumulators
   uint32_t tmem_slot;
@@ -101,6 +106,7 @@ __device__ __forceinline__ void attn_init_bars(AttnBars* b) {
     mbar_init(&b->p_full[i], 8);
     mbar_init(&b->buf_free[i], 1);
   }
+  mbar_init(&b->acc_issued, 1);
   mbar_init(&b->acc_done, 1);
   mbar_init(&b->acc_free, 16);
   b->abort_flag = 0;
@@ -244,6 +250,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_cons
     for (int item; ok && (item = snake_item(static_cast<int>(it))) < n_items; ++it) {
       const int qt = n_qt - 1 - item / HB;
       const int n_steps = 2 * (qt + 1);
+      if (it > 0 && !mbar_wait_warp(&bars->acc_issued, (it - 1u) & 1u, abort_flag, 43)) { ok = false; break; }
       if (!mbar_wait_warp(&bars->stat_full, it & 1u, abort_flag, 37)) { ok = false; break; }
       for (int u = 0; u < n_steps; ++u) {
         if ((u & 1) == 0 && !mbar_wait_warp(&bars->str_full[st], st_phase, abort_flag, 35)) { ok = false; break; }
@@ -285,7 +292,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_cons
           umma_f16_ts_warp(tmem_base + DQ_COL, t_s + (ks >> 1) * 32 + (ks & 1) * 8, desc_offset(dkt, kstep_mnmajor(ks)), idesc_q, (u | ks) != 0);
         umma_commit_warp(&bars->buf_free[buf]);
         if ((u & 1) != 0) umma_commit_warp(&bars->str_empty[st]);
-        if (u == n_steps - 1) umma_commit_warp(&bars->acc_done);
+        if (u == n_steps - 1) {
+          umma_commit_warp(&bars->acc_done);
+          if (lane == 0) mbar_arrive(&bars->acc_issued);
+        }
         if (++buf == NBUF) { buf = 0; buf_phase ^= 1u; }
         if ((u & 1) != 0 && ++st == L::STAGES) st = 0;
       }
@@ -500,6 +510,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_cons
     for (int item; ok && (item = snake_item(static_cast<int>(it))) < n_items; ++it) {
       const int kt = item / HB;
       const int n_sub = p.S_pad / KV_QSUB - kt * (ATT_BM / KV_QSUB);
+      if (it > 0 && !mbar_wait_warp(&bars->acc_issued, (it - 1u) & 1u, abort_flag, 75)) { ok = false; break; }
       if (!mbar_wait_warp(&bars->stat_full, it & 1u, abort_flag, 69)) { ok = false; break; }
       for (int t = 0; t < n_sub; ++t) {
         if (!mbar_wait_warp(&bars->str_full[st], st_phase, abort_flag, 67)) { ok = false; break; }
@@ -543,7 +554,10 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_cons
           umma_f16_ts_warp(tmem_base + DK_COL, t_s + 64 + (ks >> 1) * 32 + (ks & 1) * 8, desc_offset(dqt, kstep_mnmajor(ks)), idesc_a, (t | ks) != 0);
         umma_commit_warp(&bars->buf_free[buf]);
         umma_commit_warp(&bars->str_empty[st]);
-        if (t == n_sub - 1) umma_commit_warp(&bars->acc_done);
+        if (t == n_sub - 1) {
+          umma_commit_warp(&bars->acc_done);
+          if (lane == 0) mbar_arrive(&bars->acc_issued);
+        }
         if (++buf == NBUF) { buf = 0; buf_phase ^= 1u; }
         if (++st == L::STAGES) st = 0;
       }

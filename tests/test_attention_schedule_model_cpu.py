@@ -409,3 +409,25 @@ def test_forward_with_two_issuers_is_safe_and_live(items):
 def test_model_notices_two_issuers_without_their_barriers():
     assert any(explore(split_backward_programs([4, 4], 2, 4, 1, drop=("buf_free",)))[:2])
     assert any(explore(split_forward_programs([(2, True), (1, True)], drop=("pass_wait",)))[:2])
+
+
+def followed_backward_programs(items, nbuf, stages, steps_per_load):
+    """... and the score products of an item wait until the accumulating ones of the item before have been issued."""
+    (producer, scores, sums, *sets), counts = split_backward_programs(items, nbuf, stages, steps_per_load)
+    after = []
+    for op in scores:
+        if op[:2] == ("wait", "stat_full") and op[3] > 1:
+            after.append(("wait", "acc_issued", (op[3] - 2) & 1, op[3] - 1))
+        after.append(op)
+    told = [o for op in sums for o in ([op, ("arrive", "acc_issued")] if op == ("commit", "acc_done") else [op])]
+    return [producer, after, told, *sets], counts
+
+
+@pytest.mark.parametrize("nbuf,stages,per_load,items", [(3, 4, 2, [6, 2, 2]), (2, 2, 2, [2, 2, 2]), (3, 6, 1, [6, 2]), (2, 4, 1, [2, 2, 2])],
+                         ids=["dq64", "dq128", "dkv64", "dkv128"])
+def test_backward_issuers_that_follow_one_another_are_safe_and_live(nbuf, stages, per_load, items):
+    programs, counts = followed_backward_programs(items, nbuf, stages, per_load)
+    assert sum(op[1] == "acc_issued" for op in programs[1]) == len(items) - 1 and programs[2].count(("arrive", "acc_issued")) == len(items)
+    problems, deadlocks, states = explore((programs, counts))
+    assert states > 100
+    assert not problems and deadlocks == 0, (sorted(map(str, problems))[:3], deadlocks)
