@@ -940,6 +940,37 @@ def test_attention_adds_a_row_up_in_the_order_of_its_keys(S, D):
     assert np.abs(lse.cpu().numpy()[0, 0].astype(np.float64) - np.log(want)).max() < 1e-8
 
 
+@pytest.mark.parametrize("plan", [1, 2])
+@pytest.mark.parametrize("M,N,K", [(256, 264, 72), (300, 264, 72), (520, 1032, 200)])
+def test_packed_gelu_is_the_scalar_one_to_the_bit(M, N, K, plan):
+    """GELU and GELU' of whole 16-byte pieces are computed two values per instruction, those of a matrix whose width is no multiple of
+    eight one at a time: one column less must not change a bit of the others.  Inputs reach the constant ends of the polynomial."""
+    from ctypes import c_int, c_void_p
+
+    from fairscale_b200.ops import _bind
+
+    _bind._SIGNATURES.setdefault("fsb_gemm_bf16_plan", [c_void_p] * 6 + [c_int] * 13 + [c_void_p] * 2)
+    torch.manual_seed(M + N)
+    a, b, z = (torch.randn(*s, device=_dev()).bfloat16() for s in ((M, K), (N, K), (M, N)))
+    b, z, bias = b * (2.0 / K**0.5), z * 2, torch.randn(N, device=_dev()).bfloat16()
+
+    def run(epi, n):
+        c = torch.full((M, N), float("nan"), device=_dev(), dtype=torch.bfloat16)
+        pre = torch.empty_like(c)
+        _bind.call("fsb_gemm_bf16_plan", a.data_ptr(), b.data_ptr(), c.data_ptr(), bias.data_ptr() if epi == 2 else None, z.data_ptr() if epi == 4 else None,
+                   pre.data_ptr() if epi == 2 else None, M, n, K, K, K, N, N, 0, 0, epi, 0, 0, plan, _bind.status_ptr(_dev()), _bind.stream_ptr(_dev()))
+        return c, pre
+
+    for epi in (2, 4):
+        (packed, pre), (scalar, pre_scalar) = run(epi, N), run(epi, N - 1)
+        _status_ok()
+        assert scalar[:, N - 1].isnan().all() and not packed.isnan().any()
+        assert torch.equal(packed[:, : N - 1], scalar[:, : N - 1])
+        if epi == 2:
+            assert torch.equal(pre[:, : N - 1], pre_scalar[:, : N - 1])
+            assert (pre.float().abs() > 5).any()
+
+
 @pytest.mark.parametrize("rms", [False, True])
 @pytest.mark.parametrize("H", [8, 264, 1024, 2048, 2056, 3000, 4096])
 def test_a_row_is_normalised_alike_however_many_there_are(H, rms):

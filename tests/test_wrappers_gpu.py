@@ -277,3 +277,34 @@ def test_allocated_memory_per_phase_of_an_fsdp_step():
     expect_full = mb(layers * (2 * batch * 4 * d + 2 * batch * d) * 4)
     assert act_ckpt < 0.45 * act_full, results
     assert 0.6 * expect_full < act_full < 1.6 * expect_full, (act_full, expect_full)
+
+
+def test_stream_helpers_of_fsdp_are_those_of_torch():
+    """``_on_stream`` and ``_current_stream`` call private entry points: nested, left by an exception, on the default stream, and inside
+    ``torch.cuda.stream``, the current stream has to be what torch's own functions make it."""
+    from fairscale_b200.nn.data_parallel import fully_sharded_data_parallel as fsdp
+
+    a, b = torch.cuda.Stream(_dev()), torch.cuda.Stream(_dev(), priority=-1)
+    before = torch.cuda.current_stream(_dev())
+
+    def now():
+        want = torch.cuda.current_stream(_dev())
+        for dev in (_dev(), torch.device("cuda")):
+            got = fsdp._current_stream(dev)
+            assert got == want and got.cuda_stream == want.cuda_stream and got.device == want.device
+        return want
+
+    assert now() == before
+    with fsdp._on_stream(a):
+        assert now() == a
+        with pytest.raises(ValueError):
+            with fsdp._on_stream(b):
+                assert now() == b
+                with torch.cuda.stream(a), fsdp._on_stream(before):
+                    assert now() == before
+                assert now() == b
+                raise ValueError
+        assert now() == a
+        with fsdp._on_stream(None), fsdp._on_stream(fsdp._NULL_STREAM):
+            assert now() == a
+    assert now() == before
