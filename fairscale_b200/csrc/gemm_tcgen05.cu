@@ -418,6 +418,8 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
     if (BATCHED) tma_load_3d_pair_warp(dst, map, bar, x, y, z);
     else         tma_load_2d_pair_warp(dst, map, bar, x, y);
   };
+  // Whole lines of C; in a batch every problem's base has to keep the alignment of the first one
+  const bool coalesce = MH == 2 || (epilogue_can_coalesce(p) && (!BATCHED || (p.stride_c % 8 == 0 && p.stride_aux % 8 == 0)));
   // Index of this pair's first tile (lane 0 of the leader's producer warp): on its way while the pair sets itself up.
   unsigned int* const sched = g_sched_counters + 2 * p.sched_slot;
   const bool counted = p.sched_slot != 0;
@@ -524,7 +526,10 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
     // The next index is fetched before the loads of the current tile and handed on behind the first of them, when the ring of
     // loads is full: the atomic's round trip and the way to the peer hide, the readers find theirs without waiting, and neither
     // holds up a tile's first loads.
-    const int publish_kb = num_kb < PAIR_STAGES ? num_kb : PAIR_STAGES;
+    // (Not where the epilogue stores a row per thread, fp32 or off the 16-byte pieces, and takes longer than the products: 16384 x
+    // 6144 x 2048 fp32 398 us handed on before the loads, 464 behind them; odd rows 341 and 392.  With whole lines it is 502 and 490
+    // us at 16384 x 8192 x 2048 with a residual.)
+    const int publish_kb = !coalesce ? 0 : num_kb < PAIR_STAGES ? num_kb : PAIR_STAGES;
     int b_upto = -1;  // highest B piece known to have arrived
     int tile;
     if (leader) {
@@ -656,8 +661,6 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const 
     const int quad = warp & 3;            // TMEM lane quadrant this warp may access
     const int half = (warp - 2) >> 2;     // which 128 columns of the 256 this warp drains
     uint8_t* stage = smem + L::EPI_OFFSET + (warp - 2) * 4096;
-    // in a batch every problem's base has to keep the alignment of the first one
-    const bool coalesce = epilogue_can_coalesce(p) && (!BATCHED || (p.stride_c % 8 == 0 && p.stride_aux % 8 == 0));
     int acc = 0;
     uint32_t acc_phase = 0;
     int q = 0;

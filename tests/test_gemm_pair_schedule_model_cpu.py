@@ -17,10 +17,11 @@ DEPTH = 2  # slots of a CTA's ring (the kernel has four)
 KERNEL = {"mail_full": ("cluster", "cluster"), "mail_empty": ("cluster", "cluster"), "tmem_empty": ("relaxed", "relaxed")}
 
 
-def pair_programs(row_blocks, tiles, num_kb, stages, drop=()):
-    """Programs as ``explore`` takes them: ``row_blocks`` 1, tiles of 256 rows with two accumulators; 2, tiles of 512 rows."""
+def pair_programs(row_blocks, tiles, num_kb, stages, drop=(), publish_kb=None):
+    """Programs as ``explore`` takes them: ``row_blocks`` 1, tiles of 256 rows with two accumulators; 2, tiles of 512 rows.
+    The next index is handed on behind the first ``publish_kb`` loads of a tile, a ring of them unless given."""
     prods, mma, epis = ([], []), [], ([], [])
-    publish_kb = min(num_kb, stages)
+    publish_kb = min(num_kb, stages) if publish_kb is None else publish_kb
     order = list(range(tiles)) + [-1]
     need = {f"full{s}": 2 for s in range(stages)}  # the bytes of both CTAs
     need.update({f"tmem_empty{a}": 2 for a in (0, 1)})  # an epilogue of each CTA
@@ -197,3 +198,14 @@ def test_accesses_across_the_pair_are_ordered(row_blocks, tiles, num_kb, stages)
 def test_cta_scope_does_not_order_the_two_ctas(signal, weaker):
     """What the kernel gave its hand-out before: arrivals and waits of CTA scope between the CTAs."""
     assert any(races(pair_programs(1, 6, 3, 4), {**KERNEL, signal: weaker}, seed) for seed in range(20))
+
+
+@pytest.mark.parametrize("row_blocks,tiles,num_kb,stages", [s for s in SHAPES if s[0] == 1] + [(1, 4, 1, 1)])
+def test_indices_handed_on_before_the_loads_are_safe_and_live(row_blocks, tiles, num_kb, stages):
+    """As the kernel does where the epilogue stores a row per thread."""
+    programs = pair_programs(row_blocks, tiles, num_kb, stages, publish_kb=0)
+    problems, deadlocks, states = explore(programs)
+    assert states > 100
+    assert not problems and deadlocks == 0, (sorted(map(str, problems))[:3], deadlocks)
+    for seed in range(20):
+        assert not races(programs, KERNEL, seed)
