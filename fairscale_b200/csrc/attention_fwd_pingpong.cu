@@ -33,7 +33,7 @@
 // (In place, the chain exponentials -> PV -> S -> maximum kept the exponential unit, which bounds this head size, at 57 %.)  Each
 // tile has an issuer of its own: one for both held up the products of one tile behind its waits for the other (B16 S512 H16 D64
 // 44 -> 33 us together with the two threads a row).  With head size 128, in place and bound by the products, strict turns are the
-// faster order (B8 S2048 H16 D128 162 us, 177 with two issuers).
+// faster order (B8 S2048 H16 D128 168 us, 177 with two issuers).
 //
 // Any sequence length: the tensor map is three-dimensional (columns, positions, batch), so a tile that overhangs the
 // sequence reads zeros instead of the next sequence's rows; keys past the end lie above every real query's diagonal and

@@ -812,8 +812,8 @@ static bool pair_enabled() {  // FSB_GEMM_PAIR=0 disables the CTA-pair kernel
   return on;
 }
 
-// Kernel for a product that is not streamed and has no CTA cap (choose_persistent goes on from here).  Measured on B200 (us; 64-wide K blocks = kb), small products
-// back to back:
+// Kernel for a product that is not streamed and has no CTA cap; plan_product has what decides when.  Measured on B200 (us; 64-wide K
+// blocks = kb), small products back to back:
 //
 //   M, N, K              pair   one CTA 128x256   cluster split-K, block_n / splits
 //   77, 1024, 4096         -         24.6          64/1 20.5   64/2 15.0   64/4 11.7   128/4 12.8   128/8 12.3
@@ -831,30 +831,27 @@ static bool pair_enabled() {  // FSB_GEMM_PAIR=0 disables the CTA-pair kernel
 // of a slower MMA issue, all by the same quarter; with them the rule takes the fastest column of every row above, or one
 // within 5 %.)
 //
-// From 90 tiles on it is one CTA per tile or a pair per 256 x 256 tile.  Aligned rows, in a loop of a second at the card's power
-// limit, with the median SM clock in MHz:
+// From 90 tiles on, where choose_persistent below does not come in (fp32 results, rows in no 16-byte pieces, K below 256), it is one
+// CTA per tile or a pair per 256 x 256 tile (us, one CTA / pair, in loops of 0.2 s; * operands MN-major):
 //
-//   M, N, K                 one CTA      pair             M, N, K                        one CTA       pair
-//   4096, 2048, 2048       32.2 @1720   37.5 @1860        16384, 6144, 2048             348.1 @1342   349.2 @1385
-//   8192, 4096, 1024       67.4 @1485   75.0 @1635        16384, 8192, 2048             470.8 @1320   459.6 @1380
-//   5970, 6144, 2048      132.5 @1415   136.6 @1485       16384, 2048, 8192             461.4 @1260   457.5 @1220
-//   16384, 2048, 2048     121.5 @1370   124.8 @1462       4096, 12288, 4096             346.2 @1368   326.4 @1408
-//   8192, 8192, 2048      237.8 @1342   234.5 @1413       8192, 2048, 16384 (wgrad)     527.5 @1500   508.3 @1443
-//   8192, 16384, 512      159.8 @1485   199.0 @1723       6144, 2048, 16384 (wgrad)     400.0 @1511   386.2 @1511
-//   16384, 16384, 576     332.6 @1387   404.2 @1616       16384, 50304, 2048           2911.8 @1271  2783.5 @1331
-//   16384, 16384, 768     418.2 @1384   452.2 @1500       16384, 16384, 1280            628.1 @1368   627.0 @1428
-//   16384, 8192, 1024     256.6 @1447   274.0 @1479       16384, 8192, 1280             306.8 @1414   320.4 @1471
-//   16384, 16384, 1024    522.5 @1395   534.4 @1471       16384, 16384, 1536            729.3 @1365   711.6 @1413
+//   M, N, K                    fp32          bf16, N - 1       M, N, K                  fp32          bf16, N - 1
+//   952, 12048, 704         32.7 / 35.9      24.3 / 28.3       16384, 6144, 2048      430 / 428       379 / 382
+//   8192, 4096, 1024        90.6 / 100       79.1 / 79.3       16384, 8192, 2048      572 / 549       505 / 496
+//   5968, 2048, 2048        56.4 / 59.2      53.8 / 56.8       4096, 12288, 4096      391 / 365       367 / 342
+//   16384, 2048, 2048        146 / 149        137 / 136        8192, 2048, 16384 *    503 / 505       496 / 500
+//   8192, 8192, 2048         288 / 284        254 / 255        2048, 6144, 16384 *    376 / 375       370 / 366
+//   16384, 16384, 768        629 / 657        480 / 476        50304, 2048, 16384 *  2924 / 3065     2898 / 2994
+//   16384, 16384, 1400      1136 / 1025      1032 / 864        2992, 1976, 13208 *    237 / 183       230 / 179
+//   13640, 13184, 616        489 / 477        382 / 358        1936, 5872, 4360       152 / 125       139 / 113
 //
 // A pair costs some 6 us more per launch and rounds up to larger tiles, but moves a third less operand data.  That counts once
 // a product is long enough to run at the power limit, and much sooner where the operands' rows do not start on 128-byte lines
 // (a leading dimension that is no multiple of 64): every 128-byte row of a tile is then two lines.  Up to K about 1400 the
-// output, which one CTA drains in smaller pieces, is what takes the time.  (Stacked products, 16 x 2048 x 8192 x 1024: 510
-// against 547 us, 16 x 2048 x 2048 x 8192: 972 against 937 us.)  pair_pays puts that into two lines: us per K block and wave of
-// tiles, by the number of operands off the lines, and the pair's extra cost.  Over 197 products (M and N 256 .. 16384, K 512 ..
-// 16384, half of them with MN-major operands, most of odd sizes) the rule takes 0.6 % longer than the faster kernel would on
-// average, 12 % at worst; a single line at 2.56e11 operations took 4.7 %, and up to 44 % (2992 x 1976 x 13208 238 against 169 us,
-// 1936 x 5872 x 4360 139 against 110 us), always the pair 8 %, never 7 %.
+// output is what takes the time.  pair_pays puts that into two lines: us per K block and wave of tiles, by the number of operands
+// off the lines, and the pair's extra cost.  Over 33 products (M and N 328 .. 50304, K 256 .. 16384) the rule takes 0.7 % longer with
+// fp32 results than the faster kernel would on average, 1.1 % with ragged bf16 ones; at worst 11 and 19 %, both at 16384 x 16384 x
+// 1400, where the line in K lies.  (It was fitted to slower kernels of both kinds; a single line in operations costs 4.7 %, always the
+// pair 8 %, never 7 %.)
 struct GemmPlan {
   enum Kind { PAIR, ONE_CTA, CLUSTER_K, WIDE_PAIR } kind;
   int block_n, splits;

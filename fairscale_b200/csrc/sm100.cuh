@@ -137,8 +137,8 @@ template <int N> __device__ __forceinline__ void tma_store_wait_read() {
 template <int N> __device__ __forceinline__ void tma_store_wait() {
   asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
 }
-// The same for a whole converged warp: every lane calls, one elected lane issues (see umma_f16_ss_warp); addresses and
-// coordinates are warp-uniform.
+// The loads and expect_tx above for a whole converged warp: every lane calls, one elected lane issues (see umma_f16_ss_warp);
+// addresses and coordinates are warp-uniform.
 __device__ __forceinline__ void mbar_expect_tx_warp(uint32_t bar, uint32_t bytes) {
   asm volatile(
       "{\n\t.reg .pred q;\n\t"

@@ -38,10 +38,12 @@ def _native_available() -> bool:
 
 def _native_is_faster(B: int, S: int, H: int, inference: bool) -> bool:
     """For a length that is no multiple of 128: the kernels here or torch's operator, which needs q, k and v permuted and their
-    gradients concatenated?  Forward + backward on B200 (us, torch / here): B4 S1543 H16 D128 553 / 296, B2 S4095 H16 D64 581 / 501,
-    B4 S5000 H16 D64 1553 / 1448, but B4 S7000 H16 D64 2579 / 2773 and B1 S8000 H2 D64 253 / 330 - the backward here makes the scores
-    twice, and few heads leave one long chain.  The forward alone is up to 30 % faster in torch's operator from S 500 on (B4 S1543
-    H16 D64 55 / 61, B2 S4095 H16 D64 98 / 124, short ones are bound by the host, B1 S77 33 / 27).  Only inference mode may go by that: a
+    gradients concatenated?  Forward + backward on B200 (us, torch / here): B4 S1543 H16 D128 540 / 292, B2 S4095 H16 D64 573 / 423,
+    B4 S5000 H16 D64 1568 / 1286, B1 S8000 H2 D64 249 / 254, B1 S8000 H2 D128 316 / 368 - the backward here makes the scores twice, and
+    few heads leave one long chain.  The lines at 5500 and 8 heads are those of a slower backward: beyond them the kernels here now
+    take as long or less where there are heads enough (B4 S7000 H16 D64 2601 / 2430, B2 S7000 H16 D128 2048 / 1965, B1 S3000 H2 D64
+    145 / 112).  The forward alone is up to 30 % faster in torch's operator from S 1500 on (B4 S1543 H16 D128 58 / 72, B2 S4095 H16
+    D64 97 / 113, short ones are bound by the host, B1 S77 23 / 18, B4 S1000 H16 D64 27 / 26).  Only inference mode may go by that: a
     forward without gradients may be the first pass of a checkpointed block, whose repetition has to compute the same."""
     if inference:
         return S <= 1024 and B * H * S <= 65536
